@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/gdf.h"
+#include "gdf_charlim.cuh"
 #include "gdf_kernels.cuh"
 #include "gdf_mlp.cuh"
 
@@ -686,33 +687,12 @@ __device__ __forceinline__ void gather_features(const Consts& K, const float* __
 // fused, for one interior cell. S is the pre-limit state (ghosts as the
 // reference leaves them), D receives the limited state.
 constexpr int LIM_BS = 64;
-// the second limiter pass (gated cells only) with rolled 8x8 products and
-// one out-of-line eigenmatrix (same arithmetic, smaller instruction
-// stream); off by default: measured the same as the unrolled form (rotor
-// 512^2 steps 104-203, k_limit_tvb 0.606 against 0.612 ms per launch)
-#ifndef GDF_TVB_ROLLED
-#define GDF_TVB_ROLLED false
-#endif
 // dynamic shared memory of a learned-mode limiter block: X, W1t, W2t, H1
 // tiles (BF16) and the LIM_BS logits
 constexpr size_t LIMIT_SMEM_LEARNED = (size_t)(LIM_BS + MLP_H) * MLP_LDX * 2 + (size_t)(MLP_H + LIM_BS) * MLP_LDH * 2 +
                                       LIM_BS * sizeof(float);
 
-template <bool ROLLED = false>
 __device__ __forceinline__ void matvec8(const double* A, const double* x, double* y) {
-  if (ROLLED) {
-    // the same sums with the row loop kept as a loop: the second limiter
-    // pass (k_limit_tvb) waits on instruction fetch when its twelve 8x8
-    // products are unrolled
-#pragma unroll 1
-    for (int r = 0; r < 8; ++r) {
-      double acc = 0.0;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) acc = acc + A[r + 8 * k] * x[k];
-      y[r] = acc;
-    }
-    return;
-  }
 #pragma unroll
   for (int r = 0; r < 8; ++r) {
     double acc = 0.0;
@@ -720,13 +700,6 @@ __device__ __forceinline__ void matvec8(const double* A, const double* x, double
     for (int k = 0; k < 8; ++k) acc = acc + A[r + 8 * k] * x[k];
     y[r] = acc;
   }
-}
-
-// eigenmatrix as one out-of-line copy, for the rolled limiter
-static __device__ __noinline__ void eigenmatrix_call(const Phys& P, int dir, double rho, double u1, double u2,
-                                                     double u3, double E, double B1, double B2, double B3,
-                                                     double* R, double* L) {
-  eigenmatrix(P, dir, rho, u1, u2, u3, E, B1, B2, B3, R, L);
 }
 
 __device__ __forceinline__ void trace8(const Consts& K, const double* __restrict__ S, long long c,
@@ -936,6 +909,13 @@ static __device__ void pp_cell(const Consts& K, double (*m)[NP]) {
     for (int d = 1; d < NP; ++d) m[n][d] = eta * m[n][d];
 }
 
+__device__ __forceinline__ void lim_load(const Consts& K, const double* __restrict__ S, long long c, double (*m)[NP]) {
+#pragma unroll
+  for (int n = 0; n < NE; ++n)
+#pragma unroll
+    for (int d = 0; d < NP; ++d) m[n][d] = live_mode(n, d) ? S[c + K.plane * (d + 10 * n)] : 0.0;
+}
+
 // One interior cell (item < nx*ny). LIM_INFER: called by every thread of a
 // LIM_BS-thread block on LIM_BS consecutive items (those past nx*ny idle),
 // with lsm the block's LIMIT_SMEM_LEARNED bytes of dynamic shared memory.
@@ -957,7 +937,6 @@ __device__ __forceinline__ bool lim_gate(const Consts& K, const double* __restri
                                          float* __restrict__ pnet, float t_lo, float t_hi, long long item,
                                          unsigned char* lsm, bool valid, long long c, double (*m)[NP],
                                          int32_t& word) {
-  const long long pl = K.plane;
   float p_net = 0.f;
   if (LM == LIM_INFER) {
     // the learned indicator for the block's 64 cells on the tensor cores
@@ -1008,10 +987,7 @@ __device__ __forceinline__ bool lim_gate(const Consts& K, const double* __restri
     if (valid) p_net = pnet[item];
   }
   if (!valid) return false;
-#pragma unroll
-  for (int n = 0; n < NE; ++n)
-#pragma unroll
-    for (int d = 0; d < NP; ++d) m[n][d] = live_mode(n, d) ? S[c + pl * (d + 10 * n)] : 0.0;
+  lim_load(K, S, c, m);
   word = 0;
   bool gate = true;
   if (K.detector == GDF_DETECT_KXRCF) {
@@ -1032,8 +1008,8 @@ __device__ __forceinline__ bool lim_gate(const Consts& K, const double* __restri
 
 // TVB_Limiter_P1.f90:19-90: characteristic minmod of the two slopes only;
 // a changed variable keeps its limited slopes and loses every higher mode
-__device__ __forceinline__ void lim_tvb_p1(const Consts& K, const double* __restrict__ S, long long c,
-                                           double (*m)[NP], int32_t& word) {
+static __device__ __noinline__ void lim_tvb_p1(const Consts& K, const double* __restrict__ S, long long c,
+                                              double (*m)[NP], int32_t& word) {
   const long long pl = K.plane;
   const double rhoij = m[0][0];
   const double u1 = m[1][0] / rhoij, u2 = m[2][0] / rhoij, u3 = dv(m[3][0], rhoij);
@@ -1089,7 +1065,8 @@ __device__ __forceinline__ void lim_tvb_p1(const Consts& K, const double* __rest
 // (:24-55 x, :57-90 y): the face slopes Dp (mean to + face) and Dm (- face
 // to mean) limited against the mean differences DR, DL in the
 // characteristic variables of the cell mean (minmod with the bound Mh2),
-// back in conserved variables as Yp, Ym. The left eigenvectors are built
+// back in conserved variables as Yp, Ym: the general path behind
+// char_limit_sparse. The left eigenvectors are built
 // and used in the four products with L before the right ones are built, so
 // one 8x8 matrix is live at a time; the products and sums are those of
 // eigenmatrix's R and L. With the identity fallback of eigenmatrix.f90:
@@ -1139,141 +1116,128 @@ __device__ __forceinline__ void char_limit_dir(const Consts& K, int dir, double 
   matvec8(R, mod, Ym);
 }
 
-// STREAM: lim_tvb through char_limit_dir (one eigenvector matrix live at a
-// time) instead of both matrices at once; same values. GDF_TVB_STREAM=1
-// (the default) gives it to the second limiter pass: with the paired
-// residual loads, the developed rotor 512^2 (steps 104-303) runs 4.86
-// against 4.94 ms per step (k_limit_tvb 0.48 against 0.51 ms per launch)
-// and the blast 2048^2 step, which never launches that kernel, is unchanged
-// (45.64 against 45.65 ms), two A/B pairs with equal hashes. An earlier
-// build without the paired loads had measured that blast step 46.3 against
-// 45.5 ms with it.
-#ifndef GDF_TVB_STREAM
-#define GDF_TVB_STREAM 1
-#endif
-// the same for the characteristic limiter run inline by the one-pass
-// limiter (the learned gate, and the reference's all-cells limiter):
-// Orszag-Tang 512^2 (every cell limited) 3.64 against 3.67 ms per step, but
-// the learned blast 2048^2 45.9 against 45.6 ms and the learned blast 512^2
-// 5.70 against 5.68 (two A/B pairs, equal hashes), so it stays off
-#ifndef GDF_TVB_STREAM_INLINE
-#define GDF_TVB_STREAM_INLINE 0
-#endif
+// Operands of one direction for cell c: mean differences to the + and -
+// neighbours (stride st) and the two face slopes of modes 2+dir, 4+2*dir.
+__device__ __forceinline__ void tvb_operands(const Consts& K, const double* __restrict__ S, long long c, int dir,
+                                             double* DR, double* DL, double* Dp, double* Dm) {
+  const long long pl = K.plane, st = dir ? K.nx2 : 1;
+  const double c23 = 2.0 / 3.0;
+  const double* lo = S + c + pl * (1 + dir);
+  const double* hi = S + c + pl * (3 + 2 * dir);
+#pragma unroll
+  for (int n = 0; n < NE; ++n) {
+    const long long o = pl * (10 * n);
+    const double m0 = S[c + o], m1 = lo[o], m2 = hi[o];
+    DR[n] = S[c + st + o] - m0;
+    DL[n] = m0 - S[c - st + o];
+    Dp[n] = m1 + c23 * m2;
+    Dm[n] = m1 - c23 * m2;
+  }
+}
+// which variables one direction's limited slopes change (TVB_Limiter_P2.f90:
+// 45-52, 78-85), and the modes they give: res[n] = the slope, res[8 + n] = the
+// quadratic mode
+__device__ __forceinline__ unsigned tvb_change(const Consts& K, const double* Dp, const double* Dm, const double* Yp,
+                                               const double* Ym, double* res) {
+  unsigned change = 0;
+#pragma unroll
+  for (int n = 0; n < NE; ++n) {
+    if (fabs(Yp[n] - Dp[n]) > 1e-6 || fabs(Ym[n] - Dm[n]) > 1e-6) change |= 1u << n;
+    res[n] = 0.5 * (Yp[n] + Ym[n]);
+    res[NE + n] = K.tvb_slope * (Yp[n] - Ym[n]);
+  }
+  return change;
+}
+// both directions through the general path (cells char_limit_sparse refuses)
+static __device__ __noinline__ unsigned tvb_general(const Consts& K, const double* __restrict__ S, long long c,
+                                                    double* res) {
+  double m[NE];
+#pragma unroll
+  for (int n = 0; n < NE; ++n) m[n] = S[c + K.plane * (10 * n)];
+  const double u1 = m[1] / m[0], u2 = m[2] / m[0], u3 = m[3] / m[0];
+  unsigned change = 0;
+#pragma unroll 1
+  for (int dir = 0; dir < 2; ++dir) {
+    double DR[NE], DL[NE], Dp[NE], Dm[NE], Yp[NE], Ym[NE];
+    tvb_operands(K, S, c, dir, DR, DL, Dp, Dm);
+    const bool z = dir == 1 && K.eig_y_zero_w;
+    if (dir == 0)
+      char_limit_dir(K, 0, m[0], u1, u2, u3, m[4], m[5], m[6], m[7], DR, DL, Dp, Dm, K.Mh2x, Yp, Ym);
+    else
+      char_limit_dir(K, 1, m[0], u1, u2, z ? 0.0 : u3, m[4], m[5], m[6], z ? 0.0 : m[7], DR, DL, Dp, Dm, K.Mh2y, Yp,
+                     Ym);
+    change |= tvb_change(K, Dp, Dm, Yp, Ym, res + 2 * NE * dir);
+  }
+  return change;
+}
 
-template <bool ROLLED = false, bool STREAM = false>
+// both directions through one copy of char_limit_sparse; false where it refuses
+template <class DIV>
+__device__ __forceinline__ bool tvb_sparse(const Consts& K, const double* __restrict__ S, long long c, double* res,
+                                           unsigned& change) {
+  unsigned bad = 0;
+  change = 0;
+  double m[NE];
+#pragma unroll
+  for (int n = 0; n < NE; ++n) m[n] = S[c + K.plane * (10 * n)];
+  const auto rr = DIV::by(m[0], bad);
+  const double u1 = DIV::div(m[1], rr, bad), u2 = DIV::div(m[2], rr, bad), u3 = DIV::div(m[3], rr, bad);
+#pragma unroll 1
+  for (int dir = 0; dir < 2; ++dir) {
+    double DR[NE], DL[NE], Dp[NE], Dm[NE], Yp[NE], Ym[NE];
+    tvb_operands(K, S, c, dir, DR, DL, Dp, Dm);
+    const bool z = dir == 1 && K.eig_y_zero_w;
+    const Minmod mm{dir ? K.Mh2y : K.Mh2x};
+    bad |= (unsigned)!char_limit_sparse<DIV>(K.P, dir, m[0], u1, u2, z ? 0.0 : u3, m[4], m[5], m[6], z ? 0.0 : m[7],
+                                             rr, DR, DL, Dp, Dm, mm, Yp, Ym);
+    change |= tvb_change(K, Dp, Dm, Yp, Ym, res + 2 * NE * dir);
+  }
+  return !bad;
+}
+// the cells tvb_sparse<SharedRcp> refuses
+static __device__ __noinline__ unsigned tvb_refused(const Consts& K, const double* __restrict__ S, long long c,
+                                                    double* res) {
+  unsigned change;
+  return tvb_sparse<IeeeDiv>(K, S, c, res, change) ? change : tvb_general(K, S, c, res);
+}
+
+// TVB_Limiter_P2.f90:24-90: the limited slopes and quadratic modes of cell c
+// in both directions (res[dir][slope 8, quadratic 8]); returns the changed
+// variables.
+__device__ __forceinline__ unsigned tvb_slopes(const Consts& K, const double* __restrict__ S, long long c,
+                                               double* res) {
+  unsigned change;
+  return tvb_sparse<SharedRcp>(K, S, c, res, change) ? change : tvb_refused(K, S, c, res);
+}
+
+// the modes of the changed variables from tvb_slopes (TVB_Limiter_P2.f90:92-121)
+__device__ __forceinline__ void tvb_apply(unsigned change, const double* res, double (*m)[NP]) {
+#pragma unroll
+  for (int n = 0; n < NE; ++n) {
+    if (change & (1u << n)) {
+#pragma unroll
+      for (int d = 6; d < NP; ++d) m[n][d] = 0.0;
+      m[n][4] = 0.0;
+      m[n][1] = res[n];
+      m[n][2] = res[2 * NE + n];
+      m[n][3] = res[NE + n];
+      m[n][5] = res[3 * NE + n];
+    }
+  }
+}
+
+// the limiter of a gated cell whose modes m are loaded
 __device__ __forceinline__ void lim_tvb(const Consts& K, const double* __restrict__ S, long long c,
                                         double (*m)[NP], int32_t& word) {
   if (K.tvb_p1) {
     lim_tvb_p1(K, S, c, m, word);
     return;
   }
-  const long long pl = K.plane;
-    const double c23 = 2.0 / 3.0;
-    const double rhoij = m[0][0];
-    const double u1 = m[1][0] / rhoij, u2 = m[2][0] / rhoij, u3 = dv(m[3][0], rhoij);
-    const double Eij = m[4][0], B1 = m[5][0], B2 = m[6][0], B3 = m[7][0];
-    double R[64], L[64];
-    double DR[NE], DL[NE], Dp[NE], Dm[NE], t1[NE], t2[NE], tu[NE], mod[NE];
-    double Rp[NE], Rm[NE], Up[NE], Um[NE];
-    unsigned change = 0;
-    if (!ROLLED && STREAM) {
-#pragma unroll
-      for (int n = 0; n < NE; ++n) {
-        DR[n] = S[c + 1 + pl * (10 * n)] - m[n][0];
-        DL[n] = m[n][0] - S[c - 1 + pl * (10 * n)];
-        Dp[n] = m[n][1] + c23 * m[n][3];
-        Dm[n] = m[n][1] - c23 * m[n][3];
-      }
-      char_limit_dir(K, 0, rhoij, u1, u2, u3, Eij, B1, B2, B3, DR, DL, Dp, Dm, K.Mh2x, Rp, Rm);
-#pragma unroll
-      for (int d = 0; d < NE; ++d)
-        if (fabs(Rp[d] - Dp[d]) > 1e-6 || fabs(Rm[d] - Dm[d]) > 1e-6) change |= 1u << d;
-#pragma unroll
-      for (int n = 0; n < NE; ++n) {
-        DR[n] = S[c + K.nx2 + pl * (10 * n)] - m[n][0];
-        DL[n] = m[n][0] - S[c - K.nx2 + pl * (10 * n)];
-        Dp[n] = m[n][2] + c23 * m[n][5];
-        Dm[n] = m[n][2] - c23 * m[n][5];
-      }
-      if (K.eig_y_zero_w)
-        char_limit_dir(K, 1, rhoij, u1, u2, 0.0, Eij, B1, B2, 0.0, DR, DL, Dp, Dm, K.Mh2y, Up, Um);
-      else
-        char_limit_dir(K, 1, rhoij, u1, u2, u3, Eij, B1, B2, B3, DR, DL, Dp, Dm, K.Mh2y, Up, Um);
-#pragma unroll
-      for (int d = 0; d < NE; ++d)
-        if (fabs(Up[d] - Dp[d]) > 1e-6 || fabs(Um[d] - Dm[d]) > 1e-6) change |= 1u << d;
-    } else {
-    // x direction
-    if (ROLLED) eigenmatrix_call(K.P, 0, rhoij, u1, u2, u3, Eij, B1, B2, B3, R, L);
-    else eigenmatrix(K.P, 0, rhoij, u1, u2, u3, Eij, B1, B2, B3, R, L);
-#pragma unroll
-    for (int n = 0; n < NE; ++n) {
-      DR[n] = S[c + 1 + pl * (10 * n)] - m[n][0];
-      DL[n] = m[n][0] - S[c - 1 + pl * (10 * n)];
-      Dp[n] = m[n][1] + c23 * m[n][3];
-      Dm[n] = m[n][1] - c23 * m[n][3];
-    }
-    matvec8<ROLLED>(L, DR, t1);
-    matvec8<ROLLED>(L, DL, t2);
-    matvec8<ROLLED>(L, Dp, tu);
-#pragma unroll
-    for (int k = 0; k < NE; ++k) mod[k] = minmod1(tu[k], t1[k], t2[k], K.Mh2x);
-    matvec8<ROLLED>(R, mod, Rp);
-#pragma unroll
-    for (int d = 0; d < NE; ++d)
-      if (fabs(Rp[d] - Dp[d]) > 1e-6) change |= 1u << d;
-    matvec8<ROLLED>(L, Dm, tu);
-#pragma unroll
-    for (int k = 0; k < NE; ++k) mod[k] = minmod1(tu[k], t1[k], t2[k], K.Mh2x);
-    matvec8<ROLLED>(R, mod, Rm);
-#pragma unroll
-    for (int d = 0; d < NE; ++d)
-      if (fabs(Rm[d] - Dm[d]) > 1e-6) change |= 1u << d;
-    // y direction
-    if (ROLLED)
-      eigenmatrix_call(K.P, 1, rhoij, u1, u2, K.eig_y_zero_w ? 0.0 : u3, Eij, B1, B2, K.eig_y_zero_w ? 0.0 : B3, R, L);
-    else if (K.eig_y_zero_w)
-      eigenmatrix(K.P, 1, rhoij, u1, u2, 0.0, Eij, B1, B2, 0.0, R, L);
-    else
-      eigenmatrix(K.P, 1, rhoij, u1, u2, u3, Eij, B1, B2, B3, R, L);
-#pragma unroll
-    for (int n = 0; n < NE; ++n) {
-      DR[n] = S[c + K.nx2 + pl * (10 * n)] - m[n][0];
-      DL[n] = m[n][0] - S[c - K.nx2 + pl * (10 * n)];
-      Dp[n] = m[n][2] + c23 * m[n][5];
-      Dm[n] = m[n][2] - c23 * m[n][5];
-    }
-    matvec8<ROLLED>(L, DR, t1);
-    matvec8<ROLLED>(L, DL, t2);
-    matvec8<ROLLED>(L, Dp, tu);
-#pragma unroll
-    for (int k = 0; k < NE; ++k) mod[k] = minmod1(tu[k], t1[k], t2[k], K.Mh2y);
-    matvec8<ROLLED>(R, mod, Up);
-#pragma unroll
-    for (int d = 0; d < NE; ++d)
-      if (fabs(Up[d] - Dp[d]) > 1e-6) change |= 1u << d;
-    matvec8<ROLLED>(L, Dm, tu);
-#pragma unroll
-    for (int k = 0; k < NE; ++k) mod[k] = minmod1(tu[k], t1[k], t2[k], K.Mh2y);
-    matvec8<ROLLED>(R, mod, Um);
-#pragma unroll
-    for (int d = 0; d < NE; ++d)
-      if (fabs(Um[d] - Dm[d]) > 1e-6) change |= 1u << d;
-    }
-#pragma unroll
-    for (int n = 0; n < NE; ++n) {
-      if (change & (1u << n)) {
-#pragma unroll
-        for (int d = 6; d < NP; ++d) m[n][d] = 0.0;
-        m[n][4] = 0.0;
-        m[n][1] = 0.5 * (Rp[n] + Rm[n]);
-        m[n][2] = 0.5 * (Up[n] + Um[n]);
-        m[n][3] = K.tvb_slope * (Rp[n] - Rm[n]);
-        m[n][5] = K.tvb_slope * (Up[n] - Um[n]);
-      }
-    }
-    word |= (int32_t)change;
-  }
+  double res[4 * NE];
+  const unsigned change = tvb_slopes(K, S, c, res);
+  tvb_apply(change, res, m);
+  word |= (int32_t)change;
+}
 
 __device__ __forceinline__ void lim_finish(const Consts& K, double* __restrict__ D, const double* __restrict__ BX,
                                            const double* __restrict__ BY, int32_t* __restrict__ flags, int stage,
@@ -1324,19 +1288,27 @@ __device__ __forceinline__ void lim_finish(const Consts& K, double* __restrict__
   if (!(m[0][0] > 0.0) || !isfinite(m[4][0])) atomicOr(&sc->status, 1);
 }
 
-// Appends the gated cells among the calling warp's active lanes to list
+// Cells left to a later pass: list entries are tag + item.
+template <class T>
+struct LimList {
+  T* list;
+  int32_t* count;
+  T tag;
+};
+
+// Appends the gated cells among the calling warp's active lanes to the list
 // (one atomic per warp); true for a gated cell.
-__device__ __forceinline__ bool lim_defer(bool gate, long long item, int32_t* __restrict__ list,
-                                          int32_t* __restrict__ count) {
+template <class T>
+__device__ __forceinline__ bool lim_defer(bool gate, long long item, const LimList<T>& l) {
   const unsigned act = __activemask();
   const unsigned bal = __ballot_sync(act, gate);
   if (!gate) return false;
   const int lane = threadIdx.x & 31;
   const int leader = __ffs(bal) - 1;
   int base = 0;
-  if (lane == leader) base = atomicAdd(count, __popc(bal));
+  if (lane == leader) base = atomicAdd(l.count, __popc(bal));
   base = __shfl_sync(bal, base, leader);
-  list[base + __popc(bal & ((1u << lane) - 1u))] = (int32_t)item;
+  l.list[base + __popc(bal & ((1u << lane) - 1u))] = l.tag + (T)item;
   return true;
 }
 
@@ -1344,15 +1316,14 @@ __device__ __forceinline__ bool lim_defer(bool gate, long long item, int32_t* __
 // to list (limit_tvb_item finishes it in a second pass over full warps, so
 // the characteristic limiter never runs beside idle lanes); an ungated one
 // is finished here.
-template <int LM, bool COMPACT = false>
+template <int LM, bool COMPACT, class T = int32_t>
 __device__ __forceinline__ void limit_item(const Consts& K, const double* __restrict__ S, double* __restrict__ D,
                                            const double* __restrict__ BX, const double* __restrict__ BY,
                                            int32_t* __restrict__ flags, int32_t* __restrict__ trouble, int stage,
                                            int divfree, Scal* __restrict__ sc, const MlpDev* __restrict__ net,
                                            const float* __restrict__ QM, float* __restrict__ pnet,
                                            float t_lo, float t_hi, long long item, unsigned char* lsm,
-                                           int32_t* __restrict__ list = nullptr,
-                                           int32_t* __restrict__ count = nullptr) {
+                                           const LimList<T>& defer = LimList<T>{}) {
   const bool valid = item < (long long)K.nx * K.ny;
   const int i = valid ? (int)(item % K.nx) + 1 : 1;
   const int j = valid ? (int)(item / K.nx) + 1 : 1;
@@ -1362,32 +1333,36 @@ __device__ __forceinline__ void limit_item(const Consts& K, const double* __rest
   const bool gate = lim_gate<LM>(K, S, trouble, net, QM, pnet, t_lo, t_hi, item, lsm, valid, c, m, word);
   if (!valid) return;
   if (COMPACT) {
-    if (lim_defer(gate, item, list, count)) return;
+    if (lim_defer(gate, item, defer)) return;
   } else if (gate) {
-    lim_tvb<false, GDF_TVB_STREAM_INLINE != 0>(K, S, c, m, word);
+    lim_tvb(K, S, c, m, word);
   }
   lim_finish(K, D, BX, BY, flags, stage, divfree, sc, item, i, j, c, m, word);
 }
 
-// The second pass for a cell limit_item<LM, true> deferred: its pre-limit
-// modes again, the detector bit lim_gate set for it (KXRCF and the learned
-// gate set it; GDF_DETECT_ALL does not), the characteristic limiter and the
-// finish.
+// A cell every thread of the limiting pass limits: one limit_item<LM, true>
+// deferred, or with GDF_DETECT_ALL any. The detector bit is the one lim_gate
+// sets (KXRCF and the learned gate set it; GDF_DETECT_ALL does not). The modes
+// are loaded after the characteristic part, which needs few of them.
 __device__ __forceinline__ void limit_tvb_item(const Consts& K, const double* __restrict__ S, double* __restrict__ D,
                                                const double* __restrict__ BX, const double* __restrict__ BY,
                                                int32_t* __restrict__ flags, int stage, int divfree,
                                                Scal* __restrict__ sc, long long item) {
-  const long long pl = K.plane;
   const int i = (int)(item % K.nx) + 1;
   const int j = (int)(item / K.nx) + 1;
   const long long c = i + (long long)K.nx2 * j;
   double m[NE][NP];
-#pragma unroll
-  for (int n = 0; n < NE; ++n)
-#pragma unroll
-    for (int d = 0; d < NP; ++d) m[n][d] = live_mode(n, d) ? S[c + pl * (d + 10 * n)] : 0.0;
   int32_t word = K.detector != GDF_DETECT_ALL ? (1 << 24) : 0;
-  lim_tvb<GDF_TVB_ROLLED, GDF_TVB_STREAM != 0>(K, S, c, m, word);
+  if (K.tvb_p1) {
+    lim_load(K, S, c, m);
+    lim_tvb_p1(K, S, c, m, word);
+  } else {
+    double res[4 * NE];
+    const unsigned change = tvb_slopes(K, S, c, res);
+    lim_load(K, S, c, m);
+    tvb_apply(change, res, m);
+    word |= (int32_t)change;
+  }
   lim_finish(K, D, BX, BY, flags, stage, divfree, sc, item, i, j, c, m, word);
 }
 

@@ -77,6 +77,8 @@ struct EnsArgs {
   const int* off;                 // [EK_N][n + 1] tile prefix sums
   unsigned long long* amax;       // [2n] bit patterns of the x / y speed maxima
   EnsSync* sync;
+  long long* lim_list;            // (instance << 40) + cell: gated cells, for the limiting pass
+  int32_t* lim_count;
   const MlpDev* net;
   unsigned long long timeout_ns;
   int n;
@@ -118,7 +120,7 @@ __device__ __noinline__ void call_limit(const Consts& K, const double* S, double
                                         int32_t* flags, int32_t* trouble, int stage, int divfree, Scal* sc,
                                         const MlpDev* net, const float* QM, float* pnet, float t_lo, float t_hi,
                                         long long item) {
-  limit_item<LM>(K, S, D, BX, BY, flags, trouble, stage, divfree, sc, net, QM, pnet, t_lo, t_hi, item, ens_sm);
+  limit_item<LM, false>(K, S, D, BX, BY, flags, trouble, stage, divfree, sc, net, QM, pnet, t_lo, t_hi, item, ens_sm);
 }
 __device__ __noinline__ void call_dt(const Consts& K, const double* U, long long item, double& ax, double& ay,
                                      Scal* sc) {
@@ -475,11 +477,23 @@ __global__ void __launch_bounds__(ENS_BS) k_ep_qmodes(const __grid_constant__ En
 template <int LM>
 __global__ void __launch_bounds__(ENS_BS) k_ep_limit(const __grid_constant__ EnsArgs A, int stage) {
   extern __shared__ __align__(16) unsigned char lsm[];
-  for_tiles<true>(A, EK_LIM, [&](int, const EnsInst& I, const Consts& K, long long base, int) {
-    limit_item<LM>(K, I.UI, I.U, I.BX, I.BY, I.flags, I.trouble, stage, K.faceb ? 0 : 1, I.sc, A.net, I.QM, I.pnet,
-                   A.t_lo, A.t_hi, base + threadIdx.x, lsm);
+  for_tiles<true>(A, EK_LIM, [&](int i, const EnsInst& I, const Consts& K, long long base, int) {
+    limit_item<LM, true>(K, I.UI, I.U, I.BX, I.BY, I.flags, I.trouble, stage, K.faceb ? 0 : 1, I.sc, A.net, I.QM,
+                         I.pnet, A.t_lo, A.t_hi, base + threadIdx.x, lsm,
+                         LimList<long long>{A.lim_list, A.lim_count, (long long)i << 40});
     if (LM == LIM_INFER) __syncthreads();
   });
+}
+
+// the cells of every instance k_ep_limit listed, one per thread; resident
+// blocks walk the list
+__global__ void __launch_bounds__(ENS_BS) k_ep_limit_tvb(const __grid_constant__ EnsArgs A, int stage) {
+  const int n = *A.lim_count;
+  for (long long k = (long long)blockIdx.x * ENS_BS + threadIdx.x; k < n; k += (long long)gridDim.x * ENS_BS) {
+    const long long e = A.lim_list[k];
+    const EnsInst& I = A.inst[e >> 40];
+    limit_tvb_item(*I.K, I.UI, I.U, I.BX, I.BY, I.flags, stage, I.K->faceb ? 0 : 1, I.sc, e & ((1LL << 40) - 1));
+  }
 }
 
 __global__ void __launch_bounds__(ENS_BS) k_ep_faceb(const __grid_constant__ EnsArgs A) {
@@ -538,6 +552,8 @@ struct GdfEnsemble {
   int learned = 0;
   float t_lo = 0.5f, t_hi = 0.5f;
   int any_faceb = 0;
+  long long* lim_list = nullptr;
+  int32_t* lim_count = nullptr;
   int uploaded = 0;
   // tile shape
   int ctas_per_sm = 0;         // 0: the occupancy limit
@@ -628,6 +644,8 @@ int ens_layout(GdfEnsemble* e) {
   A.timeout_ns = std::max(2000000000ull, 200ull * cells);
   A.n = n;
   A.any_faceb = e->any_faceb;
+  A.lim_list = e->lim_list;
+  A.lim_count = e->lim_count;
   A.t_lo = e->t_lo;
   A.t_hi = e->t_hi;
   if (e->graph) {
@@ -684,6 +702,7 @@ int launch_stage_phases(GdfEnsemble* e, int stage) {
     n += 3;
   }
   const int ls = stage == 0 ? 1 : stage;
+  ECK(cudaMemsetAsync(A.lim_count, 0, sizeof(int32_t), st));
   if (e->learned && stage <= 1) {
     k_ep_qmodes<<<tiles_of(A, EK_QM), ENS_BS, 0, st>>>(A);
     k_ep_limit<LIM_INFER><<<tiles_of(A, EK_LIM), ENS_BS, LIMIT_SMEM_LEARNED, st>>>(A, ls);
@@ -695,6 +714,8 @@ int launch_stage_phases(GdfEnsemble* e, int stage) {
     k_ep_limit<LIM_PLAIN><<<tiles_of(A, EK_LIM), ENS_BS, 0, st>>>(A, ls);
     ++n;
   }
+  k_ep_limit_tvb<<<tiles_of(A, EK_LIM), ENS_BS, 0, st>>>(A, ls);
+  ++n;
   if (A.any_faceb) {
     bc(EK_BCF, 0);
     k_ep_faceb<<<tiles_of(A, EK_FB), ENS_BS, 0, st>>>(A);
@@ -800,7 +821,8 @@ int gdf_ens_destroy(GdfEnsemble* e) {
     for (void* p : bufs)
       if (p) cudaFree(p);
   }
-  void* bufs[] = {e->dK, e->dInst, e->sc, e->amax, e->sync, e->off, e->net, e->sc_save};
+  void* bufs[] = {e->dK, e->dInst, e->sc, e->amax, e->sync, e->off, e->net, e->sc_save,
+                  e->lim_list, e->lim_count};
   for (void* p : bufs)
     if (p) cudaFree(p);
   if (e->sc_host) cudaFreeHost(e->sc_host);
@@ -840,12 +862,14 @@ int gdf_ens_create(const GdfConfig* cfgs, int32_t n, GdfEnsemble** out) {
   ok = ok && alloc((void**)&e->sync, sizeof(EnsSync)) && alloc((void**)&e->off, (size_t)EK_N * (n + 1) * sizeof(int));
   ok = ok && cudaMallocHost((void**)&e->sc_host, (size_t)n * sizeof(Scal)) == cudaSuccess;
   std::vector<EnsInst> hi(n);
+  long long cells = 0;
   for (int i = 0; ok && i < n; ++i) {
     InstBufs& b = e->in[i];
     b.cfg = cfgs[i];
     consts_for(cfgs[i], b.K);
     if (i == 0) ok = ok && upload_basis_once(b.K, true) == cudaSuccess;
     if (b.K.faceb) e->any_faceb = 1;
+    cells += (long long)cfgs[i].nx * cfgs[i].ny;
     const Consts& K = b.K;
     const GdfConfig& c = cfgs[i];
     EnsInst& d = b.d;
@@ -862,6 +886,8 @@ int gdf_ens_create(const GdfConfig* cfgs, int32_t n, GdfEnsemble** out) {
     hi[i] = d;
     if (ok) ok = cudaMemcpy(e->dK + i, &b.K, sizeof(Consts), cudaMemcpyHostToDevice) == cudaSuccess;
   }
+  ok = ok && alloc((void**)&e->lim_list, (size_t)cells * sizeof(long long)) &&
+       alloc((void**)&e->lim_count, sizeof(int32_t));
   if (!ok) {
     cudaGetLastError();
     gdf_ens_destroy(e);

@@ -77,16 +77,6 @@
 #ifndef GDF_LIMIT_MINB
 #define GDF_LIMIT_MINB 1
 #endif
-// the learned indicator's stage-1 inference in its own kernel (k_infer)
-// ahead of the limiter, instead of inside the 255-register limiter blocks
-#ifndef GDF_INFER_APART
-#define GDF_INFER_APART 1
-#endif
-// the learned gate's limiter in two passes as KXRCF's (gated cells listed,
-// then limited over full warps); 0: one pass
-#ifndef GDF_LEARNED_TWO_PASS
-#define GDF_LEARNED_TWO_PASS 0
-#endif
 
 
 namespace gdf {
@@ -252,23 +242,25 @@ __global__ void __launch_bounds__(LIM_BS) k_infer(const __grid_constant__ Consts
   }
 }
 
-template <int LM, bool COMPACT>
+// The gating pass: cells the detector leaves alone are finished, the others
+// listed for k_limit_tvb (full warps, and none of the characteristic
+// limiter's registers here).
+template <int LM>
 __global__ void __launch_bounds__(LIM_BS, GDF_LIMIT_MINB) k_limit(const __grid_constant__ Consts K, const double* __restrict__ S,
                                                   double* __restrict__ D, const double* __restrict__ BX,
                                                   const double* __restrict__ BY, int32_t* __restrict__ flags,
                                                   int32_t* __restrict__ trouble, int stage, int divfree,
                                                   const Scal* __restrict__ gate_sc, Scal* __restrict__ sc,
-                                                  const MlpDev* __restrict__ net, const float* __restrict__ QM,
                                                   float* __restrict__ pnet, float t_lo, float t_hi,
                                                   int32_t* __restrict__ list, int32_t* __restrict__ count) {
-  extern __shared__ __align__(16) unsigned char lsm[];
   if (gate_sc && !gate_sc->active) return;
-  limit_item<LM, COMPACT>(K, S, D, BX, BY, flags, trouble, stage, divfree, sc, net, QM, pnet, t_lo, t_hi, gtid(), lsm,
-                          list, count);
+  limit_item<LM, true>(K, S, D, BX, BY, flags, trouble, stage, divfree, sc, nullptr, nullptr, pnet, t_lo, t_hi, gtid(),
+                       nullptr, LimList<int32_t>{list, count, 0});
 }
 
-// The cells k_limit<LM, true> deferred, one per thread (the grid covers
-// every interior cell; threads past the count return).
+// The limiting pass, one cell per thread: the cells k_limit<LM, true> deferred
+// (the grid covers every interior cell; threads past the count return), or,
+// with list null (GDF_DETECT_ALL), every interior cell.
 __global__ void __launch_bounds__(LIM_BS, GDF_LIMIT_MINB) k_limit_tvb(const __grid_constant__ Consts K,
                                                   const double* __restrict__ S, double* __restrict__ D,
                                                   const double* __restrict__ BX, const double* __restrict__ BY,
@@ -278,8 +270,8 @@ __global__ void __launch_bounds__(LIM_BS, GDF_LIMIT_MINB) k_limit_tvb(const __gr
                                                   const int32_t* __restrict__ count) {
   if (gate_sc && !gate_sc->active) return;
   const long long t = gtid();
-  if (t >= *count) return;
-  limit_tvb_item(K, S, D, BX, BY, flags, stage, divfree, sc, list[t]);
+  if (t >= (list ? (long long)*count : (long long)K.nx * K.ny)) return;
+  limit_tvb_item(K, S, D, BX, BY, flags, stage, divfree, sc, list ? list[t] : t);
 }
 
 __global__ void k_faceb_limit(const __grid_constant__ Consts K, const double* __restrict__ S,
@@ -558,6 +550,7 @@ static void build_consts(const GdfConfig& c, Consts& K) {
   K.P.kml_w = c.kml_w_term;
   K.P.eig_p_typo = c.eig_p_typo;
   K.P.eig_identity = c.eig_identity;
+  set_eig_consts(K.P);
   // get_GLP.f90:38-56 (5-point branch)
   const double lam[NG] = {-0.9061798459386639927976269, -0.5384693101056830910363144, 0,
                           0.5384693101056830910363144, 0.9061798459386639927976269};
@@ -717,76 +710,50 @@ static int launch_limit(GdfHandle* h, const double* S, double* D, int stage, con
   const Consts& K = h->K;
   const long long ncell = (long long)K.nx * K.ny;
   const int fused_divfree = K.faceb ? 0 : 1;
-  size_t smem = 0;
   // the network runs at the first stage of a step (and at the start-up
   // limiting); stages 2 and 3 reuse its probabilities
-  const int infer = stage <= 1 ? 1 : 0;
   if (K.detector == GDF_DETECT_LEARNED) {
     if (!h->net || !h->QM) return fail(GDF_ERR_STATE, "detector GDF_DETECT_LEARNED needs gdf_set_indicator first");
-    if (infer) {
+    if (stage <= 1) {
       int rq = run_kernel(h, GDF_K_LIMIT, [&] { k_qmodes<<<nblk(K.plane, 128), 128, 0, h->st>>>(K, S, h->QM); });
-      if (!rq && GDF_INFER_APART) {
-        const long long tiles = (long long)nblk(ncell, LIM_BS);
-        int per_sm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_infer, LIM_BS, LIMIT_SMEM_LEARNED) !=
-                cudaSuccess ||
-            per_sm <= 0) {
-          cudaGetLastError();
-          per_sm = 1;
-        }
-        const unsigned nb = (unsigned)std::min<long long>(tiles, (long long)per_sm * h->sms);
-        rq = run_kernel(h, GDF_K_LIMIT, [&] {
-          k_infer<<<nb, LIM_BS, LIMIT_SMEM_LEARNED, h->st>>>(K, h->net, h->QM, h->pnet, sc_gate);
-        });
-      }
       if (rq) return rq;
-      smem = LIMIT_SMEM_LEARNED;
+      const long long tiles = (long long)nblk(ncell, LIM_BS);
+      int per_sm = 0;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_infer, LIM_BS, LIMIT_SMEM_LEARNED) != cudaSuccess ||
+          per_sm <= 0) {
+        cudaGetLastError();
+        per_sm = 1;
+      }
+      const unsigned nb = (unsigned)std::min<long long>(tiles, (long long)per_sm * h->sms);
+      rq = run_kernel(h, GDF_K_LIMIT, [&] {
+        k_infer<<<nb, LIM_BS, LIMIT_SMEM_LEARNED, h->st>>>(K, h->net, h->QM, h->pnet, sc_gate);
+      });
+      if (rq) return rq;
     }
   }
-  // KXRCF: the gated cells go to a second pass over full warps (the sticky
-  // flags leave mixed warps for most of a run: the developed 512^2 rotor's
-  // limiter 1.8x faster). The learned gate stays in one pass by default
-  // (GDF_LEARNED_TWO_PASS): two passes are faster while few cells are gated
-  // (learned blast 512^2, steps 1-1200, 5.41 against 5.67 ms per step;
-  // blast 2048^2 45.4 against 45.6 ms) but slower once most are (the whole
-  // 512^2 blast run to t = 0.01, 87% gated late: 7.86 against 7.13 ms per
-  // step, two bench runs whose plain steps took 7.15 and 7.14 ms), same
-  // values either way.
-  const bool compact = K.detector == GDF_DETECT_KXRCF ||
-                       (GDF_LEARNED_TWO_PASS && K.detector == GDF_DETECT_LEARNED && (GDF_INFER_APART || !infer));
-  if (compact) CK(cudaMemsetAsync(h->lim_count, 0, sizeof(int32_t), h->st));
+  // two passes: the detector lists the gated cells, which the limiting pass
+  // takes over full warps (a sticky KXRCF flag leaves mixed warps for most of
+  // a run)
+  const bool all = K.detector == GDF_DETECT_ALL;   // no gate: the limiting pass over every cell
   int32_t *L = h->lim_list, *N = h->lim_count;
-  int rc0 = run_kernel(h, GDF_K_LIMIT, [&] {
-    const unsigned nb = nblk(ncell, LIM_BS);
-    if (K.detector == GDF_DETECT_LEARNED && infer && !GDF_INFER_APART)
-      k_limit<LIM_INFER, false><<<nb, LIM_BS, smem, h->st>>>(K, S, D, h->BX, h->BY, h->flags, h->trouble, stage,
-                                                             fused_divfree, sc_gate, h->sc, h->net, h->QM, h->pnet,
-                                                             h->t_lo, h->t_hi, nullptr, nullptr);
-    else if (K.detector == GDF_DETECT_LEARNED && compact)
-      k_limit<LIM_PNET, true><<<nb, LIM_BS, 0, h->st>>>(K, S, D, h->BX, h->BY, h->flags, h->trouble, stage,
-                                                        fused_divfree, sc_gate, h->sc, h->net, h->QM, h->pnet,
-                                                        h->t_lo, h->t_hi, L, N);
-    else if (K.detector == GDF_DETECT_LEARNED)
-      k_limit<LIM_PNET, false><<<nb, LIM_BS, 0, h->st>>>(K, S, D, h->BX, h->BY, h->flags, h->trouble, stage,
-                                                         fused_divfree, sc_gate, h->sc, h->net, h->QM, h->pnet,
-                                                         h->t_lo, h->t_hi, nullptr, nullptr);
-    else if (compact)
-      k_limit<LIM_PLAIN, true><<<nb, LIM_BS, 0, h->st>>>(K, S, D, h->BX, h->BY, h->flags, h->trouble, stage,
-                                                         fused_divfree, sc_gate, h->sc, nullptr, nullptr, nullptr,
-                                                         0.f, 0.f, L, N);
-    else
-      k_limit<LIM_PLAIN, false><<<nb, LIM_BS, 0, h->st>>>(K, S, D, h->BX, h->BY, h->flags, h->trouble, stage,
-                                                          fused_divfree, sc_gate, h->sc, nullptr, nullptr, nullptr,
-                                                          0.f, 0.f, nullptr, nullptr);
+  if (!all) {
+    CK(cudaMemsetAsync(N, 0, sizeof(int32_t), h->st));
+    int rc = run_kernel(h, GDF_K_LIMIT, [&] {
+      const unsigned nb = nblk(ncell, LIM_BS);
+      if (K.detector == GDF_DETECT_LEARNED)
+        k_limit<LIM_PNET><<<nb, LIM_BS, 0, h->st>>>(K, S, D, h->BX, h->BY, h->flags, h->trouble, stage, fused_divfree,
+                                                    sc_gate, h->sc, h->pnet, h->t_lo, h->t_hi, L, N);
+      else
+        k_limit<LIM_PLAIN><<<nb, LIM_BS, 0, h->st>>>(K, S, D, h->BX, h->BY, h->flags, h->trouble, stage, fused_divfree,
+                                                     sc_gate, h->sc, nullptr, 0.f, 0.f, L, N);
+    });
+    if (rc) return rc;
+  }
+  int rc0 = run_kernel(h, GDF_K_LIMIT_TVB, [&] {
+    k_limit_tvb<<<nblk(ncell, LIM_BS), LIM_BS, 0, h->st>>>(K, S, D, h->BX, h->BY, h->flags, stage, fused_divfree,
+                                                           sc_gate, h->sc, all ? nullptr : L, N);
   });
   if (rc0) return rc0;
-  if (compact) {
-    rc0 = run_kernel(h, GDF_K_LIMIT_TVB, [&] {
-      k_limit_tvb<<<nblk(ncell, LIM_BS), LIM_BS, 0, h->st>>>(K, S, D, h->BX, h->BY, h->flags, stage, fused_divfree,
-                                                             sc_gate, h->sc, L, N);
-    });
-    if (rc0) return rc0;
-  }
   if (K.faceb) {
     // TVB_Limiter_P2.f90:126-187 then div_free: set_bc on the limited state,
     // face-B minmod, div-free reconstruction

@@ -15,6 +15,7 @@
 
 #include <math.h>
 #include <stdint.h>
+#include <string.h>
 
 #if defined(__CUDACC__)
 #define GDF_HD __host__ __device__ __forceinline__
@@ -76,6 +77,12 @@ GDF_HD double sqz(double x) {
   return ZF ? sqrt0(x) : sqrt(x);
 }
 
+// Constants of the eigenvectors that depend on gflux alone (eigenmatrix.f90);
+// set_eig_consts fills them with the values eigen_left and eigen_right form.
+struct EigC {
+  double sqgam, gu1sq, sqg2, sq1og, sq12, sq2, rg1;   // rg1: RN(1 / (gflux - 1))
+};
+
 // Run-time physics constants shared by every kernel.
 struct Phys {
   double gamma, gamma1;   // com.txt:7-8
@@ -85,7 +92,12 @@ struct Phys {
   int kml_w;              // Lh.f90:126 w-term in KML
   int eig_p_typo;         // eigenmatrix.f90:21 DF form
   int eig_identity;       // eigenmatrix.f90:397-404
+  EigC ec;
 };
+GDF_HD void set_eig_consts(Phys& P) {
+  const double gm = P.gflux, g1 = gm - 1.0;
+  P.ec = {sqrt(g1 / gm), sqrt(1.0 / gm), sqrt(1.0 / (2.0 * gm)), sqrt(1.0 / gm), sqrt(0.5), sqrt(2.0), 1.0 / g1};
+}
 
 // ------------------------------------------------------------- state -----
 // A conservative state with the primitives every routine of the reference

@@ -793,6 +793,9 @@ static __device__ bool kxrcf_flag(const Consts& K, const double* __restrict__ S,
   return flag;
 }
 
+__device__ __forceinline__ void divfree_item(const Consts& K, double* __restrict__ D, const double* __restrict__ BX,
+                                             const double* __restrict__ BY, long long item);
+
 // calculate_tq of pp_Limiter.f90:101-126
 static __device__ double pp_tq(const Consts& K, const double* ubar, const double* uq) {
   double ta = 0.0, tb = 1.0;
@@ -808,7 +811,20 @@ static __device__ double pp_tq(const Consts& K, const double* ubar, const double
   return ta;
 }
 
-// pp_Limiter.f90:10-81 for one cell's modes (in place)
+// pp_Limiter.f90:58-72: the share of u_q - u_bar that keeps the pressure of
+// one point with pq < 0 positive
+static __device__ double pp_point(const Consts& K, const double* ubar, const double* uq) {
+  const double tq = pp_tq(K, ubar, uq);
+  double n1 = 0.0, n2 = 0.0;
+#pragma unroll
+  for (int n = 0; n < NE; ++n) {
+    const double sqv = tq * uq[n] + (1 - tq) * ubar[n];
+    n1 = n1 + sq(sqv - ubar[n]);
+    n2 = n2 + sq(uq[n] - ubar[n]);
+  }
+  return sqrt(n1) / sqrt(n2);
+}
+
 // Bound on |u_q - u_bar| over the 50 GLL-mixed points for variable n:
 // sum_d |m_d| max_q |phi_d(q)|, inflated to cover the rounding of the point
 // sums (relative error < 2.3e-15 of |u_bar| + the bound).
@@ -820,54 +836,59 @@ __device__ __forceinline__ double pp_spread(const Consts& K, const double (*m)[N
   return b * (1.0 + 1e-12) + 1e-12 * fabs(m[n][0]);
 }
 
-// pp_Limiter.f90:10-81 for one cell's modes (in place). The density part
-// acts only if some point has |rho_bar - rho_q| > rho_bar - 1e-13, and the
-// pressure part only if some point has a negative pressure; when the
-// bounds of pp_spread rule that out (with margins far above rounding) the
-// point evaluations are skipped and the cell is left exactly as the full
-// evaluation would leave it.
+// Whether pp_Limiter.f90 leaves a cell alone: the density part acts only if
+// some point has |rho_bar - rho_q| > rho_bar - 1e-13, the pressure part only
+// if some point has a negative pressure. Where the bounds of pp_spread rule
+// both out (with margins far above rounding) the point evaluations would
+// change nothing.
+__device__ __forceinline__ bool pp_rho_safe(const Consts& K, const double (*m)[NP]) {
+  return pp_spread(K, m, 0) < (m[0][0] - 1e-13) * (1.0 - 1e-12);
+}
+// a lower bound of the pressure at every point, from bounds on the point
+// values; positive beyond rounding: no point has pq < 0
+__device__ __forceinline__ bool pp_pressure_safe(const Consts& K, const double (*m)[NP]) {
+  double dv[NE];
+#pragma unroll
+  for (int n = 0; n < NE; ++n) dv[n] = pp_spread(K, m, n);
+  const double rho_lo = m[0][0] - dv[0];
+  if (!(rho_lo > 0.0)) return false;
+  const double e_lo = m[4][0] - dv[4];
+  const double k_hi = 0.5 * (sq(fabs(m[1][0]) + dv[1]) + sq(fabs(m[2][0]) + dv[2]) + sq(fabs(m[3][0]) + dv[3])) /
+                      rho_lo * (1.0 + 1e-12);
+  const double b_hi = 0.5 * (sq(fabs(m[5][0]) + dv[5]) + sq(fabs(m[6][0]) + dv[6]) + sq(fabs(m[7][0]) + dv[7])) *
+                      (1.0 + 1e-12);
+  const double p_lo = e_lo - k_hi - b_hi;
+  return p_lo > 1e-10 * (fabs(e_lo) + k_hi + b_hi);
+}
+
+// pp_Limiter.f90:10-81 for one cell's modes (in place), by one thread: the
+// ensemble's persistent stage kernel, whose limiter phase has no pass of its
+// own for these cells (elsewhere pp_item_warp takes them).
 static __device__ void pp_cell(const Consts& K, double (*m)[NP]) {
   const double epsilon = 1e-13;
   double eta = 1.0;
   const double rb = m[0][0];
-  const bool rho_safe = pp_spread(K, m, 0) < (rb - epsilon) * (1.0 - 1e-12);
-  if (!rho_safe) {
+  if (!pp_rho_safe(K, m)) {
 #pragma unroll 1
-  for (int a = 0; a < NG; ++a)
+    for (int a = 0; a < NG; ++a)
 #pragma unroll 1
-    for (int b = 0; b < NG; ++b)
+      for (int b = 0; b < NG; ++b)
 #pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        double rq = 0.0;
+        for (int s = 0; s < 2; ++s) {
+          double rq = 0.0;
 #pragma unroll
-        for (int d = 0; d < NP; ++d)
-          if (live_mode(0, d)) rq = rq + m[0][d] * c_basis.phiGLL[s][a][b][d];
-        const double eta1 = fabs((rb - epsilon) / (rb - rq));
-        if (eta1 < 1) eta = eta1;
-      }
-  if (eta < 1) {
-    const double f = 0.5 * eta;
+          for (int d = 0; d < NP; ++d)
+            if (live_mode(0, d)) rq = rq + m[0][d] * c_basis.phiGLL[s][a][b][d];
+          const double eta1 = fabs((rb - epsilon) / (rb - rq));
+          if (eta1 < 1) eta = eta1;
+        }
+    if (eta < 1) {
+      const double f = 0.5 * eta;
 #pragma unroll
-    for (int d = 1; d < NP; ++d) m[0][d] = f * m[0][d];
-  }
-  }
-  {
-    // lower bound of the pressure at every point from bounds on the point
-    // values; a positive bound (beyond rounding) means no point has pq < 0
-    double dv[NE];
-#pragma unroll
-    for (int n = 0; n < NE; ++n) dv[n] = pp_spread(K, m, n);
-    const double rho_lo = m[0][0] - dv[0];
-    if (rho_lo > 0.0) {
-      const double e_lo = m[4][0] - dv[4];
-      const double k_hi = 0.5 * (sq(fabs(m[1][0]) + dv[1]) + sq(fabs(m[2][0]) + dv[2]) + sq(fabs(m[3][0]) + dv[3])) /
-                          rho_lo * (1.0 + 1e-12);
-      const double b_hi = 0.5 * (sq(fabs(m[5][0]) + dv[5]) + sq(fabs(m[6][0]) + dv[6]) + sq(fabs(m[7][0]) + dv[7])) *
-                          (1.0 + 1e-12);
-      const double p_lo = e_lo - k_hi - b_hi;
-      if (p_lo > 1e-10 * (fabs(e_lo) + k_hi + b_hi)) return;   // eta stays 1: nothing changes
+      for (int d = 1; d < NP; ++d) m[0][d] = f * m[0][d];
     }
   }
+  if (pp_pressure_safe(K, m)) return;   // eta stays 1: nothing changes
   double ubar[NE];
 #pragma unroll
   for (int n = 0; n < NE; ++n) ubar[n] = m[n][0];
@@ -888,18 +909,7 @@ static __device__ void pp_cell(const Consts& K, double (*m)[NP]) {
             if (live_mode(n, d)) acc = acc + m[n][d] * c_basis.phiGLL[s][a][b][d];
           uq[n] = acc;
         }
-        const double pq = pressure(K.P.gamma, uq);
-        if (pq < 0) {
-          const double tq = pp_tq(K, ubar, uq);
-          double n1 = 0.0, n2 = 0.0;
-#pragma unroll
-          for (int n = 0; n < NE; ++n) {
-            const double sqv = tq * uq[n] + (1 - tq) * ubar[n];
-            n1 = n1 + sq(sqv - ubar[n]);
-            n2 = n2 + sq(uq[n] - ubar[n]);
-          }
-          eta1 = sqrt(n1) / sqrt(n2);
-        }
+        if (pressure(K.P.gamma, uq) < 0) eta1 = pp_point(K, ubar, uq);
         if (eta1 < eta) eta = eta1;
       }
   if (eta < 1) eta = 0.5 * eta;
@@ -907,6 +917,109 @@ static __device__ void pp_cell(const Consts& K, double (*m)[NP]) {
   for (int n = 0; n < NE; ++n)
 #pragma unroll
     for (int d = 1; d < NP; ++d) m[n][d] = eta * m[n][d];
+}
+
+// The 50 GLL-mixed points of pp_Limiter.f90 in its loop order, p = 2*(5*a +
+// b) + s, transposed ([mode][point]) so that 32 lanes at 32 points read 32
+// banks.
+constexpr int PP_POINTS = 2 * NG * NG;
+constexpr int PP_BS = 128;   // four cells per block
+__device__ __forceinline__ void pp_stage_points(double* sb /* [NP * PP_POINTS] */) {
+  for (int k = threadIdx.x; k < NP * PP_POINTS; k += blockDim.x) {
+    const int d = k / PP_POINTS, p = k - d * PP_POINTS;
+    sb[k] = c_basis.phiGLL[p & 1][p / (2 * NG)][(p >> 1) % NG][d];
+  }
+}
+
+// pp_Limiter.f90:10-81 for one cell whose limited modes are in D, by one
+// warp: a lane per point in two rounds, instead of one thread walking 50
+// points of which each one with a negative pressure costs 47 dependent
+// bisection steps. The density part keeps the last eta1 < 1 in point order
+// (the highest lane of the later round that has one); the pressure part's
+// running minimum is the same in any order. Then the div-free
+// reconstruction where the limiter fuses it. sm: the warp's NLIVE doubles.
+__device__ __forceinline__ void pp_item_warp(const Consts& K, double* __restrict__ D, const double* __restrict__ BX,
+                                             const double* __restrict__ BY, int divfree, long long item,
+                                             const double* sb, double* sm) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int i = (int)(item % K.nx) + 1, j = (int)(item / K.nx) + 1;
+  const long long c = i + (long long)K.nx2 * j, pl = K.plane;
+  for (int s = lane; s < NLIVE; s += 32) sm[s] = D[c + pl * (c_live_d[s] + 10 * c_live_n[s])];
+  __syncwarp();
+  const double epsilon = 1e-13, rb = sm[0];
+  bool changed = false;
+  double spread = 0.0;   // pp_spread of the density
+#pragma unroll
+  for (int d = 1; d < NP; ++d)
+    if (live_mode(0, d)) spread = spread + fabs(sm[LI(0, d)]) * c_basis.ppM[d];
+  spread = spread * (1.0 + 1e-12) + 1e-12 * fabs(rb);
+  if (!(spread < (rb - epsilon) * (1.0 - 1e-12))) {
+    double eta = 1.0;
+#pragma unroll 1
+    for (int r = 1; r >= 0; --r) {
+      const int p = lane + 32 * r;
+      double eta1 = 1.0;
+      if (p < PP_POINTS) {
+        double rq = 0.0;
+#pragma unroll
+        for (int d = 0; d < NP; ++d)
+          if (live_mode(0, d)) rq = rq + sm[LI(0, d)] * sb[d * PP_POINTS + p];
+        eta1 = fabs((rb - epsilon) / (rb - rq));
+      }
+      const unsigned hit = __ballot_sync(full, eta1 < 1);
+      if (hit) {
+        eta = __shfl_sync(full, eta1, 31 - __clz(hit));
+        break;
+      }
+    }
+    if (eta < 1) {
+      changed = true;
+      const double f = 0.5 * eta;
+      __syncwarp();
+      if (lane >= 1 && lane < 6) sm[lane] = f * sm[lane];
+      __syncwarp();
+    }
+  }
+  double eta = 1.0;
+#pragma unroll 1
+  for (int r = 0; r < 2; ++r) {
+    const int p = lane + 32 * r;
+    if (p >= PP_POINTS) break;
+    double uq[NE], ubar[NE];
+#pragma unroll
+    for (int n = 0; n < NE; ++n) {
+      double acc = 0.0;
+#pragma unroll
+      for (int d = 0; d < NP; ++d)
+        if (live_mode(n, d)) acc = acc + sm[LI(n, d)] * sb[d * PP_POINTS + p];
+      uq[n] = acc;
+      ubar[n] = sm[LI(n, 0)];
+    }
+    if (pressure(K.P.gamma, uq) < 0) {
+      const double eta1 = pp_point(K, ubar, uq);
+      if (eta1 < eta) eta = eta1;
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double e = __shfl_xor_sync(full, eta, o);
+    if (e < eta) eta = e;
+  }
+  if (eta < 1) {
+    changed = true;
+    eta = 0.5 * eta;
+  }
+  // modes 2.. of every variable scaled (eta = 1: by nothing)
+  if (changed)
+    for (int s = lane; s < NLIVE; s += 32) {
+      const int n = c_live_n[s], d = c_live_d[s];
+      if (d == 0 || (divfree && (n == 5 || n == 6))) continue;
+      D[c + pl * (d + 10 * n)] = eta * sm[s];
+    }
+  if (divfree && lane == 0) divfree_item(K, D, BX, BY, item);
+  __syncwarp();
 }
 
 __device__ __forceinline__ void lim_load(const Consts& K, const double* __restrict__ S, long long c, double (*m)[NP]) {
@@ -1239,12 +1352,47 @@ __device__ __forceinline__ void lim_tvb(const Consts& K, const double* __restric
   word |= (int32_t)change;
 }
 
+// Cells left to a later pass: list entries are tag + item.
+template <class T>
+struct LimList {
+  T* list;
+  int32_t* count;
+  T tag;
+};
+
+// Appends the gated cells among the calling warp's active lanes to the list
+// (one atomic per warp); true for a gated cell.
+template <class T>
+__device__ __forceinline__ bool lim_defer(bool gate, long long item, const LimList<T>& l) {
+  const unsigned act = __activemask();
+  const unsigned bal = __ballot_sync(act, gate);
+  if (!gate) return false;
+  const int lane = threadIdx.x & 31;
+  const int leader = __ffs(bal) - 1;
+  int base = 0;
+  if (lane == leader) base = atomicAdd(l.count, __popc(bal));
+  base = __shfl_sync(bal, base, leader);
+  l.list[base + __popc(bal & ((1u << lane) - 1u))] = l.tag + (T)item;
+  return true;
+}
+
+// PPD: a cell the positivity limiter may change is stored as it is and listed
+// in pp (pp_item_warp limits and finishes it in a pass of its own); otherwise
+// it is limited here.
+template <bool PPD>
 __device__ __forceinline__ void lim_finish(const Consts& K, double* __restrict__ D, const double* __restrict__ BX,
                                            const double* __restrict__ BY, int32_t* __restrict__ flags, int stage,
                                            int divfree, Scal* __restrict__ sc, long long item, int i, int j,
-                                           long long c, double (*m)[NP], int32_t word) {
+                                           long long c, double (*m)[NP], int32_t word,
+                                           const LimList<long long>& pp) {
   const long long pl = K.plane;
-  if (K.pp) pp_cell(K, m);
+  if (K.pp) {
+    if (PPD) {
+      if (lim_defer(!(pp_rho_safe(K, m) && pp_pressure_safe(K, m)), item, pp)) divfree = 0;
+    } else {
+      pp_cell(K, m);
+    }
+  }
   if (divfree) {
     // div_free_Balsara.f90:30-75 from the four face polynomials
     const long long fxp = K.fxplane, fyp = K.fyplane;
@@ -1288,30 +1436,6 @@ __device__ __forceinline__ void lim_finish(const Consts& K, double* __restrict__
   if (!(m[0][0] > 0.0) || !isfinite(m[4][0])) atomicOr(&sc->status, 1);
 }
 
-// Cells left to a later pass: list entries are tag + item.
-template <class T>
-struct LimList {
-  T* list;
-  int32_t* count;
-  T tag;
-};
-
-// Appends the gated cells among the calling warp's active lanes to the list
-// (one atomic per warp); true for a gated cell.
-template <class T>
-__device__ __forceinline__ bool lim_defer(bool gate, long long item, const LimList<T>& l) {
-  const unsigned act = __activemask();
-  const unsigned bal = __ballot_sync(act, gate);
-  if (!gate) return false;
-  const int lane = threadIdx.x & 31;
-  const int leader = __ffs(bal) - 1;
-  int base = 0;
-  if (lane == leader) base = atomicAdd(l.count, __popc(bal));
-  base = __shfl_sync(bal, base, leader);
-  l.list[base + __popc(bal & ((1u << lane) - 1u))] = l.tag + (T)item;
-  return true;
-}
-
 // One interior cell of the limiter. COMPACT: a gated cell is only appended
 // to list (limit_tvb_item finishes it in a second pass over full warps, so
 // the characteristic limiter never runs beside idle lanes); an ungated one
@@ -1323,7 +1447,8 @@ __device__ __forceinline__ void limit_item(const Consts& K, const double* __rest
                                            int divfree, Scal* __restrict__ sc, const MlpDev* __restrict__ net,
                                            const float* __restrict__ QM, float* __restrict__ pnet,
                                            float t_lo, float t_hi, long long item, unsigned char* lsm,
-                                           const LimList<T>& defer = LimList<T>{}) {
+                                           const LimList<T>& defer = LimList<T>{},
+                                           const LimList<long long>& pp = LimList<long long>{}) {
   const bool valid = item < (long long)K.nx * K.ny;
   const int i = valid ? (int)(item % K.nx) + 1 : 1;
   const int j = valid ? (int)(item / K.nx) + 1 : 1;
@@ -1337,7 +1462,7 @@ __device__ __forceinline__ void limit_item(const Consts& K, const double* __rest
   } else if (gate) {
     lim_tvb(K, S, c, m, word);
   }
-  lim_finish(K, D, BX, BY, flags, stage, divfree, sc, item, i, j, c, m, word);
+  lim_finish<COMPACT>(K, D, BX, BY, flags, stage, divfree, sc, item, i, j, c, m, word, pp);
 }
 
 // A cell every thread of the limiting pass limits: one limit_item<LM, true>
@@ -1347,7 +1472,8 @@ __device__ __forceinline__ void limit_item(const Consts& K, const double* __rest
 __device__ __forceinline__ void limit_tvb_item(const Consts& K, const double* __restrict__ S, double* __restrict__ D,
                                                const double* __restrict__ BX, const double* __restrict__ BY,
                                                int32_t* __restrict__ flags, int stage, int divfree,
-                                               Scal* __restrict__ sc, long long item) {
+                                               Scal* __restrict__ sc, long long item,
+                                               const LimList<long long>& pp) {
   const int i = (int)(item % K.nx) + 1;
   const int j = (int)(item / K.nx) + 1;
   const long long c = i + (long long)K.nx2 * j;
@@ -1363,7 +1489,7 @@ __device__ __forceinline__ void limit_tvb_item(const Consts& K, const double* __
     tvb_apply(change, res, m);
     word |= (int32_t)change;
   }
-  lim_finish(K, D, BX, BY, flags, stage, divfree, sc, item, i, j, c, m, word);
+  lim_finish<true>(K, D, BX, BY, flags, stage, divfree, sc, item, i, j, c, m, word, pp);
 }
 
 // Face-B TVB limiter of TVB_Limiter_P2.f90:128-187 (applied when enabled):

@@ -77,8 +77,8 @@ struct EnsArgs {
   const int* off;                 // [EK_N][n + 1] tile prefix sums
   unsigned long long* amax;       // [2n] bit patterns of the x / y speed maxima
   EnsSync* sync;
-  long long* lim_list;            // (instance << 40) + cell: gated cells, for the limiting pass
-  int32_t* lim_count;
+  long long *lim_list, *pp_list;  // (instance << 40) + cell: gated cells, cells left to the positivity pass
+  int32_t* lim_count;             // [0] and [1]: their counts
   const MlpDev* net;
   unsigned long long timeout_ns;
   int n;
@@ -480,7 +480,8 @@ __global__ void __launch_bounds__(ENS_BS) k_ep_limit(const __grid_constant__ Ens
   for_tiles<true>(A, EK_LIM, [&](int i, const EnsInst& I, const Consts& K, long long base, int) {
     limit_item<LM, true>(K, I.UI, I.U, I.BX, I.BY, I.flags, I.trouble, stage, K.faceb ? 0 : 1, I.sc, A.net, I.QM,
                          I.pnet, A.t_lo, A.t_hi, base + threadIdx.x, lsm,
-                         LimList<long long>{A.lim_list, A.lim_count, (long long)i << 40});
+                         LimList<long long>{A.lim_list, A.lim_count, (long long)i << 40},
+                         LimList<long long>{A.pp_list, A.lim_count + 1, (long long)i << 40});
     if (LM == LIM_INFER) __syncthreads();
   });
 }
@@ -492,7 +493,26 @@ __global__ void __launch_bounds__(ENS_BS) k_ep_limit_tvb(const __grid_constant__
   for (long long k = (long long)blockIdx.x * ENS_BS + threadIdx.x; k < n; k += (long long)gridDim.x * ENS_BS) {
     const long long e = A.lim_list[k];
     const EnsInst& I = A.inst[e >> 40];
-    limit_tvb_item(*I.K, I.UI, I.U, I.BX, I.BY, I.flags, stage, I.K->faceb ? 0 : 1, I.sc, e & ((1LL << 40) - 1));
+    limit_tvb_item(*I.K, I.UI, I.U, I.BX, I.BY, I.flags, stage, I.K->faceb ? 0 : 1, I.sc, e & ((1LL << 40) - 1),
+                   LimList<long long>{A.pp_list, A.lim_count + 1, (e >> 40) << 40});
+  }
+}
+
+// the positivity limiter of every instance's listed cells, one warp per cell
+// (as k_pp)
+__global__ void __launch_bounds__(PP_BS) k_ep_pp(const __grid_constant__ EnsArgs A) {
+  __shared__ double sb[NP * PP_POINTS];
+  __shared__ double sm[PP_BS / 32][NLIVE];
+  const int n = A.lim_count[1];
+  constexpr int W = PP_BS / 32;
+  if ((int)blockIdx.x * W >= n) return;
+  pp_stage_points(sb);
+  __syncthreads();
+  const int w = threadIdx.x >> 5;
+  for (long long k = (long long)blockIdx.x * W + w; k < n; k += (long long)gridDim.x * W) {
+    const long long e = A.pp_list[k];
+    const EnsInst& I = A.inst[e >> 40];
+    pp_item_warp(*I.K, I.U, I.BX, I.BY, I.K->faceb ? 0 : 1, e & ((1LL << 40) - 1), sb, sm[w]);
   }
 }
 
@@ -552,7 +572,8 @@ struct GdfEnsemble {
   int learned = 0;
   float t_lo = 0.5f, t_hi = 0.5f;
   int any_faceb = 0;
-  long long* lim_list = nullptr;
+  int any_pp = 0;
+  long long *lim_list = nullptr, *pp_list = nullptr;
   int32_t* lim_count = nullptr;
   int uploaded = 0;
   // tile shape
@@ -646,6 +667,7 @@ int ens_layout(GdfEnsemble* e) {
   A.any_faceb = e->any_faceb;
   A.lim_list = e->lim_list;
   A.lim_count = e->lim_count;
+  A.pp_list = e->pp_list;
   A.t_lo = e->t_lo;
   A.t_hi = e->t_hi;
   if (e->graph) {
@@ -702,7 +724,7 @@ int launch_stage_phases(GdfEnsemble* e, int stage) {
     n += 3;
   }
   const int ls = stage == 0 ? 1 : stage;
-  ECK(cudaMemsetAsync(A.lim_count, 0, sizeof(int32_t), st));
+  ECK(cudaMemsetAsync(A.lim_count, 0, 2 * sizeof(int32_t), st));
   if (e->learned && stage <= 1) {
     k_ep_qmodes<<<tiles_of(A, EK_QM), ENS_BS, 0, st>>>(A);
     k_ep_limit<LIM_INFER><<<tiles_of(A, EK_LIM), ENS_BS, LIMIT_SMEM_LEARNED, st>>>(A, ls);
@@ -716,6 +738,10 @@ int launch_stage_phases(GdfEnsemble* e, int stage) {
   }
   k_ep_limit_tvb<<<tiles_of(A, EK_LIM), ENS_BS, 0, st>>>(A, ls);
   ++n;
+  if (e->any_pp) {
+    k_ep_pp<<<std::min(tiles_of(A, EK_LIM), (unsigned)(8 * e->sms)), PP_BS, 0, st>>>(A);
+    ++n;
+  }
   if (A.any_faceb) {
     bc(EK_BCF, 0);
     k_ep_faceb<<<tiles_of(A, EK_FB), ENS_BS, 0, st>>>(A);
@@ -822,7 +848,7 @@ int gdf_ens_destroy(GdfEnsemble* e) {
       if (p) cudaFree(p);
   }
   void* bufs[] = {e->dK, e->dInst, e->sc, e->amax, e->sync, e->off, e->net, e->sc_save,
-                  e->lim_list, e->lim_count};
+                  e->lim_list, e->lim_count, e->pp_list};
   for (void* p : bufs)
     if (p) cudaFree(p);
   if (e->sc_host) cudaFreeHost(e->sc_host);
@@ -869,6 +895,7 @@ int gdf_ens_create(const GdfConfig* cfgs, int32_t n, GdfEnsemble** out) {
     consts_for(cfgs[i], b.K);
     if (i == 0) ok = ok && upload_basis_once(b.K, true) == cudaSuccess;
     if (b.K.faceb) e->any_faceb = 1;
+    if (b.K.pp) e->any_pp = 1;
     cells += (long long)cfgs[i].nx * cfgs[i].ny;
     const Consts& K = b.K;
     const GdfConfig& c = cfgs[i];
@@ -887,7 +914,8 @@ int gdf_ens_create(const GdfConfig* cfgs, int32_t n, GdfEnsemble** out) {
     if (ok) ok = cudaMemcpy(e->dK + i, &b.K, sizeof(Consts), cudaMemcpyHostToDevice) == cudaSuccess;
   }
   ok = ok && alloc((void**)&e->lim_list, (size_t)cells * sizeof(long long)) &&
-       alloc((void**)&e->lim_count, sizeof(int32_t));
+       alloc((void**)&e->lim_count, 2 * sizeof(int32_t)) &&
+       (!e->any_pp || alloc((void**)&e->pp_list, (size_t)cells * sizeof(long long)));
   if (!ok) {
     cudaGetLastError();
     gdf_ens_destroy(e);

@@ -252,10 +252,11 @@ __global__ void __launch_bounds__(LIM_BS, GDF_LIMIT_MINB) k_limit(const __grid_c
                                                   int32_t* __restrict__ trouble, int stage, int divfree,
                                                   const Scal* __restrict__ gate_sc, Scal* __restrict__ sc,
                                                   float* __restrict__ pnet, float t_lo, float t_hi,
-                                                  int32_t* __restrict__ list, int32_t* __restrict__ count) {
+                                                  int32_t* __restrict__ list, int32_t* __restrict__ count,
+                                                  LimList<long long> pp) {
   if (gate_sc && !gate_sc->active) return;
   limit_item<LM, true>(K, S, D, BX, BY, flags, trouble, stage, divfree, sc, nullptr, nullptr, pnet, t_lo, t_hi, gtid(),
-                       nullptr, LimList<int32_t>{list, count, 0});
+                       nullptr, LimList<int32_t>{list, count, 0}, pp);
 }
 
 // The limiting pass, one cell per thread: the cells k_limit<LM, true> deferred
@@ -267,11 +268,34 @@ __global__ void __launch_bounds__(LIM_BS, GDF_LIMIT_MINB) k_limit_tvb(const __gr
                                                   int32_t* __restrict__ flags, int stage, int divfree,
                                                   const Scal* __restrict__ gate_sc, Scal* __restrict__ sc,
                                                   const int32_t* __restrict__ list,
-                                                  const int32_t* __restrict__ count) {
+                                                  const int32_t* __restrict__ count, LimList<long long> pp) {
   if (gate_sc && !gate_sc->active) return;
   const long long t = gtid();
   if (t >= (list ? (long long)*count : (long long)K.nx * K.ny)) return;
-  limit_tvb_item(K, S, D, BX, BY, flags, stage, divfree, sc, list ? list[t] : t);
+  limit_tvb_item(K, S, D, BX, BY, flags, stage, divfree, sc, list ? list[t] : t, pp);
+}
+
+// The positivity limiter of the cells the passes before it listed, one warp
+// per cell (pp_item_warp); resident blocks walk the list.
+// What bounds it: the 47 dependent bisection steps of a point with negative
+// pressure, a division and some ten dependent operations each. Inline in the
+// limiter one thread walked its cell's 50 points in turn while its warp
+// waited, so a single such cell set the time of the whole launch (blast 512^2
+// in mid-run: 489 us for the limiting pass, 152 us of it the pass itself).
+__global__ void __launch_bounds__(PP_BS) k_pp(const __grid_constant__ Consts K, double* __restrict__ D,
+                                              const double* __restrict__ BX, const double* __restrict__ BY,
+                                              int divfree, const Scal* __restrict__ gate_sc, LimList<long long> pp) {
+  __shared__ double sb[NP * PP_POINTS];
+  __shared__ double sm[PP_BS / 32][NLIVE];
+  if (gate_sc && !gate_sc->active) return;
+  const int n = *pp.count;
+  constexpr int W = PP_BS / 32;
+  if ((int)blockIdx.x * W >= n) return;
+  pp_stage_points(sb);
+  __syncthreads();
+  const int w = threadIdx.x >> 5;
+  for (long long k = (long long)blockIdx.x * W + w; k < n; k += (long long)gridDim.x * W)
+    pp_item_warp(K, D, BX, BY, divfree, pp.list[k], sb, sm[w]);
 }
 
 __global__ void k_faceb_limit(const __grid_constant__ Consts K, const double* __restrict__ S,
@@ -476,7 +500,8 @@ struct GdfHandle {
   MlpDev* net = nullptr;     // learned-indicator network (device copy)
   float t_lo = 0.5f, t_hi = 0.5f;
   int32_t *flags = nullptr, *trouble = nullptr;
-  int32_t *lim_list = nullptr, *lim_count = nullptr;  // cells the limiter's first pass deferred
+  int32_t *lim_list = nullptr, *lim_count = nullptr;  // cells the limiter's gate listed; [0] their count
+  long long* pp_list = nullptr;   // cells left to the positivity limiter's pass; lim_count[1] their count
   Scal* sc = nullptr;
   Scal* sc_host = nullptr;  // pinned mirror
   int uploaded = 0;
@@ -736,24 +761,32 @@ static int launch_limit(GdfHandle* h, const double* S, double* D, int stage, con
   // a run)
   const bool all = K.detector == GDF_DETECT_ALL;   // no gate: the limiting pass over every cell
   int32_t *L = h->lim_list, *N = h->lim_count;
+  const LimList<long long> pp{h->pp_list, N + 1, 0};
+  if (!all || K.pp) CK(cudaMemsetAsync(N, 0, 2 * sizeof(int32_t), h->st));
   if (!all) {
-    CK(cudaMemsetAsync(N, 0, sizeof(int32_t), h->st));
     int rc = run_kernel(h, GDF_K_LIMIT, [&] {
       const unsigned nb = nblk(ncell, LIM_BS);
       if (K.detector == GDF_DETECT_LEARNED)
         k_limit<LIM_PNET><<<nb, LIM_BS, 0, h->st>>>(K, S, D, h->BX, h->BY, h->flags, h->trouble, stage, fused_divfree,
-                                                    sc_gate, h->sc, h->pnet, h->t_lo, h->t_hi, L, N);
+                                                    sc_gate, h->sc, h->pnet, h->t_lo, h->t_hi, L, N, pp);
       else
         k_limit<LIM_PLAIN><<<nb, LIM_BS, 0, h->st>>>(K, S, D, h->BX, h->BY, h->flags, h->trouble, stage, fused_divfree,
-                                                     sc_gate, h->sc, nullptr, 0.f, 0.f, L, N);
+                                                     sc_gate, h->sc, nullptr, 0.f, 0.f, L, N, pp);
     });
     if (rc) return rc;
   }
   int rc0 = run_kernel(h, GDF_K_LIMIT_TVB, [&] {
     k_limit_tvb<<<nblk(ncell, LIM_BS), LIM_BS, 0, h->st>>>(K, S, D, h->BX, h->BY, h->flags, stage, fused_divfree,
-                                                           sc_gate, h->sc, all ? nullptr : L, N);
+                                                           sc_gate, h->sc, all ? nullptr : L, N, pp);
   });
   if (rc0) return rc0;
+  if (K.pp) {
+    const unsigned nb = (unsigned)std::min<long long>(nblk(ncell, PP_BS / 32), 8LL * h->sms);
+    rc0 = run_kernel(h, GDF_K_LIMIT_TVB, [&] {
+      k_pp<<<nb, PP_BS, 0, h->st>>>(K, D, h->BX, h->BY, fused_divfree, sc_gate, pp);
+    });
+    if (rc0) return rc0;
+  }
   if (K.faceb) {
     // TVB_Limiter_P2.f90:126-187 then div_free: set_bc on the limited state,
     // face-B minmod, div-free reconstruction
@@ -985,7 +1018,8 @@ int gdf_create(const GdfConfig* cfg, GdfHandle** out) {
   ok = ok && alloc((void**)&h->flags, (size_t)ncell * sizeof(int32_t)) &&
        alloc((void**)&h->trouble, (size_t)ncell * sizeof(int32_t));
   ok = ok && alloc((void**)&h->lim_list, (size_t)ncell * sizeof(int32_t)) &&
-       alloc((void**)&h->lim_count, sizeof(int32_t));
+       alloc((void**)&h->lim_count, 2 * sizeof(int32_t)) &&
+       (!cfg->pp_limiter || alloc((void**)&h->pp_list, (size_t)ncell * sizeof(long long)));
   ok = ok && alloc((void**)&h->sc, sizeof(Scal));
   ok = ok && cudaMallocHost((void**)&h->sc_host, sizeof(Scal)) == cudaSuccess;
   if (!ok) {
@@ -1021,6 +1055,7 @@ int gdf_destroy(GdfHandle* h) {
   if (h->trouble) cudaFree(h->trouble);
   if (h->lim_list) cudaFree(h->lim_list);
   if (h->lim_count) cudaFree(h->lim_count);
+  if (h->pp_list) cudaFree(h->pp_list);
   if (h->sc) cudaFree(h->sc);
   if (h->sc_host) cudaFreeHost(h->sc_host);
   if (h->st) cudaStreamDestroy(h->st);

@@ -702,95 +702,115 @@ __device__ __forceinline__ void matvec8(const double* A, const double* x, double
   }
 }
 
-__device__ __forceinline__ void trace8(const Consts& K, const double* __restrict__ S, long long c,
-                                       const double* phi, double* out) {
+// One face of KXRCF_Detector.f90:187-224 for one variable: I gains
+// h1 w(g) (own trace - neighbour's trace) at the five points in order. AX 0: the
+// right face (low: the left), 1: the upper (lower). m and k are the modes of the
+// cell and of its neighbour, cubic the variable's live cubic modes (0 none, 1
+// those of Bx, 2 those of By). The sums keep mode order; the tables' +-1
+// entries and the zeros at the middle point are not multiplied.
+template <int AX>
+__device__ __forceinline__ void kxrcf_face(const double* m, const double* k, bool low, int cubic, double h1,
+                                           double& I) {
+  auto flip = [](double x, bool neg) { return neg ? -x : x; };   // the odd modes' sign on a low face
+  auto trace = [&](const double* q, bool neg, int g) {
+    const double* f = AX == 0 ? c_basis.phiGR[g] : c_basis.phiGU[g];
+    const bool mid = g == 2;
+    double v = 0.0 + q[0];
+    if (AX == 0) v = v + flip(q[1], neg);
+    else if (!mid) v = v + q[1] * f[1];
+    if (AX == 1) v = v + flip(q[2], neg);
+    else if (!mid) v = v + q[2] * f[2];
+    v = v + q[3] * f[3];
+    if (!mid) v = v + flip(q[4] * f[4], neg);
+    v = v + q[5] * f[5];
+    if (cubic == 1 && (AX == 0 || !mid)) {
+      v = v + flip(q[6] * f[6], AX == 0 && neg);
+      v = v + flip(q[7] * f[8], AX == 0 && neg);
+    } else if (cubic == 2 && (AX == 1 || !mid)) {
+      v = v + flip(q[6] * f[7], AX == 1 && neg);
+      v = v + flip(q[7] * f[9], AX == 1 && neg);
+    }
+    return v;
+  };
 #pragma unroll
-  for (int n = 0; n < NE; ++n) {
-    double a = 0.0;
-#pragma unroll
-    for (int d = 0; d < NP; ++d)
-      if (live_mode(n, d)) a = a + S[c + K.plane * (d + 10 * n)] * phi[d];
-    out[n] = a;
-  }
+  for (int g = 0; g < NG; ++g) I = I + h1 * c_basis.w[g] * (trace(m, low, g) - trace(k, !low, g));
 }
 
-// KXRCF_Detector.f90:187-236 for cell c (interior), given its modes m.
-static __device__ bool kxrcf_flag(const Consts& K, const double* __restrict__ S, long long c, const double (*m)[NP],
-                           bool prev) {
-  double I[NE];
-#pragma unroll
-  for (int n = 0; n < NE; ++n) I[n] = 0.0;
-  double Lij = 1e-12;
-  double A[NE], B[NE];
+// KXRCF_Detector.f90:187-236 for cell c (interior): flagged when some |I(n)| /
+// (pow L uinf(n)) reaches Ck, I the jump of the inflow faces, uinf the largest
+// |value| of the cell at its 25 Gauss points. That maximum lies between two
+// bounds that cost a few operations: the root mean square over the points (the
+// basis is orthogonal) and the sum of |mode| max |phi|. Where a bound decides
+// (with a margin of 1e-9, far above rounding) the points are not evaluated.
+// One variable at a time, so that a cell's 52 modes are never held and the
+// gating pass fits 128 registers. What bounded the detector was its loads, some
+// 2,000 per cell (every face point re-read both cells' modes), at 8 warps per
+// SM: the gating pass took 277 us on the rotor 512^2 after 100 steps, 177 with
+// each face's modes read once, 126 as it is.
+static __device__ bool kxrcf_flag(const Consts& K, const double* __restrict__ S, long long c) {
   const long long pl = K.plane;
-  if (S[c + 1 + pl * 10] < 0) {  // uh(i+1,j,1,2) < 0: right side inflow
-#pragma unroll 1
-    for (int g = 0; g < NG; ++g) {
-      trace8(K, S, c, c_basis.phiGR[g], A);
-      trace8(K, S, c + 1, c_basis.phiGL[g], B);
+  const bool r = S[c + 1 + pl * 10] < 0, l = S[c - 1 + pl * 10] > 0;            // uh(i+1,j,1,2) < 0: right side inflow
+  const bool u = S[c + K.nx2 + pl * 20] < 0, w = S[c - K.nx2 + pl * 20] > 0;
+  double Lij = 1e-12;
 #pragma unroll
-      for (int n = 0; n < NE; ++n) I[n] = I[n] + K.hy1 * c_basis.w[g] * (A[n] - B[n]);
-      Lij = Lij + K.hy;
-    }
+  for (int g = 0; g < 4 * NG; ++g) {
+    const int side = g / NG;
+    if (side == 0 ? r : side == 1 ? l : side == 2 ? u : w) Lij = Lij + (side < 2 ? K.hy : K.hx);
   }
-  if (S[c - 1 + pl * 10] > 0) {
+  const double pL = K.pow_hxhy * Lij;
+  const double cd = K.ck * pL;
 #pragma unroll 1
-    for (int g = 0; g < NG; ++g) {
-      trace8(K, S, c, c_basis.phiGL[g], A);
-      trace8(K, S, c - 1, c_basis.phiGR[g], B);
-#pragma unroll
-      for (int n = 0; n < NE; ++n) I[n] = I[n] + K.hy1 * c_basis.w[g] * (A[n] - B[n]);
-      Lij = Lij + K.hy;
-    }
-  }
-  if (S[c + K.nx2 + pl * 20] < 0) {
-#pragma unroll 1
-    for (int g = 0; g < NG; ++g) {
-      trace8(K, S, c, c_basis.phiGU[g], A);
-      trace8(K, S, c + K.nx2, c_basis.phiGD[g], B);
-#pragma unroll
-      for (int n = 0; n < NE; ++n) I[n] = I[n] + K.hx1 * c_basis.w[g] * (A[n] - B[n]);
-      Lij = Lij + K.hx;
-    }
-  }
-  if (S[c - K.nx2 + pl * 20] > 0) {
-#pragma unroll 1
-    for (int g = 0; g < NG; ++g) {
-      trace8(K, S, c, c_basis.phiGD[g], A);
-      trace8(K, S, c - K.nx2, c_basis.phiGU[g], B);
-#pragma unroll
-      for (int n = 0; n < NE; ++n) I[n] = I[n] + K.hx1 * c_basis.w[g] * (A[n] - B[n]);
-      Lij = Lij + K.hx;
-    }
-  }
-  // with every integral zero each ratio is exactly 0 (the denominator is
-  // positive), so the flag is decided without the point maxima
-  bool all_zero = true;
-#pragma unroll
-  for (int n = 0; n < NE; ++n) all_zero = all_zero && (I[n] == 0.0);
-  if (all_zero) return prev || (0.0 >= K.ck);
-  double uinf[NE];
-#pragma unroll
-  for (int n = 0; n < NE; ++n) uinf[n] = 0.0;
-#pragma unroll 1
-  for (int a = 0; a < NG; ++a)
-#pragma unroll 1
-    for (int b = 0; b < NG; ++b)
-#pragma unroll
-      for (int n = 0; n < NE; ++n) {
-        double v = 0.0;
-#pragma unroll
-        for (int d = 0; d < NP; ++d)
-          if (live_mode(n, d)) v = v + m[n][d] * c_basis.phiG[a][b][d];
-        if (fabs(v) + 1e-12 > uinf[n]) uinf[n] = fabs(v) + 1e-12;
-      }
-  bool flag = prev;
-#pragma unroll
   for (int n = 0; n < NE; ++n) {
-    const double r = dv(fabs(I[n]), K.pow_hxhy * Lij * uinf[n]);
-    if (r >= K.ck) flag = true;
+    const int cubic = n == 5 ? 1 : n == 6 ? 2 : 0;
+    const double* Sn = S + c + pl * (10 * n);
+    const long long x0 = pl * (cubic == 2 ? 7 : 6), x1 = pl * (cubic == 2 ? 9 : 8);
+    auto load = [&](const double* q, double* m) {
+#pragma unroll
+      for (int d = 0; d < 6; ++d) m[d] = q[pl * d];
+      m[6] = cubic ? q[x0] : 0.0;
+      m[7] = cubic ? q[x1] : 0.0;
+    };
+    double m[8], k[8], I = 0.0;
+    load(Sn, m);
+    if (r) { load(Sn + 1, k); kxrcf_face<0>(m, k, false, cubic, K.hy1, I); }
+    if (l) { load(Sn - 1, k); kxrcf_face<0>(m, k, true, cubic, K.hy1, I); }
+    if (u) { load(Sn + K.nx2, k); kxrcf_face<1>(m, k, false, cubic, K.hx1, I); }
+    if (w) { load(Sn - K.nx2, k); kxrcf_face<1>(m, k, true, cubic, K.hx1, I); }
+    // a zero integral gives the ratio 0 (the denominator is positive)
+    if (I == 0.0) {
+      if (0.0 >= K.ck) return true;
+      continue;
+    }
+    double up = fabs(m[0]), ms = m[0] * m[0];
+#pragma unroll
+    for (int d = 1; d < 6; ++d) {
+      up = up + fabs(m[d]) * c_basis.ppM[d];
+      ms = ms + m[d] * m[d] * c_basis.mm[d];
+    }
+    const int d6 = cubic == 2 ? 7 : 6, d7 = cubic == 2 ? 9 : 8;
+    if (cubic) {
+      up = up + fabs(m[6]) * c_basis.ppM[d6] + fabs(m[7]) * c_basis.ppM[d7];
+      ms = ms + m[6] * m[6] * c_basis.mm[d6] + m[7] * m[7] * c_basis.mm[d7];
+    }
+    const double a = fabs(I);
+    if (a > cd * (up + 1e-12) * (1.0 + 1e-9)) return true;
+    if (cd > 0.0 && (a < cd * 1e-12 * (1.0 - 1e-9) || a * a < cd * cd * ms * (1.0 - 1e-8))) continue;
+    double uinf = 0.0;
+#pragma unroll 1
+    for (int q = 0; q < NG * NG; ++q) {
+      const double* f = &c_basis.phiG[0][0][0] + NP * q;
+      double v = 0.0;
+#pragma unroll
+      for (int d = 0; d < 6; ++d) v = v + m[d] * f[d];
+      if (cubic) {
+        v = v + m[6] * f[d6];
+        v = v + m[7] * f[d7];
+      }
+      if (fabs(v) + 1e-12 > uinf) uinf = fabs(v) + 1e-12;
+    }
+    if (dv(a, pL * uinf) >= K.ck) return true;
   }
-  return flag;
+  return false;
 }
 
 __device__ __forceinline__ void divfree_item(const Consts& K, double* __restrict__ D, const double* __restrict__ BX,
@@ -828,12 +848,15 @@ static __device__ double pp_point(const Consts& K, const double* ubar, const dou
 // Bound on |u_q - u_bar| over the 50 GLL-mixed points for variable n:
 // sum_d |m_d| max_q |phi_d(q)|, inflated to cover the rounding of the point
 // sums (relative error < 2.3e-15 of |u_bar| + the bound).
+__device__ __forceinline__ double pp_spread_of(double b, double mean) {
+  return b * (1.0 + 1e-12) + 1e-12 * fabs(mean);
+}
 __device__ __forceinline__ double pp_spread(const Consts& K, const double (*m)[NP], int n) {
   double b = 0.0;
 #pragma unroll
   for (int d = 1; d < NP; ++d)
     if (live_mode(n, d)) b = b + fabs(m[n][d]) * c_basis.ppM[d];
-  return b * (1.0 + 1e-12) + 1e-12 * fabs(m[n][0]);
+  return pp_spread_of(b, m[n][0]);
 }
 
 // Whether pp_Limiter.f90 leaves a cell alone: the density part acts only if
@@ -841,24 +864,32 @@ __device__ __forceinline__ double pp_spread(const Consts& K, const double (*m)[N
 // if some point has a negative pressure. Where the bounds of pp_spread rule
 // both out (with margins far above rounding) the point evaluations would
 // change nothing.
-__device__ __forceinline__ bool pp_rho_safe(const Consts& K, const double (*m)[NP]) {
-  return pp_spread(K, m, 0) < (m[0][0] - 1e-13) * (1.0 - 1e-12);
+__device__ __forceinline__ bool pp_rho_safe(double mean, double spread) {
+  return spread < (mean - 1e-13) * (1.0 - 1e-12);
 }
-// a lower bound of the pressure at every point, from bounds on the point
-// values; positive beyond rounding: no point has pq < 0
-__device__ __forceinline__ bool pp_pressure_safe(const Consts& K, const double (*m)[NP]) {
-  double dv[NE];
-#pragma unroll
-  for (int n = 0; n < NE; ++n) dv[n] = pp_spread(K, m, n);
-  const double rho_lo = m[0][0] - dv[0];
+// a lower bound of the pressure at every point, from the variables' means and
+// spreads; positive beyond rounding: no point has pq < 0
+__device__ __forceinline__ bool pp_pressure_safe(const double* mean, const double* spread) {
+  const double rho_lo = mean[0] - spread[0];
   if (!(rho_lo > 0.0)) return false;
-  const double e_lo = m[4][0] - dv[4];
-  const double k_hi = 0.5 * (sq(fabs(m[1][0]) + dv[1]) + sq(fabs(m[2][0]) + dv[2]) + sq(fabs(m[3][0]) + dv[3])) /
-                      rho_lo * (1.0 + 1e-12);
-  const double b_hi = 0.5 * (sq(fabs(m[5][0]) + dv[5]) + sq(fabs(m[6][0]) + dv[6]) + sq(fabs(m[7][0]) + dv[7])) *
-                      (1.0 + 1e-12);
+  const double e_lo = mean[4] - spread[4];
+  auto top = [&](int n) { return sq(fabs(mean[n]) + spread[n]); };
+  const double k_hi = 0.5 * (top(1) + top(2) + top(3)) / rho_lo * (1.0 + 1e-12);
+  const double b_hi = 0.5 * (top(5) + top(6) + top(7)) * (1.0 + 1e-12);
   const double p_lo = e_lo - k_hi - b_hi;
   return p_lo > 1e-10 * (fabs(e_lo) + k_hi + b_hi);
+}
+__device__ __forceinline__ bool pp_pressure_safe(const Consts& K, const double (*m)[NP]) {
+  double mean[NE], spread[NE];
+#pragma unroll
+  for (int n = 0; n < NE; ++n) {
+    mean[n] = m[n][0];
+    spread[n] = pp_spread(K, m, n);
+  }
+  return pp_pressure_safe(mean, spread);
+}
+__device__ __forceinline__ bool pp_quiet(const Consts& K, const double (*m)[NP]) {
+  return pp_rho_safe(m[0][0], pp_spread(K, m, 0)) && pp_pressure_safe(K, m);
 }
 
 // pp_Limiter.f90:10-81 for one cell's modes (in place), by one thread: the
@@ -868,7 +899,7 @@ static __device__ void pp_cell(const Consts& K, double (*m)[NP]) {
   const double epsilon = 1e-13;
   double eta = 1.0;
   const double rb = m[0][0];
-  if (!pp_rho_safe(K, m)) {
+  if (!pp_rho_safe(rb, pp_spread(K, m, 0))) {
 #pragma unroll 1
     for (int a = 0; a < NG; ++a)
 #pragma unroll 1
@@ -949,12 +980,11 @@ __device__ __forceinline__ void pp_item_warp(const Consts& K, double* __restrict
   __syncwarp();
   const double epsilon = 1e-13, rb = sm[0];
   bool changed = false;
-  double spread = 0.0;   // pp_spread of the density
+  double spread = 0.0;
 #pragma unroll
   for (int d = 1; d < NP; ++d)
     if (live_mode(0, d)) spread = spread + fabs(sm[LI(0, d)]) * c_basis.ppM[d];
-  spread = spread * (1.0 + 1e-12) + 1e-12 * fabs(rb);
-  if (!(spread < (rb - epsilon) * (1.0 - 1e-12))) {
+  if (!pp_rho_safe(rb, pp_spread_of(spread, rb))) {
     double eta = 1.0;
 #pragma unroll 1
     for (int r = 1; r >= 0; --r) {
@@ -1039,17 +1069,16 @@ __device__ __forceinline__ void lim_load(const Consts& K, const double* __restri
 // and 3: the network sees the step's stage-1 pre-limit state).
 constexpr int LIM_PLAIN = 0, LIM_INFER = 1, LIM_PNET = 2;
 // Limiter of one interior cell in three pieces, composed by limit_item:
-//   lim_gate    loads the pre-limit modes and decides the gate (detector,
-//               sticky KXRCF flag, learned probability); LIM_INFER runs the
-//               network for the block first (block-cooperative)
+//   lim_gate    decides the gate (detector, sticky KXRCF flag, learned
+//               probability); LIM_INFER runs the network for the block first
+//               (block-cooperative)
 //   lim_tvb     characteristic TVB limiting of a gated cell
 //   lim_finish  positivity limiter, div-free reconstruction, store, flags
 template <int LM>
 __device__ __forceinline__ bool lim_gate(const Consts& K, const double* __restrict__ S, int32_t* __restrict__ trouble,
                                          const MlpDev* __restrict__ net, const float* __restrict__ QM,
                                          float* __restrict__ pnet, float t_lo, float t_hi, long long item,
-                                         unsigned char* lsm, bool valid, long long c, double (*m)[NP],
-                                         int32_t& word) {
+                                         unsigned char* lsm, bool valid, long long c, int32_t& word) {
   float p_net = 0.f;
   if (LM == LIM_INFER) {
     // the learned indicator for the block's 64 cells on the tensor cores
@@ -1100,19 +1129,17 @@ __device__ __forceinline__ bool lim_gate(const Consts& K, const double* __restri
     if (valid) p_net = pnet[item];
   }
   if (!valid) return false;
-  lim_load(K, S, c, m);
   word = 0;
   bool gate = true;
   if (K.detector == GDF_DETECT_KXRCF) {
-    const bool prev = K.sticky ? (trouble[item] != 0) : false;
     // a set sticky flag stays set whatever the detector finds
-    gate = prev ? true : kxrcf_flag(K, S, c, m, prev);
+    gate = (K.sticky && trouble[item] != 0) || kxrcf_flag(K, S, c);
     trouble[item] = gate ? 1 : 0;
     if (gate) word |= (1 << 24);
   } else if (LM != LIM_PLAIN) {
     // confident network answers decide; KXRCF decides in the uncertain band
     if (p_net >= t_hi) gate = true;
-    else if (p_net >= t_lo) gate = kxrcf_flag(K, S, c, m, false);
+    else if (p_net >= t_lo) gate = kxrcf_flag(K, S, c);
     else gate = false;
     if (gate) word |= (1 << 24);
   }
@@ -1352,6 +1379,18 @@ __device__ __forceinline__ void lim_tvb(const Consts& K, const double* __restric
   word |= (int32_t)change;
 }
 
+// the cell's flag word (its byte of this stage and gate bit) and the health of
+// its means
+__device__ __forceinline__ void lim_flags(int32_t* __restrict__ flags, int stage, Scal* __restrict__ sc, long long item,
+                                          int32_t word, double rho, double E) {
+  if (flags) {
+    int32_t w = (word & 0xff) << (8 * (stage - 1));
+    if (word & (1 << 24)) w |= (1 << (23 + stage));
+    if (stage <= 1) flags[item] = w; else flags[item] |= w;
+  }
+  if (!(rho > 0.0) || !isfinite(E)) atomicOr(&sc->status, 1);
+}
+
 // Cells left to a later pass: list entries are tag + item.
 template <class T>
 struct LimList {
@@ -1388,7 +1427,7 @@ __device__ __forceinline__ void lim_finish(const Consts& K, double* __restrict__
   const long long pl = K.plane;
   if (K.pp) {
     if (PPD) {
-      if (lim_defer(!(pp_rho_safe(K, m) && pp_pressure_safe(K, m)), item, pp)) divfree = 0;
+      if (lim_defer(!pp_quiet(K, m), item, pp)) divfree = 0;
     } else {
       pp_cell(K, m);
     }
@@ -1428,41 +1467,69 @@ __device__ __forceinline__ void lim_finish(const Consts& K, double* __restrict__
 #pragma unroll
     for (int d = 0; d < NP; ++d)
       if (live_mode(n, d)) D[c + pl * (d + 10 * n)] = m[n][d];
-  if (flags) {
-    int32_t w = (word & 0xff) << (8 * (stage - 1));
-    if (word & (1 << 24)) w |= (1 << (23 + stage));
-    if (stage <= 1) flags[item] = w; else flags[item] |= w;
-  }
-  if (!(m[0][0] > 0.0) || !isfinite(m[4][0])) atomicOr(&sc->status, 1);
+  lim_flags(flags, stage, sc, item, word, m[0][0], m[4][0]);
 }
 
-// One interior cell of the limiter. COMPACT: a gated cell is only appended
-// to list (limit_tvb_item finishes it in a second pass over full warps, so
-// the characteristic limiter never runs beside idle lanes); an ungated one
-// is finished here.
-template <int LM, bool COMPACT, class T = int32_t>
+// One interior cell of the limiter in one pass (the ensemble's persistent stage
+// kernel).
+template <int LM>
 __device__ __forceinline__ void limit_item(const Consts& K, const double* __restrict__ S, double* __restrict__ D,
                                            const double* __restrict__ BX, const double* __restrict__ BY,
                                            int32_t* __restrict__ flags, int32_t* __restrict__ trouble, int stage,
                                            int divfree, Scal* __restrict__ sc, const MlpDev* __restrict__ net,
                                            const float* __restrict__ QM, float* __restrict__ pnet,
-                                           float t_lo, float t_hi, long long item, unsigned char* lsm,
-                                           const LimList<T>& defer = LimList<T>{},
-                                           const LimList<long long>& pp = LimList<long long>{}) {
+                                           float t_lo, float t_hi, long long item, unsigned char* lsm) {
   const bool valid = item < (long long)K.nx * K.ny;
   const int i = valid ? (int)(item % K.nx) + 1 : 1;
   const int j = valid ? (int)(item / K.nx) + 1 : 1;
   const long long c = i + (long long)K.nx2 * j;
   double m[NE][NP];
   int32_t word = 0;
-  const bool gate = lim_gate<LM>(K, S, trouble, net, QM, pnet, t_lo, t_hi, item, lsm, valid, c, m, word);
+  const bool gate = lim_gate<LM>(K, S, trouble, net, QM, pnet, t_lo, t_hi, item, lsm, valid, c, word);
   if (!valid) return;
-  if (COMPACT) {
-    if (lim_defer(gate, item, defer)) return;
-  } else if (gate) {
-    lim_tvb(K, S, c, m, word);
+  lim_load(K, S, c, m);
+  if (gate) lim_tvb(K, S, c, m, word);
+  lim_finish<false>(K, D, BX, BY, flags, stage, divfree, sc, item, i, j, c, m, word, LimList<long long>{});
+}
+
+// The gating pass: a gated cell is only listed in defer (limit_tvb_item
+// finishes it over full warps, so the characteristic limiter never runs beside
+// idle lanes); an ungated one is finished here, a variable at a time: its modes
+// copied to D, the bounds of the positivity limiter gathered on the way, the
+// cell left to pp where they do not rule it out.
+template <int LM, class T>
+__device__ __forceinline__ void limit_gate_item(const Consts& K, const double* __restrict__ S, double* __restrict__ D,
+                                                const double* __restrict__ BX, const double* __restrict__ BY,
+                                                int32_t* __restrict__ flags, int32_t* __restrict__ trouble, int stage,
+                                                int divfree, Scal* __restrict__ sc, const MlpDev* __restrict__ net,
+                                                const float* __restrict__ QM, float* __restrict__ pnet, float t_lo,
+                                                float t_hi, long long item, unsigned char* lsm,
+                                                const LimList<T>& defer, const LimList<long long>& pp) {
+  const bool valid = item < (long long)K.nx * K.ny;
+  const int i = valid ? (int)(item % K.nx) + 1 : 1;
+  const int j = valid ? (int)(item / K.nx) + 1 : 1;
+  const long long c = i + (long long)K.nx2 * j, pl = K.plane;
+  int32_t word = 0;
+  const bool gate = lim_gate<LM>(K, S, trouble, net, QM, pnet, t_lo, t_hi, item, lsm, valid, c, word);
+  if (!valid) return;
+  if (lim_defer(gate, item, defer)) return;
+  double mean[NE], spread[NE];
+#pragma unroll
+  for (int n = 0; n < NE; ++n) {
+    double b = 0.0;
+#pragma unroll
+    for (int d = 0; d < NP; ++d) {
+      if (!live_mode(n, d)) continue;
+      const double v = S[c + pl * (d + 10 * n)];
+      D[c + pl * (d + 10 * n)] = v;
+      if (d == 0) mean[n] = v;
+      else b = b + fabs(v) * c_basis.ppM[d];
+    }
+    spread[n] = pp_spread_of(b, mean[n]);
   }
-  lim_finish<COMPACT>(K, D, BX, BY, flags, stage, divfree, sc, item, i, j, c, m, word, pp);
+  if (K.pp && lim_defer(!(pp_rho_safe(mean[0], spread[0]) && pp_pressure_safe(mean, spread)), item, pp)) divfree = 0;
+  if (divfree) divfree_item(K, D, BX, BY, item);
+  lim_flags(flags, stage, sc, item, word, mean[0], mean[4]);
 }
 
 // A cell every thread of the limiting pass limits: one limit_item<LM, true>

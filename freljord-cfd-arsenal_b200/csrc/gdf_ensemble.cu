@@ -120,7 +120,7 @@ __device__ __noinline__ void call_limit(const Consts& K, const double* S, double
                                         int32_t* flags, int32_t* trouble, int stage, int divfree, Scal* sc,
                                         const MlpDev* net, const float* QM, float* pnet, float t_lo, float t_hi,
                                         long long item) {
-  limit_item<LM, false>(K, S, D, BX, BY, flags, trouble, stage, divfree, sc, net, QM, pnet, t_lo, t_hi, item, ens_sm);
+  limit_item<LM>(K, S, D, BX, BY, flags, trouble, stage, divfree, sc, net, QM, pnet, t_lo, t_hi, item, ens_sm);
 }
 __device__ __noinline__ void call_dt(const Consts& K, const double* U, long long item, double& ax, double& ay,
                                      Scal* sc) {
@@ -478,10 +478,10 @@ template <int LM>
 __global__ void __launch_bounds__(ENS_BS) k_ep_limit(const __grid_constant__ EnsArgs A, int stage) {
   extern __shared__ __align__(16) unsigned char lsm[];
   for_tiles<true>(A, EK_LIM, [&](int i, const EnsInst& I, const Consts& K, long long base, int) {
-    limit_item<LM, true>(K, I.UI, I.U, I.BX, I.BY, I.flags, I.trouble, stage, K.faceb ? 0 : 1, I.sc, A.net, I.QM,
-                         I.pnet, A.t_lo, A.t_hi, base + threadIdx.x, lsm,
-                         LimList<long long>{A.lim_list, A.lim_count, (long long)i << 40},
-                         LimList<long long>{A.pp_list, A.lim_count + 1, (long long)i << 40});
+    limit_gate_item<LM>(K, I.UI, I.U, I.BX, I.BY, I.flags, I.trouble, stage, K.faceb ? 0 : 1, I.sc, A.net, I.QM,
+                        I.pnet, A.t_lo, A.t_hi, base + threadIdx.x, lsm,
+                        LimList<long long>{A.lim_list, A.lim_count, (long long)i << 40},
+                        LimList<long long>{A.pp_list, A.lim_count + 1, (long long)i << 40});
     if (LM == LIM_INFER) __syncthreads();
   });
 }

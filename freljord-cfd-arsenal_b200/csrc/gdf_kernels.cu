@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(LIM_BS) k_infer(const __grid_constant__ Consts
 // listed for k_limit_tvb (full warps, and none of the characteristic
 // limiter's registers here).
 template <int LM>
-__global__ void __launch_bounds__(LIM_BS, GDF_LIMIT_MINB) k_limit(const __grid_constant__ Consts K, const double* __restrict__ S,
+__global__ void __launch_bounds__(LIM_BS, 8) k_limit(const __grid_constant__ Consts K, const double* __restrict__ S,
                                                   double* __restrict__ D, const double* __restrict__ BX,
                                                   const double* __restrict__ BY, int32_t* __restrict__ flags,
                                                   int32_t* __restrict__ trouble, int stage, int divfree,
@@ -255,8 +255,8 @@ __global__ void __launch_bounds__(LIM_BS, GDF_LIMIT_MINB) k_limit(const __grid_c
                                                   int32_t* __restrict__ list, int32_t* __restrict__ count,
                                                   LimList<long long> pp) {
   if (gate_sc && !gate_sc->active) return;
-  limit_item<LM, true>(K, S, D, BX, BY, flags, trouble, stage, divfree, sc, nullptr, nullptr, pnet, t_lo, t_hi, gtid(),
-                       nullptr, LimList<int32_t>{list, count, 0}, pp);
+  limit_gate_item<LM>(K, S, D, BX, BY, flags, trouble, stage, divfree, sc, nullptr, nullptr, pnet, t_lo, t_hi, gtid(),
+                      nullptr, LimList<int32_t>{list, count, 0}, pp);
 }
 
 // The limiting pass, one cell per thread: the cells k_limit<LM, true> deferred

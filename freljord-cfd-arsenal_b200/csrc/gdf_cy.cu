@@ -38,7 +38,7 @@
 #include <vector>
 
 #include "../../include/gdf_cy.h"
-#include "gdf_physics.cuh"
+#include "gdf_charlim.cuh"
 
 namespace gdf {
 int set_last_error(int code, const char* msg);
@@ -722,7 +722,12 @@ __device__ __forceinline__ void mv8(const double* A, const double* x, double* y)
   }
 }
 
-// characteristic limiting in one direction (TVB_Limiter_P2.f90:57-125):
+// the P2 mode d of variable n with r*B replaced by B (the projection)
+__device__ __forceinline__ double modeB(const KC& K, const double* U, const double* BP, long long c, int n, int d) {
+  return (n == 5 || n == 6) ? ld(BP + c + K.ncp * (NQC * (n - 5) + d)) : ld(U + c + K.ncp * (NQC * n + d));
+}
+
+// one direction through the full matrices (cells char_limit_sparse refuses):
 // L of the differences, minmod, R; the left vectors are built and used
 // before the right ones (the same values, one matrix live at a time)
 __device__ __forceinline__ void char_dir(const Phys& P, int dir, const double* m, const double* DR, const double* DL,
@@ -750,11 +755,78 @@ __device__ __forceinline__ void char_dir(const Phys& P, int dir, const double* m
   mv8(R, mod, Ym);
 }
 
-// the P2 mode d of variable n with r*B replaced by B (the projection)
-__device__ __forceinline__ double modeB(const KC& K, const double* U, const double* BP, long long c, int n, int d) {
-  return (n == 5 || n == 6) ? ld(BP + c + K.ncp * (NQC * (n - 5) + d)) : ld(U + c + K.ncp * (NQC * n + d));
+// Operands of one direction for the cell plane at c: mean differences to the
+// neighbours and the two face slopes (TVB_Limiter_P2.f90:57-66, 91-100)
+__device__ __forceinline__ void cy_operands(const KC& K, const double* U, const double* BP, long long c, int dir,
+                                            double* DR, double* DL, double* Dp, double* Dm) {
+  const double c23 = 2.0 / 3.0;
+  const long long st = dir ? K.nx2 : 1;
+#pragma unroll
+  for (int n = 0; n < NE; ++n) {
+    const double m0 = modeB(K, U, BP, c, n, 0);
+    DR[n] = modeB(K, U, BP, c + st, n, 0) - m0;
+    DL[n] = m0 - modeB(K, U, BP, c - st, n, 0);
+    const double m1 = modeB(K, U, BP, c, n, 1 + dir), m2 = modeB(K, U, BP, c, n, 3 + 2 * dir);
+    Dp[n] = m1 + c23 * m2;
+    Dm[n] = m1 - c23 * m2;
+  }
+}
+// what one direction changes, and the modes it gives: res[n] the slope,
+// res[8 + n] the quadratic mode
+__device__ __forceinline__ int cy_change(const KC& K, const double* Dp, const double* Dm, const double* Yp,
+                                         const double* Ym, double* res) {
+  int change = 0;
+#pragma unroll
+  for (int n = 0; n < NE; ++n) {
+    if (fabs(Yp[n] - Dp[n]) > K.change_tol || fabs(Ym[n] - Dm[n]) > K.change_tol) change |= 1 << n;
+    res[n] = 0.5 * (Yp[n] + Ym[n]);
+    res[NE + n] = (3.0 / 4.0) * (Yp[n] - Ym[n]);
+  }
+  return change;
+}
+// both directions through one copy of char_limit_sparse; false where it refuses
+template <class DIV>
+__device__ __forceinline__ bool cy_sparse(const KC& K, const double* U, const double* BP, long long c, double* res,
+                                          int& change) {
+  unsigned bad = 0;
+  change = 0;
+  double m[NE];
+#pragma unroll
+  for (int n = 0; n < NE; ++n) m[n] = modeB(K, U, BP, c, n, 0);
+  const auto rr = DIV::by(m[0], bad);
+  const double u1 = DIV::div(m[1], rr, bad), u2 = DIV::div(m[2], rr, bad), u3 = DIV::div(m[3], rr, bad);
+#pragma unroll 1
+  for (int dir = 0; dir < 2; ++dir) {
+    double DR[NE], DL[NE], Dp[NE], Dm[NE], Yp[NE], Ym[NE];
+    cy_operands(K, U, BP, c, dir, DR, DL, Dp, Dm);
+    const gdf::Minmod mm{dir ? K.Mh2z : K.Mh2r};
+    bad |= (unsigned)!gdf::char_limit_sparse<DIV>(K.P, dir, m[0], u1, u2, u3, m[4], m[5], m[6], m[7], rr, DR, DL, Dp,
+                                                  Dm, mm, Yp, Ym);
+    change |= cy_change(K, Dp, Dm, Yp, Ym, res + 2 * NE * dir);
+  }
+  return !bad;
+}
+static __device__ __noinline__ int cy_refused(const KC& K, const double* U, const double* BP, long long c,
+                                              double* res) {
+  int change;
+  if (cy_sparse<gdf::IeeeDiv>(K, U, BP, c, res, change)) return change;
+  double m[NE];
+#pragma unroll
+  for (int n = 0; n < NE; ++n) m[n] = modeB(K, U, BP, c, n, 0);
+  change = 0;
+#pragma unroll 1
+  for (int dir = 0; dir < 2; ++dir) {
+    double DR[NE], DL[NE], Dp[NE], Dm[NE], Yp[NE], Ym[NE];
+    cy_operands(K, U, BP, c, dir, DR, DL, Dp, Dm);
+    if (dir == 0) char_dir(K.P, 0, m, DR, DL, Dp, Dm, K.Mh2r, Yp, Ym);
+    else char_dir(K.P, 1, m, DR, DL, Dp, Dm, K.Mh2z, Yp, Ym);
+    change |= cy_change(K, Dp, Dm, Yp, Ym, res + 2 * NE * dir);
+  }
+  return change;
 }
 
+// In place: it writes modes 2-6 (and the cubic slots of a changed r*B) of its
+// own cell plane, the neighbours read mode 1.
 __global__ void __launch_bounds__(64) k_cy_tvb(const __grid_constant__ KC K, double* __restrict__ U,
                                                const double* __restrict__ BP, int32_t* __restrict__ flags,
                                                const ScalC* __restrict__ sc) {
@@ -765,52 +837,17 @@ __global__ void __launch_bounds__(64) k_cy_tvb(const __grid_constant__ KC K, dou
   const long long r = q / K.nx;
   const int j = (int)(r % K.ny) + 1, kk = (int)(r / K.ny);
   const long long c = cp_of(K, i, j, kk);
-  const long long cE = cp_of(K, i + 1, j, kk), cW = cp_of(K, i - 1, j, kk);
-  const long long cN = cp_of(K, i, j + 1, kk), cS = cp_of(K, i, j - 1, kk);
-  double m[NE];
-#pragma unroll
-  for (int n = 0; n < NE; ++n) m[n] = modeB(K, U, BP, c, n, 0);
-  const double c23 = 2.0 / 3.0;
-  int change = 0;
-  double Xp[NE], Xm[NE], Yp[NE], Ym[NE];
-  {
-    double DR[NE], DL[NE], Dp[NE], Dm[NE];
-#pragma unroll
-    for (int n = 0; n < NE; ++n) {
-      DR[n] = modeB(K, U, BP, cE, n, 0) - m[n];
-      DL[n] = m[n] - modeB(K, U, BP, cW, n, 0);
-      const double m2 = modeB(K, U, BP, c, n, 1), m4 = modeB(K, U, BP, c, n, 3);
-      Dp[n] = m2 + c23 * m4;
-      Dm[n] = m2 - c23 * m4;
-    }
-    char_dir(K.P, 0, m, DR, DL, Dp, Dm, K.Mh2r, Xp, Xm);
-#pragma unroll
-    for (int n = 0; n < NE; ++n)
-      if (fabs(Xp[n] - Dp[n]) > K.change_tol || fabs(Xm[n] - Dm[n]) > K.change_tol) change |= 1 << n;
-  }
-  {
-    double DR[NE], DL[NE], Dp[NE], Dm[NE];
-#pragma unroll
-    for (int n = 0; n < NE; ++n) {
-      DR[n] = modeB(K, U, BP, cN, n, 0) - m[n];
-      DL[n] = m[n] - modeB(K, U, BP, cS, n, 0);
-      const double m3 = modeB(K, U, BP, c, n, 2), m6 = modeB(K, U, BP, c, n, 5);
-      Dp[n] = m3 + c23 * m6;
-      Dm[n] = m3 - c23 * m6;
-    }
-    char_dir(K.P, 1, m, DR, DL, Dp, Dm, K.Mh2z, Yp, Ym);
-#pragma unroll
-    for (int n = 0; n < NE; ++n)
-      if (fabs(Yp[n] - Dp[n]) > K.change_tol || fabs(Ym[n] - Dm[n]) > K.change_tol) change |= 1 << n;
-  }
+  double res[4 * NE];
+  int change;
+  if (!cy_sparse<gdf::SharedRcp>(K, U, BP, c, res, change)) change = cy_refused(K, U, BP, c, res);
 #pragma unroll
   for (int n = 0; n < NE; ++n)
     if (change & (1 << n)) {
-      U[c + K.ncp * (NQC * n + 1)] = 0.5 * (Xp[n] + Xm[n]);
-      U[c + K.ncp * (NQC * n + 2)] = 0.5 * (Yp[n] + Ym[n]);
-      U[c + K.ncp * (NQC * n + 3)] = (3.0 / 4.0) * (Xp[n] - Xm[n]);
+      U[c + K.ncp * (NQC * n + 1)] = res[n];
+      U[c + K.ncp * (NQC * n + 2)] = res[2 * NE + n];
+      U[c + K.ncp * (NQC * n + 3)] = res[NE + n];
       U[c + K.ncp * (NQC * n + 4)] = 0.0;
-      U[c + K.ncp * (NQC * n + 5)] = (3.0 / 4.0) * (Yp[n] - Ym[n]);
+      U[c + K.ncp * (NQC * n + 5)] = res[3 * NE + n];
       if (n == 5)
         for (int s = 48; s < 51; ++s) U[c + K.ncp * s] = 0.0;
       if (n == 6)
@@ -1219,6 +1256,7 @@ void build_kc(const GdfCyConfig& c, KC& K) {
   K.P.kml_w = 1;
   K.P.eig_p_typo = 0;
   K.P.eig_identity = 0;    // eigenmatrix.f90:396-402 commented out
+  gdf::set_eig_consts(K.P);
   // get_basis.f90:191-196 (host sin/cos, as the reference's)
   const double pi = 4 * std::atan(1.0), hphi = 2 * pi / K.nph;
   for (int kk = 0; kk < K.nph; ++kk) K.phi[kk] = kk * hphi;

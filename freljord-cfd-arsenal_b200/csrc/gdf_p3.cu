@@ -32,7 +32,7 @@
 
 #include "../../include/gdf_p3.h"
 #include "gdf_p3_basis.h"
-#include "gdf_physics.cuh"
+#include "gdf_charlim.cuh"
 
 namespace gdf {
 int set_last_error(int code, const char* msg);
@@ -551,14 +551,67 @@ __global__ void __launch_bounds__(128) k3_faceb_limit(const __grid_constant__ K3
 }
 
 // ------------------------------------------------------------- limiter -----
-// One direction of TVB_Limiter's characteristic part: the face slopes X1
-// (mean to + face) and X2 (- face to mean) limited against the mean
-// differences DR, DL in the characteristic variables of the cell mean,
-// back in conserved variables as Y1, Y2. The left eigenvectors are built
-// and used in the four products with L (main.f90:3319-3321, 3337), then
-// the right ones for the two products with R: one 8x8 matrix live at a
-// time, the same products and sums as with both (this eigenmatrix has no
-// identity fallback that would tie R to L).
+// Operands of one direction of TVB_Limiter's characteristic part for cell c
+// (main.f90:3312-3320, 3347-3355): the mean differences DR, DL and the face
+// slopes X1 (mean to + face), X2 (- face to mean).
+__device__ __forceinline__ void tvb3_operands(const K3& K, const double* __restrict__ S, long long c, int dir,
+                                              double* DR, double* DL, double* X1, double* X2) {
+  const long long pl = K.plane, st = dir ? K.nx2 : 1;
+#pragma unroll
+  for (int n = 0; n < NE; ++n) {
+    const double* q = S + c + pl * slot3(n, 0);
+    const double m0 = q[0];
+    DR[n] = q[st] - m0;
+    DL[n] = m0 - q[-st];
+    // modes 2, 4, 7 (x) or 3, 6, 10 (y): the first ten slots of a variable are
+    // its first ten modes
+    const double a = q[pl * (dir ? 2 : 1)], b = q[pl * (dir ? 5 : 3)], d = q[pl * (dir ? 9 : 6)];
+    X1[n] = a + (2.0 / 3.0) * b + (2.0 / 5.0) * d;
+    X2[n] = a - (2.0 / 3.0) * b + (2.0 / 5.0) * d;
+  }
+}
+__device__ __forceinline__ unsigned tvb3_change(const K3& K, const double* X1, const double* X2, const double* Y1,
+                                                const double* Y2) {
+  unsigned change = 0;
+#pragma unroll
+  for (int n = 0; n < NE; ++n)
+    if (fabs(Y1[n] - X1[n]) > K.change_tol || fabs(Y2[n] - X2[n]) > K.change_tol) change |= 1u << n;
+  return change;
+}
+
+// The limited face slopes of cell c in both directions, Y = (Y1, Y2) of x, then
+// of y (8 each), and the changed variables, through one copy of
+// char_limit_sparse; false where it refuses.
+template <class DIV>
+__device__ __forceinline__ bool tvb3_sparse(const K3& K, const double* __restrict__ S, long long c, double* Y,
+                                            unsigned& change) {
+  unsigned bad = 0;
+  change = 0;
+  double m[NE];
+#pragma unroll
+  for (int n = 0; n < NE; ++n) m[n] = S[c + K.plane * slot3(n, 0)];
+  const auto rr = DIV::by(m[0], bad);
+  const double u1 = DIV::div(m[1], rr, bad), u2 = DIV::div(m[2], rr, bad), u3 = DIV::div(m[3], rr, bad);
+#pragma unroll 1
+  for (int dir = 0; dir < 2; ++dir) {
+    double DR[NE], DL[NE], X1[NE], X2[NE], Y1[NE], Y2[NE];
+    tvb3_operands(K, S, c, dir, DR, DL, X1, X2);
+    const gdf::MinmodBeta mm{dir ? K.Mh2y : K.Mh2x, K.beta};
+    bad |= (unsigned)!gdf::char_limit_sparse<DIV>(K.P, dir, m[0], u1, u2, u3, m[4], m[5], m[6], m[7], rr, DR, DL, X1,
+                                                  X2, mm, Y1, Y2);
+    change |= tvb3_change(K, X1, X2, Y1, Y2);
+    double* o = Y + 2 * NE * dir;
+#pragma unroll
+    for (int n = 0; n < NE; ++n) { o[n] = Y1[n]; o[NE + n] = Y2[n]; }
+  }
+  return !bad;
+}
+
+// One direction through the full matrices (cells char_limit_sparse refuses).
+// The left eigenvectors are built and used in the four products with L
+// (main.f90:3319-3321, 3337), then the right ones for the two products with R:
+// one 8x8 matrix live at a time, the same products and sums as with both (this
+// eigenmatrix has no identity fallback that would tie R to L).
 __device__ __forceinline__ void char_limit(const Phys& P, int dir, double rho, double u1, double u2, double u3,
                                            const double* m0, const double* DR, const double* DL, const double* X1,
                                            const double* X2, double Mh2, double beta, double* Y1, double* Y2) {
@@ -583,6 +636,30 @@ __device__ __forceinline__ void char_limit(const Phys& P, int dir, double rho, d
   mv8(R, mod1, Y1);
   mv8(R, mod2, Y2);
 }
+static __device__ __noinline__ unsigned tvb3_refused(const K3& K, const double* __restrict__ S, long long c,
+                                                     double* Y) {
+  unsigned change;
+  if (tvb3_sparse<gdf::IeeeDiv>(K, S, c, Y, change)) return change;
+  double m[NE];
+#pragma unroll
+  for (int n = 0; n < NE; ++n) m[n] = S[c + K.plane * slot3(n, 0)];
+  const double u1 = m[1] / m[0], u2 = m[2] / m[0], u3 = m[3] / m[0];
+  change = 0;
+#pragma unroll 1
+  for (int dir = 0; dir < 2; ++dir) {
+    double DR[NE], DL[NE], X1[NE], X2[NE], Y1[NE], Y2[NE];
+    tvb3_operands(K, S, c, dir, DR, DL, X1, X2);
+    if (dir == 0)
+      char_limit(K.P, 0, m[0], u1, u2, u3, m, DR, DL, X1, X2, K.Mh2x, K.beta, Y1, Y2);
+    else
+      char_limit(K.P, 1, m[0], u1, u2, u3, m, DR, DL, X1, X2, K.Mh2y, K.beta, Y1, Y2);
+    change |= tvb3_change(K, X1, X2, Y1, Y2);
+    double* o = Y + 2 * NE * dir;
+#pragma unroll
+    for (int n = 0; n < NE; ++n) { o[n] = Y1[n]; o[NE + n] = Y2[n]; }
+  }
+  return change;
+}
 
 // TVB_Limiter's cell part (main.f90:3295-3428) on the pre-limit state S
 // (ghosts set) for one interior cell, then div_free_Balsara for it from the
@@ -598,40 +675,13 @@ __global__ void __launch_bounds__(64) k3_limit(const __grid_constant__ K3 K, con
   const int i = (int)(item % K.nx) + 1, j = (int)(item / K.nx) + 1;
   const long long c = i + (long long)K.nx2 * j, pl = K.plane;
   auto at = [&](long long cc, int n, int d) { return S[cc + pl * slot3(n, d)]; };
+  double Y[4 * NE];
+  unsigned change;
+  if (!tvb3_sparse<gdf::SharedRcp>(K, S, c, Y, change)) change = tvb3_refused(K, S, c, Y);
+  const double *Rm = Y, *Lm = Y + NE, *Um = Y + 2 * NE, *Dm = Y + 3 * NE;
   double m0[NE];
 #pragma unroll
   for (int n = 0; n < NE; ++n) m0[n] = at(c, n, 0);
-  const double rhoij = m0[0];
-  const double u1 = m0[1] / rhoij, u2 = m0[2] / rhoij, u3 = m0[3] / rhoij;
-  double DR[NE], DL[NE], X1[NE], X2[NE];
-  double Rm[NE], Lm[NE], Um[NE], Dm[NE];
-  unsigned change = 0;
-  // x direction (main.f90:3312-3345)
-#pragma unroll
-  for (int n = 0; n < NE; ++n) {
-    DR[n] = at(c + 1, n, 0) - m0[n];
-    DL[n] = m0[n] - at(c - 1, n, 0);
-    const double a2 = at(c, n, 1), a4 = at(c, n, 3), a7 = at(c, n, 6);
-    X1[n] = a2 + (2.0 / 3.0) * a4 + (2.0 / 5.0) * a7;
-    X2[n] = a2 - (2.0 / 3.0) * a4 + (2.0 / 5.0) * a7;
-  }
-  char_limit(K.P, 0, rhoij, u1, u2, u3, m0, DR, DL, X1, X2, K.Mh2x, K.beta, Rm, Lm);
-#pragma unroll
-  for (int n = 0; n < NE; ++n)
-    if (fabs(Rm[n] - X1[n]) > K.change_tol || fabs(Lm[n] - X2[n]) > K.change_tol) change |= 1u << n;
-  // y direction (main.f90:3347-3380)
-#pragma unroll
-  for (int n = 0; n < NE; ++n) {
-    DR[n] = at(c + K.nx2, n, 0) - m0[n];
-    DL[n] = m0[n] - at(c - K.nx2, n, 0);
-    const double a3 = at(c, n, 2), a6 = at(c, n, 5), a10 = at(c, n, 9);
-    X1[n] = a3 + (2.0 / 3.0) * a6 + (2.0 / 5.0) * a10;
-    X2[n] = a3 - (2.0 / 3.0) * a6 + (2.0 / 5.0) * a10;
-  }
-  char_limit(K.P, 1, rhoij, u1, u2, u3, m0, DR, DL, X1, X2, K.Mh2y, K.beta, Um, Dm);
-#pragma unroll
-  for (int n = 0; n < NE; ++n)
-    if (fabs(Um[n] - X1[n]) > K.change_tol || fabs(Dm[n] - X2[n]) > K.change_tol) change |= 1u << n;
   // reconstruction (main.f90:3382-3425); the cell B's modes 2 and 3 only
   // feed omega of the divergence-free rebuild below
   unsigned p3 = 0;
@@ -947,6 +997,7 @@ void build_k3(const GdfP3Config& c, K3& K) {
   K.P.kml_w = 1;
   K.P.eig_p_typo = 0;
   K.P.eig_identity = 0;      // this eigenmatrix has no identity fallback
+  gdf::set_eig_consts(K.P);
   build_basis_p3(hx1, hy1, &K.B);
 }
 

@@ -74,6 +74,13 @@ GDF_HD double rdiv(double a, const Rcp& d, unsigned& bad) {
 #endif
 }
 
+// the same where the caller keeps no flag: an operand out of range divides
+// itself
+GDF_HD double rdiv_any(double a, const Rcp& d, unsigned bad = 0) {
+  const double q = rdiv(a, d, bad);
+  return bad ? a / d.b : q;
+}
+
 // How char_limit_sparse divides: by shared reciprocals, or with the IEEE
 // division itself for the cells in which an operand leaves rdiv's ranges
 // (a disturbance spreading into a quiet region passes through a ring of

@@ -49,6 +49,7 @@ namespace gdfc {
 using gdf::fmax2;
 using gdf::fmin2;
 using gdf::Phys;
+using gdf::Rcp;
 using gdf::sq;
 
 constexpr int NG = 5, NE = 8, NQC = 6, NPC = 10;
@@ -76,7 +77,7 @@ struct BasisC {
   double phiGLL[2][NG][NG][NPC];
   double phiGR[NG][NQC], phiGL[NG][NQC], phiGU[NG][NQC], phiGD[NG][NQC];
   double phiRU[NPC], phiLU[NPC], phiRD[NPC], phiLD[NPC];
-  double mm[NPC];
+  double mm[NPC], rmm[NPC];   // rmm: RN(1 / mm)
   double EzG[NG][3], EzxG[NG][3], EzyG[NG][3], mmE[3], EzR[3], EzL[3], EzU[3], EzD[3];
 };
 
@@ -165,16 +166,26 @@ __device__ __forceinline__ double fourier(const KC& K, double v, int kk, double 
 struct PrimC {
   double rho, u, v, w, E, B1, B2, B3, rB1, rB2, rB3, S, T, K;
 };
-__device__ __forceinline__ void prim_c(const Phys& P, const double* U, double rad, bool dquirk, PrimC& q) {
+__device__ __forceinline__ void prim_c(const Phys& P, const double* U, double rad, const Rcp& rrad, bool dquirk,
+                                       PrimC& q) {
   q.rho = U[0];
-  q.u = U[1] / q.rho;
-  q.v = U[2] / q.rho;
-  q.w = U[3] / q.rho;
   q.E = U[4];
   q.rB1 = U[5];
   q.rB2 = U[6];
-  q.B1 = q.rB1 / rad;
-  q.B2 = q.rB2 / rad;
+  unsigned bad = 0;
+  const Rcp rr = gdf::rcp_of(q.rho, bad);
+  q.u = gdf::rdiv(U[1], rr, bad);
+  q.v = gdf::rdiv(U[2], rr, bad);
+  q.w = gdf::rdiv(U[3], rr, bad);
+  q.B1 = gdf::rdiv(q.rB1, rrad, bad);
+  q.B2 = gdf::rdiv(q.rB2, rrad, bad);
+  if (bad) {   // an operand out of rdiv's range: the IEEE division itself
+    q.u = U[1] / q.rho;
+    q.v = U[2] / q.rho;
+    q.w = U[3] / q.rho;
+    q.B1 = q.rB1 / rad;
+    q.B2 = q.rB2 / rad;
+  }
   q.B3 = U[7];
   q.rB3 = q.B3 * rad;
   const double BB = sq(q.B1) + sq(q.B2) + sq(q.B3);
@@ -253,41 +264,41 @@ __device__ __forceinline__ double xghost(const KC& K, const double* __restrict__
   return (flip != odd) ? -v : v;
 }
 
+// One thread per slot and ghost cell plane: a slot's ghosts come from interior
+// cells only (corner ghosts compose the row source with the column rule), so
+// no thread waits for another. One thread per ghost cell plane, walking its 54
+// slots, took 30 us at 192^2 x 2 (a chain of dependent loads and stores per
+// thread, two blocks' worth of threads), nine times per step.
 __global__ void __launch_bounds__(128) k_cy_set_bc(const __grid_constant__ KC K, double* __restrict__ U,
                                                    const ScalC* __restrict__ sc) {
   if (sc && !sc->active) return;
-  const long long q = gtid();
   const long long nxg = 2LL * K.ny * K.nph, nyg = 2LL * K.nx2 * K.nph;
+  const long long t = gtid();
+  if (t >= (nxg + nyg) * NSC) return;
+  const int s = (int)(t / (nxg + nyg));
+  const long long q = t - s * (nxg + nyg);
   if (q < nxg) {
-    const int kk = (int)(q % K.nph);
-    const long long r = q / K.nph;
-    const int right = r < K.ny ? 1 : 0;
-    const int j = (int)(r % K.ny) + 1;
-    const int gi = right ? K.nx + 1 : 0;
-    double* dst = U + cp_of(K, gi, j, kk);
-    for (int s = 0; s < NSC; ++s) dst[K.ncp * s] = xghost(K, U, right, j, kk, s);
+    // rows fastest within a plane and side
+    const int j = (int)(q % K.ny) + 1;
+    const long long r = q / K.ny;
+    const int right = (int)(r & 1), kk = (int)(r >> 1);
+    U[cp_of(K, right ? K.nx + 1 : 0, j, kk) + K.ncp * s] = xghost(K, U, right, j, kk, s);
     return;
   }
-  if (q >= nxg + nyg) return;
   const long long q2 = q - nxg;
-  const int kk = (int)(q2 % K.nph);
-  const long long r = q2 / K.nph;
-  const int top = r < K.nx2 ? 1 : 0;
-  const int i = (int)(r % K.nx2);
+  const int i = (int)(q2 % K.nx2);
+  const long long r = q2 / K.nx2;
+  const int top = (int)(r & 1), kk = (int)(r >> 1);
   const int bc = top ? K.bc_u : K.bc_d;
   const int src = top ? (bc == 1 ? 1 : K.ny) : (bc == 1 ? K.ny : 1);
-  const int gj = top ? K.ny + 1 : 0;
-  double* dst = U + cp_of(K, i, gj, kk);
   const bool inlet = !top && bc == 4 && i >= 1 && i <= K.nx && K.ra + i * K.hr <= K.jet_r;
-  for (int s = 0; s < NSC; ++s) {
-    double v;
-    if (i >= 1 && i <= K.nx)
-      v = ld(U + cp_of(K, i, src, kk) + K.ncp * s);
-    else
-      v = xghost(K, U, i == K.nx + 1, src, kk, s);
-    if (inlet && !(s < 48 && s % NQC == 0)) v = 0.0;
-    dst[K.ncp * s] = v;
-  }
+  double v;
+  if (i >= 1 && i <= K.nx)
+    v = ld(U + cp_of(K, i, src, kk) + K.ncp * s);
+  else
+    v = xghost(K, U, i == K.nx + 1, src, kk, s);
+  if (inlet && !(s < 48 && s % NQC == 0)) v = 0.0;
+  U[cp_of(K, i, top ? K.ny + 1 : 0, kk) + K.ncp * s] = v;
 }
 
 // ------------------------------------------------------------- faces -------
@@ -331,8 +342,10 @@ __global__ void __launch_bounds__(128) k_cy_face(const __grid_constant__ KC K, c
     }
     const double re = DIR == 0 ? K.ra + i * K.hr : K.ra + (i - 0.5) * K.hr + K.hr1 * K.B.lam[g];
     PrimC pa, pb;
-    prim_c(K.P, UA, re, false, pa);
-    prim_c(K.P, UB, re, DIR == 1, pb);   // Lh.f90:284: the D side's pressure takes -w^2
+    unsigned far = 0;
+    const Rcp rre = gdf::rcp_of(re, far);
+    prim_c(K.P, UA, re, rre, false, pa);
+    prim_c(K.P, UB, re, rre, DIR == 1, pb);   // Lh.f90:284: the D side's pressure takes -w^2
     double FA[NE], FB[NE];
     if (DIR == 0) { flux_r(pa, UA, FA); flux_r(pb, UB, FB); }
     else { flux_z(pa, UA, FA); flux_z(pb, UB, FB); }
@@ -483,6 +496,8 @@ __global__ void __launch_bounds__(CY_CELL_BS) k_cy_cell(const __grid_constant__ 
 #pragma unroll 1
   for (int a = 0; a < NG; ++a) {
     const double rad = rc + K.hr1 * K.B.lam[a];
+    unsigned far = 0;
+    const Rcp rrad = gdf::rcp_of(rad, far);
 #pragma unroll 1
     for (int b = 0; b < NG; ++b) {
       const double* G = K.B.phiG[a][b];
@@ -500,7 +515,7 @@ __global__ void __launch_bounds__(CY_CELL_BS) k_cy_cell(const __grid_constant__ 
         Uv[n] = s;
       }
       PrimC pq;
-      prim_c(K.P, Uv, rad, false, pq);
+      prim_c(K.P, Uv, rad, rrad, false, pq);
       double Fx[NE], Fy[NE], Fz[NE];
       flux_r(pq, Uv, Fx);
       flux_z(pq, Uv, Fy);
@@ -517,24 +532,40 @@ __global__ void __launch_bounds__(CY_CELL_BS) k_cy_cell(const __grid_constant__ 
         C[5] = rad * S6f(rad, zz, ph, trk);
         C[6] = rad * S7f(rad, ph, trk);
       }
+      // RHS of Lh.f90:73-77: geometric source, then the phi derivative, over the
+      // radius (var 8 has none)
+      double R[7];
+      unsigned bad = far;
+#pragma unroll
+      for (int n = 0; n < 7; ++n) {
+        double r;
+        if (n == 1) r = Fz[3] - Fx[1];
+        else if (n == 3) r = -Fx[3] - Fx[3];
+        else if (n < 5) r = 0.0 - Fx[n];
+        else r = 0.0;
+        R[n] = fourier<LP>(K, Fz[n], kk, r, true);
+      }
+      double Q[7];
+#pragma unroll
+      for (int n = 0; n < 7; ++n) Q[n] = gdf::rdiv(R[n], rrad, bad);
+      if (bad) {
+#pragma unroll
+        for (int n = 0; n < 7; ++n) Q[n] = R[n] / rad;
+      }
+      const double* PX = K.B.phixG[a][b];
+      const double* PY = K.B.phiyG[a][b];
 #pragma unroll
       for (int n = 0; n < NE; ++n) {
-        // RHS of Lh.f90:73-77: geometric source, then the phi derivative
-        double R;
-        if (n == 0) R = 0.0 - Fx[0];
-        else if (n == 1) R = Fz[3] - Fx[1];
-        else if (n == 2) R = 0.0 - Fx[2];
-        else if (n == 3) R = -Fx[3] - Fx[3];
-        else if (n == 4) R = 0.0 - Fx[4];
-        else R = 0.0;
-        if (n < 7) R = fourier<LP>(K, Fz[n], kk, R, true);
-        R = R / rad + C[n];
-        const double* PX = K.B.phixG[a][b];
-        const double* PY = K.B.phiyG[a][b];
+        const double wR = n < 7 ? wab * (Q[n] + C[n]) : 0.0;
 #pragma unroll
         for (int d = 0; d < NQC; ++d) {
-          if (d > 0) du[n][d] = du[n][d] + wab * (Fx[n] * PX[d] + Fy[n] * PY[d]);
-          if (n < 7) du[n][d] = du[n][d] + wab * R * G[d];
+          // phixG vanishes for modes 1, 3, 6, phiyG for 1, 2, 4, Fx(6) and
+          // Fy(7) always: those products contribute +-0 and are left out
+          const bool hx = n != 5 && (d == 1 || d == 3 || d == 4), hy = n != 6 && (d == 2 || d == 4 || d == 5);
+          if (hx && hy) du[n][d] = du[n][d] + wab * (Fx[n] * PX[d] + Fy[n] * PY[d]);
+          else if (hx) du[n][d] = du[n][d] + wab * (Fx[n] * PX[d]);
+          else if (hy) du[n][d] = du[n][d] + wab * (Fy[n] * PY[d]);
+          if (n < 7) du[n][d] = du[n][d] + (d == 0 ? wR : wR * G[d]);
         }
       }
     }
@@ -565,8 +596,15 @@ __global__ void __launch_bounds__(CY_CELL_BS) k_cy_cell(const __grid_constant__ 
         else
           acc = acc + K.czs * K.B.w[g] * (u1 * K.B.phiGU[g][d] - d1 * K.B.phiGD[g][d]);
       }
-      du[n][d] = acc / K.B.mm[d];
+      du[n][d] = acc;
     }
+    // the mass matrix (mm(1) = 1), by its reciprocals
+    unsigned bad = 0;
+    double Q[NQC];
+#pragma unroll
+    for (int d = 1; d < NQC; ++d) Q[d] = gdf::rdiv(du[n][d], Rcp{K.B.mm[d], K.B.rmm[d]}, bad);
+#pragma unroll
+    for (int d = 1; d < NQC; ++d) du[n][d] = bad ? du[n][d] / K.B.mm[d] : Q[d];
   }
   if (KIND == KIND_LH) {
 #pragma unroll
@@ -576,17 +614,38 @@ __global__ void __launch_bounds__(CY_CELL_BS) k_cy_cell(const __grid_constant__ 
     for (int s = 48; s < NSC; ++s) T[cp + K.ncp * s] = 0.0;
     return;
   }
+  // the stage's combination, a variable's (then the cubic slots') six values
+  // at a time: their loads are all under way before the first store (192^2 x
+  // 2: 153-156 us per launch, 149-201 with each value stored before the next
+  // was loaded)
   const double dt = sc->dt;
 #pragma unroll
-  for (int n = 0; n < NE; ++n)
+  for (int n = 0; n <= NE; ++n) {
+    const double* u = U + cp + K.ncp * (NQC * n);
+    double a[NQC], x[NQC], u0[NQC];
 #pragma unroll
     for (int d = 0; d < NQC; ++d) {
       const long long o = cp + K.ncp * (NQC * n + d);
-      U[o] = combine(KIND, U[o], du[n][d], dt, X, U0, o);
+      if (KIND == KIND_S1) a[d] = u[K.ncp * d];
+      if (KIND != KIND_S1) { x[d] = X[o]; u0[d] = U0[o]; }
     }
-  for (int s = 48; s < NSC; ++s) {
-    const long long o = cp + K.ncp * s;
-    U[o] = combine(KIND, U[o], 0.0, dt, X, U0, o);
+#pragma unroll
+    for (int d = 0; d < NQC; ++d) {
+      const long long o = cp + K.ncp * (NQC * n + d);
+      const double dd = n < NE ? du[n < NE ? n : 0][d] : 0.0;
+      if (KIND == KIND_S1) {
+        const double v = a[d] + dt * dd;
+        U0[o] = a[d];
+        X[o] = v;
+        U[o] = v;
+      } else if (KIND == KIND_S2) {
+        const double v = (3.0 / 4.0) * u0[d] + (1.0 / 4.0) * (x[d] + dt * dd);
+        X[o] = v;
+        U[o] = v;
+      } else {
+        U[o] = (1.0 / 3.0) * u0[d] + (2.0 / 3.0) * (x[d] + dt * dd);
+      }
+    }
   }
 }
 
@@ -679,30 +738,40 @@ __global__ void __launch_bounds__(128) k_cy_bproj(const __grid_constant__ KC K, 
   const long long q = gtid();
   if (q >= K.ncp) return;
   const int i = (int)(q % K.nx2);
-  double acc[2][NQC];
+  double acc[2][NQC], m[2][NPC];
 #pragma unroll
   for (int v = 0; v < 2; ++v)
 #pragma unroll
-    for (int d = 0; d < NQC; ++d) acc[v][d] = 0.0;
+    for (int d = 0; d < NPC; ++d) {
+      const int sl = slotc(5 + v, d);
+      m[v][d] = sl >= 0 ? ld(U + q + K.ncp * sl) : 0.0;
+      if (d < NQC) acc[v][d] = 0.0;
+    }
   const double r0 = K.ra + (i - 0.5) * K.hr;
 #pragma unroll 1
   for (int a = 0; a < NG; ++a) {
     const double rad = r0 + K.hr1 * K.B.lam[a];
+    unsigned far = 0;
+    const Rcp rrad = gdf::rcp_of(rad, far);
 #pragma unroll 1
     for (int b = 0; b < NG; ++b) {
       const double* G = K.B.phiG[a][b];
       const double wab = 0.25 * K.B.w[a] * K.B.w[b];
 #pragma unroll
       for (int v = 0; v < 2; ++v) {
-        const int n = 5 + v;
         double s = 0.0;
 #pragma unroll
-        for (int d = 0; d < NPC; ++d) {
-          const int sl = slotc(n, d);
-          if (sl >= 0) s = s + ld(U + q + K.ncp * sl) * G[d];
-        }
+        for (int d = 0; d < NPC; ++d)
+          if (slotc(5 + v, d) >= 0) s = s + m[v][d] * G[d];
+        // + wab s / rad G(d) / mm(d): both divisors known ahead (mm(1) = 1)
+        const double t = gdf::rdiv_any(wab * s, rrad, far);
+        unsigned bad = 0;
+        double Q[NQC];
 #pragma unroll
-        for (int d = 0; d < NQC; ++d) acc[v][d] = acc[v][d] + wab * s / rad * G[d] / K.B.mm[d];
+        for (int d = 1; d < NQC; ++d) Q[d] = gdf::rdiv(t * G[d], Rcp{K.B.mm[d], K.B.rmm[d]}, bad);
+        acc[v][0] = acc[v][0] + t;
+#pragma unroll
+        for (int d = 1; d < NQC; ++d) acc[v][d] = acc[v][d] + (bad ? t * G[d] / K.B.mm[d] : Q[d]);
       }
     }
   }
@@ -920,8 +989,12 @@ __global__ void __launch_bounds__(128) k_cy_divfree(const __grid_constant__ KC K
       for (int d = 0; d < NQC; ++d) s = s + m8[d] * G[d];
       const double dv = fourier<LP>(K, s, kk, 0.0, false);
       const double wab = 0.25 * K.B.w[a] * K.B.w[b];
+      unsigned bad = 0;
+      double Q[NQC];
 #pragma unroll
-      for (int d = 0; d < NQC; ++d) bpp[d] = bpp[d] + wab * dv * G[d] / K.B.mm[d];
+      for (int d = 1; d < NQC; ++d) Q[d] = gdf::rdiv(wab * dv * G[d], Rcp{K.B.mm[d], K.B.rmm[d]}, bad);
+#pragma unroll
+      for (int d = 1; d < NQC; ++d) bpp[d] = bpp[d] + (bad ? wab * dv * G[d] / K.B.mm[d] : Q[d]);
     }
   if (!valid) return;
   auto br = [&](int ii, int d) { return ld(BR + ii + (K.nx + 1) * ((long long)(j - 1) + (long long)K.ny * (kk + (long long)K.nph * d))); };
@@ -1266,6 +1339,7 @@ void build_kc(const GdfCyConfig& c, KC& K) {
       K.cosk[d - 1][kk] = std::cos(d * K.phi[kk]);
     }
   build_basis(K.hr1, K.hz1, K.B);
+  for (int d = 0; d < NPC; ++d) K.B.rmm[d] = 1.0 / K.B.mm[d];
 }
 
 template <class F>
@@ -1280,7 +1354,7 @@ int run(GdfCyHandle* h, F&& launch) {
 int launch_set_bc(GdfCyHandle* h, const ScalC* sc) {
   const KC& K = h->K;
   const long long n = (2LL * K.ny + 2LL * K.nx2) * K.nph;
-  return run(h, [&] { k_cy_set_bc<<<nblk(n, 128), 128, 0, h->st>>>(K, h->U, sc); });
+  return run(h, [&] { k_cy_set_bc<<<nblk(n * NSC, 128), 128, 0, h->st>>>(K, h->U, sc); });
 }
 
 // set_bc, then Lh + LhEz of U fused with the stage's combination (kind)

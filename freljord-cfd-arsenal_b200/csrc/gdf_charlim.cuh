@@ -12,97 +12,6 @@
 
 namespace gdf {
 
-// ------------------------------------------------- division by a shared divisor
-// a / b with the IEEE result from r = RN(1/b): q0 = RN(a r), e = b q0 - a (one
-// fused operation), q = RN(q0 - e r). That this is the correctly rounded
-// quotient when nothing over- or underflows is Markstein's theorem (IBM J. Res.
-// Dev. 34, 1990) in the form of Brisebarre, Muller and Raina, "Accelerating
-// correctly rounded floating-point division when the divisor is known in
-// advance" (IEEE Trans. Comput. 53, 2004), algorithm 1.
-// The operands' ranges keep every step away from over- and underflow: |b| in
-// [2^-60, 2^60], a zero or |a| in [2^-960, 2^960] (a quotient is then normal,
-// and e, a multiple of 2^-1065, exact). The numerators' range is this wide
-// because a disturbance spreading into a quiet region decays by many orders of
-// magnitude per cell. An operand outside raises
-// `bad`, and the caller takes its general path. A zero a gives a zero quotient
-// whose sign may differ from the IEEE one where b < 0; no caller's value
-// depends on it.
-// One division costs three FP64 operations here; the compiler's own takes about
-// nine, a branch and a call for its special cases, per site.
-constexpr uint32_t RD_B_LO = (1023 - 60) << 20, RD_B_N = 120u << 20;
-constexpr uint32_t RD_A_LO = (1023 - 960) << 20, RD_A_N = 1920u << 20;
-
-GDF_HD uint32_t hi_of(double x) {
-#if defined(__CUDA_ARCH__)
-  return (uint32_t)__double2hiint(x);
-#else
-  uint64_t u;
-  memcpy(&u, &x, 8);
-  return (uint32_t)(u >> 32);
-#endif
-}
-GDF_HD uint32_t lo_of(double x) {
-#if defined(__CUDA_ARCH__)
-  return (uint32_t)__double2loint(x);
-#else
-  uint64_t u;
-  memcpy(&u, &x, 8);
-  return (uint32_t)u;
-#endif
-}
-
-struct Rcp {
-  double b, r;
-};
-GDF_HD Rcp rcp_of(double b, unsigned& bad) {
-  bad |= (unsigned)((hi_of(b) & 0x7fffffffu) - RD_B_LO >= RD_B_N);
-#if defined(__CUDA_ARCH__)
-  return {b, __drcp_rn(b)};
-#else
-  return {b, 1.0 / b};
-#endif
-}
-GDF_HD double rdiv(double a, const Rcp& d, unsigned& bad) {
-  const uint32_t h = hi_of(a) & 0x7fffffffu;
-  bad |= (unsigned)(h - RD_A_LO >= RD_A_N) & (unsigned)((h | lo_of(a)) != 0);
-#if defined(__CUDA_ARCH__)
-  const double q = __dmul_rn(a, d.r);
-  return __fma_rn(-__fma_rn(d.b, q, -a), d.r, q);
-#else
-  const double q = a * d.r;
-  return fma(-fma(d.b, q, -a), d.r, q);
-#endif
-}
-
-// the same where the caller keeps no flag: an operand out of range divides
-// itself
-GDF_HD double rdiv_any(double a, const Rcp& d, unsigned bad = 0) {
-  const double q = rdiv(a, d, bad);
-  return bad ? a / d.b : q;
-}
-
-// How char_limit_sparse divides: by shared reciprocals, or with the IEEE
-// division itself for the cells in which an operand leaves rdiv's ranges
-// (a disturbance spreading into a quiet region passes through a ring of
-// numerators below 2^-960).
-struct SharedRcp {
-  typedef Rcp Divisor;
-  static GDF_HD Divisor by(double b, unsigned& bad) { return rcp_of(b, bad); }
-  static GDF_HD Divisor known(double b, double r) { return {b, r}; }
-  static GDF_HD double div(double a, const Divisor& d, unsigned& bad) { return rdiv(a, d, bad); }
-  static GDF_HD double inverse(double b, unsigned& bad) { return rcp_of(b, bad).r; }
-};
-struct IeeeDiv {
-  typedef double Divisor;
-  static GDF_HD Divisor by(double b, unsigned& bad) {
-    bad |= (unsigned)!(b != 0.0 && fabs(b) < 1e300);
-    return b;
-  }
-  static GDF_HD Divisor known(double b, double) { return b; }
-  static GDF_HD double div(double a, Divisor d, unsigned&) { return a / d; }
-  static GDF_HD double inverse(double b, unsigned& bad) { return 1.0 / by(b, bad); }
-};
-
 // |a| and |b| as gfortran's MIN takes them (a NaN first operand gives the
 // second): non-negative doubles order as their bit patterns, NaN above all
 GDF_HD double min_abs(double a, double b) {

@@ -97,14 +97,9 @@ __host__ __device__ __forceinline__ long long face_items(const Consts& K) {
 // mL(n, d) (the cell on the low side) and mR(n, d) (the high side); o is the
 // face's offset in its plane. The arithmetic is that of Lh.f90:72-265 and
 // LhEz.f90:6-31 whichever memory the modes come from.
-// SMB: the face basis is read from sb, a copy in shared memory of the low
-// cell's table (phiGR / phiGU) followed by the high cell's (phiGL / phiGD),
-// [2][NG][NP], for lanes whose points g differ (the constant cache would
-// serialise their addresses).
-template <int DIR, bool SMB = false, class ML, class MR>
-__device__ __forceinline__ void face_point(const Consts& K, ML mL, MR mR, int g, double* __restrict__ Fh_out,
-                                           double* __restrict__ Ez_out, long long o,
-                                           const double* __restrict__ sb = nullptr) {
+template <int DIR, class DIV, class ML, class MR>
+__device__ __forceinline__ bool face_point(const Consts& K, ML mL, MR mR, int g, double* __restrict__ Fh_out,
+                                           double* __restrict__ Ez_out, long long o) {
   double uL[NE], uR[NE];
 #pragma unroll
   for (int n = 0; n < NE; ++n) {
@@ -112,8 +107,8 @@ __device__ __forceinline__ void face_point(const Consts& K, ML mL, MR mR, int g,
 #pragma unroll
     for (int d = 0; d < NP; ++d) {
       if (!live_mode(n, d)) continue;
-      const double pl = SMB ? sb[g * NP + d] : DIR == 0 ? c_basis.phiGR[g][d] : c_basis.phiGU[g][d];
-      const double pr = SMB ? sb[(NG + g) * NP + d] : DIR == 0 ? c_basis.phiGL[g][d] : c_basis.phiGD[g][d];
+      const double pl = DIR == 0 ? c_basis.phiGR[g][d] : c_basis.phiGU[g][d];
+      const double pr = DIR == 0 ? c_basis.phiGL[g][d] : c_basis.phiGD[g][d];
       // the face basis is 1 for mode 1, and for mode 2 (x faces) or 3 (y
       // faces) 1 on the low cell's face and -1 on the high cell's
       // (get_basis.f90): those products are exact and written out
@@ -132,11 +127,12 @@ __device__ __forceinline__ void face_point(const Consts& K, ML mL, MR mR, int g,
     uL[n] = a;
     uR[n] = b;
   }
-  Side L, R;
-  make_side<true>(K.P, uL, L);
-  make_side<true>(K.P, uR, R);
+  SideOf<DIV> L, R;
+  unsigned bad = 0;
+  make_side(K.P, uL, L, bad);
+  make_side(K.P, uR, R, bad);
   double Fh[NE], fL[NE], fR[NE];
-  face_flux_sides<true>(K.P, L, R, DIR, Fh, fL, fR);
+  face_flux_sides(K.P, L, R, DIR, Fh, fL, fR, bad);
   const long long fp = DIR == 0 ? K.fxplane : K.fyplane;
 #pragma unroll
   for (int n = 0; n < NE; ++n) Fh_out[(n * NG + g) * fp + o] = Fh[n];
@@ -157,30 +153,15 @@ __device__ __forceinline__ void face_point(const Consts& K, ML mL, MR mR, int g,
     }
   }
   Ez_out[g * fp + o] = ez;
+  return !bad;
 }
 
-// GFAST: items run point-fastest (item = g + NG * face), so the five points
-// of a face sit on adjacent lanes and their loads of the two cells' modes
-// are served by the same cache lines; the face basis then comes from sb
-// (see face_point). Otherwise faces run fastest (item = face + nf * (g + NG
-// * row)) and every lane of a warp has the same g.
-template <int DIR, bool GFAST = false>
-__device__ __forceinline__ void face_item(const Consts& K, const double* __restrict__ U, double* __restrict__ Fh_out,
-                                          double* __restrict__ Ez_out, long long item,
-                                          const double* __restrict__ sb = nullptr) {
+// Face f (in plane order) at point g; false where an operand left rdiv's ranges.
+template <int DIR, class DIV>
+__device__ __forceinline__ bool face_solve(const Consts& K, const double* __restrict__ U, double* __restrict__ Fh_out,
+                                        double* __restrict__ Ez_out, long long f, int g) {
   const int nf = DIR == 0 ? K.nx + 1 : K.nx;
-  int i0, g, j0;
-  if (GFAST) {
-    g = (int)(item % NG);
-    const long long f = item / NG;
-    i0 = (int)(f % nf);
-    j0 = (int)(f / nf);
-  } else {
-    i0 = (int)(item % nf);
-    const long long r = item / nf;
-    g = (int)(r % NG);
-    j0 = (int)(r / NG);
-  }
+  const int i0 = (int)(f % nf), j0 = (int)(f / nf);
   long long cL, cR;
   if (DIR == 0) {
     cL = i0 + (long long)K.nx2 * (j0 + 1);
@@ -190,44 +171,33 @@ __device__ __forceinline__ void face_item(const Consts& K, const double* __restr
     cR = cL + K.nx2;
   }
   const long long pl = K.plane;
-  face_point<DIR, GFAST>(
+  return face_point<DIR, DIV>(
       K, [&](int n, int d) { return U[pl * (d + 10 * n) + cL]; }, [&](int n, int d) { return U[pl * (d + 10 * n) + cR]; },
-      g, Fh_out, Ez_out, i0 + (long long)nf * j0, sb);
+      g, Fh_out, Ez_out, f);
 }
 
-// Faces of one block, staged: FACE_TILE faces of one face row at all NG
-// points (FACE_TILE * NG threads of a 128-thread block). The modes of the
-// cells they touch are copied once into shared memory with coalesced loads
-// (x faces: the FACE_TILE + 1 cells of one cell row; y faces: FACE_TILE
-// cells of the two cell rows), and every face point reads its two cells
-// from there instead of issuing 104 scattered global loads of its own.
-constexpr int FACE_TILE = 25;
-constexpr int FACE_TILE_W = FACE_TILE + 1;   // cells per staged row
+// A face whose operands leave rdiv's ranges is solved again with IEEE divisions
+// (out of line: rare, and its code stays out of the instruction cache).
 template <int DIR>
-__device__ __forceinline__ void face_tile(const Consts& K, const double* __restrict__ U, double* __restrict__ Fh_out,
-                                          double* __restrict__ Ez_out, int f0, int j0,
-                                          double (*ms)[2 * FACE_TILE_W]) {
+static __device__ __noinline__ void face_refused(const Consts& K, const double* __restrict__ U,
+                                                 double* __restrict__ Fh_out, double* __restrict__ Ez_out, long long f,
+                                                 int g) {
+  face_solve<DIR, IeeeDiv>(K, U, Fh_out, Ez_out, f, g);
+}
+template <int DIR>
+__device__ __forceinline__ void face_at(const Consts& K, const double* __restrict__ U, double* __restrict__ Fh_out,
+                                        double* __restrict__ Ez_out, long long f, int g) {
+  if (!face_solve<DIR, SharedRcp>(K, U, Fh_out, Ez_out, f, g)) face_refused<DIR>(K, U, Fh_out, Ez_out, f, g);
+}
+
+// the same from an item number, faces of a row fastest, then its points (the
+// ensemble's tiles)
+template <int DIR>
+__device__ __forceinline__ void face_item(const Consts& K, const double* __restrict__ U, double* __restrict__ Fh_out,
+                                          double* __restrict__ Ez_out, long long item) {
   const int nf = DIR == 0 ? K.nx + 1 : K.nx;
-  const int rows = DIR == 0 ? 1 : 2;
-  const int ncx = DIR == 0 ? min(FACE_TILE_W, nf + 1 - f0) : min(FACE_TILE, nf - f0);
-  const long long pl = K.plane;
-  const int per_slot = rows * ncx;
-  for (int q = threadIdx.x; q < NLIVE * per_slot; q += blockDim.x) {
-    const int s = q / per_slot, rk = q - s * per_slot;
-    const int r = rk / ncx, k = rk - r * ncx;
-    const long long cell = DIR == 0 ? f0 + k + (long long)K.nx2 * (j0 + 1) : (f0 + 1 + k) + (long long)K.nx2 * (j0 + r);
-    ms[s][r * FACE_TILE_W + k] = U[cell + pl * (c_live_d[s] + 10 * c_live_n[s])];
-  }
-  __syncthreads();
-  const int t = threadIdx.x;
-  if (t >= FACE_TILE * NG) return;
-  const int f = t % FACE_TILE, g = t / FACE_TILE;
-  const int i0 = f0 + f;
-  if (i0 >= nf) return;
-  const int kR = DIR == 0 ? f + 1 : FACE_TILE_W + f;
-  face_point<DIR>(
-      K, [&](int n, int d) { return ms[LI(n, d)][f]; }, [&](int n, int d) { return ms[LI(n, d)][kR]; }, g, Fh_out,
-      Ez_out, i0 + (long long)nf * j0);
+  const long long r = item / nf;
+  face_at<DIR>(K, U, Fh_out, Ez_out, item - r * nf + (r / NG) * nf, (int)(r % NG));
 }
 
 // ------------------------------------------------------- vertex Ez -------
@@ -267,6 +237,10 @@ __device__ __forceinline__ void vertex_item(const Consts& K, const double* __res
     }
     URU[n] = a; ULU[n] = b; URD[n] = c; ULD[n] = e;
   }
+  // IEEE divisions: four solvers' worth of live state leaves no registers for
+  // the reciprocals (168 without spills; with them 352 bytes of spills, 1.27
+  // against 1.31 ms on the blast 2048^2 but 165 against 107 us on the rotor
+  // 512^2, whose quiet region sends a ring of vertices to the IEEE copy)
   EzV[item] = vertex_ez(K.P, URU, ULU, URD, ULD);
 }
 
@@ -489,26 +463,34 @@ __device__ __forceinline__ void cell_item(const Consts& K, const double* __restr
     }
     return;
   }
+  // the stage's combination, a variable at a time: its loads are all under way
+  // before its first store
   const double dt = sc->dt;
 #pragma unroll
-  for (int n = 0; n < NE; ++n)
+  for (int n = 0; n < NE; ++n) {
+    double a[NP], b[NP];
 #pragma unroll
     for (int d = 0; d < NP; ++d) {
       if (!live_mode(n, d)) continue;
       const long long c = item + K.plane * (d + 10 * n);
-      const double dd = du[LI(n, d)];
+      a[d] = stage == 1 ? U[c] : UI[c];
+      b[d] = stage == 1 ? 0.0 : U0[c];
+    }
+#pragma unroll
+    for (int d = 0; d < NP; ++d) {
+      if (!live_mode(n, d)) continue;
+      const long long c = item + K.plane * (d + 10 * n);
+      const double v = a[d] + dt * du[LI(n, d)];
       if (stage == 1) {
-        const double u0 = U[c];
-        U0[c] = u0;
-        UI[c] = u0 + dt * dd;
+        U0[c] = a[d];
+        UI[c] = v;
       } else if (stage == 2) {
-        const double v = UI[c] + dt * dd;
-        UI[c] = (3.0 / 4.0) * U0[c] + (1.0 / 4.0) * v;
+        UI[c] = (3.0 / 4.0) * b[d] + (1.0 / 4.0) * v;
       } else {
-        const double v = UI[c] + dt * dd;
-        UI[c] = (1.0 / 3.0) * U0[c] + (2.0 / 3.0) * v;
+        UI[c] = (1.0 / 3.0) * b[d] + (2.0 / 3.0) * v;
       }
     }
+  }
 }
 
 // --------------------------------------------------- face-B update -------

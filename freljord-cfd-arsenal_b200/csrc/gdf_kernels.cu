@@ -43,20 +43,7 @@
 // Faces at 4 blocks (128 registers, ~300 B spilled) ran 20% faster than at
 // the unconstrained 168 registers; the residual kernel gained nothing.
 #ifndef GDF_FACE_MINB
-#define GDF_FACE_MINB 4
-#endif
-// faces through the shared-memory staged kernel (k_face_tile) or one
-// thread per face point reading global memory (k_face, the default: the
-// staged form measured 30% slower, blast 2048^2, same values)
-#ifndef GDF_FACE_STAGED
-#define GDF_FACE_STAGED 0
-#endif
-// face points numbered point-fastest, the five points of a face on
-// adjacent lanes (face_item<DIR, true>): face kernels 3.04 / 3.21 against
-// 2.83 / 2.91 ms on the blast 2048^2 (step 47.8 against 45.6 ms, same
-// values), so the product keeps faces fastest
-#ifndef GDF_FACE_GFAST
-#define GDF_FACE_GFAST 0
+#define GDF_FACE_MINB 3
 #endif
 // vertex kernel at 3 blocks (168 registers, no spill): timed alone a
 // launch is 10% slower than at 4 blocks, but the blast 2048^2 step replayed
@@ -92,37 +79,18 @@ __global__ void k_set_bc(const __grid_constant__ Consts K, double* __restrict__ 
   set_bc_item(K, U, zeroB, t);
 }
 
+// A block takes 32 consecutive faces, one point per warp: the five warps read
+// the same two cells' modes, so four of the five reads hit L1, and a warp's
+// point is uniform (its basis values come from the constant cache).
+constexpr int FACE_BS = 32 * NG;
 template <int DIR>
-__global__ void __launch_bounds__(128, GDF_FACE_MINB) k_face(const __grid_constant__ Consts K, const double* __restrict__ U,
+__global__ void __launch_bounds__(FACE_BS, GDF_FACE_MINB) k_face(const __grid_constant__ Consts K, const double* __restrict__ U,
                                               double* __restrict__ Fh_out, double* __restrict__ Ez_out,
                                               const Scal* __restrict__ sc) {
   if (sc && !sc->active) return;
-  const long long item = gtid();
-  if (GDF_FACE_GFAST) {
-    // the face basis of this direction in shared memory: low cell's table,
-    // then the high cell's
-    __shared__ double sb[2 * NG * NP];
-    const double* lo = DIR == 0 ? &c_basis.phiGR[0][0] : &c_basis.phiGU[0][0];
-    const double* hi = DIR == 0 ? &c_basis.phiGL[0][0] : &c_basis.phiGD[0][0];
-    for (int k = threadIdx.x; k < 2 * NG * NP; k += blockDim.x) sb[k] = k < NG * NP ? lo[k] : hi[k - NG * NP];
-    __syncthreads();
-    if (item >= face_items<DIR>(K)) return;
-    face_item<DIR, true>(K, U, Fh_out, Ez_out, item, sb);
-    return;
-  }
-  if (item >= face_items<DIR>(K)) return;
-  face_item<DIR>(K, U, Fh_out, Ez_out, item);
-}
-
-// The staged form of k_face: block (bx, by) takes faces bx*FACE_TILE ..
-// of face row by at all quadrature points.
-template <int DIR>
-__global__ void __launch_bounds__(128, GDF_FACE_MINB) k_face_tile(const __grid_constant__ Consts K,
-                                                    const double* __restrict__ U, double* __restrict__ Fh_out,
-                                                    double* __restrict__ Ez_out, const Scal* __restrict__ sc) {
-  __shared__ double ms[NLIVE][2 * FACE_TILE_W];
-  if (sc && !sc->active) return;
-  face_tile<DIR>(K, U, Fh_out, Ez_out, (int)blockIdx.x * FACE_TILE, (int)blockIdx.y, ms);
+  const long long f = (long long)blockIdx.x * 32 + (threadIdx.x & 31);
+  if (f >= (DIR == 0 ? K.fxplane : K.fyplane)) return;
+  face_at<DIR>(K, U, Fh_out, Ez_out, f, threadIdx.x >> 5);
 }
 
 __global__ void __launch_bounds__(128, GDF_VERTEX_MINB) k_vertex(const __grid_constant__ Consts K, const double* __restrict__ U,
@@ -710,17 +678,12 @@ static int launch_set_bc(GdfHandle* h, double* U, int zeroB, const Scal* sc) {
 // Lh traces/Riemann (Fxhat, Fyhat, EzRL, EzUD) and LhEz vertex Ez on U
 static int launch_faces(GdfHandle* h, const double* U, const Scal* sc) {
   const Consts& K = h->K;
-  const long long nfx = (long long)(K.nx + 1) * NG * K.ny;
-  const long long nfy = (long long)K.nx * NG * (K.ny + 1);
-  int rc;
-  if (GDF_FACE_STAGED && K.ny + 1 <= 65535) {
-    const dim3 gx((unsigned)nblk(K.nx + 1, FACE_TILE), (unsigned)K.ny), gy((unsigned)nblk(K.nx, FACE_TILE), (unsigned)(K.ny + 1));
-    rc = run_kernel(h, GDF_K_FACE_X, [&] { k_face_tile<0><<<gx, 128, 0, h->st>>>(K, U, h->Fxh, h->EzRL, sc); });
-    if (!rc) rc = run_kernel(h, GDF_K_FACE_Y, [&] { k_face_tile<1><<<gy, 128, 0, h->st>>>(K, U, h->Fyh, h->EzUD, sc); });
-  } else {
-    rc = run_kernel(h, GDF_K_FACE_X, [&] { k_face<0><<<nblk(nfx, 128), 128, 0, h->st>>>(K, U, h->Fxh, h->EzRL, sc); });
-    if (!rc) rc = run_kernel(h, GDF_K_FACE_Y, [&] { k_face<1><<<nblk(nfy, 128), 128, 0, h->st>>>(K, U, h->Fyh, h->EzUD, sc); });
-  }
+  int rc = run_kernel(h, GDF_K_FACE_X, [&] {
+    k_face<0><<<nblk(K.fxplane, 32), FACE_BS, 0, h->st>>>(K, U, h->Fxh, h->EzRL, sc);
+  });
+  if (!rc) rc = run_kernel(h, GDF_K_FACE_Y, [&] {
+    k_face<1><<<nblk(K.fyplane, 32), FACE_BS, 0, h->st>>>(K, U, h->Fyh, h->EzUD, sc);
+  });
   if (!rc) rc = run_kernel(h, GDF_K_VERTEX, [&] { k_vertex<<<nblk(K.vplane, 128), 128, 0, h->st>>>(K, U, h->EzV, sc); });
   return rc;
 }
@@ -1273,8 +1236,8 @@ int gdf_lh_noalloc(const GdfConfig* cfg, const double* d_uh, double* d_du, void*
   // the scratch left by an earlier call needs no clearing; du's ghost and
   // dead slots must read 0
   CK(cudaMemsetAsync(d_du, 0, uh_bytes(*cfg), st));
-  k_face<0><<<nblk(fx * NG, 128), 128, 0, st>>>(K, d_uh, Fxh, ezx, nullptr);
-  k_face<1><<<nblk(fy * NG, 128), 128, 0, st>>>(K, d_uh, Fyh, ezy, nullptr);
+  k_face<0><<<nblk(fx, 32), FACE_BS, 0, st>>>(K, d_uh, Fxh, ezx, nullptr);
+  k_face<1><<<nblk(fy, 32), FACE_BS, 0, st>>>(K, d_uh, Fyh, ezy, nullptr);
   k_cell<<<nblk(K.plane, CELL_BS), CELL_BS, 0, st>>>(K, d_uh, nullptr, nullptr, Fxh, Fyh, d_du, nullptr, 0);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(GDF_ERR_CUDA, std::string("gdf_lh_noalloc launch: ") + cudaGetErrorString(e));

@@ -42,7 +42,9 @@ namespace gdf3 {
 
 using gdf::fmax2;
 using gdf::fmin2;
+using gdf::IeeeDiv;
 using gdf::Phys;
+using gdf::SharedRcp;
 using gdf::sgn1;
 using gdf::Side;
 using gdf::sq;
@@ -115,17 +117,18 @@ __device__ __forceinline__ void flux3(const Side& s, double* F) {
 
 // one face point: uL = trace of the cell on the -normal side (the
 // reference's UL1), uR = the +normal side (UR1); Fh = Fhat1
-template <int DIR>
-__device__ __forceinline__ void face_flux3(const Phys& P, const double* uL, const double* uR, double* Fh) {
-  Side L, R;
-  gdf::make_side(P, uL, L);
-  gdf::make_side(P, uR, R);
+template <int DIR, class DIV>
+__device__ __forceinline__ void face_flux3(const Phys& P, const double* uL, const double* uR, double* Fh,
+                                           unsigned& bad) {
+  gdf::SideOf<DIV> L, R;
+  gdf::make_side(P, uL, L, bad);
+  gdf::make_side(P, uR, R, bad);
   double fL[NE], fR[NE];
   flux3<DIR>(L, fL);
   flux3<DIR>(R, fR);
   double a1, a2, b1, b2;
-  gdf::side_speeds(P, L, DIR, a1, a2);   // SRmax, SRmin (from the left cell's trace)
-  gdf::side_speeds(P, R, DIR, b1, b2);   // SLmax, SLmin
+  gdf::side_speeds(P, L, DIR, a1, a2, bad);   // SRmax, SRmin (from the left cell's trace)
+  gdf::side_speeds(P, R, DIR, b1, b2, bad);   // SLmax, SLmin
   const double SR = fmax2(a1, b1);
   const double SL = fmin2(a2, b2);
   if (P.flux == 1) {
@@ -140,16 +143,18 @@ __device__ __forceinline__ void face_flux3(const Phys& P, const double* uL, cons
 #pragma unroll
       for (int n = 0; n < NE; ++n) Fh[n] = fL[n];
     } else {
-      const double den = SR - SL, sls = SL * SR;
+      const auto rS = DIV::by(SR - SL, bad);
+      const double sls = SL * SR;
 #pragma unroll
-      for (int n = 0; n < NE; ++n) Fh[n] = (SR * fL[n] - SL * fR[n] + sls * (R.U[n] - L.U[n])) / den;
+      for (int n = 0; n < NE; ++n)
+        Fh[n] = DIV::div(SR * fL[n] - SL * fR[n] + sls * (R.U[n] - L.U[n]), rS, bad);
     }
   } else {
     double Ust[NE];
     if (P.flux == 3)
-      gdf::hllcd_flux<false>(P, R, L, fR, fL, SR, SL, DIR, Fh, Ust);
+      gdf::hllcd_flux<false, DIV>(P, R, L, fR, fL, SR, SL, DIR, Fh, Ust, bad);
     else
-      gdf::hllcd_flux<true>(P, R, L, fR, fL, SR, SL, DIR, Fh, Ust);
+      gdf::hllcd_flux<true, DIV>(P, R, L, fR, fL, SR, SL, DIR, Fh, Ust, bad);
   }
 }
 
@@ -261,16 +266,11 @@ __global__ void __launch_bounds__(128) k3_set_bc(const __grid_constant__ K3 K, d
 }
 
 // ---------------------------------------------------------------- faces ----
-// item = g * (faces) + face: a warp covers consecutive faces at one point.
-template <int DIR>
-__global__ void __launch_bounds__(128) k3_face(const __grid_constant__ K3 K, const double* __restrict__ U,
-                                               double* __restrict__ Fh, const Scal3* __restrict__ sc) {
-  if (sc && !sc->active) return;
+// Face f at point g; false where an operand left rdiv's ranges.
+template <int DIR, class DIV>
+__device__ __forceinline__ bool face_solve3(const K3& K, const double* __restrict__ U, double* __restrict__ Fh,
+                                            long long f, int g) {
   const long long nf = DIR == 0 ? K.fxplane : K.fyplane;
-  const long long item = gtid();
-  if (item >= nf * NG) return;
-  const int g = (int)(item / nf);
-  const long long f = item - (long long)g * nf;
   long long cl, cr;
   if (DIR == 0) {
     const int i = (int)(f % (K.nx + 1)), j = (int)(f / (K.nx + 1)) + 1;
@@ -282,11 +282,49 @@ __global__ void __launch_bounds__(128) k3_face(const __grid_constant__ K3 K, con
     cr = cl + K.nx2;
   }
   double uL[NE], uR[NE], F[NE];
+  unsigned bad = 0;
   trace3(K, U, cl, DIR == 0 ? K.B.phiGR[g] : K.B.phiGU[g], uL);
   trace3(K, U, cr, DIR == 0 ? K.B.phiGL[g] : K.B.phiGD[g], uR);
-  face_flux3<DIR>(K.P, uL, uR, F);
+  face_flux3<DIR, DIV>(K.P, uL, uR, F, bad);
 #pragma unroll
   for (int n = 0; n < NE; ++n) Fh[(long long)(g * NE + n) * nf + f] = F[n];
+  return !bad;
+}
+template <int DIR>
+static __device__ __noinline__ void face_refused3(const K3& K, const double* __restrict__ U, double* __restrict__ Fh,
+                                                  long long f, int g) {
+  face_solve3<DIR, IeeeDiv>(K, U, Fh, f, g);
+}
+// y faces: a block takes 32 consecutive faces, one point per warp (as the P2
+// faces), so that the five points' reads of the two cells' 168 modes meet in
+// L1: 81 against 119 us per launch at 480 x 240. x faces: consecutive faces at
+// one point per block of 128; neighbouring lanes share a cell's modes already,
+// and with 254 registers the loads run far ahead (80 us; 109 in the other
+// shape at 168 registers, 156 at 128).
+template <int DIR>
+struct Face3 {
+  static constexpr int BS = DIR == 0 ? 128 : 32 * NG, MINB = DIR == 0 ? 1 : 2;
+};
+template <int DIR>
+__global__ void __launch_bounds__(Face3<DIR>::BS, Face3<DIR>::MINB) k3_face(const __grid_constant__ K3 K,
+                                                                          const double* __restrict__ U,
+                                                                          double* __restrict__ Fh,
+                                                                          const Scal3* __restrict__ sc) {
+  if (sc && !sc->active) return;
+  const long long nf = DIR == 0 ? K.fxplane : K.fyplane;
+  long long f;
+  int g;
+  if (DIR == 0) {
+    const long long item = gtid();
+    g = (int)(item / nf);
+    f = item - (long long)g * nf;
+    if (g >= NG) return;
+  } else {
+    f = (long long)blockIdx.x * 32 + (threadIdx.x & 31);
+    g = threadIdx.x >> 5;
+    if (f >= nf) return;
+  }
+  if (!face_solve3<DIR, SharedRcp>(K, U, Fh, f, g)) face_refused3<DIR>(K, U, Fh, f, g);
 }
 
 // -------------------------------------------------------------- vertices ---
@@ -348,8 +386,14 @@ __global__ void __launch_bounds__(64) k3_cell(const __grid_constant__ K3 K, doub
 #else
       trace3(K, U, c, K.B.phiG[a][b], uG);
 #endif
-      Side s;
-      gdf::make_side(K.P, uG, s);
+      gdf::SideOf<SharedRcp> s;
+      unsigned bad = 0;
+      gdf::make_side(K.P, uG, s, bad);
+      if (bad) {
+        gdf::SideOf<IeeeDiv> e;
+        gdf::make_side(K.P, uG, e, bad);
+        static_cast<Side&>(s) = e;
+      }
       double Fx[NE], Fy[NE];
       flux3<0>(s, Fx);
       flux3<1>(s, Fy);
@@ -1033,8 +1077,8 @@ int launch_set_bc(GdfP3Handle* h, double* S, double* SX, double* SY, const Scal3
 // Lh of U (ghosts as they are) into the stage's outputs (kind)
 int launch_lh_body(GdfP3Handle* h, int kind, const Scal3* sc) {
   const K3& K = h->K;
-  int rc = run(h, [&] { k3_face<0><<<nblk(K.fxplane * NG, 128), 128, 0, h->st>>>(K, h->U, h->Fxh, sc); });
-  if (!rc) rc = run(h, [&] { k3_face<1><<<nblk(K.fyplane * NG, 128), 128, 0, h->st>>>(K, h->U, h->Fyh, sc); });
+  int rc = run(h, [&] { k3_face<0><<<nblk(K.fxplane * NG, Face3<0>::BS), Face3<0>::BS, 0, h->st>>>(K, h->U, h->Fxh, sc); });
+  if (!rc) rc = run(h, [&] { k3_face<1><<<nblk(K.fyplane, 32), Face3<1>::BS, 0, h->st>>>(K, h->U, h->Fyh, sc); });
   if (!rc) rc = run(h, [&] { k3_vertex<<<nblk(K.vplane, 128), 128, 0, h->st>>>(K, h->U, h->EzV, sc); });
   if (rc) return rc;
   const unsigned nc = nblk((long long)K.nx * K.ny, 64), nf = nblk(K.fxplane + K.fyplane, 128);

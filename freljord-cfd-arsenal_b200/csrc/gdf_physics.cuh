@@ -45,14 +45,10 @@ GDF_HD double sgn1(double b) { return copysign(1.0, b); }
 // x / y and sqrt(x) with their IEEE results. On the device a zero x is
 // answered directly (the signed zero the operation would return), because
 // the hardware sequences send a zero operand down their slow path; a 2-D run
-// (w = Bz = 0 everywhere, u = v = 0 in quiet regions) feeds the face solvers
-// a zero numerator in a large share of their divisions. Every other operand
-// goes through the correctly rounded operation itself.
-#ifndef GDF_DV_FAST
-#define GDF_DV_FAST 1
-#endif
+// (w = Bz = 0 everywhere, u = v = 0 in quiet regions) has many. Every other
+// operand goes through the correctly rounded operation itself.
 GDF_HD double dv(double x, double y) {
-#if defined(__CUDA_ARCH__) && GDF_DV_FAST
+#if defined(__CUDA_ARCH__)
   if (x == 0.0 && y == y && y != 0.0)
     return __longlong_as_double((long long)(((unsigned long long)__double_as_longlong(x) ^
                                              (unsigned long long)__double_as_longlong(y)) & 0x8000000000000000ull));
@@ -60,22 +56,106 @@ GDF_HD double dv(double x, double y) {
   return x / y;
 }
 GDF_HD double sqrt0(double x) {
-#if defined(__CUDA_ARCH__) && GDF_DV_FAST
-  if (x == 0.0) return x;
+#if defined(__CUDA_ARCH__)
+  if ((((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) == 0u) return x;
 #endif
   return sqrt(x);
 }
-// The face solvers take the shortcut (ZF); elsewhere the plain operation
-// measured faster (the vertex solver and the limiter's eigenvectors meet
-// few exact zeros and their code grows with the extra test).
-template <bool ZF>
-GDF_HD double dvz(double x, double y) {
-  return ZF ? dv(x, y) : x / y;
+
+// ------------------------------------------------- division by a shared divisor
+// a / b with the IEEE result from r = RN(1/b): q0 = RN(a r), e = b q0 - a (one
+// fused operation), q = RN(q0 - e r). That this is the correctly rounded
+// quotient when nothing over- or underflows is Markstein's theorem (IBM J. Res.
+// Dev. 34, 1990) in the form of Brisebarre, Muller and Raina, "Accelerating
+// correctly rounded floating-point division when the divisor is known in
+// advance" (IEEE Trans. Comput. 53, 2004), algorithm 1.
+// The operands' ranges keep every step away from over- and underflow: |b| in
+// [2^-60, 2^60], a zero or |a| in [2^-960, 2^960] (a quotient is then normal,
+// and e, a multiple of 2^-1065, exact). The numerators' range is this wide
+// because a disturbance spreading into a quiet region decays by many orders of
+// magnitude per cell. An operand outside raises
+// `bad`, and the caller takes its general path. A zero a gives a zero quotient
+// whose sign may differ from the IEEE one where b < 0; no caller's value
+// depends on it.
+// One division costs three FP64 operations here; the compiler's own takes about
+// nine, a branch and a call for its special cases, per site.
+constexpr uint32_t RD_B_LO = (1023 - 60) << 20, RD_B_N = 120u << 20;
+constexpr uint32_t RD_A_LO = (1023 - 960) << 20, RD_A_N = 1920u << 20;
+
+GDF_HD uint32_t hi_of(double x) {
+#if defined(__CUDA_ARCH__)
+  return (uint32_t)__double2hiint(x);
+#else
+  uint64_t u;
+  memcpy(&u, &x, 8);
+  return (uint32_t)(u >> 32);
+#endif
 }
-template <bool ZF>
-GDF_HD double sqz(double x) {
-  return ZF ? sqrt0(x) : sqrt(x);
+GDF_HD uint32_t lo_of(double x) {
+#if defined(__CUDA_ARCH__)
+  return (uint32_t)__double2loint(x);
+#else
+  uint64_t u;
+  memcpy(&u, &x, 8);
+  return (uint32_t)u;
+#endif
 }
+
+struct Rcp {
+  double b, r;
+};
+GDF_HD Rcp rcp_of(double b, unsigned& bad) {
+  bad |= (unsigned)((hi_of(b) & 0x7fffffffu) - RD_B_LO >= RD_B_N);
+#if defined(__CUDA_ARCH__)
+  return {b, __drcp_rn(b)};
+#else
+  return {b, 1.0 / b};
+#endif
+}
+GDF_HD double rdiv(double a, const Rcp& d, unsigned& bad) {
+  const uint32_t h = hi_of(a) & 0x7fffffffu;
+  bad |= (unsigned)(h - RD_A_LO >= RD_A_N) & (unsigned)((h | lo_of(a)) != 0);
+#if defined(__CUDA_ARCH__)
+  const double q = __dmul_rn(a, d.r);
+  return __fma_rn(-__fma_rn(d.b, q, -a), d.r, q);
+#else
+  const double q = a * d.r;
+  return fma(-fma(d.b, q, -a), d.r, q);
+#endif
+}
+
+// the same where the caller keeps no flag: an operand out of range divides
+// itself
+GDF_HD double rdiv_any(double a, const Rcp& d, unsigned bad = 0) {
+  const double q = rdiv(a, d, bad);
+  return bad ? a / d.b : q;
+}
+
+// How the solvers divide: by shared reciprocals, or with the IEEE division
+// itself for the items in which an operand leaves rdiv's ranges (a disturbance
+// spreading into a quiet region passes through a ring of numerators below
+// 2^-960).
+struct SharedRcp {
+  typedef Rcp Divisor;
+  static GDF_HD Divisor by(double b, unsigned& bad) { return rcp_of(b, bad); }
+  static GDF_HD Divisor known(double b, double r) { return {b, r}; }
+  static GDF_HD double div(double a, const Divisor& d, unsigned& bad) { return rdiv(a, d, bad); }
+  static GDF_HD double inverse(double b, unsigned& bad) { return rcp_of(b, bad).r; }
+  static GDF_HD double root(double x) { return sqrt0(x); }
+};
+struct IeeeDiv {
+  typedef double Divisor;
+  static GDF_HD Divisor by(double b, unsigned& bad) {
+    bad |= (unsigned)!(b != 0.0 && fabs(b) < 1e300);
+    return b;
+  }
+  static GDF_HD Divisor known(double b, double) { return b; }
+  static GDF_HD double div(double a, Divisor d, unsigned&) { return a / d; }
+  static GDF_HD double inverse(double b, unsigned& bad) { return 1.0 / by(b, bad); }
+  static GDF_HD double root(double x) { return sqrt(x); }
+};
+
+GDF_HD double quot(double x, double y) { return x / y; }
 
 // Constants of the eigenvectors that depend on gflux alone (eigenmatrix.f90);
 // set_eig_consts fills them with the values eigen_left and eigen_right form.
@@ -109,14 +189,21 @@ struct Side {
   double rho, u, v, w, E, B1, B2, B3, BB, p;
 };
 
-template <bool ZF = false>
-GDF_HD void make_side(const Phys& P, const double* U, Side& s) {
+// a state with the divisor its primitives and speeds share
+template <class DIV>
+struct SideOf : Side {
+  typename DIV::Divisor rr;
+};
+
+template <class DIV>
+GDF_HD void make_side(const Phys& P, const double* U, SideOf<DIV>& s, unsigned& bad) {
 #pragma unroll
   for (int n = 0; n < NE; ++n) s.U[n] = U[n];
   s.rho = U[0];
-  s.u = dvz<ZF>(U[1], s.rho);
-  s.v = dvz<ZF>(U[2], s.rho);
-  s.w = dvz<ZF>(U[3], s.rho);
+  s.rr = DIV::by(s.rho, bad);
+  s.u = DIV::div(U[1], s.rr, bad);
+  s.v = DIV::div(U[2], s.rr, bad);
+  s.w = DIV::div(U[3], s.rr, bad);
   s.E = U[4];
   s.B1 = U[5];
   s.B2 = U[6];
@@ -183,15 +270,15 @@ GDF_HD void side_flux_hard(const Phys& P, const Side& s, double* Fx, double* Fy)
 }
 
 // eigenvalueMm.f90 from a state's primitives (normal x: dir 0, y: dir 1)
-template <bool ZF = false>
-GDF_HD void side_speeds(const Phys& P, const Side& s, int dir, double& amax, double& amin) {
+template <class DIV>
+GDF_HD void side_speeds(const Phys& P, const SideOf<DIV>& s, int dir, double& amax, double& amin, unsigned& bad) {
   const double Bn = dir == 0 ? s.B1 : s.B2;
   const double un = dir == 0 ? s.u : s.v;
-  const double c = sqz<ZF>(fabs(dvz<ZF>(P.gamma * s.p, s.rho)));
+  const double c = DIV::root(fabs(DIV::div(P.gamma * s.p, s.rr, bad)));
   const double c2 = sq(c);
-  const double br = dvz<ZF>(s.BB, s.rho);
+  const double br = DIV::div(s.BB, s.rr, bad);
   const double X = c2 + br;
-  const double cf = sqz<ZF>(fabs(0.5 * (c2 + br + sqz<ZF>(sq(X) - dvz<ZF>(4 * c2 * sq(Bn), s.rho)))));
+  const double cf = DIV::root(fabs(0.5 * (c2 + br + DIV::root(sq(X) - DIV::div(4 * c2 * sq(Bn), s.rr, bad)))));
   amax = un + cf;
   amin = un - cf;
 }
@@ -200,16 +287,16 @@ GDF_HD void side_speeds(const Phys& P, const Side& s, int dir, double& amax, dou
 // eigenvalueMm.f90:1-25 for the normal (1,0) (dir 0) or (0,1) (dir 1).
 GDF_HD void fast_speeds(const Phys& P, const double* U, int dir, double& amax, double& amin) {
   const double rho = U[0];
-  const double u = dvz<false>(U[1], rho), v = dvz<false>(U[2], rho), w = dvz<false>(U[3], rho);
+  const double u = quot(U[1], rho), v = quot(U[2], rho), w = quot(U[3], rho);
   const double B1 = U[5], B2 = U[6], B3 = U[7];
   const double BP = sq(B1) + sq(B2) + sq(B3);
   const double Bn = dir == 0 ? B1 : B2;
   const double un = dir == 0 ? u : v;
   const double p = P.gamma1 * (U[4] - 0.5 * rho * (sq(u) + sq(v) + sq(w)) - 0.5 * BP);
-  const double c = sqz<false>(fabs(dvz<false>(P.gamma * p, rho)));
+  const double c = sqrt(fabs(quot(P.gamma * p, rho)));
   const double c2 = sq(c);
-  const double X = c2 + dvz<false>(BP, rho);
-  const double cf = sqz<false>(fabs(0.5 * (c2 + dvz<false>(BP, rho) + sqz<false>(sq(X) - dvz<false>(4 * c2 * sq(Bn), rho)))));
+  const double X = c2 + quot(BP, rho);
+  const double cf = sqrt(fabs(0.5 * (c2 + quot(BP, rho) + sqrt(sq(X) - quot(4 * c2 * sq(Bn), rho)))));
   amax = un + cf;
   amin = un - cf;
 }
@@ -218,9 +305,9 @@ GDF_HD void fast_speeds(const Phys& P, const double* U, int dir, double& amax, d
 // HLLC_Flux.f90:9-106 and HLLD_Flux.f90:14-189 share the first stage.
 // dir 0 = normal x (reference direction 1), 1 = normal y (direction 2).
 // Fh gets the flux, Ust the star state (Ustar of the reference).
-template <bool HLLD, bool ZF = false>
+template <bool HLLD, class DIV>
 GDF_HD void hllcd_flux(const Phys& P, const Side& R, const Side& L, const double* FR, const double* FL, double SR,
-                       double SL, int dir, double* Fh, double* Ust) {
+                       double SL, int dir, double* Fh, double* Ust, unsigned& bad) {
   if (SR < 0) {
 #pragma unroll
     for (int n = 0; n < NE; ++n) { Fh[n] = FR[n]; Ust[n] = R.U[n]; }
@@ -234,20 +321,23 @@ GDF_HD void hllcd_flux(const Phys& P, const Side& R, const Side& L, const double
   const double* UR1 = R.U;
   const double* UL1 = L.U;
   double Us[NE];
+  const auto rS = DIV::by(SR - SL, bad);
 #pragma unroll
-  for (int n = 0; n < NE; ++n) Us[n] = dvz<ZF>(SR * UR1[n] - SL * UL1[n] + FL[n] - FR[n], SR - SL);
+  for (int n = 0; n < NE; ++n) Us[n] = DIV::div(SR * UR1[n] - SL * UL1[n] + FL[n] - FR[n], rS, bad);
   const double rhoR = R.rho, u1R = R.u, u2R = R.v, u3R = R.w, ER = R.E;
   const double B1R = R.B1, B2R = R.B2, B3R = R.B3;
   const double rhoL = L.rho, u1L = L.u, u2L = L.v, u3L = L.w, EL = L.E;
   const double B1L = L.B1, B2L = L.B2, B3L = L.B3;
-  const double Sstar = dvz<ZF>(dir == 0 ? Us[1] : Us[2], Us[0]);
+  const double Sstar = DIV::div(dir == 0 ? Us[1] : Us[2], DIV::by(Us[0], bad), bad);
   const double uRbot = dir == 0 ? u1R : u2R, uLbot = dir == 0 ? u1L : u2L;
   const double BRbot = dir == 0 ? B1R : B2R, BLbot = dir == 0 ? B1L : B2L;
   const double Bsb = dir == 0 ? Us[5] : Us[6];
   const double dR = SR - uRbot, dL = SL - uLbot;      // (SR - uRbot), (SL - uLbot)
   const double eR = SR - Sstar, eL = SL - Sstar;      // (SR - Sstar), (SL - Sstar)
-  const double rhoRs = dvz<ZF>(rhoR * dR, eR);
-  const double rhoLs = dvz<ZF>(rhoL * dL, eL);
+  const auto reR = DIV::by(eR, bad), reL = DIV::by(eL, bad);
+  const double rhoRs = DIV::div(rhoR * dR, reR, bad);
+  const double rhoLs = DIV::div(rhoL * dL, reL, bad);
+  const auto rrR = DIV::by(rhoRs, bad), rrL = DIV::by(rhoLs, bad);
   const double PtotR = P.gamma1 * (ER - 0.5 * rhoR * (sq(u1R) + sq(u2R) + sq(u3R)));
   const double PtotL = P.gamma1 * (EL - 0.5 * rhoL * (sq(u1L) + sq(u2L) + sq(u3L)));
   const double PtotRs = PtotR + rhoR * dR * (Sstar - uRbot) + sq(Bsb) - sq(BRbot);
@@ -255,48 +345,49 @@ GDF_HD void hllcd_flux(const Phys& P, const Side& R, const Side& L, const double
   double B1Rs, B1Ls, B2Rs, B2Ls, B3Rs, B3Ls;
   double SRs = 0, SLs = 0;
   if (HLLD) {
-    SRs = Sstar + sqz<ZF>(dvz<ZF>(sq(Bsb), rhoRs));
-    SLs = Sstar - sqz<ZF>(dvz<ZF>(sq(Bsb), rhoLs));
+    SRs = Sstar + DIV::root(DIV::div(sq(Bsb), rrR, bad));
+    SLs = Sstar - DIV::root(DIV::div(sq(Bsb), rrL, bad));
     const double AR = rhoR * sq(dR) - Bsb * BRbot;
     const double AL = rhoL * sq(dL) - Bsb * BLbot;
     const double CR = rhoR * dR * (BRbot - Bsb);
     const double CL = rhoL * dL * (BLbot - Bsb);
     const double DR = rhoR * dR * eR - sq(Bsb) + 1e-15;
     const double DL = rhoL * dL * eL - sq(Bsb) + 1e-15;
+    const auto rDR = DIV::by(DR, bad), rDL = DIV::by(DL, bad);
     if (dir == 0) {
       B1Rs = Bsb; B1Ls = Bsb;
-      B2Rs = dvz<ZF>(AR * B2R + CR * u2R, DR);
-      B2Ls = dvz<ZF>(AL * B2L + CL * u2L, DL);
+      B2Rs = DIV::div(AR * B2R + CR * u2R, rDR, bad);
+      B2Ls = DIV::div(AL * B2L + CL * u2L, rDL, bad);
     } else {
-      B1Rs = dvz<ZF>(AR * B1R + CR * u1R, DR);
-      B1Ls = dvz<ZF>(AL * B1L + CL * u1L, DL);
+      B1Rs = DIV::div(AR * B1R + CR * u1R, rDR, bad);
+      B1Ls = DIV::div(AL * B1L + CL * u1L, rDL, bad);
       B2Rs = Bsb; B2Ls = Bsb;
     }
-    B3Rs = dvz<ZF>(AR * B3R + CR * u3R, DR);
-    B3Ls = dvz<ZF>(AL * B3L + CL * u3L, DL);
+    B3Rs = DIV::div(AR * B3R + CR * u3R, rDR, bad);
+    B3Ls = DIV::div(AL * B3L + CL * u3L, rDL, bad);
   } else {
     B1Rs = Us[5]; B1Ls = Us[5]; B2Rs = Us[6]; B2Ls = Us[6]; B3Rs = Us[7]; B3Ls = Us[7];
   }
   double URs[NE], ULs[NE];
   if (dir == 0) {
-    URs[1] = dvz<ZF>(UR1[1] * dR + PtotRs - PtotR + BRbot * B1R - Bsb * B1Rs, eR);
-    URs[2] = dvz<ZF>(UR1[2] * dR + BRbot * B2R - Bsb * B2Rs, eR);
-    ULs[1] = dvz<ZF>(UL1[1] * dL + PtotLs - PtotL + BLbot * B1L - Bsb * B1Ls, eL);
-    ULs[2] = dvz<ZF>(UL1[2] * dL + BLbot * B2L - Bsb * B2Ls, eL);
+    URs[1] = DIV::div(UR1[1] * dR + PtotRs - PtotR + BRbot * B1R - Bsb * B1Rs, reR, bad);
+    URs[2] = DIV::div(UR1[2] * dR + BRbot * B2R - Bsb * B2Rs, reR, bad);
+    ULs[1] = DIV::div(UL1[1] * dL + PtotLs - PtotL + BLbot * B1L - Bsb * B1Ls, reL, bad);
+    ULs[2] = DIV::div(UL1[2] * dL + BLbot * B2L - Bsb * B2Ls, reL, bad);
   } else {
-    URs[1] = dvz<ZF>(UR1[1] * dR + BRbot * B1R - Bsb * B1Rs, eR);
-    URs[2] = dvz<ZF>(UR1[2] * dR + PtotRs - PtotR + BRbot * B2R - Bsb * B2Rs, eR);
-    ULs[1] = dvz<ZF>(UL1[1] * dL + BLbot * B1L - Bsb * B1Ls, eL);
-    ULs[2] = dvz<ZF>(UL1[2] * dL + PtotLs - PtotL + BLbot * B2L - Bsb * B2Ls, eL);
+    URs[1] = DIV::div(UR1[1] * dR + BRbot * B1R - Bsb * B1Rs, reR, bad);
+    URs[2] = DIV::div(UR1[2] * dR + PtotRs - PtotR + BRbot * B2R - Bsb * B2Rs, reR, bad);
+    ULs[1] = DIV::div(UL1[1] * dL + BLbot * B1L - Bsb * B1Ls, reL, bad);
+    ULs[2] = DIV::div(UL1[2] * dL + PtotLs - PtotL + BLbot * B2L - Bsb * B2Ls, reL, bad);
   }
-  URs[3] = dvz<ZF>(UR1[3] * dR + BRbot * B3R - Bsb * B3Rs, eR);
-  ULs[3] = dvz<ZF>(UL1[3] * dL + BLbot * B3L - Bsb * B3Ls, eL);
-  const double u1Rs = dvz<ZF>(URs[1], rhoRs), u2Rs = dvz<ZF>(URs[2], rhoRs), u3Rs = dvz<ZF>(URs[3], rhoRs);
-  const double u1Ls = dvz<ZF>(ULs[1], rhoLs), u2Ls = dvz<ZF>(ULs[2], rhoLs), u3Ls = dvz<ZF>(ULs[3], rhoLs);
-  const double ERs = dvz<ZF>(dR * ER - PtotR * uRbot + PtotRs * Sstar + BRbot * (u1R * B1R + u2R * B2R + u3R * B3R) -
-                            Bsb * (u1Rs * B1Rs + u2Rs * B2Rs + u3Rs * B3Rs), eR);
-  const double ELs = dvz<ZF>(dL * EL - PtotL * uLbot + PtotLs * Sstar + BLbot * (u1L * B1L + u2L * B2L + u3L * B3L) -
-                            Bsb * (u1Ls * B1Ls + u2Ls * B2Ls + u3Ls * B3Ls), eL);
+  URs[3] = DIV::div(UR1[3] * dR + BRbot * B3R - Bsb * B3Rs, reR, bad);
+  ULs[3] = DIV::div(UL1[3] * dL + BLbot * B3L - Bsb * B3Ls, reL, bad);
+  const double u1Rs = DIV::div(URs[1], rrR, bad), u2Rs = DIV::div(URs[2], rrR, bad), u3Rs = DIV::div(URs[3], rrR, bad);
+  const double u1Ls = DIV::div(ULs[1], rrL, bad), u2Ls = DIV::div(ULs[2], rrL, bad), u3Ls = DIV::div(ULs[3], rrL, bad);
+  const double ERs = DIV::div(dR * ER - PtotR * uRbot + PtotRs * Sstar + BRbot * (u1R * B1R + u2R * B2R + u3R * B3R) -
+                            Bsb * (u1Rs * B1Rs + u2Rs * B2Rs + u3Rs * B3Rs), reR, bad);
+  const double ELs = DIV::div(dL * EL - PtotL * uLbot + PtotLs * Sstar + BLbot * (u1L * B1L + u2L * B2L + u3L * B3L) -
+                            Bsb * (u1Ls * B1Ls + u2Ls * B2Ls + u3Ls * B3Ls), reL, bad);
   URs[0] = rhoRs; URs[4] = ERs;
   ULs[0] = rhoLs; ULs[4] = ELs;
 #pragma unroll
@@ -313,14 +404,14 @@ GDF_HD void hllcd_flux(const Phys& P, const Side& R, const Side& L, const double
       // second stage (HLLD_Flux.f90:134-176)
       const double sL = sqrt(fabs(rhoLs)), sR = sqrt(fabs(rhoRs));
       const double sg = sgn1(Bsb);
-      const double den = sL + sR;
-      const double u1ss = dvz<ZF>(sL * u1Ls + sR * u1Rs + sg * (B1Rs - B1Ls), den);
-      const double u2ss = dvz<ZF>(sL * u2Ls + sR * u2Rs + sg * (B2Rs - B2Ls), den);
-      const double u3ss = dvz<ZF>(sL * u3Ls + sR * u3Rs + sg * (B3Rs - B3Ls), den);
+      const auto rden = DIV::by(sL + sR, bad);
+      const double u1ss = DIV::div(sL * u1Ls + sR * u1Rs + sg * (B1Rs - B1Ls), rden, bad);
+      const double u2ss = DIV::div(sL * u2Ls + sR * u2Rs + sg * (B2Rs - B2Ls), rden, bad);
+      const double u3ss = DIV::div(sL * u3Ls + sR * u3Rs + sg * (B3Rs - B3Ls), rden, bad);
       const double sLR = sqrt(fabs(rhoLs * rhoRs));
-      const double B1ss = dvz<ZF>(sL * B1Ls + sR * B1Rs + sg * sLR * (u1Rs - u1Ls), den);
-      const double B2ss = dvz<ZF>(sL * B2Ls + sR * B2Rs + sg * sLR * (u2Rs - u2Ls), den);
-      const double B3ss = dvz<ZF>(sL * B3Ls + sR * B3Rs + sg * sLR * (u3Rs - u3Ls), den);
+      const double B1ss = DIV::div(sL * B1Ls + sR * B1Rs + sg * sLR * (u1Rs - u1Ls), rden, bad);
+      const double B2ss = DIV::div(sL * B2Ls + sR * B2Rs + sg * sLR * (u2Rs - u2Ls), rden, bad);
+      const double B3ss = DIV::div(sL * B3Ls + sR * B3Rs + sg * sLR * (u3Rs - u3Ls), rden, bad);
       if (Sstar > 0) {
         const double ELss = ELs - sL * (u1Ls * B1Ls + u2Ls * B2Ls + u3Ls * B3Ls - u1ss * B1ss - u2ss * B2ss -
                                         u3ss * B3ss) * sg;
@@ -358,9 +449,9 @@ GDF_HD void hllcd_flux(const Phys& P, const Side& R, const Side& L, const double
 // reference's UL1), uR = +normal side (UR1); dir 0 = x, 1 = y. Writes the
 // numerical flux Fh and returns the fluxes of both sides in fL / fR and the
 // normal velocities of both sides in unL / unR (used by the face Ez).
-template <bool ZF = false>
-GDF_HD void face_flux_sides(const Phys& P, const Side& L, const Side& R, int dir, double* Fh, double* fL,
-                            double* fR) {
+template <class DIV>
+GDF_HD void face_flux_sides(const Phys& P, const SideOf<DIV>& L, const SideOf<DIV>& R, int dir, double* Fh, double* fL,
+                            double* fR, unsigned& bad) {
   if (dir == 0) {
     side_flux_x(L, fL, false);
     side_flux_x(R, fR, !P.kml_w);
@@ -369,8 +460,8 @@ GDF_HD void face_flux_sides(const Phys& P, const Side& L, const Side& R, int dir
     side_flux_y(P, R, fR, true);
   }
   double a1, a2, b1, b2;
-  side_speeds<ZF>(P, L, dir, a1, a2);   // SRmax/SRmin of the reference (from UR(i) = left side)
-  side_speeds<ZF>(P, R, dir, b1, b2);   // SLmax/SLmin (from UL(i+1) = right side)
+  side_speeds(P, L, dir, a1, a2, bad);   // SRmax/SRmin of the reference (from UR(i) = left side)
+  side_speeds(P, R, dir, b1, b2, bad);   // SLmax/SLmin (from UL(i+1) = right side)
   const double SR = fmax2(a1, b1);
   const double SL = fmin2(a2, b2);
   double Ust[NE];
@@ -386,43 +477,49 @@ GDF_HD void face_flux_sides(const Phys& P, const Side& L, const Side& R, int dir
 #pragma unroll
       for (int n = 0; n < NE; ++n) Fh[n] = fL[n];
     } else {
-      const double den = SR - SL, sls = SL * SR;
+      const auto rS = DIV::by(SR - SL, bad);
+      const double sls = SL * SR;
 #pragma unroll
-      for (int n = 0; n < NE; ++n) Fh[n] = dvz<ZF>(SR * fL[n] - SL * fR[n] + sls * (R.U[n] - L.U[n]), den);
+      for (int n = 0; n < NE; ++n) Fh[n] = DIV::div(SR * fL[n] - SL * fR[n] + sls * (R.U[n] - L.U[n]), rS, bad);
     }
   } else if (P.flux == 3) {
-    hllcd_flux<false, ZF>(P, R, L, fR, fL, SR, SL, dir, Fh, Ust);
+    hllcd_flux<false, DIV>(P, R, L, fR, fL, SR, SL, dir, Fh, Ust, bad);
   } else {
-    hllcd_flux<true, ZF>(P, R, L, fR, fL, SR, SL, dir, Fh, Ust);
+    hllcd_flux<true, DIV>(P, R, L, fR, fL, SR, SL, dir, Fh, Ust, bad);
   }
 }
 
 GDF_HD void face_flux(const Phys& P, const double* uL, const double* uR, int dir, double* Fh, double* fL,
                       double* fR) {
-  Side L, R;
-  make_side(P, uL, L);
-  make_side(P, uR, R);
-  face_flux_sides(P, L, R, dir, Fh, fL, fR);
+  SideOf<IeeeDiv> L, R;
+  unsigned any = 0;
+  make_side(P, uL, L, any);
+  make_side(P, uR, R, any);
+  face_flux_sides(P, L, R, dir, Fh, fL, fR, any);
 }
 
 // ------------------------------------------------------ 2-D vertex Ez -----
 // HLL1.f90:1-15 restricted to what the vertex solver reads: component k of
 // the HLL state and component m of the HLL flux.
+template <class DIV>
 GDF_HD void hll1_cm(const double* UR, const double* UL, const double* FR, const double* FL, double SR, double SL,
-                    int k, int m, double& uk, double& fm) {
+                    int k, int m, double& uk, double& fm, unsigned& bad) {
   if (SR < 0) {
     uk = UR[k]; fm = FR[m];
   } else if (SL > 0) {
     uk = UL[k]; fm = FL[m];
   } else {
-    fm = dvz<false>(SR * FL[m] - SL * FR[m] + SL * SR * (UR[m] - UL[m]), SR - SL);
-    uk = dvz<false>(SR * UR[k] - SL * UL[k] - (FR[k] - FL[k]), SR - SL);
+    const auto rS = DIV::by(SR - SL, bad);
+    fm = DIV::div(SR * FL[m] - SL * FR[m] + SL * SR * (UR[m] - UL[m]), rS, bad);
+    uk = DIV::div(SR * UR[k] - SL * UL[k] - (FR[k] - FL[k]), rS, bad);
   }
 }
 
 // LhEz.f90:50-69 for one vertex: states in the four quadrants around it
 // (RU = upper right, ...). LF_Flux_2D.f90, HLL_Flux_2D.f90, HLLC/HLLD_Flux_2D.f90.
-GDF_HD double vertex_ez(const Phys& P, const double* URU, const double* ULU, const double* URD, const double* ULD) {
+template <class DIV>
+GDF_HD double vertex_ez(const Phys& P, const double* URU, const double* ULU, const double* URD, const double* ULD,
+                        unsigned& bad) {
   if (P.flux == 1) {
     const double ax = fmax2(fmax2(fmax2(fabs(URU[1] / URU[0]), fabs(ULU[1] / ULU[0])), fabs(URD[1] / URD[0])),
                             fabs(ULD[1] / ULD[0]));
@@ -436,20 +533,20 @@ GDF_HD double vertex_ez(const Phys& P, const double* URU, const double* ULU, con
     return 0.25 * (EzRU + EzLU + EzRD + EzLD) - 0.25 * ay * (0.5 * (URU[5] + ULU[5]) - 0.5 * (URD[5] + ULD[5])) +
            0.25 * ax * (0.5 * (URU[6] + URD[6]) - 0.5 * (ULU[6] + ULD[6]));
   }
-  Side sRU, sLU, sRD, sLD;
-  make_side(P, URU, sRU);
-  make_side(P, ULU, sLU);
-  make_side(P, URD, sRD);
-  make_side(P, ULD, sLD);
+  SideOf<DIV> sRU, sLU, sRD, sLD;
+  make_side(P, URU, sRU, bad);
+  make_side(P, ULU, sLU, bad);
+  make_side(P, URD, sRD, bad);
+  make_side(P, ULD, sLD, bad);
   double axRU, bxRU, ayRU, byRU, axLU, bxLU, ayLU, byLU, axRD, bxRD, ayRD, byRD, axLD, bxLD, ayLD, byLD;
-  side_speeds(P, sRU, 0, axRU, bxRU);
-  side_speeds(P, sRU, 1, ayRU, byRU);
-  side_speeds(P, sLU, 0, axLU, bxLU);
-  side_speeds(P, sLU, 1, ayLU, byLU);
-  side_speeds(P, sRD, 0, axRD, bxRD);
-  side_speeds(P, sRD, 1, ayRD, byRD);
-  side_speeds(P, sLD, 0, axLD, bxLD);
-  side_speeds(P, sLD, 1, ayLD, byLD);
+  side_speeds(P, sRU, 0, axRU, bxRU, bad);
+  side_speeds(P, sRU, 1, ayRU, byRU, bad);
+  side_speeds(P, sLU, 0, axLU, bxLU, bad);
+  side_speeds(P, sLU, 1, ayLU, byLU, bad);
+  side_speeds(P, sRD, 0, axRD, bxRD, bad);
+  side_speeds(P, sRD, 1, ayRD, byRD, bad);
+  side_speeds(P, sLD, 0, axLD, bxLD, bad);
+  side_speeds(P, sLD, 1, ayLD, byLD, bad);
   const double SR = fmax2(fmax2(fmax2(axRU, axLU), axRD), axLD);
   const double SL = fmin2(fmin2(fmin2(bxRU, bxLU), bxRD), bxLD);
   const double SU = fmax2(fmax2(fmax2(ayRU, ayLU), ayRD), ayLD);
@@ -462,10 +559,10 @@ GDF_HD double vertex_ez(const Phys& P, const double* URU, const double* ULU, con
   double EzRs, EzLs, EzUs, EzDs;
   if (P.flux == 2) {
     double BxUs, BxDs, ByRs, ByLs, fU7, fD7;
-    hll1_cm(URU, ULU, FxRU, FxLU, SR, SL, 5, 6, BxUs, fU7);
-    hll1_cm(URD, ULD, FxRD, FxLD, SR, SL, 5, 6, BxDs, fD7);
-    hll1_cm(URU, URD, FyRU, FyRD, SU, SD, 6, 5, ByRs, EzRs);
-    hll1_cm(ULU, ULD, FyLU, FyLD, SU, SD, 6, 5, ByLs, EzLs);
+    hll1_cm<DIV>(URU, ULU, FxRU, FxLU, SR, SL, 5, 6, BxUs, fU7, bad);
+    hll1_cm<DIV>(URD, ULD, FxRD, FxLD, SR, SL, 5, 6, BxDs, fD7, bad);
+    hll1_cm<DIV>(URU, URD, FyRU, FyRD, SU, SD, 6, 5, ByRs, EzRs, bad);
+    hll1_cm<DIV>(ULU, ULD, FyLU, FyLD, SU, SD, 6, 5, ByLs, EzLs, bad);
     EzUs = -fU7;
     EzDs = -fD7;
     if (SL > 0) return EzLs;
@@ -478,18 +575,19 @@ GDF_HD double vertex_ez(const Phys& P, const double* URU, const double* ULU, con
     const double BxRU = URU[5], BxLU = ULU[5], BxRD = URD[5], BxLD = ULD[5];
     const double ByRU = URU[6], ByLU = ULU[6], ByRD = URD[6], ByLD = ULD[6];
     const double den = 2 * (SR - SL) * (SU - SD);
-    const double BxSS = dvz<false>(2 * SR * SU * BxRU - 2 * SL * SU * BxLU + 2 * SL * SD * BxLD - 2 * SR * SD * BxRD -
-                               SR * (z - z) + SL * (z - z) - (SR - SL) * (EzUs - EzDs), den);
-    const double BySS = dvz<false>(2 * SR * SU * ByRU - 2 * SL * SU * ByLU + 2 * SL * SD * ByLD - 2 * SR * SD * ByRD +
-                               SU * (z - z) - SD * (z - z) + (SU - SD) * (EzRs - EzLs), den);
+    const auto rden = DIV::by(den, bad);
+    const double BxSS = DIV::div(2 * SR * SU * BxRU - 2 * SL * SU * BxLU + 2 * SL * SD * BxLD - 2 * SR * SD * BxRD -
+                               SR * (z - z) + SL * (z - z) - (SR - SL) * (EzUs - EzDs), rden, bad);
+    const double BySS = DIV::div(2 * SR * SU * ByRU - 2 * SL * SU * ByLU + 2 * SL * SD * ByLD - 2 * SR * SD * ByRD +
+                               SU * (z - z) - SD * (z - z) + (SU - SD) * (EzRs - EzLs), rden, bad);
     return 0.25 * (EzRs + EzLs + EzUs + EzDs) - 0.25 * SU * (BxUs - BxSS) - 0.25 * SD * (BxDs - BxSS) +
            0.25 * SR * (ByRs - BySS) + 0.25 * SL * (ByLs - BySS);
   }
   // HLLC / HLLD vertex solvers: four 1-D solves, plain average for Ez**
   double Fh[NE], Us[NE];
   auto solve = [&](const Side& r, const Side& l, const double* Fr, const double* Fl, double sr, double sl, int dir) {
-    if (P.flux == 3) hllcd_flux<false>(P, r, l, Fr, Fl, sr, sl, dir, Fh, Us);
-    else hllcd_flux<true>(P, r, l, Fr, Fl, sr, sl, dir, Fh, Us);
+    if (P.flux == 3) hllcd_flux<false, DIV>(P, r, l, Fr, Fl, sr, sl, dir, Fh, Us, bad);
+    else hllcd_flux<true, DIV>(P, r, l, Fr, Fl, sr, sl, dir, Fh, Us, bad);
   };
   solve(sRU, sLU, FxRU, FxLU, SR, SL, 0);
   EzUs = -Fh[6];
@@ -504,6 +602,11 @@ GDF_HD double vertex_ez(const Phys& P, const double* URU, const double* ULU, con
   if (SD > 0) return EzDs;
   if (SU < 0) return EzUs;
   return 0.25 * (EzRs + EzLs + EzUs + EzDs);
+}
+
+GDF_HD double vertex_ez(const Phys& P, const double* URU, const double* ULU, const double* URD, const double* ULD) {
+  unsigned any = 0;
+  return vertex_ez<IeeeDiv>(P, URU, ULU, URD, ULD, any);
 }
 
 // ------------------------------------------------------- eigenmatrix ------
@@ -569,12 +672,12 @@ GDF_HD void eigen_right(int dir, const EigFrame& f, double rho, double u1, doubl
     const double sqpr = sqrt(fabs(p)) / rho;
     const double sqpor = sqrt(fabs(p / rho));
     const double sq1og = sqrt(1.0 / gm);
-    const double b1s = dvz<false>(B1, rhosq), b2s = dvz<false>(B2, rhosq), b3s = dvz<false>(B3, rhosq);
+    const double b1s = quot(B1, rhosq), b2s = quot(B2, rhosq), b3s = quot(B3, rhosq);
     const double bN = dir == 0 ? b1s : b2s;
     const double d = a2 + (sq(b1s) + sq(b2s) + sq(b3s));
     const double disc = sqrt(fabs(sq(d) - 4.0 * a2 * sq(bN)));
-    const double cf = sqz<false>(0.5 * fabs(d + disc));
-    const double cs = sqz<false>(0.5 * fabs(d - disc));
+    const double cf = sqrt(0.5 * fabs(d + disc));
+    const double cs = sqrt(0.5 * fabs(d - disc));
     const double bNsum = dir == 0 ? ((b1s + b2s * 0.0) + b3s * 0.0) : ((b1s * 0.0 + b2s) + b3s * 0.0);
     const double beta1 = sgn1(bNsum * 1.0);
     double alphaf, alphas;
@@ -582,9 +685,9 @@ GDF_HD void eigen_right(int dir, const EigFrame& f, double rho, double u1, doubl
       alphaf = 0x1.6a09e667f3bccp-1;
       alphas = 0x1.6a09e667f3bcdp-1;
     } else {
-      const double den = sqz<false>(fabs(cf * cf - cs * cs));
-      alphaf = dvz<false>(sqz<false>(fabs(a2 - cs * cs)), den);
-      alphas = dvz<false>(sqz<false>(fabs(cf * cf - a2)), den);
+      const double den = sqrt(fabs(cf * cf - cs * cs));
+      alphaf = quot(sqrt(fabs(a2 - cs * cs)), den);
+      alphas = quot(sqrt(fabs(cf * cf - a2)), den);
     }
     const double bst = (b1s * t1 + b2s * t2 + b3s * t3);
     const double rc = rhosq * cf;
@@ -609,9 +712,9 @@ GDF_HD void eigen_right(int dir, const EigFrame& f, double rho, double u1, doubl
       const double m1 = dir == 0 ? (afa2 + asa * (bst - bN * t1)) : (asa * (-(bN * t1)));
       const double m2 = dir == 1 ? (afa2 + asa * (bst - bN * t2)) : (asa * (-(bN * t2)));
       const double m3 = asa * (-(bN * t3));
-      ru[1][4] = dvz<false>(sqg2 * m1, rc);
-      ru[2][4] = dvz<false>(sqg2 * m2, rc);
-      ru[3][4] = dvz<false>(sqg2 * m3, rc);
+      ru[1][4] = quot(sqg2 * m1, rc);
+      ru[2][4] = quot(sqg2 * m2, rc);
+      ru[3][4] = quot(sqg2 * m3, rc);
     }
     ru[0][4] = sqg2 * alphaf * rhosq;
     ru[4][4] = sqg2 * alphaf * rhosq * a2;
@@ -625,9 +728,9 @@ GDF_HD void eigen_right(int dir, const EigFrame& f, double rho, double u1, doubl
       const double k1 = dir == 0 ? (alphaf * cf2 * t1 + a * alphas * bN) : (alphaf * cf2 * t1);
       const double k2 = dir == 1 ? (alphaf * cf2 * t2 + alphas * a * bN) : (alphaf * cf2 * t2);
       const double k3 = alphaf * cf2 * t3;
-      ru[1][6] = dvz<false>(bs * k1, rc);
-      ru[2][6] = dvz<false>(bs * k2, rc);
-      ru[3][6] = dvz<false>(bs * k3, rc);
+      ru[1][6] = quot(bs * k1, rc);
+      ru[2][6] = quot(bs * k2, rc);
+      ru[3][6] = quot(bs * k3, rc);
     }
     ru[0][6] = sqg2 * alphas * rhosq;
     ru[4][6] = sq(a) * sqg2 * alphas * rhosq;
@@ -649,15 +752,15 @@ GDF_HD void eigen_right(int dir, const EigFrame& f, double rho, double u1, doubl
     const double k2 = sq(u1) + sq(u2) + sq(u3);
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
-      R[0 + 8 * m] = dvz<false>(ru[0][m], g1);
-      R[1 + 8 * m] = dvz<false>(ru[0][m] * u1 + ru[1][m] * rho, g1);
-      R[2 + 8 * m] = dvz<false>(ru[0][m] * u2 + ru[2][m] * rho, g1);
-      R[3 + 8 * m] = dvz<false>(ru[0][m] * u3 + ru[3][m] * rho, g1);
-      R[4 + 8 * m] = dvz<false>(dvz<false>(ru[4][m], g1) + B1 * ru[5][m] + B2 * ru[6][m] + B3 * ru[7][m] + 0.5 * ru[0][m] * k2 +
+      R[0 + 8 * m] = quot(ru[0][m], g1);
+      R[1 + 8 * m] = quot(ru[0][m] * u1 + ru[1][m] * rho, g1);
+      R[2 + 8 * m] = quot(ru[0][m] * u2 + ru[2][m] * rho, g1);
+      R[3 + 8 * m] = quot(ru[0][m] * u3 + ru[3][m] * rho, g1);
+      R[4 + 8 * m] = quot(quot(ru[4][m], g1) + B1 * ru[5][m] + B2 * ru[6][m] + B3 * ru[7][m] + 0.5 * ru[0][m] * k2 +
                             ru[1][m] * u1 * rho + ru[2][m] * u2 * rho + ru[3][m] * u3 * rho, g1);
-      R[5 + 8 * m] = dvz<false>(ru[5][m], g1);
-      R[6 + 8 * m] = dvz<false>(ru[6][m], g1);
-      R[7 + 8 * m] = dvz<false>(ru[7][m], g1);
+      R[5 + 8 * m] = quot(ru[5][m], g1);
+      R[6 + 8 * m] = quot(ru[6][m], g1);
+      R[7 + 8 * m] = quot(ru[7][m], g1);
     }
   }
 }
@@ -670,21 +773,21 @@ GDF_HD void eigen_left(int dir, const EigFrame& f, double rho, double u1, double
     const double rhosq = sqrt(rho);
     const double a2 = fabs(gm * p / rho);
     const double a = sqrt(a2);
-    const double b1s = dvz<false>(B1, rhosq), b2s = dvz<false>(B2, rhosq), b3s = dvz<false>(B3, rhosq);
+    const double b1s = quot(B1, rhosq), b2s = quot(B2, rhosq), b3s = quot(B3, rhosq);
     const double BNs = dir == 0 ? b1s : b2s;
     const double BN = dir == 0 ? B1 : B2;
     const double d = a2 + (sq(b1s) + sq(b2s) + sq(b3s));
     const double disc = sqrt(fabs(sq(d) - 4.0 * a2 * sq(BNs)));
-    const double cf = sqz<false>(0.5 * fabs(d + disc));
-    const double cs = sqz<false>(0.5 * fabs(d - disc));
+    const double cf = sqrt(0.5 * fabs(d + disc));
+    const double cs = sqrt(0.5 * fabs(d - disc));
     double alphaf, alphas;
     if (fabs(cf * cf - cs * cs) <= 1.0e-12) {
       alphaf = 0x1.6a09e667f3bccp-1;
       alphas = 0x1.6a09e667f3bcdp-1;
     } else {
-      const double den = sqz<false>(fabs(cf * cf - cs * cs));
-      alphaf = dvz<false>(sqz<false>(fabs(a2 - cs * cs)), den);
-      alphas = dvz<false>(sqz<false>(fabs(cf * cf - a2)), den);
+      const double den = sqrt(fabs(cf * cf - cs * cs));
+      alphaf = quot(sqrt(fabs(a2 - cs * cs)), den);
+      alphas = quot(sqrt(fabs(cf * cf - a2)), den);
     }
     const double twosq = sqrt(2.0);
     // sign(1, BNs*1): BNs summed as (b1s*n1 + b2s*n2) + b3s*n3 so that the
@@ -705,30 +808,30 @@ GDF_HD void eigen_left(int dir, const EigFrame& f, double rho, double u1, double
     const double nen = dir == 0 ? (sq(t2) + sq(t3)) : (sq(t1) + sq(t3));
     const double nen2 = a * gu1sq * nen;
     if (dir == 0) {
-      lu[1][5] = dvz<false>(sq(t2) + sq(t3), nen2);
-      lu[1][6] = dvz<false>(-(t2 * t1), nen2);
-      lu[1][7] = dvz<false>(-(t1 * t3), nen2);
+      lu[1][5] = quot(sq(t2) + sq(t3), nen2);
+      lu[1][6] = quot(-(t2 * t1), nen2);
+      lu[1][7] = quot(-(t1 * t3), nen2);
     } else {
-      lu[1][5] = dvz<false>(-(t1 * t2), nen2);
-      lu[1][6] = dvz<false>(sq(t1) + sq(t3), nen2);
-      lu[1][7] = dvz<false>(-(t2 * t3), nen2);
+      lu[1][5] = quot(-(t1 * t2), nen2);
+      lu[1][6] = quot(sq(t1) + sq(t3), nen2);
+      lu[1][7] = quot(-(t2 * t3), nen2);
     }
     const double nen3 = sqrt(2.0) * sqrt(fabs(p)) * nen;
     const double nen31 = nen3 / sqrt(fabs(rho));
-    lu[2][1] = dvz<false>(rho * (-TxN1), nen3);
-    lu[2][2] = dvz<false>(rho * (-TxN2), nen3);
-    lu[2][3] = dvz<false>(rho * (-TxN3), nen3);
-    lu[2][5] = dvz<false>(TxN1, nen31);
-    lu[2][6] = dvz<false>(TxN2, nen31);
-    lu[2][7] = dvz<false>(TxN3, nen31);
+    lu[2][1] = quot(rho * (-TxN1), nen3);
+    lu[2][2] = quot(rho * (-TxN2), nen3);
+    lu[2][3] = quot(rho * (-TxN3), nen3);
+    lu[2][5] = quot(TxN1, nen31);
+    lu[2][6] = quot(TxN2, nen31);
+    lu[2][7] = quot(TxN3, nen31);
     const double cf2 = sq(cf);
     const double q = a * sq(BN) * sq(alphas) + rhosq * cf2 * alphaf * (a * rhosq * alphaf + BT * alphas);
     const double nen51 = twosq * a * nen * gu1sq * q;
     const double nen52 = twosq * a * gu1sq * (sq(alphaf) + sq(alphas)) * nen;
     const double nen71 = twosq * beta1 * nen * gu1sq * q;
     const double rcf = rho * cf;
-    const double Term54 = dvz<false>(alphaf, twosq * sq(a) * gu1sq * rhosq * (sq(alphaf) + sq(alphas)));
-    const double Term74 = dvz<false>(alphas, twosq * sq(a) * gu1sq * rhosq * (sq(alphaf) + sq(alphas)));
+    const double Term54 = quot(alphaf, twosq * sq(a) * gu1sq * rhosq * (sq(alphaf) + sq(alphas)));
+    const double Term74 = quot(alphas, twosq * sq(a) * gu1sq * rhosq * (sq(alphaf) + sq(alphas)));
     // Term51..Term77 of eigenmatrix.f90:287-351 with the zero normal
     // components removed
     double T51, T52, T53, T55, T56, T57, T71, T72, T73, T75, T76, T77;
@@ -759,20 +862,20 @@ GDF_HD void eigen_left(int dir, const EigFrame& f, double rho, double u1, double
       T76 = 0.0;
       T77 = -alphaf * t3;
     }
-    lu[4][1] = dvz<false>(-T51, nen51);
-    lu[4][2] = dvz<false>(T52, nen51);
-    lu[4][3] = dvz<false>(T53, nen51);
+    lu[4][1] = quot(-T51, nen51);
+    lu[4][2] = quot(T52, nen51);
+    lu[4][3] = quot(T53, nen51);
     lu[4][4] = Term54;
-    lu[4][5] = dvz<false>(T55, nen52);
-    lu[4][6] = dvz<false>(T56, nen52);
-    lu[4][7] = dvz<false>(T57, nen52);
-    lu[6][1] = dvz<false>(T71, nen71);
-    lu[6][2] = dvz<false>(T72, nen71);
-    lu[6][3] = dvz<false>(T73, nen71);
+    lu[4][5] = quot(T55, nen52);
+    lu[4][6] = quot(T56, nen52);
+    lu[4][7] = quot(T57, nen52);
+    lu[6][1] = quot(T71, nen71);
+    lu[6][2] = quot(T72, nen71);
+    lu[6][3] = quot(T73, nen71);
     lu[6][4] = Term74;
-    lu[6][5] = dvz<false>(T75, nen52);
-    lu[6][6] = dvz<false>(T76, nen52);
-    lu[6][7] = dvz<false>(T77, nen52);
+    lu[6][5] = quot(T75, nen52);
+    lu[6][6] = quot(T76, nen52);
+    lu[6][7] = quot(T77, nen52);
 #pragma unroll
     for (int pr = 2; pr <= 6; pr += 2) {
       lu[pr + 1][0] = lu[pr][0];
@@ -789,10 +892,10 @@ GDF_HD void eigen_left(int dir, const EigFrame& f, double rho, double u1, double
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
       const double* l = lu[m];
-      L[m + 8 * 0] = l[0] * g1 - dvz<false>(l[1] * u1 * g1, rho) - dvz<false>(l[2] * u2 * g1, rho) - dvz<false>(l[3] * u3 * g1, rho) + l[4] * g12 * k2 * .5;
-      L[m + 8 * 1] = -l[4] * u1 * g12 + dvz<false>(l[1] * g1, rho);
-      L[m + 8 * 2] = -l[4] * u2 * g12 + dvz<false>(l[2] * g1, rho);
-      L[m + 8 * 3] = -l[4] * u3 * g12 + dvz<false>(l[3] * g1, rho);
+      L[m + 8 * 0] = l[0] * g1 - quot(l[1] * u1 * g1, rho) - quot(l[2] * u2 * g1, rho) - quot(l[3] * u3 * g1, rho) + l[4] * g12 * k2 * .5;
+      L[m + 8 * 1] = -l[4] * u1 * g12 + quot(l[1] * g1, rho);
+      L[m + 8 * 2] = -l[4] * u2 * g12 + quot(l[2] * g1, rho);
+      L[m + 8 * 3] = -l[4] * u3 * g12 + quot(l[3] * g1, rho);
       L[m + 8 * 4] = l[4] * g12;
       L[m + 8 * 5] = l[5] * g1 - B1 * l[4] * g12;
       L[m + 8 * 6] = l[6] * g1 - B2 * l[4] * g12;

@@ -74,6 +74,7 @@ struct K3 {
   int bc_r, bc_l, bc_u, bc_d;
   Phys P;
   BasisP3 B;
+  double rmm[NP3];   // RN(1 / mm)
 };
 
 struct Scal3 {
@@ -169,21 +170,6 @@ __device__ __forceinline__ void trace3(const K3& K, const double* __restrict__ U
     for (int d = 0; d < NP3; ++d) {
       const int s = slot3(n, d);
       if (s >= 0) acc = acc + __ldg(&U[c + K.plane * s]) * phi[d];
-    }
-    out[n] = acc;
-  }
-}
-
-// the same from a thread's copy of its cell's 84 slots in shared memory
-// (slot s at sm[s * 64])
-__device__ __forceinline__ void trace3s(const double* sm, const double* phi, double* out) {
-#pragma unroll
-  for (int n = 0; n < NE; ++n) {
-    double acc = 0.0;
-#pragma unroll
-    for (int d = 0; d < NP3; ++d) {
-      const int s = slot3(n, d);
-      if (s >= 0) acc = acc + sm[s * 64] * phi[d];
     }
     out[n] = acc;
   }
@@ -346,30 +332,38 @@ __global__ void __launch_bounds__(128) k3_vertex(const __grid_constant__ K3 K, c
 // ------------------------------------------------------------------ cells --
 // du of one interior cell: each du(d, n) is one chain of additions in the
 // reference's order (volume points i1 then j1, x faces, y faces, then the
-// mass matrix), held in registers; then the stage's combination.
-// GDF_P3_CELL_SMEM: each thread first copies its cell's 84 slots to shared
-// memory and evaluates the 25 points from there (same values)
-#ifndef GDF_P3_CELL_SMEM
-#define GDF_P3_CELL_SMEM 0
-#endif
-constexpr size_t CELL_SMEM = GDF_P3_CELL_SMEM ? (size_t)NS3 * 64 * sizeof(double) : 0;
+// mass matrix), held in registers (160 of them, which is what keeps the kernel
+// at 8 warps per SM); then the stage's combination. The cell's 84 slots are
+// staged in shared memory two by two (slot s at sm[2*(64*(s/2) + thread) +
+// s%2]) and read there at the 25 points, a pair per 128-bit load. Products
+// with the structural zeros of the derivative basis and of the fluxes' own B
+// components contribute +-0 and are left out; the face basis is the same on both
+// faces up to the sign of the modes odd across them, and 1 for mode 1; u, v, w
+// share a reciprocal and the mass matrix has known ones.
+// 480 x 240: 254 us per launch, 286 with every slot read through L1 at every
+// point and none of the sharing.
+__device__ constexpr bool px3_zero(int d) { return d == 0 || d == 2 || d == 5 || d == 9; }
+__device__ constexpr bool py3_zero(int d) { return d == 0 || d == 1 || d == 3 || d == 6; }
+// modes odd across an x face (1, 4, 6, 8) and across a y face (2, 4, 7, 9)
+__device__ constexpr bool odd3(int d, bool x) {
+  return x ? (d == 1 || d == 4 || d == 6 || d == 8) : (d == 2 || d == 4 || d == 7 || d == 9);
+}
 
 template <int KIND>
 __global__ void __launch_bounds__(64) k3_cell(const __grid_constant__ K3 K, double* __restrict__ U,
                                               double* __restrict__ T, double* __restrict__ UII,
                                               const double* __restrict__ Fxh, const double* __restrict__ Fyh,
                                               const Scal3* __restrict__ sc) {
+  __shared__ __align__(16) double sm[NS3 * 64];
   if (sc && !sc->active) return;
   const long long item = gtid();
   if (item >= (long long)K.nx * K.ny) return;
   const int i = (int)(item % K.nx) + 1, j = (int)(item / K.nx) + 1;
   const long long c = i + (long long)K.nx2 * j;
-#if GDF_P3_CELL_SMEM
-  extern __shared__ double cell_sm[];
-  double* my = cell_sm + threadIdx.x;
-#pragma unroll 4
-  for (int q = 0; q < NS3; ++q) my[q * 64] = U[c + K.plane * q];
-#endif
+  const int tid = threadIdx.x;
+#pragma unroll 12
+  for (int q = 0; q < NS3; q += 2)
+    reinterpret_cast<double2*>(sm)[64 * (q >> 1) + tid] = make_double2(U[c + K.plane * q], U[c + K.plane * (q + 1)]);
   double du[NQ3][NE];
 #pragma unroll
   for (int d = 0; d < NQ3; ++d)
@@ -380,20 +374,45 @@ __global__ void __launch_bounds__(64) k3_cell(const __grid_constant__ K3 K, doub
   for (int a = 0; a < NG; ++a)
 #pragma unroll 1
     for (int b = 0; b < NG; ++b) {
+      const double* f = K.B.phiG[a][b];
       double uG[NE];
-#if GDF_P3_CELL_SMEM
-      trace3s(my, K.B.phiG[a][b], uG);
-#else
-      trace3(K, U, c, K.B.phiG[a][b], uG);
-#endif
-      gdf::SideOf<SharedRcp> s;
-      unsigned bad = 0;
-      gdf::make_side(K.P, uG, s, bad);
-      if (bad) {
-        gdf::SideOf<IeeeDiv> e;
-        gdf::make_side(K.P, uG, e, bad);
-        static_cast<Side&>(s) = e;
+#pragma unroll
+      for (int n = 0; n < NE; ++n) {
+        // a variable's slots are consecutive, its first ten modes, then (Bx,
+        // By) modes 11 and 14 or 12 and 15
+        double m[12];
+#pragma unroll
+        for (int k = 0; k < (n == 5 || n == 6 ? 12 : 10); k += 2) {
+          const double2 t = reinterpret_cast<const double2*>(sm)[64 * ((slot3(n, 0) + k) >> 1) + tid];
+          m[k] = t.x;
+          m[k + 1] = t.y;
+        }
+        double acc = 0.0 + m[0];
+#pragma unroll
+        for (int d = 1; d < NP3; ++d) {
+          const int s = slot3(n, d);
+          if (s >= 0) acc = acc + m[s >= 0 ? s - slot3(n, 0) : 0] * f[d];
+        }
+        uG[n] = acc;
       }
+      Side s;
+      s.rho = uG[0];
+      unsigned bad = 0;
+      const gdf::Rcp rr = gdf::rcp_of(s.rho, bad);
+      s.u = gdf::rdiv(uG[1], rr, bad);
+      s.v = gdf::rdiv(uG[2], rr, bad);
+      s.w = gdf::rdiv(uG[3], rr, bad);
+      if (bad) {   // an operand out of rdiv's range: the IEEE division itself
+        s.u = uG[1] / s.rho;
+        s.v = uG[2] / s.rho;
+        s.w = uG[3] / s.rho;
+      }
+      s.E = uG[4];
+      s.B1 = uG[5];
+      s.B2 = uG[6];
+      s.B3 = uG[7];
+      s.BB = sq(s.B1) + sq(s.B2) + sq(s.B3);
+      s.p = K.P.gamma1 * (s.E - 0.5 * s.rho * (sq(s.u) + sq(s.v) + sq(s.w)) - 0.5 * s.BB);
       double Fx[NE], Fy[NE];
       flux3<0>(s, Fx);
       flux3<1>(s, Fy);
@@ -402,52 +421,63 @@ __global__ void __launch_bounds__(64) k3_cell(const __grid_constant__ K3 K, doub
       for (int d = 1; d < NQ3; ++d) {
         const double px = K.B.phixG[a][b][d], py = K.B.phiyG[a][b][d];
 #pragma unroll
-        for (int n = 0; n < NE; ++n) du[d][n] = du[d][n] + wab * (Fx[n] * px + Fy[n] * py);
+        for (int n = 0; n < NE; ++n) {
+          const bool hx = n != 5 && !px3_zero(d), hy = n != 6 && !py3_zero(d);
+          if (hx && hy) du[d][n] = du[d][n] + wab * (Fx[n] * px + Fy[n] * py);
+          else if (hx) du[d][n] = du[d][n] + wab * (Fx[n] * px);
+          else if (hy) du[d][n] = du[d][n] + wab * (Fy[n] * py);
+        }
       }
     }
-  // surface integrals (main.f90:2232-2258): x faces of the cell, then y faces
+  // surface integrals (main.f90:2232-2258): x faces of the cell, then y faces;
+  // F1 the flux on the high face, F0 on the low one
+  auto surface = [&](const double* F1, const double* F0, double cw, const double* f, bool x) {
+#pragma unroll
+    for (int n = 0; n < NE; ++n) {
+      du[0][n] = du[0][n] - cw * (F1[n] - F0[n]);
+#pragma unroll
+      for (int d = 1; d < NQ3; ++d) {
+        const double h = F1[n] * f[d], l = F0[n] * f[d];
+        du[d][n] = du[d][n] - cw * (odd3(d, x) ? h + l : h - l);
+      }
+    }
+  };
   {
     const long long fr = i + (long long)(K.nx + 1) * (j - 1), fl = fr - 1;
 #pragma unroll 1
     for (int g = 0; g < NG; ++g) {
-      const double cw = K.cxs * K.B.weight[g];
       double Fr[NE], Fl[NE];
 #pragma unroll
       for (int n = 0; n < NE; ++n) {
         Fr[n] = Fxh[(long long)(g * NE + n) * K.fxplane + fr];
         Fl[n] = Fxh[(long long)(g * NE + n) * K.fxplane + fl];
       }
-#pragma unroll
-      for (int d = 0; d < NQ3; ++d) {
-        const double pr = K.B.phiGR[g][d], pl = K.B.phiGL[g][d];
-#pragma unroll
-        for (int n = 0; n < NE; ++n) du[d][n] = du[d][n] - cw * (Fr[n] * pr - Fl[n] * pl);
-      }
+      surface(Fr, Fl, K.cxs * K.B.weight[g], K.B.phiGR[g], true);
     }
   }
   {
     const long long fu = (i - 1) + (long long)K.nx * j, fd = fu - K.nx;
 #pragma unroll 1
     for (int g = 0; g < NG; ++g) {
-      const double cw = K.cys * K.B.weight[g];
       double Fu[NE], Fd[NE];
 #pragma unroll
       for (int n = 0; n < NE; ++n) {
         Fu[n] = Fyh[(long long)(g * NE + n) * K.fyplane + fu];
         Fd[n] = Fyh[(long long)(g * NE + n) * K.fyplane + fd];
       }
-#pragma unroll
-      for (int d = 0; d < NQ3; ++d) {
-        const double pu = K.B.phiGU[g][d], pd = K.B.phiGD[g][d];
-#pragma unroll
-        for (int n = 0; n < NE; ++n) du[d][n] = du[d][n] - cw * (Fu[n] * pu - Fd[n] * pd);
-      }
+      surface(Fu, Fd, K.cys * K.B.weight[g], K.B.phiGU[g], false);
     }
   }
+  // the mass matrix (mm(1) = 1), by its reciprocals
 #pragma unroll
-  for (int d = 0; d < NQ3; ++d)
+  for (int n = 0; n < NE; ++n) {
+    unsigned bad = 0;
+    double q[NQ3];
 #pragma unroll
-    for (int n = 0; n < NE; ++n) du[d][n] = du[d][n] / K.B.mm[d];
+    for (int d = 1; d < NQ3; ++d) q[d] = gdf::rdiv(du[d][n], gdf::Rcp{K.B.mm[d], K.rmm[d]}, bad);
+#pragma unroll
+    for (int d = 1; d < NQ3; ++d) du[d][n] = bad ? du[d][n] / K.B.mm[d] : q[d];
+  }
   // the stage's combination over the 84 live slots (du = 0 beyond mode 10)
   const double c6 = KIND == KIND_LH ? 0.0 : sc->c6;
   const double c10 = KIND == KIND_LAST ? sc->c10 : 0.0;
@@ -1056,6 +1086,7 @@ void build_k3(const GdfP3Config& c, K3& K) {
   K.P.eig_identity = 0;      // this eigenmatrix has no identity fallback
   gdf::set_eig_consts(K.P);
   build_basis_p3(hx1, hy1, &K.B);
+  for (int d = 0; d < NP3; ++d) K.rmm[d] = 1.0 / K.B.mm[d];
 }
 
 template <class F>
@@ -1086,27 +1117,27 @@ int launch_lh_body(GdfP3Handle* h, int kind, const Scal3* sc) {
   return run(h, [&] {
     switch (kind) {
       case KIND_LH:
-        k3_cell<KIND_LH><<<nc, 64, CELL_SMEM, h->st>>>(K, h->U, h->T, h->UII, h->Fxh, h->Fyh, sc);
+        k3_cell<KIND_LH><<<nc, 64, 0, h->st>>>(K, h->U, h->T, h->UII, h->Fxh, h->Fyh, sc);
         k3_bface<KIND_LH><<<nf, 128, 0, h->st>>>(K, h->Fxh, h->Fyh, h->EzV, h->BX, h->BXT, h->BXII, h->BY, h->BYT,
                                                   h->BYII, sc);
         break;
       case KIND_FIRST:
-        k3_cell<KIND_FIRST><<<nc, 64, CELL_SMEM, h->st>>>(K, h->U, h->T, h->UII, h->Fxh, h->Fyh, sc);
+        k3_cell<KIND_FIRST><<<nc, 64, 0, h->st>>>(K, h->U, h->T, h->UII, h->Fxh, h->Fyh, sc);
         k3_bface<KIND_FIRST><<<nf, 128, 0, h->st>>>(K, h->Fxh, h->Fyh, h->EzV, h->BX, h->BXT, h->BXII, h->BY,
                                                      h->BYT, h->BYII, sc);
         break;
       case KIND_STAGE:
-        k3_cell<KIND_STAGE><<<nc, 64, CELL_SMEM, h->st>>>(K, h->U, h->T, h->UII, h->Fxh, h->Fyh, sc);
+        k3_cell<KIND_STAGE><<<nc, 64, 0, h->st>>>(K, h->U, h->T, h->UII, h->Fxh, h->Fyh, sc);
         k3_bface<KIND_STAGE><<<nf, 128, 0, h->st>>>(K, h->Fxh, h->Fyh, h->EzV, h->BX, h->BXT, h->BXII, h->BY,
                                                      h->BYT, h->BYII, sc);
         break;
       case KIND_FIVE:
-        k3_cell<KIND_FIVE><<<nc, 64, CELL_SMEM, h->st>>>(K, h->U, h->T, h->UII, h->Fxh, h->Fyh, sc);
+        k3_cell<KIND_FIVE><<<nc, 64, 0, h->st>>>(K, h->U, h->T, h->UII, h->Fxh, h->Fyh, sc);
         k3_bface<KIND_FIVE><<<nf, 128, 0, h->st>>>(K, h->Fxh, h->Fyh, h->EzV, h->BX, h->BXT, h->BXII, h->BY,
                                                     h->BYT, h->BYII, sc);
         break;
       default:
-        k3_cell<KIND_LAST><<<nc, 64, CELL_SMEM, h->st>>>(K, h->U, h->T, h->UII, h->Fxh, h->Fyh, sc);
+        k3_cell<KIND_LAST><<<nc, 64, 0, h->st>>>(K, h->U, h->T, h->UII, h->Fxh, h->Fyh, sc);
         k3_bface<KIND_LAST><<<nf, 128, 0, h->st>>>(K, h->Fxh, h->Fyh, h->EzV, h->BX, h->BXT, h->BXII, h->BY,
                                                     h->BYT, h->BYII, sc);
         break;

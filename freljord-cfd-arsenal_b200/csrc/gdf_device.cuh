@@ -74,11 +74,6 @@ __device__ __forceinline__ void set_bc_item(const Consts& K, double* __restrict_
   U[off + i + (long long)K.nx2 * j] = v;
 }
 
-// k_cell asks for its faces' fluxes in L2 before its volume loop
-#ifndef GDF_CELL_PREFETCH
-#define GDF_CELL_PREFETCH 1
-#endif
-
 // Products with the exact 1 and -1 entries of the basis tables written as
 // the value itself (x * 1 == x, x * -1 == -x for every double)
 #ifndef GDF_FOLD_UNIT
@@ -250,78 +245,42 @@ __device__ __forceinline__ void vertex_item(const Consts& K, const double* __res
 // du = 0, as Lh leaves them). stage 0 writes du instead (gdf_lh).
 constexpr int CELL_BS = 64;
 
-// The residual kernels read their staged modes in pairs, one 128-bit
-// shared-memory load per two modes: blast 2048^2 step 45.6 against 46.5 ms,
-// same values (GDF_CELL_PAIRS=0: one 64-bit load per mode).
-#ifndef GDF_CELL_PAIRS
-#define GDF_CELL_PAIRS 1
-#endif
+// A thread's 52 staged modes, two by two at ms[2*(CELL_BS*(k/2) + tid) + k%2]
+// (one 128-bit load per pair).
+constexpr int CELL_SLOTS = NLIVE;
 
-// ms: the block's NLIVE * CELL_BS staging array (blockDim.x == CELL_BS).
-// PAIRS: ms holds the live slots in pairs (2L, 2L+1) per thread, 16-byte
-// aligned, and the volume loop reads a pair with one 128-bit load (ms must
-// then be 16-byte aligned). SHFL: the x-face fluxes are loaded once per face:
-// each lane reads its cell's right face and takes its left face, the right
-// face of cell i-1, from the lane below by a warp shuffle (lane 0 reads its
-// own); every lane of the warp must then call with consecutive items, valid
-// or not (valid = false: a lane past the array's end, no work). Both leave
-// every value and the order of every sum as they are.
-template <bool SHFL = false, bool PAIRS = false>
+// The point values and fluxes of the volume term take a third of the residual's
+// operations, the 52 sums du the rest: they hold 104 registers, which is what
+// keeps the kernel at 8 warps per SM. Sums keep the reference's order (the 25
+// points with b fastest, then x faces, then y faces, then the mass matrix); what
+// is shared between points or modes is shared before a sum, never across one: a face flux times lambda
+// (modes 3 and 5, or 2 and 5) or times P2 (modes 6 and 9, or 4 and 8), one
+// reciprocal per point for u, v, w, known reciprocals for the mass matrix.
+// Blast 2048^2: 5.66 ms per launch, 5.95-6.05 before; rotor
+// 512^2 366 us, 387 before. (Keeping a column's parts in shared memory as well:
+// 6.47 ms; forming the next point's values beside this one's primitives: 6.67.)
+// ms: the block's CELL_SLOTS * CELL_BS doubles, 16-byte aligned (blockDim.x ==
+// CELL_BS).
 __device__ __forceinline__ void cell_item(const Consts& K, const double* __restrict__ U, double* __restrict__ U0,
                                           double* __restrict__ UI, const double* __restrict__ Fxh,
                                           const double* __restrict__ Fyh, double* __restrict__ duout,
-                                          const Scal* __restrict__ sc, int stage, long long item, double* ms,
-                                          bool valid = true) {
+                                          const Scal* __restrict__ sc, int stage, long long item, double* ms) {
   const int tid = threadIdx.x;
   const int i = (int)(item % K.nx2);
   const int j = (int)(item / K.nx2);
-  const bool interior = valid && i >= 1 && i <= K.nx && j >= 1 && j <= K.ny;
-  auto msi = [&](int L) { return PAIRS ? ((L >> 1) * CELL_BS + tid) * 2 + (L & 1) : L * CELL_BS + tid; };
+  const bool interior = i >= 1 && i <= K.nx && j >= 1 && j <= K.ny;
+  auto at = [&](int k) -> double& { return ms[2 * (CELL_BS * (k >> 1) + tid) + (k & 1)]; };
+  auto pair = [&](int k) { return reinterpret_cast<const double2*>(ms)[CELL_BS * (k >> 1) + tid]; };   // k even
   double du[NLIVE];
 #pragma unroll
   for (int k = 0; k < NLIVE; ++k) du[k] = 0.0;
-  // Lh.f90:268-304 for variable n from the fluxes of the cell's four faces
-  auto surface = [&](int n, const double* fr, const double* fl, const double* fu, const double* fd) {
-#pragma unroll
-    for (int d = 0; d < NP; ++d) {
-      if (!live_mode(n, d)) continue;
-      double acc = du[LI(n, d)];
-      // at the middle point (lambda = 0) the face basis of modes 3, 5, 8,
-      // 10 (x faces) and 2, 5, 9, 7 (y faces) vanishes on both sides
-#pragma unroll
-      for (int g = 0; g < NG; ++g) {
-        if (g == 2 && (d == 2 || d == 4 || d == 7 || d == 9)) continue;
-        // modes 1 and 2 of the x-face basis are 1 on the right face and
-        // +-1 on the left (get_basis.f90): x * 1 and x * -1 are exact, so
-        // those products are written out
-        const double t = (GDF_FOLD_UNIT && d == 0) ? fr[g] - fl[g]
-                         : (GDF_FOLD_UNIT && d == 1) ? fr[g] - (-fl[g])
-                                                     : fr[g] * c_basis.phiGR[g][d] - fl[g] * c_basis.phiGL[g][d];
-        acc = acc - K.cxs * c_basis.w[g] * t;
-      }
-#pragma unroll
-      for (int g = 0; g < NG; ++g) {
-        if (g == 2 && (d == 1 || d == 4 || d == 8 || d == 6)) continue;
-        // modes 1 and 3 of the y-face basis: 1 on the upper face, +-1 on
-        // the lower
-        const double t = (GDF_FOLD_UNIT && d == 0) ? fu[g] - fd[g]
-                         : (GDF_FOLD_UNIT && d == 2) ? fu[g] - (-fd[g])
-                                                     : fu[g] * c_basis.phiGU[g][d] - fd[g] * c_basis.phiGD[g][d];
-        acc = acc - K.cys * c_basis.w[g] * t;
-      }
-      // mm(1) = 1 (get_basis.f90): x / 1 == x
-      du[LI(n, d)] = (GDF_FOLD_UNIT && d == 0) ? acc
-                     : (n == 3 || n == 7)     ? dv(acc, c_basis.mm[d])
-                                              : acc / c_basis.mm[d];
-    }
-  };
   if (interior) {
 #pragma unroll
     for (int n = 0; n < NE; ++n)
 #pragma unroll
       for (int d = 0; d < NP; ++d)
-        if (live_mode(n, d)) ms[msi(LI(n, d))] = U[item + K.plane * (d + 10 * n)];
-    if (GDF_CELL_PREFETCH) {
+        if (live_mode(n, d)) at(LI(n, d)) = U[item + K.plane * (d + 10 * n)];
+    {
       // the surface term reads the fluxes of the cell's four faces after the
       // volume loop: ask for them in L2 now, so the loads that follow the
       // volume work do not wait on DRAM
@@ -339,33 +298,33 @@ __device__ __forceinline__ void cell_item(const Consts& K, const double* __restr
     for (int a = 0; a < NG; ++a) {
 #pragma unroll 1
       for (int b = 0; b < NG; ++b) {
+        const double* f = c_basis.phiG[a][b];
         double v[NE];
 #pragma unroll
         for (int n = 0; n < NE; ++n) {
-          double acc = 0.0;
-          double mv[8];
-          if (PAIRS) {
-            const int nl = (n == 5 || n == 6) ? 8 : 6;
+          double m[8];
+          const int nl = (n == 5 || n == 6) ? 8 : 6;
 #pragma unroll
-            for (int k = 0; k < 8; k += 2)
-              if (k < nl) {
-                const double2 q = reinterpret_cast<const double2*>(ms)[((LI(n, 0) + k) >> 1) * CELL_BS + tid];
-                mv[k] = q.x;
-                mv[k + 1] = q.y;
-              }
+          for (int k = 0; k < nl; k += 2) {
+            const double2 q = pair(LI(n, 0) + k);
+            m[k] = q.x;
+            m[k + 1] = q.y;
           }
+          double acc = 0.0 + m[0];
 #pragma unroll
-          for (int d = 0; d < NP; ++d) {
-            if (!live_mode(n, d)) continue;
-            const double m = PAIRS ? mv[LI(n, d) - LI(n, 0)] : ms[LI(n, d) * CELL_BS + tid];
-            // mode 1 of the volume basis is 1 at every point: m * 1 == m
-            if (GDF_FOLD_UNIT && d == 0) acc = acc + m;
-            else acc = acc + m * c_basis.phiG[a][b][d];
-          }
+          for (int d = 1; d < NP; ++d)
+            if (live_mode(n, d)) acc = acc + m[LI(n, d) - LI(n, 0)] * f[d];
           v[n] = acc;
         }
         const double rho = v[0];
-        const double u = v[1] / rho, vv = v[2] / rho, w = dv(v[3], rho);   // rho w = 0 in 2-D runs
+        unsigned bad = 0;
+        const Rcp rr = rcp_of(rho, bad);
+        double u = rdiv(v[1], rr, bad), vv = rdiv(v[2], rr, bad), w = rdiv(v[3], rr, bad);
+        if (bad) {   // an operand out of rdiv's range: the IEEE division itself
+          u = v[1] / rho;
+          vv = v[2] / rho;
+          w = v[3] / rho;
+        }
         const double E = v[4], B1 = v[5], B2 = v[6], B3 = v[7];
         const double BB = sq(B1) + sq(B2) + sq(B3);
         const double p = K.P.gamma1 * (E - 0.5 * rho * (sq(u) + sq(vv) + sq(w)) - 0.5 * BB);
@@ -409,50 +368,81 @@ __device__ __forceinline__ void cell_item(const Consts& K, const double* __restr
           }
       }
     }
-    if (!SHFL) {
-      // surface terms in the reference order (x faces, then y faces), mass
-      const long long ox = (i - 1) + 1 + (long long)(K.nx + 1) * (j - 1);  // Fxhat(i,j)
-      const long long oy = (i - 1) + (long long)K.nx * j;                  // Fyhat(i,j)
+    // surface terms in the reference order (x faces, then y faces), mass.
+    // q1 the flux on the high face, q0 on the low one; the face basis is the
+    // same on both up to the sign of the modes odd in the face's direction
+    // (get_basis.f90), 1 for mode 1, +-1 for the slope across the face, and at
+    // the middle point zero for the modes odd along it.
+    const long long ox = (i - 1) + 1 + (long long)(K.nx + 1) * (j - 1);  // Fxhat(i,j)
+    const long long oy = (i - 1) + (long long)K.nx * j;                  // Fyhat(i,j)
+    // the next variable's fluxes are asked for before this one's sums
+    double nr[NG], nl[NG], nu[NG], nd[NG];
+    auto load = [&](int n) {
 #pragma unroll
-      for (int n = 0; n < NE; ++n) {
-        double fr[NG], fl[NG], fu[NG], fd[NG];
-#pragma unroll
-        for (int g = 0; g < NG; ++g) {
-          fr[g] = Fxh[(n * NG + g) * K.fxplane + ox];
-          fl[g] = Fxh[(n * NG + g) * K.fxplane + ox - 1];
-          fu[g] = Fyh[(n * NG + g) * K.fyplane + oy];
-          fd[g] = Fyh[(n * NG + g) * K.fyplane + oy - K.nx];
-        }
-        surface(n, fr, fl, fu, fd);
+      for (int g = 0; g < NG; ++g) {
+        nr[g] = Fxh[(n * NG + g) * K.fxplane + ox];
+        nl[g] = Fxh[(n * NG + g) * K.fxplane + ox - 1];
+        nu[g] = Fyh[(n * NG + g) * K.fyplane + oy];
+        nd[g] = Fyh[(n * NG + g) * K.fyplane + oy - K.nx];
       }
-    }
-  }
-  if (SHFL) {
-    // the right x face of every cell of rows 1..ny with i <= nx (ghost
-    // column 0 included: its right face is the left face of cell 1)
-    const bool has_r = valid && j >= 1 && j <= K.ny && i <= K.nx;
-    const long long ox = i + (long long)(K.nx + 1) * (j - 1);  // Fxhat(i,j)
-    const long long oy = (i - 1) + (long long)K.nx * j;        // Fyhat(i,j)
-    const bool own_l = (threadIdx.x & 31) == 0;
+    };
+    load(0);
 #pragma unroll
     for (int n = 0; n < NE; ++n) {
-      double fr[NG], fl[NG], fu[NG], fd[NG];
-#pragma unroll
-      for (int g = 0; g < NG; ++g) fr[g] = has_r ? Fxh[(n * NG + g) * K.fxplane + ox] : 0.0;
-#pragma unroll
-      for (int g = 0; g < NG; ++g) fl[g] = __shfl_up_sync(0xffffffffu, fr[g], 1);
-      if (interior) {
+      auto faces = [&](const double* q1, const double* q0, const double* cw, const double (*f)[NP], bool x) {
+        const int across = x ? 1 : 2, along = x ? 2 : 1, across2 = x ? 3 : 5, along2 = x ? 5 : 3;
 #pragma unroll
         for (int g = 0; g < NG; ++g) {
-          if (own_l) fl[g] = Fxh[(n * NG + g) * K.fxplane + ox - 1];
-          fu[g] = Fyh[(n * NG + g) * K.fyplane + oy];
-          fd[g] = Fyh[(n * NG + g) * K.fyplane + oy - K.nx];
+          const double c = cw[g];
+          auto add = [&](int d, double t) { du[LI(n, d)] = du[LI(n, d)] - c * t; };
+          add(0, q1[g] - q0[g]);
+          add(across, q1[g] + q0[g]);
+          add(across2, q1[g] * f[g][across2] - q0[g] * f[g][across2]);
+          const double s1 = q1[g] * f[g][along2], s0 = q0[g] * f[g][along2];
+          add(along2, s1 - s0);
+          if (g != 2) {
+            const double l1 = q1[g] * f[g][along], l0 = q0[g] * f[g][along];
+            add(along, l1 - l0);
+            add(4, l1 + l0);
+          }
+          // cubic modes: Bx's 7 and 9, By's 8 and 10
+          if (n == 5) {
+            if (x) {
+              add(6, q1[g] * f[g][6] + q0[g] * f[g][6]);
+              add(8, s1 + s0);
+            } else if (g != 2) {
+              add(6, q1[g] * f[g][6] - q0[g] * f[g][6]);
+              add(8, q1[g] * f[g][8] - q0[g] * f[g][8]);
+            }
+          }
+          if (n == 6) {
+            if (!x) {
+              add(7, s1 + s0);
+              add(9, q1[g] * f[g][9] + q0[g] * f[g][9]);
+            } else if (g != 2) {
+              add(7, q1[g] * f[g][7] - q0[g] * f[g][7]);
+              add(9, q1[g] * f[g][9] - q0[g] * f[g][9]);
+            }
+          }
         }
-        surface(n, fr, fl, fu, fd);
-      }
+      };
+      double fr[NG], fl[NG], fu[NG], fd[NG];
+#pragma unroll
+      for (int g = 0; g < NG; ++g) { fr[g] = nr[g]; fl[g] = nl[g]; fu[g] = nu[g]; fd[g] = nd[g]; }
+      if (n + 1 < NE) load(n + 1);
+      faces(fr, fl, K.cxw, c_basis.phiGR, true);
+      faces(fu, fd, K.cyw, c_basis.phiGU, false);
+      // mm(1) = 1 (get_basis.f90): x / 1 == x
+      unsigned bad = 0;
+      double q[NP];
+#pragma unroll
+      for (int d = 1; d < NP; ++d)
+        if (live_mode(n, d)) q[d] = rdiv(du[LI(n, d)], Rcp{c_basis.mm[d], c_basis.rmm[d]}, bad);
+#pragma unroll
+      for (int d = 1; d < NP; ++d)
+        if (live_mode(n, d)) du[LI(n, d)] = bad ? du[LI(n, d)] / c_basis.mm[d] : q[d];
     }
   }
-  if (!valid) return;
   if (stage == 0) {
     if (interior) {
 #pragma unroll
@@ -466,16 +456,24 @@ __device__ __forceinline__ void cell_item(const Consts& K, const double* __restr
   // the stage's combination, a variable at a time: its loads are all under way
   // before its first store
   const double dt = sc->dt;
-#pragma unroll
-  for (int n = 0; n < NE; ++n) {
-    double a[NP], b[NP];
+  double na[NP], nb[NP];
+  auto fetch = [&](int n) {
 #pragma unroll
     for (int d = 0; d < NP; ++d) {
       if (!live_mode(n, d)) continue;
       const long long c = item + K.plane * (d + 10 * n);
-      a[d] = stage == 1 ? U[c] : UI[c];
-      b[d] = stage == 1 ? 0.0 : U0[c];
+      na[d] = stage == 1 ? U[c] : UI[c];
+      nb[d] = stage == 1 ? 0.0 : U0[c];
     }
+  };
+  fetch(0);
+#pragma unroll
+  for (int n = 0; n < NE; ++n) {
+    double a[NP], b[NP];
+#pragma unroll
+    for (int d = 0; d < NP; ++d)
+      if (live_mode(n, d)) { a[d] = na[d]; b[d] = nb[d]; }
+    if (n + 1 < NE) fetch(n + 1);
 #pragma unroll
     for (int d = 0; d < NP; ++d) {
       if (!live_mode(n, d)) continue;

@@ -54,13 +54,6 @@
 #ifndef GDF_CELL_MINB
 #define GDF_CELL_MINB 1
 #endif
-// k_cell reads its staged modes in pairs (GDF_CELL_PAIRS, in
-// gdf_device.cuh). GDF_CELL_SHFL=1 loads every x-face flux once and passes the left
-// face of a cell from the lane below by a warp shuffle: 12% slower k_cell
-// (246 registers, the surface loads taken out of the interior branch), off.
-#ifndef GDF_CELL_SHFL
-#define GDF_CELL_SHFL 0
-#endif
 #ifndef GDF_LIMIT_MINB
 #define GDF_LIMIT_MINB 1
 #endif
@@ -105,16 +98,11 @@ __global__ void __launch_bounds__(CELL_BS, GDF_CELL_MINB) k_cell(const __grid_co
                                                   double* __restrict__ U0, double* __restrict__ UI,
                                                   const double* __restrict__ Fxh, const double* __restrict__ Fyh,
                                                   double* __restrict__ duout, const Scal* __restrict__ sc, int stage) {
-  __shared__ __align__(16) double ms[NLIVE * CELL_BS];
+  __shared__ __align__(16) double ms[CELL_SLOTS * CELL_BS];
   if (sc && !sc->active) return;
   const long long item = gtid();
-  if (GDF_CELL_SHFL) {
-    // every lane takes part in the x-face shuffles, past the end too
-    cell_item<true, GDF_CELL_PAIRS != 0>(K, U, U0, UI, Fxh, Fyh, duout, sc, stage, item, ms, item < K.plane);
-    return;
-  }
   if (item >= K.plane) return;
-  cell_item<false, GDF_CELL_PAIRS != 0>(K, U, U0, UI, Fxh, Fyh, duout, sc, stage, item, ms);
+  cell_item(K, U, U0, UI, Fxh, Fyh, duout, sc, stage, item, ms);
 }
 
 __global__ void __launch_bounds__(128) k_bface(const __grid_constant__ Consts K, const double* __restrict__ EzRL,
@@ -552,7 +540,12 @@ static void build_consts(const GdfConfig& c, Consts& K) {
   const double lamL[NG] = {-1, -0.6546536707079771437983, 0, 0.654653670707977143798, 1};
   const double hx1 = K.hx1, hy1 = K.hy1;
   const double c13 = 1.0 / 3.0, c23 = 2.0 / 3.0, c25 = 2.0 / 5.0, c35 = 3.0 / 5.0;
-  for (int a = 0; a < NG; ++a) { K.w[a] = wt[a]; K.lam[a] = lam[a]; }
+  for (int a = 0; a < NG; ++a) {
+    K.w[a] = wt[a];
+    K.lam[a] = lam[a];
+    K.cxw[a] = K.cxs * wt[a];
+    K.cyw[a] = K.cys * wt[a];
+  }
   // get_basis.f90: Legendre tensor basis values and derivatives
   auto P2 = [&](double x) { return x * x - c13; };
   auto P3 = [&](double x) { return x * x * x - 3.0 * x / 5.0; };
@@ -637,6 +630,7 @@ void consts_for(const GdfConfig& c, Consts& K) { build_consts(c, K); }
 void basis_of(const Consts& K, Basis& B) {
   std::memcpy(B.w, K.w, sizeof(B.w));
   std::memcpy(B.lam, K.lam, sizeof(B.lam));
+  for (int q = 0; q < NG * NG; ++q) B.wq[q] = 0.25 * K.w[q / NG] * K.w[q % NG];
   std::memcpy(B.phiG, K.phiG, sizeof(B.phiG));
   std::memcpy(B.phiGLL, K.phiGLL, sizeof(B.phiGLL));
   std::memcpy(B.ppM, K.ppM, sizeof(B.ppM));
@@ -649,6 +643,7 @@ void basis_of(const Consts& K, Basis& B) {
   std::memcpy(B.phiRD, K.phiRD, sizeof(B.phiRD));
   std::memcpy(B.phiLD, K.phiLD, sizeof(B.phiLD));
   std::memcpy(B.mm, K.mm, sizeof(B.mm));
+  for (int d = 0; d < NP; ++d) B.rmm[d] = 1.0 / K.mm[d];
   std::memcpy(B.mmE, K.mmE, sizeof(B.mmE));
   std::memcpy(B.EzR, K.EzR, sizeof(B.EzR));
   std::memcpy(B.EzL, K.EzL, sizeof(B.EzL));

@@ -33,6 +33,7 @@ struct Consts {
   long long plane, fxplane, fyplane, vplane;
   double hx, hy, hx1, hy1;
   double cxs, cys;          // 0.5/hx, 0.5/hy (Lh.f90:275,291)
+  double cxw[NG], cyw[NG];  // the same times the weights
   double Mh2x, Mh2y;        // M*hx**2, M*hy**2 (minmod.f90:10)
   double Mh2x_b, Mh2y_b;    // minmodB bounds: M*hy**2 for Bx, M*hx**2 for By
   double rxy, ryx;          // hx/hy, hy/hx (div_free_Balsara.f90:36-37)
@@ -55,13 +56,13 @@ struct Consts {
 // one copy (gdf_device.cuh c_basis) that every kernel reads from constant
 // memory. Consts keeps its own copy for the host.
 struct Basis {
-  double w[NG], lam[NG];
+  double w[NG], lam[NG], wq[NG * NG];   // wq: 0.25 w(a) w(b)
   double phiG[NG][NG][NP];
   double phiGLL[2][NG][NG][NP];
   double ppM[NP];
   double phiGR[NG][NP], phiGL[NG][NP], phiGU[NG][NP], phiGD[NG][NP];
   double phiRU[NP], phiLU[NP], phiRD[NP], phiLD[NP];
-  double mm[NP];
+  double mm[NP], rmm[NP];   // rmm: RN(1 / mm)
   double mmE[3], EzR[3], EzL[3], EzU[3], EzD[3];
 };
 

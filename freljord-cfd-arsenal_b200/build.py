@@ -28,6 +28,7 @@ HOST_CXX = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
 KERNEL_SRC = os.path.join(CSRC, "gdf_kernels.cu")
 MLP_SRC = os.path.join(CSRC, "gdf_mlp.cu")
 ENS_SRC = os.path.join(CSRC, "gdf_ensemble.cu")
+STAGE_SRC = os.path.join(CSRC, "gdf_stage.cu")
 PEAK_SRC = os.path.join(CSRC, "gdf_peak.cu")
 INIT_SRC = os.path.join(CSRC, "gdf_init.cu")
 MLPTC_SRC = os.path.join(CSRC, "gdf_mlp_tc.cu")
@@ -37,7 +38,7 @@ HOST_SRC = os.path.join(CSRC, "gdf_host.cpp")
 IO_SRC = os.path.join(CSRC, "gdf_io.cpp")
 CYHOST_SRC = os.path.join(CSRC, "gdf_cy_host.cpp")
 HEADERS = [os.path.join(CSRC, f) for f in ("gdf_physics.cuh", "gdf_charlim.cuh", "gdf_kernels.cuh", "gdf_device.cuh",
-                                                         "gdf_mlp.cuh", "gdf_p3_basis.h")] + [
+                                                         "gdf_mlp.cuh", "gdf_p3_basis.h", "gdf_stage.h")] + [
     os.path.join(REPO, "include", "gdf.h"), os.path.join(REPO, "include", "gdf_p3.h"),
     os.path.join(REPO, "include", "gdf_cy.h")]
 
@@ -82,7 +83,7 @@ def build(verbose: bool = False, jobs: int | None = None) -> dict:
     for name, flags in (("libgdf_b200.so", ["--fmad=false", "-DGDF_EXACT=1"]),
                         ("libgdf_b200_fma.so", ["--fmad=true"])):
         objs = []
-        for src in (KERNEL_SRC, MLP_SRC, ENS_SRC, PEAK_SRC, INIT_SRC, MLPTC_SRC, P3_SRC, CY_SRC):
+        for src in (KERNEL_SRC, MLP_SRC, ENS_SRC, PEAK_SRC, INIT_SRC, MLPTC_SRC, P3_SRC, CY_SRC, STAGE_SRC):
             obj = os.path.join(BUILD, name.replace(".so", "") + "_" + os.path.basename(src).replace(".cu", ".o"))
             if _stale(obj, [src] + HEADERS):
                 cmd = [nvcc, *ARCH, "-lineinfo", "-O3", "-std=c++17", *flags,

@@ -39,6 +39,7 @@
 
 #include "../../include/gdf_cy.h"
 #include "gdf_charlim.cuh"
+#include "gdf_stage.h"
 
 namespace gdf {
 int set_last_error(int code, const char* msg);
@@ -1184,6 +1185,7 @@ __global__ void __launch_bounds__(128) k_cy_diag(const __grid_constant__ KC K, c
 using namespace gdfc;
 
 struct GdfCyHandle {
+  gdf::StageRef stage;
   GdfCyConfig cfg{};
   KC K{};
   cudaStream_t st = nullptr;
@@ -1483,20 +1485,25 @@ size_t bz_bytes(const KC& K) { return (size_t)K.nyf * 3 * sizeof(double); }
 
 // host uh (10 modes x 8 variables of full planes) -> the 54 live slots; the
 // slots the method keeps at zero must be zero
+// (consecutive live slots are consecutive planes on both sides: one copy a run)
 int upload_cells(GdfCyHandle* h, const double* uh, double* D) {
   const size_t pl = (size_t)h->K.ncp;
   for (int n = 0; n < NE; ++n)
-    for (int d = 0; d < NPC; ++d) {
+    for (int d = 0, e; d < NPC; d = e) {
       const double* src = uh + pl * (d + (size_t)NPC * n);
       const int s = slotc(n, d);
+      e = d + 1;
       if (s < 0) {
-        for (size_t q = 0; q < pl; ++q)
-          if (src[q] != 0.0)
-            return fail(GDF_ERR_ARG, "uh slot (d=" + std::to_string(d + 1) + ", n=" + std::to_string(n + 1) +
+        while (e < NPC && slotc(n, e) < 0) ++e;
+        if (gdf::par_any_nonzero(src, pl * (e - d)))
+          for (int k = d; k < e; ++k)
+            if (gdf::par_any_nonzero(src + pl * (k - d), pl))
+              return fail(GDF_ERR_ARG, "uh slot (d=" + std::to_string(k + 1) + ", n=" + std::to_string(n + 1) +
                                          ") must be zero: the cylindrical method never fills it");
         continue;
       }
-      CKC(cudaMemcpyAsync(D + pl * s, src, pl * sizeof(double), cudaMemcpyHostToDevice, h->st));
+      while (e < NPC && slotc(n, e) == s + (e - d)) ++e;
+      CKC(gdf::h2d(D + pl * s, src, pl * (e - d) * sizeof(double), h->st));
     }
   CKC(cudaStreamSynchronize(h->st));
   return GDF_OK;
@@ -1505,14 +1512,17 @@ int upload_cells(GdfCyHandle* h, const double* uh, double* D) {
 int download_cells(GdfCyHandle* h, const double* D, double* uh) {
   const size_t pl = (size_t)h->K.ncp;
   for (int n = 0; n < NE; ++n)
-    for (int d = 0; d < NPC; ++d) {
+    for (int d = 0, e; d < NPC; d = e) {
       double* dst = uh + pl * (d + (size_t)NPC * n);
       const int s = slotc(n, d);
+      e = d + 1;
       if (s < 0) {
-        std::memset(dst, 0, pl * sizeof(double));
+        while (e < NPC && slotc(n, e) < 0) ++e;
+        gdf::par_zero(dst, pl * (e - d) * sizeof(double));
         continue;
       }
-      CKC(cudaMemcpyAsync(dst, D + pl * s, pl * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+      while (e < NPC && slotc(n, e) == s + (e - d)) ++e;
+      CKC(gdf::d2h(dst, D + pl * s, pl * (e - d) * sizeof(double), h->st));
     }
   CKC(cudaStreamSynchronize(h->st));
   return GDF_OK;
@@ -1596,8 +1606,8 @@ int gdf_cy_upload(GdfCyHandle* h, const double* uh, const double* br, const doub
   if (!h || !uh || !br || !bz) return fail(GDF_ERR_ARG, "null argument");
   int rc = upload_cells(h, uh, h->U);
   if (rc) return rc;
-  CKC(cudaMemcpyAsync(h->BR, br, br_bytes(h->K), cudaMemcpyHostToDevice, h->st));
-  CKC(cudaMemcpyAsync(h->BZ, bz, bz_bytes(h->K), cudaMemcpyHostToDevice, h->st));
+  CKC(gdf::h2d(h->BR, br, br_bytes(h->K), h->st));
+  CKC(gdf::h2d(h->BZ, bz, bz_bytes(h->K), h->st));
   h->sc_host->t = 0;
   h->sc_host->dt = 0;
   h->sc_host->active = 1;
@@ -1614,8 +1624,8 @@ int gdf_cy_download(GdfCyHandle* h, double* uh, double* br, double* bz) {
   if (!h->uploaded) return fail(GDF_ERR_STATE, "no state uploaded");
   int rc = download_cells(h, h->U, uh);
   if (rc) return rc;
-  CKC(cudaMemcpyAsync(br, h->BR, br_bytes(h->K), cudaMemcpyDeviceToHost, h->st));
-  CKC(cudaMemcpyAsync(bz, h->BZ, bz_bytes(h->K), cudaMemcpyDeviceToHost, h->st));
+  CKC(gdf::d2h(br, h->BR, br_bytes(h->K), h->st));
+  CKC(gdf::d2h(bz, h->BZ, bz_bytes(h->K), h->st));
   CKC(cudaStreamSynchronize(h->st));
   return GDF_OK;
 }
@@ -1722,8 +1732,8 @@ int gdf_cy_lh(GdfCyHandle* h, const double* uh, const double* br, const double* 
   const KC& K = h->K;
   int rc = upload_cells(h, uh, h->U);
   if (rc) return rc;
-  CKC(cudaMemcpyAsync(h->BR, br, br_bytes(K), cudaMemcpyHostToDevice, h->st));
-  CKC(cudaMemcpyAsync(h->BZ, bz, bz_bytes(K), cudaMemcpyHostToDevice, h->st));
+  CKC(gdf::h2d(h->BR, br, br_bytes(K), h->st));
+  CKC(gdf::h2d(h->BZ, bz, bz_bytes(K), h->st));
   CKC(cudaMemsetAsync(h->T, 0, cell_plane_bytes(K) * NSC, h->st));
   if ((rc = sync_scal(h))) return rc;
   h->sc_host->trk[0] = t_rk;
@@ -1731,8 +1741,8 @@ int gdf_cy_lh(GdfCyHandle* h, const double* uh, const double* br, const double* 
   if ((rc = push_scal(h))) return rc;
   if ((rc = launch_lh(h, KIND_LH, h->sc))) return rc;
   if ((rc = download_cells(h, h->T, du))) return rc;
-  CKC(cudaMemcpyAsync(dbr, h->BRX, br_bytes(K), cudaMemcpyDeviceToHost, h->st));
-  CKC(cudaMemcpyAsync(dbz, h->BZX, bz_bytes(K), cudaMemcpyDeviceToHost, h->st));
+  CKC(gdf::d2h(dbr, h->BRX, br_bytes(K), h->st));
+  CKC(gdf::d2h(dbz, h->BZX, bz_bytes(K), h->st));
   CKC(cudaStreamSynchronize(h->st));
   h->uploaded = 1;
   return GDF_OK;
@@ -1743,12 +1753,12 @@ int gdf_cy_limit(GdfCyHandle* h, double* uh, double* br, double* bz) {
   const KC& K = h->K;
   int rc = upload_cells(h, uh, h->U);
   if (rc) return rc;
-  CKC(cudaMemcpyAsync(h->BR, br, br_bytes(K), cudaMemcpyHostToDevice, h->st));
-  CKC(cudaMemcpyAsync(h->BZ, bz, bz_bytes(K), cudaMemcpyHostToDevice, h->st));
+  CKC(gdf::h2d(h->BR, br, br_bytes(K), h->st));
+  CKC(gdf::h2d(h->BZ, bz, bz_bytes(K), h->st));
   if ((rc = launch_limit(h, nullptr, nullptr))) return rc;
   if ((rc = download_cells(h, h->U, uh))) return rc;
-  CKC(cudaMemcpyAsync(br, h->BR, br_bytes(K), cudaMemcpyDeviceToHost, h->st));
-  CKC(cudaMemcpyAsync(bz, h->BZ, bz_bytes(K), cudaMemcpyDeviceToHost, h->st));
+  CKC(gdf::d2h(br, h->BR, br_bytes(K), h->st));
+  CKC(gdf::d2h(bz, h->BZ, bz_bytes(K), h->st));
   CKC(cudaStreamSynchronize(h->st));
   h->uploaded = 1;
   return GDF_OK;
@@ -1779,7 +1789,7 @@ int gdf_cy_diagnostics(GdfCyHandle* h, double* umax, double* totaldiv, double* p
   });
   if (rc) return rc;
   std::vector<double> v((size_t)n * 3);
-  CKC(cudaMemcpyAsync(v.data(), h->diag, v.size() * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+  CKC(gdf::d2h(v.data(), h->diag, v.size() * sizeof(double), h->st));
   CKC(cudaStreamSynchronize(h->st));
   // item q = kk + nph*((i-1) + nr*(j-1)); the reference's loops: j outer, i inner
   double um = 0, td = 0, pm = 1000000;

@@ -15,6 +15,10 @@
 // list-directed layout differs only in spacing and exponent style, which
 // the reference's MATLAB readers (MHD_GDF_plot/*.m, load()) ignore.
 
+#include <omp.h>
+
+#include <algorithm>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -24,7 +28,41 @@
 
 namespace gdf {
 int set_last_error(int code, const char* msg);   // gdf_kernels.cu
+
+// The host side of gdf_stage.h: up to eight threads, each with at least 256 KB.
+static int host_threads(size_t bytes) {
+  return (int)std::max<size_t>(1, std::min<size_t>({8, (size_t)omp_get_num_procs(), bytes >> 18}));
 }
+void par_memcpy(void* dst, const void* src, size_t bytes) {
+  const int nt = host_threads(bytes);
+#pragma omp parallel for num_threads(nt) schedule(static) if (nt > 1)
+  for (int t = 0; t < nt; ++t) {
+    const size_t a = (bytes / 64 * t / nt) * 64, b = t + 1 == nt ? bytes : (bytes / 64 * (t + 1) / nt) * 64;
+    std::memcpy((char*)dst + a, (const char*)src + a, b - a);
+  }
+}
+void par_zero(void* dst, size_t bytes) {
+  const int nt = host_threads(bytes);
+#pragma omp parallel for num_threads(nt) schedule(static) if (nt > 1)
+  for (int t = 0; t < nt; ++t) {
+    const size_t a = (bytes / 64 * t / nt) * 64, b = t + 1 == nt ? bytes : (bytes / 64 * (t + 1) / nt) * 64;
+    std::memset((char*)dst + a, 0, b - a);
+  }
+}
+bool par_any_nonzero(const void* words, size_t n) {
+  const uint64_t* w = (const uint64_t*)words;
+  const int nt = host_threads(n * sizeof(uint64_t));
+  int any = 0;
+#pragma omp parallel for num_threads(nt) schedule(static) reduction(| : any) if (nt > 1)
+  for (int t = 0; t < nt; ++t) {
+    const size_t a = n * t / nt, b = n * (t + 1) / nt;
+    uint64_t acc = 0;
+    for (size_t q = a; q < b; ++q) acc |= w[q] << 1;
+    any |= acc != 0;
+  }
+  return any != 0;
+}
+}  // namespace gdf
 
 namespace {
 

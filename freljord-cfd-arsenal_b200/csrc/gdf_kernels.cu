@@ -33,6 +33,7 @@
 
 #include "../../include/gdf.h"
 #include "gdf_device.cuh"
+#include "gdf_stage.h"
 
 #ifndef GDF_EXACT
 #define GDF_EXACT 0
@@ -444,6 +445,7 @@ static int fail(int code, const std::string& msg) {
   } while (0)
 
 struct GdfHandle {
+  gdf::StageRef stage;
   GdfConfig cfg{};
   Consts K{};
   cudaStream_t st = nullptr;
@@ -799,49 +801,27 @@ static size_t uh_bytes(const GdfConfig& c) { return (size_t)(c.nx + 2) * (c.ny +
 static size_t bx_bytes(const GdfConfig& c) { return (size_t)(c.nx + 1) * c.ny * 3 * sizeof(double); }
 static size_t by_bytes(const GdfConfig& c) { return (size_t)c.nx * (c.ny + 1) * 3 * sizeof(double); }
 
-// dead (mode, variable) slots must be zero in an uploaded state. The 28
-// dead planes are scanned by several host threads (a 2048^2 state has 940 MB
-// of them; one thread took longer than the upload it overlaps); the error
-// names the first failing slot in (variable, mode) order.
+// dead (mode, variable) slots must be zero in an uploaded state (+0 and -0
+// pass, anything else, NaN included, fails): each of the 28 dead planes scanned
+// by several host threads. The error names the first failing slot in
+// (variable, mode) order.
 static int check_dead_slots(const GdfConfig& c, const double* uh) {
   const size_t plane = (size_t)(c.nx + 2) * (c.ny + 2);
-  std::vector<int> dead;
   for (int n = 0; n < NE; ++n)
-    for (int d = 0; d < NP; ++d)
-      if (!live_mode(n, d)) dead.push_back(d + 10 * n);
-  // +0 and -0 pass, anything else (NaN included) fails: OR of the bit
-  // patterns without the sign bit, a loop the compiler vectorises
-  auto bad_range = [&](int slot, size_t q0, size_t q1) {
-    const uint64_t* w = reinterpret_cast<const uint64_t*>(uh + plane * slot);
-    uint64_t acc = 0;
-    for (size_t q = q0; q < q1; ++q) acc |= w[q] << 1;
-    return acc != 0;
-  };
-  const size_t total = plane * dead.size();
-  unsigned nt = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-  if (total < ((size_t)1 << 22)) nt = 1;
-  std::vector<char> bad(dead.size(), 0);
-  auto work = [&](unsigned t) {
-    // thread t scans a contiguous share of the concatenated dead planes
-    const size_t a = total * t / nt, b = total * (t + 1) / nt;
-    for (size_t k = a; k < b;) {
-      const size_t s = k / plane, q0 = k - s * plane;
-      const size_t q1 = std::min(plane, q0 + (b - k));
-      if (bad_range(dead[s], q0, q1)) bad[s] = 1;
-      k += q1 - q0;
+    for (int d = 6; d < NP;) {
+      if (live_mode(n, d)) {
+        ++d;
+        continue;
+      }
+      int e = d + 1;   // a run of dead planes is one scan
+      while (e < NP && !live_mode(n, e)) ++e;
+      if (par_any_nonzero(uh + plane * (d + 10 * n), plane * (e - d)))
+        for (; d < e; ++d)
+          if (par_any_nonzero(uh + plane * (d + 10 * n), plane))
+            return fail(GDF_ERR_ARG, "uh has a nonzero value in mode " + std::to_string(d + 1) + " of variable " +
+                                         std::to_string(n + 1) + ", which the P2 scheme never populates");
+      d = e;
     }
-  };
-  if (nt == 1) {
-    work(0);
-  } else {
-    std::vector<std::thread> th;
-    for (unsigned t = 0; t < nt; ++t) th.emplace_back(work, t);
-    for (auto& x : th) x.join();
-  }
-  for (size_t s = 0; s < dead.size(); ++s)
-    if (bad[s])
-      return fail(GDF_ERR_ARG, "uh has a nonzero value in mode " + std::to_string(dead[s] % 10 + 1) + " of variable " +
-                                   std::to_string(dead[s] / 10 + 1) + ", which the P2 scheme never populates");
   return GDF_OK;
 }
 
@@ -850,16 +830,18 @@ static int check_dead_slots(const GdfConfig& c, const double* uh) {
 static cudaError_t copy_live(double* dst, const double* uh, const GdfConfig& c, cudaStream_t st,
                              cudaMemcpyKind kind) {
   const size_t plane = (size_t)(c.nx + 2) * (c.ny + 2);
+  auto copy = [&](int slot, int planes) {
+    const size_t o = plane * slot, b = planes * plane * sizeof(double);
+    return kind == cudaMemcpyHostToDevice   ? h2d(dst + o, uh + o, b, st)
+           : kind == cudaMemcpyDeviceToHost ? d2h(dst + o, uh + o, b, st)
+                                            : cudaMemcpyAsync(dst + o, uh + o, b, kind, st);
+  };
+  // live slots of a variable are modes 0..5 plus (Bx) 6, 8 or (By) 7, 9
   for (int n = 0; n < NE; ++n) {
-    // live slots of a variable are modes 0..5 plus (Bx) 6, 8 or (By) 7, 9
-    const size_t o = plane * (10 * n);
-    cudaError_t e = cudaMemcpyAsync(dst + o, uh + o, 6 * plane * sizeof(double), kind, st);
+    cudaError_t e = copy(10 * n, 6);
+    for (int d = 6; e == cudaSuccess && d < NP; ++d)
+      if (live_mode(n, d)) e = copy(10 * n + d, 1);
     if (e != cudaSuccess) return e;
-    for (int d = 6; d < NP; ++d) {
-      if (!live_mode(n, d)) continue;
-      e = cudaMemcpyAsync(dst + o + plane * d, uh + o + plane * d, plane * sizeof(double), kind, st);
-      if (e != cudaSuccess) return e;
-    }
   }
   return cudaSuccess;
 }
@@ -1032,8 +1014,8 @@ int gdf_upload(GdfHandle* h, const double* uh, const double* bx, const double* b
     return rc;
   }
   CK(copy_live(h->U, h->UT, h->cfg, h->st, cudaMemcpyDeviceToDevice));
-  CK(cudaMemcpyAsync(h->BX, bx, bx_bytes(h->cfg), cudaMemcpyHostToDevice, h->st));
-  CK(cudaMemcpyAsync(h->BY, by, by_bytes(h->cfg), cudaMemcpyHostToDevice, h->st));
+  CK(gdf::h2d(h->BX, bx, bx_bytes(h->cfg), h->st));
+  CK(gdf::h2d(h->BY, by, by_bytes(h->cfg), h->st));
   CK(cudaStreamSynchronize(h->st));
   h->uploaded = 1;
   return GDF_OK;
@@ -1042,9 +1024,9 @@ int gdf_upload(GdfHandle* h, const double* uh, const double* bx, const double* b
 int gdf_download(GdfHandle* h, double* uh, double* bx, double* by) {
   if (!h) return fail(GDF_ERR_ARG, "null handle");
   if (!h->uploaded) return fail(GDF_ERR_STATE, "no state uploaded");
-  if (uh) CK(cudaMemcpyAsync(uh, h->U, uh_bytes(h->cfg), cudaMemcpyDeviceToHost, h->st));
-  if (bx) CK(cudaMemcpyAsync(bx, h->BX, bx_bytes(h->cfg), cudaMemcpyDeviceToHost, h->st));
-  if (by) CK(cudaMemcpyAsync(by, h->BY, by_bytes(h->cfg), cudaMemcpyDeviceToHost, h->st));
+  if (uh) CK(gdf::d2h(uh, h->U, uh_bytes(h->cfg), h->st));
+  if (bx) CK(gdf::d2h(bx, h->BX, bx_bytes(h->cfg), h->st));
+  if (by) CK(gdf::d2h(by, h->BY, by_bytes(h->cfg), h->st));
   CK(cudaStreamSynchronize(h->st));
   return GDF_OK;
 }
@@ -1053,8 +1035,8 @@ int gdf_download_live(GdfHandle* h, double* uh, double* bx, double* by) {
   if (!h) return fail(GDF_ERR_ARG, "null handle");
   if (!h->uploaded) return fail(GDF_ERR_STATE, "no state uploaded");
   if (uh) CK(copy_live(uh, h->U, h->cfg, h->st, cudaMemcpyDeviceToHost));
-  if (bx) CK(cudaMemcpyAsync(bx, h->BX, bx_bytes(h->cfg), cudaMemcpyDeviceToHost, h->st));
-  if (by) CK(cudaMemcpyAsync(by, h->BY, by_bytes(h->cfg), cudaMemcpyDeviceToHost, h->st));
+  if (bx) CK(gdf::d2h(bx, h->BX, bx_bytes(h->cfg), h->st));
+  if (by) CK(gdf::d2h(by, h->BY, by_bytes(h->cfg), h->st));
   CK(cudaStreamSynchronize(h->st));
   return GDF_OK;
 }
@@ -1063,9 +1045,9 @@ int gdf_upload_state(GdfHandle* h, const double* cells, const double* bx, const 
   if (!h || !cells || !bx || !by) return fail(GDF_ERR_ARG, "null argument");
   const Consts& K = h->K;
   const long long n = 36LL * K.nx * K.ny;
-  CK(cudaMemcpyAsync(h->UT, cells, state_bytes(h->cfg), cudaMemcpyHostToDevice, h->st));
-  CK(cudaMemcpyAsync(h->BX, bx, bx_bytes(h->cfg), cudaMemcpyHostToDevice, h->st));
-  CK(cudaMemcpyAsync(h->BY, by, by_bytes(h->cfg), cudaMemcpyHostToDevice, h->st));
+  CK(gdf::h2d(h->UT, cells, state_bytes(h->cfg), h->st));
+  CK(gdf::h2d(h->BX, bx, bx_bytes(h->cfg), h->st));
+  CK(gdf::h2d(h->BY, by, by_bytes(h->cfg), h->st));
   int rc = run_plain(h, [&] { k_unpack_state<<<nblk(n, 256), 256, 0, h->st>>>(K, h->UT, h->U); });
   // the cell B modes from the face fields (div_free_Balsara.f90:13-79), the
   // ghosts as the end of a stage leaves them (set_bc with the ghost B
@@ -1088,10 +1070,10 @@ int gdf_download_state(GdfHandle* h, double* cells, double* bx, double* by) {
     const long long n = 36LL * h->K.nx * h->K.ny;
     int rc = run_plain(h, [&] { k_pack_state<<<nblk(n, 256), 256, 0, h->st>>>(h->K, h->U, h->UT); });
     if (rc) return rc;
-    CK(cudaMemcpyAsync(cells, h->UT, state_bytes(h->cfg), cudaMemcpyDeviceToHost, h->st));
+    CK(gdf::d2h(cells, h->UT, state_bytes(h->cfg), h->st));
   }
-  if (bx) CK(cudaMemcpyAsync(bx, h->BX, bx_bytes(h->cfg), cudaMemcpyDeviceToHost, h->st));
-  if (by) CK(cudaMemcpyAsync(by, h->BY, by_bytes(h->cfg), cudaMemcpyDeviceToHost, h->st));
+  if (bx) CK(gdf::d2h(bx, h->BX, bx_bytes(h->cfg), h->st));
+  if (by) CK(gdf::d2h(by, h->BY, by_bytes(h->cfg), h->st));
   CK(cudaStreamSynchronize(h->st));
   return GDF_OK;
 }
@@ -1137,8 +1119,7 @@ int gdf_prepare(GdfHandle* h, int32_t* flags) {
   if ((rc = launch_limit(h, h->UI, h->U, 1, nullptr))) return rc;
   if ((rc = launch_set_bc(h, h->U, 1, nullptr))) return rc;
   if (flags) {
-    CK(cudaMemcpyAsync(flags, h->flags, (size_t)h->cfg.nx * h->cfg.ny * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                       h->st));
+    CK(gdf::d2h(flags, h->flags, (size_t)h->cfg.nx * h->cfg.ny * sizeof(int32_t), h->st));
   }
   rc = sync_scal(h);
   if (rc) return rc;
@@ -1153,8 +1134,7 @@ int gdf_step(GdfHandle* h, double tend, double* t, double* dt_out, int32_t* flag
   if (rc) return rc;
   if ((rc = launch_step(h))) return rc;
   if (flags) {
-    CK(cudaMemcpyAsync(flags, h->flags, (size_t)h->cfg.nx * h->cfg.ny * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                       h->st));
+    CK(gdf::d2h(flags, h->flags, (size_t)h->cfg.nx * h->cfg.ny * sizeof(int32_t), h->st));
   }
   if ((rc = sync_scal(h))) return rc;
   *t = h->sc_host->t;
@@ -1281,11 +1261,11 @@ int gdf_features(GdfHandle* h, const double* uh, float* X) {
   if (!h->QM) CK(cudaMalloc((void**)&h->QM, (size_t)QMODES * h->K.plane * sizeof(float)));
   float* dX = nullptr;
   CK(cudaMallocAsync((void**)&dX, (size_t)ncell * NFEAT * sizeof(float), h->st));
-  CK(cudaMemcpyAsync(h->UT, uh, uh_bytes(h->cfg), cudaMemcpyHostToDevice, h->st));
+  CK(copy_live(h->UT, uh, h->cfg, h->st, cudaMemcpyHostToDevice));
   rc = run_kernel(h, GDF_K_LIMIT, [&] { k_qmodes<<<nblk(h->K.plane, 128), 128, 0, h->st>>>(h->K, h->UT, h->QM); });
   if (!rc) rc = run_kernel(h, GDF_K_LIMIT, [&] { k_features<<<nblk(ncell, 128), 128, 0, h->st>>>(h->K, h->QM, dX); });
   if (!rc) {
-    cudaError_t e = cudaMemcpyAsync(X, dX, (size_t)ncell * NFEAT * sizeof(float), cudaMemcpyDeviceToHost, h->st);
+    cudaError_t e = gdf::d2h(X, dX, (size_t)ncell * NFEAT * sizeof(float), h->st);
     if (e != cudaSuccess) rc = fail(GDF_ERR_CUDA, cudaGetErrorString(e));
   }
   cudaFreeAsync(dX, h->st);
@@ -1302,16 +1282,14 @@ int gdf_config_of(GdfHandle* h, GdfConfig* out) {
 // Is_Trouble_Cell (the sticky KXRCF flags), nx*ny int32 in (i-1)+nx*(j-1) order
 int gdf_get_trouble(GdfHandle* h, int32_t* trouble) {
   if (!h || !trouble) return fail(GDF_ERR_ARG, "null argument");
-  CK(cudaMemcpyAsync(trouble, h->trouble, (size_t)h->cfg.nx * h->cfg.ny * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                     h->st));
+  CK(gdf::d2h(trouble, h->trouble, (size_t)h->cfg.nx * h->cfg.ny * sizeof(int32_t), h->st));
   CK(cudaStreamSynchronize(h->st));
   return GDF_OK;
 }
 
 int gdf_set_trouble(GdfHandle* h, const int32_t* trouble) {
   if (!h || !trouble) return fail(GDF_ERR_ARG, "null argument");
-  CK(cudaMemcpyAsync(h->trouble, trouble, (size_t)h->cfg.nx * h->cfg.ny * sizeof(int32_t), cudaMemcpyHostToDevice,
-                     h->st));
+  CK(gdf::h2d(h->trouble, trouble, (size_t)h->cfg.nx * h->cfg.ny * sizeof(int32_t), h->st));
   CK(cudaStreamSynchronize(h->st));
   return GDF_OK;
 }
@@ -1355,7 +1333,7 @@ int gdf_lh(GdfHandle* h, const double* uh, double* du) {
   int rc = check_dead_slots(h->cfg, uh);
   if (rc) return rc;
   const size_t ub = uh_bytes(h->cfg);
-  CK(cudaMemcpyAsync(h->UT, uh, ub, cudaMemcpyHostToDevice, h->st));
+  CK(copy_live(h->UT, uh, h->cfg, h->st, cudaMemcpyHostToDevice));
   CK(cudaMemsetAsync(h->UI, 0, ub, h->st));  // du (ghost and dead entries stay 0)
   if ((rc = launch_faces(h, h->UT, nullptr))) return rc;
   rc = run_kernel(h, GDF_K_CELL, [&] {
@@ -1363,7 +1341,7 @@ int gdf_lh(GdfHandle* h, const double* uh, double* du) {
                                                              nullptr, 0);
   });
   if (rc) return rc;
-  CK(cudaMemcpyAsync(du, h->UI, ub, cudaMemcpyDeviceToHost, h->st));
+  CK(gdf::d2h(du, h->UI, ub, h->st));
   CK(cudaStreamSynchronize(h->st));
   return GDF_OK;
 }
@@ -1372,7 +1350,7 @@ int gdf_lhez(GdfHandle* h, const double* uh, double* dez1, double* dez2) {
   if (!h || !uh || !dez1 || !dez2) return fail(GDF_ERR_ARG, "null argument");
   int rc = check_dead_slots(h->cfg, uh);
   if (rc) return rc;
-  CK(cudaMemcpyAsync(h->UT, uh, uh_bytes(h->cfg), cudaMemcpyHostToDevice, h->st));
+  CK(copy_live(h->UT, uh, h->cfg, h->st, cudaMemcpyHostToDevice));
   if ((rc = launch_faces(h, h->UT, nullptr))) return rc;
   double *d1 = h->BX0, *d2 = h->BY0;
   rc = run_kernel(h, GDF_K_BFACE, [&] {
@@ -1380,8 +1358,8 @@ int gdf_lhez(GdfHandle* h, const double* uh, double* dez1, double* dez2) {
         h->K, h->EzRL, h->EzUD, h->EzV, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, d1, d2, nullptr, 0);
   });
   if (rc) return rc;
-  CK(cudaMemcpyAsync(dez1, d1, bx_bytes(h->cfg), cudaMemcpyDeviceToHost, h->st));
-  CK(cudaMemcpyAsync(dez2, d2, by_bytes(h->cfg), cudaMemcpyDeviceToHost, h->st));
+  CK(gdf::d2h(dez1, d1, bx_bytes(h->cfg), h->st));
+  CK(gdf::d2h(dez2, d2, by_bytes(h->cfg), h->st));
   CK(cudaStreamSynchronize(h->st));
   return GDF_OK;
 }
@@ -1392,10 +1370,10 @@ int gdf_limit(GdfHandle* h, double* uh, double* bx, double* by, int32_t* flags) 
   if (rc) return rc;
   const size_t ub = uh_bytes(h->cfg);
   // the limiter works on the resident buffers; save and restore them
-  CK(cudaMemcpyAsync(h->UT, uh, ub, cudaMemcpyHostToDevice, h->st));
+  CK(gdf::h2d(h->UT, uh, ub, h->st));
   CK(cudaMemcpyAsync(h->U0, h->UT, ub, cudaMemcpyDeviceToDevice, h->st));
-  CK(cudaMemcpyAsync(h->BX0, bx, bx_bytes(h->cfg), cudaMemcpyHostToDevice, h->st));
-  CK(cudaMemcpyAsync(h->BY0, by, by_bytes(h->cfg), cudaMemcpyHostToDevice, h->st));
+  CK(gdf::h2d(h->BX0, bx, bx_bytes(h->cfg), h->st));
+  CK(gdf::h2d(h->BY0, by, by_bytes(h->cfg), h->st));
   double* sBX = h->BX;
   double* sBY = h->BY;
   h->BX = h->BX0;
@@ -1405,19 +1383,20 @@ int gdf_limit(GdfHandle* h, double* uh, double* bx, double* by, int32_t* flags) 
   h->BX = sBX;
   h->BY = sBY;
   if (rc) return rc;
-  CK(cudaMemcpyAsync(uh, h->U0, ub, cudaMemcpyDeviceToHost, h->st));
-  CK(cudaMemcpyAsync(bx, h->BX0, bx_bytes(h->cfg), cudaMemcpyDeviceToHost, h->st));
-  CK(cudaMemcpyAsync(by, h->BY0, by_bytes(h->cfg), cudaMemcpyDeviceToHost, h->st));
+  CK(gdf::d2h(uh, h->U0, ub, h->st));
+  CK(gdf::d2h(bx, h->BX0, bx_bytes(h->cfg), h->st));
+  CK(gdf::d2h(by, h->BY0, by_bytes(h->cfg), h->st));
   if (flags)
-    CK(cudaMemcpyAsync(flags, h->flags, (size_t)h->cfg.nx * h->cfg.ny * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                       h->st));
+    CK(gdf::d2h(flags, h->flags, (size_t)h->cfg.nx * h->cfg.ny * sizeof(int32_t), h->st));
   CK(cudaStreamSynchronize(h->st));
   return GDF_OK;
 }
 
 int gdf_dt(GdfHandle* h, const double* uh, double* dt) {
   if (!h || !uh || !dt) return fail(GDF_ERR_ARG, "null argument");
-  CK(cudaMemcpyAsync(h->UT, uh, uh_bytes(h->cfg), cudaMemcpyHostToDevice, h->st));
+  // the cell averages only (calculate_dt reads mode 1)
+  const size_t pl = (size_t)h->K.plane;
+  for (int n = 0; n < NE; ++n) CK(gdf::h2d(h->UT + 10 * n * pl, uh + 10 * n * pl, pl * sizeof(double), h->st));
   int rc = launch_dt(h, h->UT, 0);
   if (rc) return rc;
   if ((rc = sync_scal(h))) return rc;

@@ -24,6 +24,7 @@
 
 #include "../../include/gdf.h"
 #include "gdf_mlp.cuh"
+#include "gdf_stage.h"
 
 using namespace gdf;
 
@@ -414,6 +415,7 @@ __global__ void k_to_bf16(const float* __restrict__ Xf, __nv_bfloat16* __restric
 }  // namespace
 
 struct GdfMlp {
+  gdf::StageRef stage;
   cudaStream_t st = nullptr;
   float *P = nullptr, *M = nullptr, *V = nullptr, *grad = nullptr, *loss = nullptr;
   MlpDev* D = nullptr;
@@ -457,7 +459,7 @@ static int mlp_ensure(GdfMlp* m, long long n, int blocks) {
 static int mlp_upload_x(GdfMlp* m, const float* X, long long n) {
   float* tmp = nullptr;
   MCK(cudaMallocAsync((void**)&tmp, (size_t)n * MLP_IN * sizeof(float), m->st));
-  MCK(cudaMemcpyAsync(tmp, X, (size_t)n * MLP_IN * sizeof(float), cudaMemcpyHostToDevice, m->st));
+  MCK(gdf::h2d(tmp, X, (size_t)n * MLP_IN * sizeof(float), m->st));
   const long long tot = n * MLP_INP;
   k_to_bf16<<<(unsigned)((tot + 255) / 256), 256, 0, m->st>>>(tmp, m->X, n);
   MCK(cudaGetLastError());
@@ -495,7 +497,7 @@ static int fwdbwd_launch(GdfMlp* m, const int* idx, long long nsel, float pos_w,
 // the error word of the tcgen05 tiles (read back after a synchronisation)
 static int check_err(GdfMlp* m) {
   int e = 0;
-  MCK(cudaMemcpyAsync(&e, m->err, sizeof(int), cudaMemcpyDeviceToHost, m->st));
+  MCK(gdf::d2h(&e, m->err, sizeof(int), m->st));
   MCK(cudaStreamSynchronize(m->st));
   if (e) {
     MCK(cudaMemsetAsync(m->err, 0, sizeof(int), m->st));
@@ -565,7 +567,7 @@ int gdf_mlp_destroy(GdfMlp* m) {
 
 int gdf_mlp_set_params(GdfMlp* m, const float* params) {
   if (!m || !params) return mfail(GDF_ERR_ARG, "null argument");
-  MCK(cudaMemcpyAsync(m->P, params, MLP_NPARAM * sizeof(float), cudaMemcpyHostToDevice, m->st));
+  MCK(gdf::h2d(m->P, params, MLP_NPARAM * sizeof(float), m->st));
   MCK(cudaMemsetAsync(m->M, 0, MLP_NPARAM * sizeof(float), m->st));
   MCK(cudaMemsetAsync(m->V, 0, MLP_NPARAM * sizeof(float), m->st));
   m->adam_t = 0;
@@ -577,7 +579,7 @@ int gdf_mlp_set_params(GdfMlp* m, const float* params) {
 
 int gdf_mlp_get_params(GdfMlp* m, float* params) {
   if (!m || !params) return mfail(GDF_ERR_ARG, "null argument");
-  MCK(cudaMemcpyAsync(params, m->P, MLP_NPARAM * sizeof(float), cudaMemcpyDeviceToHost, m->st));
+  MCK(gdf::d2h(params, m->P, MLP_NPARAM * sizeof(float), m->st));
   MCK(cudaStreamSynchronize(m->st));
   return GDF_OK;
 }
@@ -589,13 +591,13 @@ int gdf_mlp_grad(GdfMlp* m, const float* X, const float* y, int64_t n, float pos
   int rc = mlp_ensure(m, n, nb);
   if (rc) return rc;
   if ((rc = mlp_upload_x(m, X, n))) return rc;
-  MCK(cudaMemcpyAsync(m->y, y, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, m->st));
+  MCK(gdf::h2d(m->y, y, (size_t)n * sizeof(float), m->st));
   std::vector<int> id((size_t)n);
   for (long long q = 0; q < n; ++q) id[q] = (int)q;
-  MCK(cudaMemcpyAsync(m->idx, id.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice, m->st));
+  MCK(gdf::h2d(m->idx, id.data(), (size_t)n * sizeof(int), m->st));
   if ((rc = mlp_grad_launch(m, n, pos_weight, 1.f / (float)n))) return rc;
-  MCK(cudaMemcpyAsync(grad, m->grad, MLP_NPARAM * sizeof(float), cudaMemcpyDeviceToHost, m->st));
-  if (loss) MCK(cudaMemcpyAsync(loss, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->st));
+  MCK(gdf::d2h(grad, m->grad, MLP_NPARAM * sizeof(float), m->st));
+  if (loss) MCK(gdf::d2h(loss, m->loss, sizeof(float), m->st));
   MCK(cudaStreamSynchronize(m->st));
   return check_err(m);
 }
@@ -607,7 +609,7 @@ int gdf_mlp_train(GdfMlp* m, const float* X, const float* y, int64_t n, int32_t 
   int rc = mlp_ensure(m, n, nb_max);
   if (rc) return rc;
   if ((rc = mlp_upload_x(m, X, n))) return rc;
-  MCK(cudaMemcpyAsync(m->y, y, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, m->st));
+  MCK(gdf::h2d(m->y, y, (size_t)n * sizeof(float), m->st));
   std::vector<int> id((size_t)n);
   for (long long q = 0; q < n; ++q) id[q] = (int)q;
   std::mt19937 rng((uint32_t)seed);
@@ -616,7 +618,7 @@ int gdf_mlp_train(GdfMlp* m, const float* X, const float* y, int64_t n, int32_t 
   std::vector<float> lossv;
   for (int ep = 0; ep < epochs; ++ep) {
     std::shuffle(id.begin(), id.end(), rng);
-    MCK(cudaMemcpyAsync(m->idx, id.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice, m->st));
+    MCK(gdf::h2d(m->idx, id.data(), (size_t)n * sizeof(int), m->st));
     MCK(cudaStreamSynchronize(m->st));   // id is reshuffled next epoch
     double ep_loss = 0.0;
     for (long long off = 0; off < n; off += batch) {
@@ -629,7 +631,7 @@ int gdf_mlp_train(GdfMlp* m, const float* X, const float* y, int64_t n, int32_t 
       k_mlp_adam<<<(MLP_NPARAM + 255) / 256, 256, 0, m->st>>>(m->P, m->M, m->V, m->grad, lr, b1, b2, eps, c1, c2);
       if ((rc = mlp_sync(m))) return rc;
       float l = 0.f;
-      MCK(cudaMemcpyAsync(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->st));
+      MCK(gdf::d2h(&l, m->loss, sizeof(float), m->st));
       MCK(cudaStreamSynchronize(m->st));
       ep_loss += (double)l * (double)nsel;
     }
@@ -648,7 +650,7 @@ int gdf_mlp_predict(GdfMlp* m, const float* X, int64_t n, float* p) {
   MCK(cudaMallocAsync((void**)&dp, (size_t)n * sizeof(float), m->st));
   k_mlp_predict<<<(unsigned)((n + TB - 1) / TB), MLP_THREADS, 0, m->st>>>(m->D, m->X, (int)n, dp);
   MCK(cudaGetLastError());
-  MCK(cudaMemcpyAsync(p, dp, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, m->st));
+  MCK(gdf::d2h(p, dp, (size_t)n * sizeof(float), m->st));
   MCK(cudaFreeAsync(dp, m->st));
   MCK(cudaStreamSynchronize(m->st));
   return GDF_OK;

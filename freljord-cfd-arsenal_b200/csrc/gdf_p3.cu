@@ -33,6 +33,7 @@
 #include "../../include/gdf_p3.h"
 #include "gdf_p3_basis.h"
 #include "gdf_charlim.cuh"
+#include "gdf_stage.h"
 
 namespace gdf {
 int set_last_error(int code, const char* msg);
@@ -1001,6 +1002,7 @@ __global__ void __launch_bounds__(128) k3_diag(const __grid_constant__ K3 K, con
 using namespace gdf3;
 
 struct GdfP3Handle {
+  gdf::StageRef stage;
   GdfP3Config cfg{};
   K3 K{};
   cudaStream_t st = nullptr;
@@ -1229,20 +1231,25 @@ int push_scal(GdfP3Handle* h) {
 
 // host uh (full 15-slot layout) -> device live slots; the slots the method
 // keeps at zero must be zero
+// (consecutive live slots are consecutive planes on both sides: one copy a run)
 int upload_cells(GdfP3Handle* h, const double* uh, double* D) {
   const size_t pl = (size_t)h->K.plane;
   for (int n = 0; n < NE; ++n)
-    for (int d = 0; d < NP3; ++d) {
+    for (int d = 0, e; d < NP3; d = e) {
       const double* src = uh + pl * (d + (size_t)NP3 * n);
       const int s = slot3(n, d);
+      e = d + 1;
       if (s < 0) {
-        for (size_t q = 0; q < pl; ++q)
-          if (src[q] != 0.0)
-            return fail(GDF_ERR_ARG, "uh slot (d=" + std::to_string(d + 1) + ", n=" + std::to_string(n + 1) +
+        while (e < NP3 && slot3(n, e) < 0) ++e;
+        if (gdf::par_any_nonzero(src, pl * (e - d)))
+          for (int k = d; k < e; ++k)
+            if (gdf::par_any_nonzero(src + pl * (k - d), pl))
+              return fail(GDF_ERR_ARG, "uh slot (d=" + std::to_string(k + 1) + ", n=" + std::to_string(n + 1) +
                                          ") must be zero: the k = 3 method never fills it");
         continue;
       }
-      CK3(cudaMemcpyAsync(D + pl * s, src, pl * sizeof(double), cudaMemcpyHostToDevice, h->st));
+      while (e < NP3 && slot3(n, e) == s + (e - d)) ++e;
+      CK3(gdf::h2d(D + pl * s, src, pl * (e - d) * sizeof(double), h->st));
     }
   CK3(cudaStreamSynchronize(h->st));
   return GDF_OK;
@@ -1251,14 +1258,17 @@ int upload_cells(GdfP3Handle* h, const double* uh, double* D) {
 int download_cells(GdfP3Handle* h, const double* D, double* uh) {
   const size_t pl = (size_t)h->K.plane;
   for (int n = 0; n < NE; ++n)
-    for (int d = 0; d < NP3; ++d) {
+    for (int d = 0, e; d < NP3; d = e) {
       double* dst = uh + pl * (d + (size_t)NP3 * n);
       const int s = slot3(n, d);
+      e = d + 1;
       if (s < 0) {
-        std::memset(dst, 0, pl * sizeof(double));
+        while (e < NP3 && slot3(n, e) < 0) ++e;
+        gdf::par_zero(dst, pl * (e - d) * sizeof(double));
         continue;
       }
-      CK3(cudaMemcpyAsync(dst, D + pl * s, pl * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+      while (e < NP3 && slot3(n, e) == s + (e - d)) ++e;
+      CK3(gdf::d2h(dst, D + pl * s, pl * (e - d) * sizeof(double), h->st));
     }
   CK3(cudaStreamSynchronize(h->st));
   return GDF_OK;
@@ -1346,8 +1356,8 @@ int gdf_p3_upload(GdfP3Handle* h, const double* uh, const double* bx, const doub
   if (!h || !uh || !bx || !by) return fail(GDF_ERR_ARG, "null argument");
   int rc = upload_cells(h, uh, h->U);
   if (rc) return rc;
-  CK3(cudaMemcpyAsync(h->BX, bx, bx_bytes(h->K), cudaMemcpyHostToDevice, h->st));
-  CK3(cudaMemcpyAsync(h->BY, by, by_bytes(h->K), cudaMemcpyHostToDevice, h->st));
+  CK3(gdf::h2d(h->BX, bx, bx_bytes(h->K), h->st));
+  CK3(gdf::h2d(h->BY, by, by_bytes(h->K), h->st));
   h->sc_host->t = 0;
   h->sc_host->dt = 0;
   h->sc_host->active = 1;
@@ -1364,8 +1374,8 @@ int gdf_p3_download(GdfP3Handle* h, double* uh, double* bx, double* by) {
   if (!h->uploaded) return fail(GDF_ERR_STATE, "no state uploaded");
   int rc = download_cells(h, h->U, uh);
   if (rc) return rc;
-  CK3(cudaMemcpyAsync(bx, h->BX, bx_bytes(h->K), cudaMemcpyDeviceToHost, h->st));
-  CK3(cudaMemcpyAsync(by, h->BY, by_bytes(h->K), cudaMemcpyDeviceToHost, h->st));
+  CK3(gdf::d2h(bx, h->BX, bx_bytes(h->K), h->st));
+  CK3(gdf::d2h(by, h->BY, by_bytes(h->K), h->st));
   CK3(cudaStreamSynchronize(h->st));
   return GDF_OK;
 }
@@ -1531,15 +1541,15 @@ int gdf_p3_lh(GdfP3Handle* h, const double* uh, const double* bx, const double* 
   const K3& K = h->K;
   int rc = upload_cells(h, uh, h->U);
   if (rc) return rc;
-  CK3(cudaMemcpyAsync(h->BX, bx, bx_bytes(K), cudaMemcpyHostToDevice, h->st));
-  CK3(cudaMemcpyAsync(h->BY, by, by_bytes(K), cudaMemcpyHostToDevice, h->st));
+  CK3(gdf::h2d(h->BX, bx, bx_bytes(K), h->st));
+  CK3(gdf::h2d(h->BY, by, by_bytes(K), h->st));
   CK3(cudaMemsetAsync(h->T, 0, (size_t)K.plane * NS3 * sizeof(double), h->st));
   CK3(cudaMemsetAsync(h->BXT, 0, bx_bytes(K), h->st));
   CK3(cudaMemsetAsync(h->BYT, 0, by_bytes(K), h->st));
   if ((rc = launch_lh(h, KIND_LH, nullptr))) return rc;
   if ((rc = download_cells(h, h->T, du))) return rc;
-  CK3(cudaMemcpyAsync(dbx, h->BXT, bx_bytes(K), cudaMemcpyDeviceToHost, h->st));
-  CK3(cudaMemcpyAsync(dby, h->BYT, by_bytes(K), cudaMemcpyDeviceToHost, h->st));
+  CK3(gdf::d2h(dbx, h->BXT, bx_bytes(K), h->st));
+  CK3(gdf::d2h(dby, h->BYT, by_bytes(K), h->st));
   CK3(cudaStreamSynchronize(h->st));
   h->uploaded = 1;
   return GDF_OK;
@@ -1550,8 +1560,8 @@ int gdf_p3_limit(GdfP3Handle* h, double* uh, double* bx, double* by) {
   const K3& K = h->K;
   int rc = upload_cells(h, uh, h->T);
   if (rc) return rc;
-  CK3(cudaMemcpyAsync(h->BXT, bx, bx_bytes(K), cudaMemcpyHostToDevice, h->st));
-  CK3(cudaMemcpyAsync(h->BYT, by, by_bytes(K), cudaMemcpyHostToDevice, h->st));
+  CK3(gdf::h2d(h->BXT, bx, bx_bytes(K), h->st));
+  CK3(gdf::h2d(h->BYT, by, by_bytes(K), h->st));
   // the cells' ghosts keep the values set_bc gives them
   if ((rc = launch_set_bc(h, h->T, h->BXT, h->BYT, nullptr))) return rc;
   CK3(cudaMemcpyAsync(h->U, h->T, (size_t)K.plane * NS3 * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
@@ -1559,8 +1569,8 @@ int gdf_p3_limit(GdfP3Handle* h, double* uh, double* bx, double* by) {
   CK3(cudaMemcpyAsync(h->BY, h->BYT, by_bytes(K), cudaMemcpyDeviceToDevice, h->st));
   if ((rc = launch_limit(h, nullptr, nullptr))) return rc;
   if ((rc = download_cells(h, h->U, uh))) return rc;
-  CK3(cudaMemcpyAsync(bx, h->BX, bx_bytes(K), cudaMemcpyDeviceToHost, h->st));
-  CK3(cudaMemcpyAsync(by, h->BY, by_bytes(K), cudaMemcpyDeviceToHost, h->st));
+  CK3(gdf::d2h(bx, h->BX, bx_bytes(K), h->st));
+  CK3(gdf::d2h(by, h->BY, by_bytes(K), h->st));
   CK3(cudaStreamSynchronize(h->st));
   h->uploaded = 1;
   return GDF_OK;
@@ -1584,7 +1594,7 @@ int gdf_p3_diagnostics(GdfP3Handle* h, double* umax, double* totaldiv) {
   int rc = run(h, [&] { k3_diag<<<nblk(nc, 128), 128, 0, h->st>>>(K, h->U, h->diag, h->diag + nc); });
   if (rc) return rc;
   std::vector<double> v((size_t)nc * 2);
-  CK3(cudaMemcpyAsync(v.data(), h->diag, v.size() * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+  CK3(gdf::d2h(v.data(), h->diag, v.size() * sizeof(double), h->st));
   CK3(cudaStreamSynchronize(h->st));
   // the reference's loop order: i outer, j inner
   double um = 0, td = 0;

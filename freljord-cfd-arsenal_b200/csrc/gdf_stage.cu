@@ -1,0 +1,131 @@
+// gdf_stage.cu -- the pinned ring behind gdf_stage.h.
+//
+// One ring per device. A copy holds the ring for its whole length; a copy that
+// finds it taken (another thread's) goes to cudaMemcpyAsync, so threads never
+// wait for each other here. A slot is reused when the event recorded behind its
+// last transfer has passed, whatever stream that was on.
+#include "gdf_stage.h"
+
+#include <algorithm>
+#include <mutex>
+
+namespace gdf {
+namespace {
+
+struct Ring {
+  std::mutex mu;
+  int holders = 0;
+  char* buf[STAGE_SLOTS] = {};
+  cudaEvent_t ev[STAGE_SLOTS] = {};
+  bool ready = false;
+};
+constexpr int MAX_DEV = 64;
+Ring g_ring[MAX_DEV];
+
+void drop(Ring& r) {
+  for (int k = 0; k < STAGE_SLOTS; ++k) {
+    if (r.ev[k]) {
+      cudaEventSynchronize(r.ev[k]);
+      cudaEventDestroy(r.ev[k]);
+    }
+    if (r.buf[k]) cudaFreeHost(r.buf[k]);
+    r.ev[k] = nullptr;
+    r.buf[k] = nullptr;
+  }
+  r.ready = false;
+  cudaGetLastError();
+}
+
+bool make(Ring& r) {
+  if (r.ready) return true;
+  bool ok = true;
+  for (int k = 0; ok && k < STAGE_SLOTS; ++k)
+    ok = cudaHostAlloc((void**)&r.buf[k], STAGE_CHUNK, cudaHostAllocPortable) == cudaSuccess &&
+         cudaEventCreateWithFlags(&r.ev[k], cudaEventDisableTiming) == cudaSuccess;
+  if (!ok) {
+    drop(r);
+    return false;
+  }
+  r.ready = true;
+  return true;
+}
+
+// the current device's ring, locked in lk, for a pageable array of this size;
+// null: copy plainly
+Ring* take(const void* host, size_t bytes, std::unique_lock<std::mutex>& lk) {
+  if (bytes < STAGE_MIN) return nullptr;
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (a.type != cudaMemoryTypeUnregistered) return nullptr;
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEV) return nullptr;
+  Ring& r = g_ring[dev];
+  lk = std::unique_lock<std::mutex>(r.mu, std::try_to_lock);
+  if (!lk.owns_lock() || r.holders == 0 || !make(r)) return nullptr;
+  return &r;
+}
+
+}  // namespace
+
+StageRef::StageRef() : dev(-1) {
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEV) {
+    cudaGetLastError();
+    dev = -1;
+    return;
+  }
+  std::lock_guard<std::mutex> lk(g_ring[dev].mu);
+  ++g_ring[dev].holders;
+}
+
+StageRef::~StageRef() {
+  if (dev < 0) return;
+  std::lock_guard<std::mutex> lk(g_ring[dev].mu);
+  if (--g_ring[dev].holders == 0) drop(g_ring[dev]);
+}
+
+cudaError_t h2d(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+  std::unique_lock<std::mutex> lk;
+  Ring* r = take(src, bytes, lk);
+  if (!r) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+  int k = 0;
+  for (size_t o = 0; o < bytes; o += STAGE_CHUNK, k = (k + 1) % STAGE_SLOTS) {
+    const size_t n = std::min(STAGE_CHUNK, bytes - o);
+    cudaError_t e = cudaEventSynchronize(r->ev[k]);
+    if (e != cudaSuccess) return e;
+    par_memcpy(r->buf[k], (const char*)src + o, n);
+    e = cudaMemcpyAsync((char*)dst + o, r->buf[k], n, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaEventRecord(r->ev[k], st);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+cudaError_t d2h(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+  std::unique_lock<std::mutex> lk;
+  Ring* r = take(dst, bytes, lk);
+  if (!r) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
+  const size_t chunks = (bytes + STAGE_CHUNK - 1) / STAGE_CHUNK;
+  auto issue = [&](size_t c) {
+    const int k = (int)(c % STAGE_SLOTS);
+    const size_t o = c * STAGE_CHUNK, n = std::min(STAGE_CHUNK, bytes - o);
+    cudaError_t e = cudaEventSynchronize(r->ev[k]);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(r->buf[k], (const char*)src + o, n, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaEventRecord(r->ev[k], st);
+    return e;
+  };
+  cudaError_t e = cudaSuccess;
+  for (size_t c = 0; e == cudaSuccess && c < std::min(chunks, (size_t)STAGE_SLOTS); ++c) e = issue(c);
+  for (size_t c = 0; e == cudaSuccess && c < chunks; ++c) {
+    const size_t o = c * STAGE_CHUNK, n = std::min(STAGE_CHUNK, bytes - o);
+    e = cudaEventSynchronize(r->ev[c % STAGE_SLOTS]);
+    if (e != cudaSuccess) break;
+    par_memcpy((char*)dst + o, r->buf[c % STAGE_SLOTS], n);
+    if (c + STAGE_SLOTS < chunks) e = issue(c + STAGE_SLOTS);
+  }
+  return e;
+}
+
+}  // namespace gdf

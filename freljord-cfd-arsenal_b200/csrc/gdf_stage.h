@@ -1,0 +1,48 @@
+// gdf_stage.h -- copies between host arrays and the device.
+//
+// A caller's arrays are ordinary (pageable) memory as a rule. The driver copies
+// those through its own staging buffer with one host thread, 12 GB/s here (less
+// into pages not yet touched), well under the link. h2d / d2h take large
+// pageable arrays through a ring of pinned buffers instead: several threads fill
+// (empty) one while the link moves another. Small arrays, and memory that is
+// already pinned or on a device, go to cudaMemcpyAsync as they are.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+
+namespace gdf {
+
+// Keeps the current device's ring for as long as it lives: the ring (STAGE_SLOTS
+// x STAGE_CHUNK bytes, made on first use) is freed with the last of its holders.
+// Every handle holds one.
+struct StageRef {
+  StageRef();
+  ~StageRef();
+  StageRef(const StageRef&) = delete;
+  StageRef& operator=(const StageRef&) = delete;
+
+ private:
+  int dev;
+};
+
+constexpr size_t STAGE_CHUNK = (size_t)4 << 20;
+constexpr int STAGE_SLOTS = 4;
+constexpr size_t STAGE_MIN = (size_t)1 << 20;   // below: one plain copy (the ring's hand-overs cost more)
+
+// host -> device, ordered on st; src may be reused on return
+cudaError_t h2d(void* dst, const void* src, size_t bytes, cudaStream_t st);
+// device -> host after st's earlier work; a pageable dst of STAGE_MIN bytes or
+// more is complete on return
+cudaError_t d2h(void* dst, const void* src, size_t bytes, cudaStream_t st);
+
+// memcpy over several threads (gdf_io.cpp)
+void par_memcpy(void* dst, const void* src, size_t bytes);
+// zeros over several threads (gdf_io.cpp)
+void par_zero(void* dst, size_t bytes);
+// whether any of n 64-bit words has a bit besides the sign set, over several
+// threads (gdf_io.cpp)
+bool par_any_nonzero(const void* words, size_t n);
+
+}  // namespace gdf

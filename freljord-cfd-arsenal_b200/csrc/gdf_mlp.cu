@@ -6,8 +6,9 @@
 //   k_mlp_fwdbwd   64 samples per block: forward, loss, backward, and the
 //                  block's gradient written to its own slot (no atomics)
 //   k_mlp_reduce   gradient = sum of the block slots in block order
-//   k_mlp_adam     Adam update of the FP32 master parameters
-//   k_mlp_sync     BF16 / transposed device copy for the next step
+//   k_mlp_update   the same sum, Adam on the FP32 master parameters and their
+//                  BF16 / transposed device copies, one launch per step
+//   k_mlp_sync     those copies of given parameters
 // Roundings to BF16 (the operands of the tensor-core products): inputs X,
 // W1, W2, w3, the first hidden layer H1, and the back-propagated dZ2, dZ1.
 // Everything else is FP32. tests/test_mlp.py restates this in numpy.
@@ -91,7 +92,7 @@ __global__ void k_mlp_sync(const float* __restrict__ P, MlpDev* __restrict__ D) 
 }
 
 // Forward + backward of one 64-sample tile; block b writes its gradient to
-// partial[b * MLP_NPARAM ...] and its loss to loss_part[b].
+// partial[b * MLP_PSTRIDE ...] and its loss to loss_part[b].
 __global__ void __launch_bounds__(MLP_THREADS) k_mlp_fwdbwd(const MlpDev* __restrict__ D,
                                                             const __nv_bfloat16* __restrict__ X,
                                                             const float* __restrict__ y,
@@ -282,7 +283,7 @@ __global__ void __launch_bounds__(MLP_THREADS) k_mlp_fwdbwd(const MlpDev* __rest
       if (g == 0) S.red_b1[warp][nt * 8 + 2 * t + e] = a;
     }
   __syncthreads();
-  float* out = partial + (long long)blockIdx.x * MLP_NPARAM;
+  float* out = partial + (long long)blockIdx.x * MLP_PSTRIDE;
   // dW2t[o][i] = sum_s dZ2t[o][s] H1t[i][s]: warp rows o = 16w..16w+15
   {
     float c[8][4];
@@ -360,7 +361,7 @@ __global__ void k_mlp_reduce(const float* __restrict__ partial, int nb, float* _
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p < MLP_NPARAM) {
     float s = 0.f;
-    for (int b = 0; b < nb; ++b) s += partial[(long long)b * MLP_NPARAM + p];
+    for (int b = 0; b < nb; ++b) s += partial[(long long)b * MLP_PSTRIDE + p];
     grad[p] = s;
   }
   if (p == 0 && loss) {
@@ -370,17 +371,43 @@ __global__ void k_mlp_reduce(const float* __restrict__ partial, int nb, float* _
   }
 }
 
-__global__ void k_mlp_adam(float* __restrict__ P, float* __restrict__ M, float* __restrict__ V,
-                           const float* __restrict__ grad, float lr, float b1, float b2, float eps, float c1,
-                           float c2) {
+// One training step's end: the gradient (the block slots in block order, as
+// k_mlp_reduce), the Adam update of the FP32 parameters and their BF16 copies
+// (as k_mlp_sync), one parameter per thread; the batch's loss to *loss. Three
+// launches and a read-back of the loss before.
+__global__ void k_mlp_update(float* __restrict__ P, float* __restrict__ M, float* __restrict__ V,
+                             MlpDev* __restrict__ D, const float* __restrict__ partial, int nb,
+                             const float* __restrict__ loss_part, float* __restrict__ loss, float lr, float b1,
+                             float b2, float eps, float c1, float c2) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= MLP_NPARAM) return;
-  const float gr = grad[p];
+  float gr = 0.f;
+  for (int b = 0; b < nb; ++b) gr += partial[(long long)b * MLP_PSTRIDE + p];
   const float m = b1 * M[p] + (1.f - b1) * gr;
   const float v = b2 * V[p] + (1.f - b2) * gr * gr;
   M[p] = m;
   V[p] = v;
-  P[p] -= lr * (m / c1) / (sqrtf(v / c2) + eps);
+  const float w = P[p] - lr * (m / c1) / (sqrtf(v / c2) + eps);
+  P[p] = w;
+  const __nv_bfloat16 h = __float2bfloat16_rn(w);
+  if (p < MLP_OFF_B1) {
+    D->W1t[(p % MLP_H) * MLP_INP + p / MLP_H] = h;
+  } else if (p < MLP_OFF_W2) {
+    D->b1[p - MLP_OFF_B1] = w;
+  } else if (p < MLP_OFF_B2) {
+    const int q = p - MLP_OFF_W2;
+    D->W2t[(q % MLP_H) * MLP_H + q / MLP_H] = h;
+    D->W2n[q] = h;
+  } else if (p < MLP_OFF_W3) {
+    D->b2[p - MLP_OFF_B2] = w;
+  } else if (p < MLP_OFF_B3) {
+    D->w3[p - MLP_OFF_W3] = __bfloat162float(h);
+  } else {
+    D->b3 = w;
+    float s = 0.f;
+    for (int b = 0; b < nb; ++b) s += loss_part[b];
+    *loss = s;
+  }
 }
 
 __global__ void __launch_bounds__(MLP_THREADS) k_mlp_predict(const MlpDev* __restrict__ D,
@@ -449,7 +476,7 @@ static int mlp_ensure(GdfMlp* m, long long n, int blocks) {
     if (m->partial) cudaFree(m->partial);
     if (m->loss_part) cudaFree(m->loss_part);
     m->partial = nullptr; m->loss_part = nullptr;
-    MCK(cudaMalloc((void**)&m->partial, (size_t)blocks * MLP_NPARAM * sizeof(float)));
+    MCK(cudaMalloc((void**)&m->partial, (size_t)blocks * MLP_PSTRIDE * sizeof(float)));
     MCK(cudaMalloc((void**)&m->loss_part, (size_t)blocks * sizeof(float)));
     m->part_blocks = blocks;
   }
@@ -610,35 +637,49 @@ int gdf_mlp_train(GdfMlp* m, const float* X, const float* y, int64_t n, int32_t 
   if (rc) return rc;
   if ((rc = mlp_upload_x(m, X, n))) return rc;
   MCK(gdf::h2d(m->y, y, (size_t)n * sizeof(float), m->st));
-  std::vector<int> id((size_t)n);
+  std::vector<int> id((size_t)n), next;
   for (long long q = 0; q < n; ++q) id[q] = (int)q;
   std::mt19937 rng((uint32_t)seed);
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   if ((rc = fwdbwd_attr())) return rc;
-  std::vector<float> lossv;
-  for (int ep = 0; ep < epochs; ++ep) {
-    std::shuffle(id.begin(), id.end(), rng);
+  // an epoch is enqueued whole: its losses stay on the device until its end,
+  // and the next epoch is shuffled while it runs
+  const long long nbatch = (n + batch - 1) / batch;
+  float* dloss = nullptr;
+  MCK(cudaMallocAsync((void**)&dloss, (size_t)nbatch * sizeof(float), m->st));
+  std::vector<float> lossv((size_t)nbatch);
+  auto epoch = [&](int ep) -> int {
+    if (ep == 0) std::shuffle(id.begin(), id.end(), rng);
     MCK(gdf::h2d(m->idx, id.data(), (size_t)n * sizeof(int), m->st));
-    MCK(cudaStreamSynchronize(m->st));   // id is reshuffled next epoch
-    double ep_loss = 0.0;
-    for (long long off = 0; off < n; off += batch) {
-      const long long nsel = std::min<long long>(batch, n - off);
+    for (long long k = 0; k < nbatch; ++k) {
+      const long long off = k * batch, nsel = std::min<long long>(batch, n - off);
       int nb = 0;
-      if ((rc = fwdbwd_launch(m, m->idx + off, nsel, pos_weight, 1.f / (float)nsel, nb))) return rc;
-      k_mlp_reduce<<<(MLP_NPARAM + 255) / 256, 256, 0, m->st>>>(m->partial, nb, m->grad, m->loss_part, m->loss);
+      int r = fwdbwd_launch(m, m->idx + off, nsel, pos_weight, 1.f / (float)nsel, nb);
+      if (r) return r;
       m->adam_t += 1;
       const float c1 = 1.f - std::pow(b1, (float)m->adam_t), c2 = 1.f - std::pow(b2, (float)m->adam_t);
-      k_mlp_adam<<<(MLP_NPARAM + 255) / 256, 256, 0, m->st>>>(m->P, m->M, m->V, m->grad, lr, b1, b2, eps, c1, c2);
-      if ((rc = mlp_sync(m))) return rc;
-      float l = 0.f;
-      MCK(gdf::d2h(&l, m->loss, sizeof(float), m->st));
-      MCK(cudaStreamSynchronize(m->st));
-      ep_loss += (double)l * (double)nsel;
+      k_mlp_update<<<(MLP_NPARAM + 63) / 64, 64, 0, m->st>>>(m->P, m->M, m->V, m->D, m->partial, nb, m->loss_part,
+                                                             dloss + k, lr, b1, b2, eps, c1, c2);
+      MCK(cudaGetLastError());
     }
+    if (ep + 1 < epochs) {
+      next = id;   // the copy of id may still be under way
+      std::shuffle(next.begin(), next.end(), rng);
+    }
+    MCK(cudaMemcpyAsync(lossv.data(), dloss, (size_t)nbatch * sizeof(float), cudaMemcpyDeviceToHost, m->st));
+    int r = check_err(m);   // waits for the epoch
+    if (r) return r;
+    id.swap(next);
+    double ep_loss = 0.0;
+    for (long long k = 0; k < nbatch; ++k)
+      ep_loss += (double)lossv[k] * (double)std::min<long long>(batch, n - k * batch);
     if (epoch_loss) epoch_loss[ep] = (float)(ep_loss / (double)n);
-    if ((rc = check_err(m))) return rc;
-  }
-  return GDF_OK;
+    return GDF_OK;
+  };
+  for (int ep = 0; !rc && ep < epochs; ++ep) rc = epoch(ep);
+  cudaStreamSynchronize(m->st);   // an epoch that failed part of the way
+  cudaFreeAsync(dloss, m->st);
+  return rc;
 }
 
 int gdf_mlp_predict(GdfMlp* m, const float* X, int64_t n, float* p) {

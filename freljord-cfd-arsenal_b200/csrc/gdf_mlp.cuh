@@ -29,9 +29,10 @@ constexpr int MLP_OFF_B2 = MLP_OFF_W2 + MLP_H * MLP_H;
 constexpr int MLP_OFF_W3 = MLP_OFF_B2 + MLP_H;
 constexpr int MLP_OFF_B3 = MLP_OFF_W3 + MLP_H;
 constexpr int MLP_NPARAM = MLP_OFF_B3 + 1;   // 10049
+constexpr int MLP_PSTRIDE = 10112;           // a block's slot of partial gradients (rows 16-byte aligned)
 
 // Device copy of the network for the kernels.
-struct MlpDev {
+struct alignas(16) MlpDev {
   __nv_bfloat16 W1t[MLP_H * MLP_INP];   // [n][k], k >= 90 zero
   __nv_bfloat16 W2t[MLP_H * MLP_H];     // [o][i]
   __nv_bfloat16 W2n[MLP_H * MLP_H];     // [i][o] (for the backward product)

@@ -3,8 +3,9 @@
 // operands in shared memory, FP32 accumulators in tensor memory), one
 // 128-sample tile per CTA.
 //
-// Per tile (rows = samples s, 128 per CTA; 128 threads, thread t <-> row t
-// <-> tensor-memory lane t):
+// Per tile (rows = samples s, 128 per CTA; 256 threads: warps w and w + 4 share
+// the rows, tensor-memory lanes, 32 (w % 4) .., warps 0-3 the first 32 columns
+// of a result, warps 4-7 the other 32):
 //   Z1 [s][n]  = X [s][k]  . W1t[n][k]      M 128, N 64, K 96   TMEM cols   0..63
 //   Z2 [s][o]  = H1[s][i]  . W2t[o][i]      M 128, N 64, K 64   TMEM cols  64..127
 //   dH1[s][i]  = dZ2[s][o] . W2n[i][o]      M 128, N 64, K 64   TMEM cols  64..127 (after Z2 is read)
@@ -14,6 +15,15 @@
 // layout: 8-row x 16-byte core matrices, element (r, k) of a tile with K
 // columns at (r/8)*(K/8)*128 + (k/8)*128 + (r%8)*16 + (k%8)*2 bytes
 // (core matrices adjacent in K 128 B apart, in M/N (K/8)*128 B apart).
+// What bounds a tile is not its products but what lies between them: 64 columns
+// of erf and exp per sample, the operands' stores, the column sums. So rows are
+// loaded and packed 16 bytes at a time, a column's erf is evaluated once per
+// pass, and the sums over 32 lanes exchange 31 values for 32 columns (a
+// halving butterfly: the additions of the full butterfly, in its order).
+// Rows of the 128-row operands Xt and H1t past the 96 / 64 in use are left as
+// they are: they feed result rows that nothing reads.
+// 61 us per tile with scalar loads, one thread per row and a shuffle tree per
+// column; 18 us so.
 // One elected thread issues the products and commits them to an mbarrier;
 // every wait on it is bounded (2 s of %globaltimer), after which the CTA
 // sets the error word, still frees its tensor memory and returns.
@@ -33,7 +43,7 @@ namespace gdf {
 namespace {
 
 constexpr int TCM = 128;          // samples per CTA (UMMA M)
-constexpr int TC_THREADS = 128;
+constexpr int TC_THREADS = 256;
 constexpr int TMEM_COLS = 256;
 constexpr unsigned long long WAIT_NS = 2000000000ull;
 
@@ -58,7 +68,7 @@ struct TcSmem {
   alignas(128) unsigned char dZ2t[SZ_T64];
   alignas(128) unsigned char dZ1t[SZ_T64];
   float b1[MLP_H], b2[MLP_H], w3[MLP_H];
-  float yv[TCM], wv[TCM], g3[TCM], lossv[TCM];
+  float yv[TCM], wv[TCM], g3[TCM], lossv[TCM], part[TCM];
   float red[3][4][MLP_H];       // per-warp column sums of db1, db2, dw3
   alignas(8) uint64_t mbar;
   uint32_t tmem_base;
@@ -159,12 +169,33 @@ __device__ __forceinline__ float gelu_df(float x) {
   return 0.5f * (1.f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
 }
 
-// column sums over the CTA's 128 rows of per-thread vectors (fixed order:
-// lanes by a shuffle tree, then the four warps in order)
-__device__ __forceinline__ void warp_colsum(float v, float* red_warp_col, int lane) {
+// Sums of 32 columns over the warp's 32 lanes; lane l gets column l's. Per step
+// a lane passes on the half it gives up and adds its partner's half to its own:
+// each sum is the one v += shfl_xor(v, 16), 8, 4, 2, 1 forms.
+__device__ __forceinline__ float warp_colsums(float* v, int lane) {
 #pragma unroll
-  for (int m = 16; m > 0; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
-  if (lane == 0) *red_warp_col = v;
+  for (int m = 16; m > 0; m >>= 1) {
+    const bool up = (lane & m) != 0;
+#pragma unroll
+    for (int k = 0; k < m; ++k) {
+      const float give = up ? v[k] : v[k + m], keep = up ? v[k + m] : v[k];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, give, m);
+    }
+  }
+  return v[0];
+}
+// columns c0 .. c0 + 31 of row r (K-major tile with K columns), rounded to BF16
+__device__ __forceinline__ void st_row32(unsigned char* tile, int r, int c0, int K, const __nv_bfloat16* h) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const __nv_bfloat162 t = __halves2bfloat162(h[8 * q + 2 * e], h[8 * q + 2 * e + 1]);
+      w[e] = *reinterpret_cast<const uint32_t*>(&t);
+    }
+    *reinterpret_cast<uint4*>(tile + cofs(r, c0 + 8 * q, K)) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
 }
 
 __global__ void __launch_bounds__(TC_THREADS, 1) k_mlp_fwdbwd_tc(const MlpDev* __restrict__ D,
@@ -188,11 +219,19 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_mlp_fwdbwd_tc(const MlpDev* _
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&S.mbar)));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  // parameters and samples into the canonical tiles
-  for (int q = tid; q < MLP_H * MLP_INP; q += TC_THREADS) st_bf16(S.W1t, q / MLP_INP, q % MLP_INP, MLP_INP, D->W1t[q]);
-  for (int q = tid; q < MLP_H * MLP_H; q += TC_THREADS) {
-    st_bf16(S.W2t, q / MLP_H, q % MLP_H, MLP_H, D->W2t[q]);
-    st_bf16(S.W2n, q / MLP_H, q % MLP_H, MLP_H, D->W2n[q]);
+  // parameters and samples into the canonical tiles, 8 columns (16 bytes) at a
+  // time, rows fastest over the threads (the shared-memory stores of a warp then
+  // fall into different banks)
+  const int row = 32 * (warp & 3) + lane, half = warp >> 2, c0 = 32 * half;
+  for (int q = tid; q < MLP_H * (MLP_INP / 8); q += TC_THREADS) {
+    const int r = q % MLP_H, k = q / MLP_H * 8;
+    *reinterpret_cast<uint4*>(S.W1t + cofs(r, k, MLP_INP)) =
+        *reinterpret_cast<const uint4*>(D->W1t + r * MLP_INP + k);
+  }
+  for (int q = tid; q < MLP_H * (MLP_H / 8); q += TC_THREADS) {
+    const int r = q % MLP_H, k = q / MLP_H * 8;
+    *reinterpret_cast<uint4*>(S.W2t + cofs(r, k, MLP_H)) = *reinterpret_cast<const uint4*>(D->W2t + r * MLP_H + k);
+    *reinterpret_cast<uint4*>(S.W2n + cofs(r, k, MLP_H)) = *reinterpret_cast<const uint4*>(D->W2n + r * MLP_H + k);
   }
   if (tid < MLP_H) {
     S.b1[tid] = D->b1[tid];
@@ -200,26 +239,33 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_mlp_fwdbwd_tc(const MlpDev* _
     S.w3[tid] = D->w3[tid];
   }
   {
-    const int q = base + tid;
+    const int q = base + row;
     const bool in = q < nsel;
-    const long long src = in ? (long long)idx[q] * MLP_INP : 0;
-    for (int k = 0; k < MLP_INP; ++k) {
-      const __nv_bfloat16 v = in ? X[src + k] : __float2bfloat16_rn(0.f);
-      st_bf16(S.X, tid, k, MLP_INP, v);
-      st_bf16(S.Xt, k, tid, TCM, v);
+    const int id = in ? idx[q] : 0;
+    const uint4* src = reinterpret_cast<const uint4*>(X + (long long)id * MLP_INP) + 6 * half;
+    uint4 v[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) v[k] = in ? src[k] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const int col = 48 * half + 8 * k;
+      *reinterpret_cast<uint4*>(S.X + cofs(row, col, MLP_INP)) = v[k];
+      const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&v[k]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) st_bf16(S.Xt, col + j, row, TCM, e[j]);
     }
-    for (int k = MLP_INP; k < 128; ++k) st_bf16(S.Xt, k, tid, TCM, __float2bfloat16_rn(0.f));
-    for (int i = MLP_H; i < 128; ++i) st_bf16(S.H1t, i, tid, TCM, __float2bfloat16_rn(0.f));
-    const float yy = in ? y[idx[q]] : 0.f;
-    S.yv[tid] = yy;
-    S.wv[tid] = in ? (yy > 0.5f ? pos_w : 1.f) : 0.f;
+    if (half == 0) {
+      const float yy = in ? y[id] : 0.f;
+      S.yv[row] = yy;
+      S.wv[row] = in ? (yy > 0.5f ? pos_w : 1.f) : 0.f;
+    }
   }
   fence_async_smem();
   tc_before_sync();
   __syncthreads();
   tc_after_sync();
   const uint32_t tm = S.tmem_base;
-  const uint32_t lane_off = (uint32_t)(32 * warp) << 16;
+  const uint32_t lane_off = (uint32_t)(32 * (warp & 3)) << 16;
   uint32_t phase = 0;
   bool ok = true;
   // issue (thread 0), commit, wait: `ok` stays uniform over the CTA; after a
@@ -246,48 +292,62 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_mlp_fwdbwd_tc(const MlpDev* _
   run([&] { gemm(tm + 0, S.X, MLP_INP, S.W1t, MLP_INP, MLP_INP, MLP_H); });
   if (ok) {
     float z[32];
-#pragma unroll 1
-    for (int h = 0; h < 2; ++h) {
-      tmem_ld32(tm + lane_off + 32 * h, z);
+    tmem_ld32(tm + lane_off + c0, z);
+    __nv_bfloat16 h[32];
 #pragma unroll
-      for (int q = 0; q < 32; ++q) {
-        const int c = 32 * h + q;
-        const __nv_bfloat16 v = __float2bfloat16_rn(gelu_f(z[q] + S.b1[c]));
-        st_bf16(S.H1, tid, c, MLP_H, v);
-        st_bf16(S.H1t, c, tid, TCM, v);
-      }
+    for (int q = 0; q < 32; ++q) {
+      h[q] = __float2bfloat16_rn(gelu_f(z[q] + S.b1[c0 + q]));
+      st_bf16(S.H1t, c0 + q, row, TCM, h[q]);
     }
+    st_row32(S.H1, row, c0, MLP_H, h);
   }
   handoff();
 
   // Z2 = H1 . W2t^T ; loss, dL/dz3, dZ2, db2, dw3
   run([&] { gemm(tm + 64, S.H1, MLP_H, S.W2t, MLP_H, MLP_H, MLP_H); });
   if (ok) {
-    float z2[MLP_H];
-    tmem_ld32(tm + lane_off + 64, z2);
-    tmem_ld32(tm + lane_off + 96, z2 + 32);
-    float s = 0.f;
+    float z2[32], er[32];   // er = 1 + erf(z2 / sqrt 2), shared by gelu and its derivative
+    tmem_ld32(tm + lane_off + 64 + c0, z2);
 #pragma unroll
-    for (int c = 0; c < MLP_H; ++c) {
-      z2[c] += S.b2[c];
-      s += gelu_f(z2[c]) * S.w3[c];
+    for (int c = 0; c < 32; ++c) {
+      z2[c] += S.b2[c0 + c];
+      er[c] = 1.f + erff(z2[c] * 0.70710678118654752f);
     }
-    const float z = s + D->b3;
-    const float p = 1.f / (1.f + expf(-z));
-    const float yy = S.yv[tid], wt = S.wv[tid];
-    const float sp_pos = fmaxf(z, 0.f) + log1pf(expf(-fabsf(z)));
-    S.lossv[tid] = wt * (yy * (sp_pos - z) + (1.f - yy) * sp_pos) * inv_b;
-    const float g3 = wt * (p - yy) * inv_b;
-    S.g3[tid] = g3;
-#pragma unroll 1
-    for (int c = 0; c < MLP_H; ++c) {
-      const float dz = g3 * S.w3[c] * gelu_df(z2[c]);
-      const __nv_bfloat16 b = __float2bfloat16_rn(dz);
-      st_bf16(S.dZ2, tid, c, MLP_H, b);
-      st_bf16(S.dZ2t, c, tid, TCM, b);
-      warp_colsum(dz, &S.red[1][warp][c], lane);
-      warp_colsum(g3 * gelu_f(z2[c]), &S.red[2][warp][c], lane);
+    // z = sum over the 64 columns in order: warps 0-3 begin it, 4-7 finish it
+    float s = 0.f;
+    if (half == 0) {
+#pragma unroll
+      for (int c = 0; c < 32; ++c) s += 0.5f * z2[c] * er[c] * S.w3[c];
+      S.part[row] = s;
     }
+    __syncthreads();
+    if (half == 1) {
+      s = S.part[row];
+#pragma unroll
+      for (int c = 0; c < 32; ++c) s += 0.5f * z2[c] * er[c] * S.w3[32 + c];
+      const float z = s + D->b3;
+      const float p = 1.f / (1.f + expf(-z));
+      const float yy = S.yv[row], wt = S.wv[row];
+      const float sp_pos = fmaxf(z, 0.f) + log1pf(expf(-fabsf(z)));
+      S.lossv[row] = wt * (yy * (sp_pos - z) + (1.f - yy) * sp_pos) * inv_b;
+      S.g3[row] = wt * (p - yy) * inv_b;
+    }
+    __syncthreads();
+    const float g3 = S.g3[row];
+    float dz[32];
+    __nv_bfloat16 b[32];
+#pragma unroll
+    for (int c = 0; c < 32; ++c) {
+      const float gd = 0.5f * er[c] + z2[c] * 0.39894228040143268f * expf(-0.5f * z2[c] * z2[c]);
+      dz[c] = g3 * S.w3[c0 + c] * gd;
+      b[c] = __float2bfloat16_rn(dz[c]);
+      st_bf16(S.dZ2t, c0 + c, row, TCM, b[c]);
+    }
+    st_row32(S.dZ2, row, c0, MLP_H, b);
+    S.red[1][warp & 3][c0 + lane] = warp_colsums(dz, lane);
+#pragma unroll
+    for (int c = 0; c < 32; ++c) dz[c] = g3 * (0.5f * z2[c] * er[c]);
+    S.red[2][warp & 3][c0 + lane] = warp_colsums(dz, lane);
   }
   handoff();
 
@@ -296,30 +356,24 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_mlp_fwdbwd_tc(const MlpDev* _
     gemm(tm + 64, S.dZ2, MLP_H, S.W2n, MLP_H, MLP_H, MLP_H);
     gemm(tm + 128, S.H1t, TCM, S.dZ2t, TCM, TCM, MLP_H);
   });
-  float* out = partial + (long long)blockIdx.x * MLP_NPARAM;
+  float* out = partial + (long long)blockIdx.x * MLP_PSTRIDE;
+  auto store32 = [&](float* o, const float* v) {   // 32 values of a result row, 16-byte aligned
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      reinterpret_cast<float4*>(o)[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+  };
   if (ok) {
     float dh[32], z1[32];
-#pragma unroll 1
-    for (int h = 0; h < 2; ++h) {
-      tmem_ld32(tm + lane_off + 64 + 32 * h, dh);
-      tmem_ld32(tm + lane_off + 32 * h, z1);
-#pragma unroll 1
-      for (int q = 0; q < 32; ++q) {
-        const int c = 32 * h + q;
-        const float dz = dh[q] * gelu_df(z1[q] + S.b1[c]);
-        st_bf16(S.dZ1t, c, tid, TCM, __float2bfloat16_rn(dz));
-        warp_colsum(dz, &S.red[0][warp][c], lane);
-      }
+    tmem_ld32(tm + lane_off + 64 + c0, dh);
+    tmem_ld32(tm + lane_off + c0, z1);
+#pragma unroll
+    for (int q = 0; q < 32; ++q) {
+      dh[q] = dh[q] * gelu_df(z1[q] + S.b1[c0 + q]);
+      st_bf16(S.dZ1t, c0 + q, row, TCM, __float2bfloat16_rn(dh[q]));
     }
-    float w2r[32];
-#pragma unroll 1
-    for (int h = 0; h < 2; ++h) {
-      tmem_ld32(tm + lane_off + 128 + 32 * h, w2r);
-      if (tid < MLP_H) {
-#pragma unroll 1
-        for (int q = 0; q < 32; ++q) out[MLP_OFF_W2 + tid * MLP_H + 32 * h + q] = w2r[q];
-      }
-    }
+    S.red[0][warp & 3][c0 + lane] = warp_colsums(dh, lane);
+    tmem_ld32(tm + lane_off + 128 + c0, z1);
+    if (row < MLP_H) store32(out + MLP_OFF_W2 + row * MLP_H + c0, z1);
   }
   handoff();
 
@@ -327,14 +381,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_mlp_fwdbwd_tc(const MlpDev* _
   run([&] { gemm(tm + 192, S.Xt, TCM, S.dZ1t, TCM, TCM, MLP_H); });
   if (ok) {
     float w1r[32];
-#pragma unroll 1
-    for (int h = 0; h < 2; ++h) {
-      tmem_ld32(tm + lane_off + 192 + 32 * h, w1r);
-      if (tid < MLP_IN) {
-#pragma unroll 1
-        for (int q = 0; q < 32; ++q) out[MLP_OFF_W1 + tid * MLP_H + 32 * h + q] = w1r[q];
-      }
-    }
+    tmem_ld32(tm + lane_off + 192 + c0, w1r);
+    if (row < MLP_IN) store32(out + MLP_OFF_W1 + row * MLP_H + c0, w1r);
   }
   tc_before_sync();
   __syncthreads();

@@ -181,11 +181,11 @@ __device__ __forceinline__ void prim_c(const Phys& P, const double* U, double ra
   q.B1 = gdf::rdiv(q.rB1, rrad, bad);
   q.B2 = gdf::rdiv(q.rB2, rrad, bad);
   if (bad) {   // an operand out of rdiv's range: the IEEE division itself
-    q.u = U[1] / q.rho;
-    q.v = U[2] / q.rho;
-    q.w = U[3] / q.rho;
-    q.B1 = q.rB1 / rad;
-    q.B2 = q.rB2 / rad;
+    q.u = gdf::ieee_div(U[1], q.rho);
+    q.v = gdf::ieee_div(U[2], q.rho);
+    q.w = gdf::ieee_div(U[3], q.rho);
+    q.B1 = gdf::ieee_div(q.rB1, rad);
+    q.B2 = gdf::ieee_div(q.rB2, rad);
   }
   q.B3 = U[7];
   q.rB3 = q.B3 * rad;
@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(CY_CELL_BS) k_cy_cell(const __grid_constant__ 
       for (int n = 0; n < 7; ++n) Q[n] = gdf::rdiv(R[n], rrad, bad);
       if (bad) {
 #pragma unroll
-        for (int n = 0; n < 7; ++n) Q[n] = R[n] / rad;
+        for (int n = 0; n < 7; ++n) Q[n] = gdf::ieee_div(R[n], rad);
       }
       const double* PX = K.B.phixG[a][b];
       const double* PY = K.B.phiyG[a][b];
@@ -572,40 +572,48 @@ __global__ void __launch_bounds__(CY_CELL_BS) k_cy_cell(const __grid_constant__ 
     }
   }
   if (!valid) return;
-  // surface terms (Lh.f90:370-407; var 8 from the edge fields, LhEz.f90:37-55)
-  const long long npx = K.nxf * NG, npy = K.nyf * NG;
+  // surface terms (Lh.f90:370-407; var 8 from the edge fields, LhEz.f90:37-55),
+  // x faces, then y faces, a point at a time for all variables: one copy of the
+  // code per direction (unrolled over the points as well it did not fit the
+  // instruction cache). The face basis is the same on both faces up to the sign
+  // of the modes odd across them, and 1 for mode 1.
   const long long fR = (long long)i + (K.nx + 1) * (long long)(j - 1), fL = fR - 1;
   const long long fU = (long long)(i - 1) + (long long)K.nx * j, fD = fU - K.nx;
+  auto faces = [&](const double* F, long long np, long long hi, long long lo, double ch, const double (*fb)[NQC],
+                   bool x) {
+#pragma unroll 1
+    for (int g = 0; g < NG; ++g) {
+      const double cw = ch * K.B.w[g];
+      const double* f = fb[g];
+      double q1[NE], q0[NE];
+#pragma unroll
+      for (int n = 0; n < NE; ++n) {
+        const double* Q = F + np * (n < 7 ? n : 8) + kk;
+        q1[n] = ld(Q + K.nph * (g + NG * hi));
+        q0[n] = ld(Q + K.nph * (g + NG * lo));
+      }
+#pragma unroll
+      for (int n = 0; n < NE; ++n)
+#pragma unroll
+        for (int d = 0; d < NQC; ++d) {
+          const bool odd = x ? (d == 1 || d == 4) : (d == 2 || d == 4);
+          const double h = d == 0 ? q1[n] : q1[n] * f[d], l = d == 0 ? q0[n] : q0[n] * f[d];
+          const double t = cw * (odd ? h + l : h - l);
+          du[n][d] = (n < 7 || x) ? du[n][d] - t : du[n][d] + t;
+        }
+    }
+  };
+  faces(FXH, K.nxf * NG, fR, fL, K.cxs, K.B.phiGR, true);
+  faces(FYH, K.nyf * NG, fU, fD, K.czs, K.B.phiGU, false);
+  // the mass matrix (mm(1) = 1), by its reciprocals
 #pragma unroll
   for (int n = 0; n < NE; ++n) {
-    const int qx = n < 7 ? n : 8, qy = n < 7 ? n : 8;
-#pragma unroll
-    for (int d = 0; d < NQC; ++d) {
-      double acc = du[n][d];
-#pragma unroll
-      for (int g = 0; g < NG; ++g) {
-        const double r1 = ld(FXH + npx * qx + kk + K.nph * (g + NG * fR));
-        const double l1 = ld(FXH + npx * qx + kk + K.nph * (g + NG * fL));
-        acc = acc - K.cxs * K.B.w[g] * (r1 * K.B.phiGR[g][d] - l1 * K.B.phiGL[g][d]);
-      }
-#pragma unroll
-      for (int g = 0; g < NG; ++g) {
-        const double u1 = ld(FYH + npy * qy + kk + K.nph * (g + NG * fU));
-        const double d1 = ld(FYH + npy * qy + kk + K.nph * (g + NG * fD));
-        if (n < 7)
-          acc = acc - K.czs * K.B.w[g] * (u1 * K.B.phiGU[g][d] - d1 * K.B.phiGD[g][d]);
-        else
-          acc = acc + K.czs * K.B.w[g] * (u1 * K.B.phiGU[g][d] - d1 * K.B.phiGD[g][d]);
-      }
-      du[n][d] = acc;
-    }
-    // the mass matrix (mm(1) = 1), by its reciprocals
     unsigned bad = 0;
     double Q[NQC];
 #pragma unroll
     for (int d = 1; d < NQC; ++d) Q[d] = gdf::rdiv(du[n][d], Rcp{K.B.mm[d], K.B.rmm[d]}, bad);
 #pragma unroll
-    for (int d = 1; d < NQC; ++d) du[n][d] = bad ? du[n][d] / K.B.mm[d] : Q[d];
+    for (int d = 1; d < NQC; ++d) du[n][d] = bad ? gdf::ieee_div(du[n][d], K.B.mm[d]) : Q[d];
   }
   if (KIND == KIND_LH) {
 #pragma unroll
@@ -772,7 +780,7 @@ __global__ void __launch_bounds__(128) k_cy_bproj(const __grid_constant__ KC K, 
         for (int d = 1; d < NQC; ++d) Q[d] = gdf::rdiv(t * G[d], Rcp{K.B.mm[d], K.B.rmm[d]}, bad);
         acc[v][0] = acc[v][0] + t;
 #pragma unroll
-        for (int d = 1; d < NQC; ++d) acc[v][d] = acc[v][d] + (bad ? t * G[d] / K.B.mm[d] : Q[d]);
+        for (int d = 1; d < NQC; ++d) acc[v][d] = acc[v][d] + (bad ? gdf::ieee_div(t * G[d], K.B.mm[d]) : Q[d]);
       }
     }
   }
@@ -995,7 +1003,7 @@ __global__ void __launch_bounds__(128) k_cy_divfree(const __grid_constant__ KC K
 #pragma unroll
       for (int d = 1; d < NQC; ++d) Q[d] = gdf::rdiv(wab * dv * G[d], Rcp{K.B.mm[d], K.B.rmm[d]}, bad);
 #pragma unroll
-      for (int d = 1; d < NQC; ++d) bpp[d] = bpp[d] + (bad ? wab * dv * G[d] / K.B.mm[d] : Q[d]);
+      for (int d = 1; d < NQC; ++d) bpp[d] = bpp[d] + (bad ? gdf::ieee_div(wab * dv * G[d], K.B.mm[d]) : Q[d]);
     }
   if (!valid) return;
   auto br = [&](int ii, int d) { return ld(BR + ii + (K.nx + 1) * ((long long)(j - 1) + (long long)K.ny * (kk + (long long)K.nph * d))); };

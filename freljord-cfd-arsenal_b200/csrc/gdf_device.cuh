@@ -256,9 +256,15 @@ constexpr int CELL_SLOTS = NLIVE;
 // is shared between points or modes is shared before a sum, never across one: a face flux times lambda
 // (modes 3 and 5, or 2 and 5) or times P2 (modes 6 and 9, or 4 and 8), one
 // reciprocal per point for u, v, w, known reciprocals for the mass matrix.
-// Blast 2048^2: 5.66 ms per launch, 5.95-6.05 before; rotor
-// 512^2 366 us, 387 before. (Keeping a column's parts in shared memory as well:
-// 6.47 ms; forming the next point's values beside this one's primitives: 6.67.)
+// The instruction cache decides much of the rest: eight warps at different places
+// of a long straight line evict each other's code. So the surface sums are one
+// copy per direction (not unrolled over the points) and the divisions behind
+// rdiv out of line.
+// Blast 2048^2: 3.80 ms per launch, 6.09 at first (5.66 with the surface sums
+// unrolled, 4.27 with the fallback divisions inline); rotor 512^2 319 us, 448 at
+// first. (Keeping a column's parts in shared memory, forming the next point's
+// values beside this one's primitives, and the mass matrix and the combination
+// as a loop over the slots in shared memory were each slower.)
 // ms: the block's CELL_SLOTS * CELL_BS doubles, 16-byte aligned (blockDim.x ==
 // CELL_BS).
 __device__ __forceinline__ void cell_item(const Consts& K, const double* __restrict__ U, double* __restrict__ U0,
@@ -321,9 +327,9 @@ __device__ __forceinline__ void cell_item(const Consts& K, const double* __restr
         const Rcp rr = rcp_of(rho, bad);
         double u = rdiv(v[1], rr, bad), vv = rdiv(v[2], rr, bad), w = rdiv(v[3], rr, bad);
         if (bad) {   // an operand out of rdiv's range: the IEEE division itself
-          u = v[1] / rho;
-          vv = v[2] / rho;
-          w = v[3] / rho;
+          u = ieee_div(v[1], rho);
+          vv = ieee_div(v[2], rho);
+          w = ieee_div(v[3], rho);
         }
         const double E = v[4], B1 = v[5], B2 = v[6], B3 = v[7];
         const double BB = sq(B1) + sq(B2) + sq(B3);
@@ -368,71 +374,67 @@ __device__ __forceinline__ void cell_item(const Consts& K, const double* __restr
           }
       }
     }
-    // surface terms in the reference order (x faces, then y faces), mass.
-    // q1 the flux on the high face, q0 on the low one; the face basis is the
-    // same on both up to the sign of the modes odd in the face's direction
+    // surface terms in the reference order (x faces, then y faces), a point at
+    // a time for all variables (one copy of the code per direction: unrolled
+    // over the points and variables the kernel did not fit the instruction
+    // cache). q1 the flux on the high face, q0 on the low one; the face basis is
+    // the same on both up to the sign of the modes odd in the face's direction
     // (get_basis.f90), 1 for mode 1, +-1 for the slope across the face, and at
     // the middle point zero for the modes odd along it.
     const long long ox = (i - 1) + 1 + (long long)(K.nx + 1) * (j - 1);  // Fxhat(i,j)
     const long long oy = (i - 1) + (long long)K.nx * j;                  // Fyhat(i,j)
-    // the next variable's fluxes are asked for before this one's sums
-    double nr[NG], nl[NG], nu[NG], nd[NG];
-    auto load = [&](int n) {
-#pragma unroll
+    auto faces = [&](const double* F, long long pl, long long o, long long low, const double* cw,
+                     const double (*fb)[NP], bool x) {
+      const int across = x ? 1 : 2, along = x ? 2 : 1, across2 = x ? 3 : 5, along2 = x ? 5 : 3;
+#pragma unroll 1
       for (int g = 0; g < NG; ++g) {
-        nr[g] = Fxh[(n * NG + g) * K.fxplane + ox];
-        nl[g] = Fxh[(n * NG + g) * K.fxplane + ox - 1];
-        nu[g] = Fyh[(n * NG + g) * K.fyplane + oy];
-        nd[g] = Fyh[(n * NG + g) * K.fyplane + oy - K.nx];
-      }
-    };
-    load(0);
+        const double c = cw[g];
+        const double* f = fb[g];
+        const double* G = F + g * pl + o;
+        double q1[NE], q0[NE];
 #pragma unroll
-    for (int n = 0; n < NE; ++n) {
-      auto faces = [&](const double* q1, const double* q0, const double* cw, const double (*f)[NP], bool x) {
-        const int across = x ? 1 : 2, along = x ? 2 : 1, across2 = x ? 3 : 5, along2 = x ? 5 : 3;
+        for (int n = 0; n < NE; ++n) {
+          q1[n] = G[n * NG * pl];
+          q0[n] = G[n * NG * pl - low];
+        }
 #pragma unroll
-        for (int g = 0; g < NG; ++g) {
-          const double c = cw[g];
+        for (int n = 0; n < NE; ++n) {
           auto add = [&](int d, double t) { du[LI(n, d)] = du[LI(n, d)] - c * t; };
-          add(0, q1[g] - q0[g]);
-          add(across, q1[g] + q0[g]);
-          add(across2, q1[g] * f[g][across2] - q0[g] * f[g][across2]);
-          const double s1 = q1[g] * f[g][along2], s0 = q0[g] * f[g][along2];
+          add(0, q1[n] - q0[n]);
+          add(across, q1[n] + q0[n]);
+          add(across2, q1[n] * f[across2] - q0[n] * f[across2]);
+          const double s1 = q1[n] * f[along2], s0 = q0[n] * f[along2];
           add(along2, s1 - s0);
-          if (g != 2) {
-            const double l1 = q1[g] * f[g][along], l0 = q0[g] * f[g][along];
+          // Bx's mode 9, By's 8
+          if (n == 5 && x) add(8, s1 + s0);
+          if (n == 6 && !x) add(7, s1 + s0);
+          if (n == 5 && x) add(6, q1[n] * f[6] + q0[n] * f[6]);
+          if (n == 6 && !x) add(9, q1[n] * f[9] + q0[n] * f[9]);
+        }
+        if (g != 2) {
+#pragma unroll
+          for (int n = 0; n < NE; ++n) {
+            auto add = [&](int d, double t) { du[LI(n, d)] = du[LI(n, d)] - c * t; };
+            const double l1 = q1[n] * f[along], l0 = q0[n] * f[along];
             add(along, l1 - l0);
             add(4, l1 + l0);
-          }
-          // cubic modes: Bx's 7 and 9, By's 8 and 10
-          if (n == 5) {
-            if (x) {
-              add(6, q1[g] * f[g][6] + q0[g] * f[g][6]);
-              add(8, s1 + s0);
-            } else if (g != 2) {
-              add(6, q1[g] * f[g][6] - q0[g] * f[g][6]);
-              add(8, q1[g] * f[g][8] - q0[g] * f[g][8]);
+            if (n == 5 && !x) {
+              add(6, q1[n] * f[6] - q0[n] * f[6]);
+              add(8, q1[n] * f[8] - q0[n] * f[8]);
             }
-          }
-          if (n == 6) {
-            if (!x) {
-              add(7, s1 + s0);
-              add(9, q1[g] * f[g][9] + q0[g] * f[g][9]);
-            } else if (g != 2) {
-              add(7, q1[g] * f[g][7] - q0[g] * f[g][7]);
-              add(9, q1[g] * f[g][9] - q0[g] * f[g][9]);
+            if (n == 6 && x) {
+              add(7, q1[n] * f[7] - q0[n] * f[7]);
+              add(9, q1[n] * f[9] - q0[n] * f[9]);
             }
           }
         }
-      };
-      double fr[NG], fl[NG], fu[NG], fd[NG];
+      }
+    };
+    faces(Fxh, K.fxplane, ox, 1, K.cxw, c_basis.phiGR, true);
+    faces(Fyh, K.fyplane, oy, K.nx, K.cyw, c_basis.phiGU, false);
+    // mm(1) = 1 (get_basis.f90): x / 1 == x
 #pragma unroll
-      for (int g = 0; g < NG; ++g) { fr[g] = nr[g]; fl[g] = nl[g]; fu[g] = nu[g]; fd[g] = nd[g]; }
-      if (n + 1 < NE) load(n + 1);
-      faces(fr, fl, K.cxw, c_basis.phiGR, true);
-      faces(fu, fd, K.cyw, c_basis.phiGU, false);
-      // mm(1) = 1 (get_basis.f90): x / 1 == x
+    for (int n = 0; n < NE; ++n) {
       unsigned bad = 0;
       double q[NP];
 #pragma unroll
@@ -440,7 +442,7 @@ __device__ __forceinline__ void cell_item(const Consts& K, const double* __restr
         if (live_mode(n, d)) q[d] = rdiv(du[LI(n, d)], Rcp{c_basis.mm[d], c_basis.rmm[d]}, bad);
 #pragma unroll
       for (int d = 1; d < NP; ++d)
-        if (live_mode(n, d)) du[LI(n, d)] = bad ? du[LI(n, d)] / c_basis.mm[d] : q[d];
+        if (live_mode(n, d)) du[LI(n, d)] = bad ? ieee_div(du[LI(n, d)], c_basis.mm[d]) : q[d];
     }
   }
   if (stage == 0) {

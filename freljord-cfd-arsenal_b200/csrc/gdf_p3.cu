@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(128) k3_vertex(const __grid_constant__ K3 K, c
 // components contribute +-0 and are left out; the face basis is the same on both
 // faces up to the sign of the modes odd across them, and 1 for mode 1; u, v, w
 // share a reciprocal and the mass matrix has known ones.
-// 480 x 240: 254 us per launch, 286 with every slot read through L1 at every
+// 480 x 240: 246 us per launch, 286 with every slot read through L1 at every
 // point and none of the sharing.
 __device__ constexpr bool px3_zero(int d) { return d == 0 || d == 2 || d == 5 || d == 9; }
 __device__ constexpr bool py3_zero(int d) { return d == 0 || d == 1 || d == 3 || d == 6; }
@@ -404,9 +404,9 @@ __global__ void __launch_bounds__(64) k3_cell(const __grid_constant__ K3 K, doub
       s.v = gdf::rdiv(uG[2], rr, bad);
       s.w = gdf::rdiv(uG[3], rr, bad);
       if (bad) {   // an operand out of rdiv's range: the IEEE division itself
-        s.u = uG[1] / s.rho;
-        s.v = uG[2] / s.rho;
-        s.w = uG[3] / s.rho;
+        s.u = gdf::ieee_div(uG[1], s.rho);
+        s.v = gdf::ieee_div(uG[2], s.rho);
+        s.w = gdf::ieee_div(uG[3], s.rho);
       }
       s.E = uG[4];
       s.B1 = uG[5];
@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(64) k3_cell(const __grid_constant__ K3 K, doub
 #pragma unroll
     for (int d = 1; d < NQ3; ++d) q[d] = gdf::rdiv(du[d][n], gdf::Rcp{K.B.mm[d], K.rmm[d]}, bad);
 #pragma unroll
-    for (int d = 1; d < NQ3; ++d) du[d][n] = bad ? du[d][n] / K.B.mm[d] : q[d];
+    for (int d = 1; d < NQ3; ++d) du[d][n] = bad ? gdf::ieee_div(du[d][n], K.B.mm[d]) : q[d];
   }
   // the stage's combination over the 84 live slots (du = 0 beyond mode 10)
   const double c6 = KIND == KIND_LH ? 0.0 : sc->c6;

@@ -37,7 +37,7 @@ CY_SRC = os.path.join(CSRC, "gdf_cy.cu")
 HOST_SRC = os.path.join(CSRC, "gdf_host.cpp")
 IO_SRC = os.path.join(CSRC, "gdf_io.cpp")
 CYHOST_SRC = os.path.join(CSRC, "gdf_cy_host.cpp")
-HEADERS = [os.path.join(CSRC, f) for f in ("gdf_physics.cuh", "gdf_charlim.cuh", "gdf_kernels.cuh", "gdf_device.cuh",
+HEADERS = [os.path.join(CSRC, f) for f in ("gdf_physics.cuh", "gdf_charlim.cuh", "gdf_vertex.cuh", "gdf_kernels.cuh", "gdf_device.cuh",
                                                          "gdf_mlp.cuh", "gdf_p3_basis.h", "gdf_stage.h")] + [
     os.path.join(REPO, "include", "gdf.h"), os.path.join(REPO, "include", "gdf_p3.h"),
     os.path.join(REPO, "include", "gdf_cy.h")]

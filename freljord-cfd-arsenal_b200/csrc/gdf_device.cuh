@@ -10,6 +10,7 @@
 #include "gdf_charlim.cuh"
 #include "gdf_kernels.cuh"
 #include "gdf_mlp.cuh"
+#include "gdf_vertex.cuh"
 
 #include <mutex>
 
@@ -198,45 +199,66 @@ __device__ __forceinline__ void face_item(const Consts& K, const double* __restr
 // ------------------------------------------------------- vertex Ez -------
 // LhEz.f90:34-69: corner traces of the four cells around vertex (i,j),
 // i = 0..Nx, j = 0..Ny, and the 2-D Riemann solver.
-__device__ __forceinline__ void vertex_item(const Consts& K, const double* __restrict__ U, double* __restrict__ EzV,
-                                            long long item) {
+// Lane q of four (see gdf_vertex.cuh). Corner values of modes 1, 2,
+// 3 and 5 are +-1 (get_basis.f90: 1, x, y and x y at the corner): their products
+// are exact and written as sign changes.
+template <int FLUX, class DIV>
+__device__ __forceinline__ bool vertex_lane_as(const Consts& K, const double* __restrict__ U, long long item, int q,
+                                               double& Ez) {
   const int i = (int)(item % (K.nx + 1));
   const int j = (int)(item / (K.nx + 1));
-  const long long cLD = i + (long long)K.nx2 * j;  // cell (i,j): its RU corner
-  const long long cRD = cLD + 1;                   // (i+1,j): LU corner
-  const long long cLU = cLD + K.nx2;               // (i,j+1): RD corner
-  const long long cRU = cLU + 1;                   // (i+1,j+1): LD corner
-  double URU[NE], ULU[NE], URD[NE], ULD[NE];
+  const bool xr = !(q & 1), yu = q < 2;      // the cell is right of, above the vertex
+  const long long c = i + xr + (long long)K.nx2 * (j + yu);
+  const int sx = xr ? (int)0x80000000 : 0, sy = yu ? (int)0x80000000 : 0;
+  double u[NE], phi[NP];
+  // in registers: a choice among the tables inside the sums is a branch that
+  // keeps one variable's loads from starting before the last one's sum
+#pragma unroll
+  for (int d = 0; d < NP; ++d) {
+    const double ru = c_basis.phiRU[d], lu = c_basis.phiLU[d], rd = c_basis.phiRD[d], ld = c_basis.phiLD[d];
+    phi[d] = xr ? (yu ? ld : lu) : (yu ? rd : ru);
+  }
 #pragma unroll
   for (int n = 0; n < NE; ++n) {
-    double a = 0, b = 0, c = 0, e = 0;
+    double a = 0;
 #pragma unroll
     for (int d = 0; d < NP; ++d) {
       if (!live_mode(n, d)) continue;
-      const long long off = K.plane * (d + 10 * n);
-      if (GDF_FOLD_UNIT && (d == 0 || d == 1 || d == 2 || d == 4)) {
-        // corner values of modes 1, 2, 3 and 5 are +-1 (get_basis.f90):
-        // phiLD = (1,-1,-1,.,1), phiRD = (1,1,-1,.,-1), phiLU = (1,-1,1,.,-1),
-        // phiRU = (1,1,1,.,1); the products are exact and written out
-        const double xa = U[off + cRU], xb = U[off + cLU], xc = U[off + cRD], xe = U[off + cLD];
-        a = a + ((d == 1 || d == 2) ? -xa : xa);
-        b = b + ((d == 2 || d == 4) ? -xb : xb);
-        c = c + ((d == 1 || d == 4) ? -xc : xc);
-        e = e + xe;
-      } else {
-        a = a + U[off + cRU] * c_basis.phiLD[d];
-        b = b + U[off + cLU] * c_basis.phiRD[d];
-        c = c + U[off + cRD] * c_basis.phiLU[d];
-        e = e + U[off + cLD] * c_basis.phiRU[d];
-      }
+      const double v = U[K.plane * (d + 10 * n) + c];
+      if (d == 0) a = a + v;
+      else if (d == 1 || d == 2 || d == 4)
+        a = a + __hiloint2double(__double2hiint(v) ^ (d == 1 ? sx : d == 2 ? sy : sx ^ sy), __double2loint(v));
+      else
+        a = a + v * phi[d];
     }
-    URU[n] = a; ULU[n] = b; URD[n] = c; ULD[n] = e;
+    u[n] = a;
   }
-  // IEEE divisions: four solvers' worth of live state leaves no registers for
-  // the reciprocals (168 without spills; with them 352 bytes of spills, 1.27
-  // against 1.31 ms on the blast 2048^2 but 165 against 107 us on the rotor
-  // 512^2, whose quiet region sends a ring of vertices to the IEEE copy)
-  EzV[item] = vertex_ez(K.P, URU, ULU, URD, ULD);
+  return vertex_quad<FLUX, DIV>(K.P, u, Ez);
+}
+template <int FLUX>
+static __device__ __noinline__ double vertex_refused(const Consts& K, const double* __restrict__ U, long long item, int q) {
+  double Ez;
+  vertex_lane_as<FLUX, IeeeDiv>(K, U, item, q, Ez);
+  return Ez;
+}
+template <int FLUX>
+__device__ __forceinline__ void vertex_lane(const Consts& K, const double* __restrict__ U, double* __restrict__ EzV,
+                                            long long item, int q) {
+  const bool live = q == 0 && item < K.vplane;
+  if (item >= K.vplane) item = K.vplane - 1;   // the whole warp takes part
+  double Ez;
+  if (!vertex_lane_as<FLUX, SharedRcp>(K, U, item, q, Ez)) Ez = vertex_refused<FLUX>(K, U, item, q);
+  if (live) EzV[item] = Ez;
+}
+// for any solver
+__device__ __forceinline__ void vertex_at(const Consts& K, const double* __restrict__ U, double* __restrict__ EzV,
+                                          long long item, int q) {
+  switch (K.P.flux) {
+    case 1: return vertex_lane<1>(K, U, EzV, item, q);
+    case 2: return vertex_lane<2>(K, U, EzV, item, q);
+    case 3: return vertex_lane<3>(K, U, EzV, item, q);
+    default: return vertex_lane<4>(K, U, EzV, item, q);
+  }
 }
 
 // ------------------------------------------------ residual + combine -----

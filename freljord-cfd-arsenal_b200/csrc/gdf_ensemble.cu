@@ -99,8 +99,8 @@ __device__ __noinline__ void call_face_x(const Consts& K, const double* U, doubl
 __device__ __noinline__ void call_face_y(const Consts& K, const double* U, double* F, double* Ez, long long item) {
   face_item<1>(K, U, F, Ez, item);
 }
-__device__ __noinline__ void call_vertex(const Consts& K, const double* U, double* EzV, long long item) {
-  vertex_item(K, U, EzV, item);
+__device__ __noinline__ void call_vertex(const Consts& K, const double* U, double* EzV, long long item, int q) {
+  vertex_at(K, U, EzV, item, q);
 }
 extern __shared__ __align__(16) unsigned char ens_sm[];   // the stage kernel's dynamic shared memory
 __device__ __noinline__ void call_cell(const Consts& K, const double* U, double* U0, double* UI, const double* Fxh,
@@ -316,10 +316,7 @@ __global__ void __launch_bounds__(ENS_BS) k_ens_stage(const __grid_constant__ En
       }
     });
     for_tiles<true>(A, EK_VX, [&](int, const EnsInst& I, const Consts& K, long long base, int per) {
-      for (int k = threadIdx.x; k < per; k += ENS_BS) {
-        const long long item = base + k;
-        if (item < K.vplane) call_vertex(K, I.U, I.EzV, item);
-      }
+      for (int k = threadIdx.x; k < 4 * per; k += ENS_BS) call_vertex(K, I.U, I.EzV, base + (k >> 2), k & 3);
     });
     if (!ens_barrier(A, &s_ok)) return;
     // residual + RK combine; dEz + face-B combine
@@ -435,10 +432,7 @@ __global__ void __launch_bounds__(ENS_BS, 8) k_ep_faces(const __grid_constant__ 
     }
   });
   for_tiles<true>(A, EK_VX, [&](int, const EnsInst& I, const Consts& K, long long base, int per) {
-    for (int k = threadIdx.x; k < per; k += ENS_BS) {
-      const long long item = base + k;
-      if (item < K.vplane) vertex_item(K, I.U, I.EzV, item);
-    }
+    for (int k = threadIdx.x; k < 4 * per; k += ENS_BS) vertex_at(K, I.U, I.EzV, base + (k >> 2), k & 3);
   });
 }
 

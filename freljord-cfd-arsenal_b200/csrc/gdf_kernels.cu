@@ -87,12 +87,12 @@ __global__ void __launch_bounds__(FACE_BS, GDF_FACE_MINB) k_face(const __grid_co
   face_at<DIR>(K, U, Fh_out, Ez_out, f, threadIdx.x >> 5);
 }
 
+template <int FLUX>
 __global__ void __launch_bounds__(128, GDF_VERTEX_MINB) k_vertex(const __grid_constant__ Consts K, const double* __restrict__ U,
                                                 double* __restrict__ EzV, const Scal* __restrict__ sc) {
   if (sc && !sc->active) return;
-  const long long item = gtid();
-  if (item >= K.vplane) return;
-  vertex_item(K, U, EzV, item);
+  const long long t = gtid();
+  vertex_lane<FLUX>(K, U, EzV, t >> 2, (int)(t & 3));
 }
 
 __global__ void __launch_bounds__(CELL_BS, GDF_CELL_MINB) k_cell(const __grid_constant__ Consts K, const double* __restrict__ U,
@@ -632,7 +632,6 @@ void consts_for(const GdfConfig& c, Consts& K) { build_consts(c, K); }
 void basis_of(const Consts& K, Basis& B) {
   std::memcpy(B.w, K.w, sizeof(B.w));
   std::memcpy(B.lam, K.lam, sizeof(B.lam));
-  for (int q = 0; q < NG * NG; ++q) B.wq[q] = 0.25 * K.w[q / NG] * K.w[q % NG];
   std::memcpy(B.phiG, K.phiG, sizeof(B.phiG));
   std::memcpy(B.phiGLL, K.phiGLL, sizeof(B.phiGLL));
   std::memcpy(B.ppM, K.ppM, sizeof(B.ppM));
@@ -681,7 +680,10 @@ static int launch_faces(GdfHandle* h, const double* U, const Scal* sc) {
   if (!rc) rc = run_kernel(h, GDF_K_FACE_Y, [&] {
     k_face<1><<<nblk(K.fyplane, 32), FACE_BS, 0, h->st>>>(K, U, h->Fyh, h->EzUD, sc);
   });
-  if (!rc) rc = run_kernel(h, GDF_K_VERTEX, [&] { k_vertex<<<nblk(K.vplane, 128), 128, 0, h->st>>>(K, U, h->EzV, sc); });
+  if (!rc) rc = run_kernel(h, GDF_K_VERTEX, [&] {
+    const auto kv = K.P.flux == 1 ? k_vertex<1> : K.P.flux == 2 ? k_vertex<2> : K.P.flux == 3 ? k_vertex<3> : k_vertex<4>;
+    kv<<<nblk(4 * K.vplane, 128), 128, 0, h->st>>>(K, U, h->EzV, sc);
+  });
   return rc;
 }
 

@@ -56,7 +56,7 @@ struct Consts {
 // one copy (gdf_device.cuh c_basis) that every kernel reads from constant
 // memory. Consts keeps its own copy for the host.
 struct Basis {
-  double w[NG], lam[NG], wq[NG * NG];   // wq: 0.25 w(a) w(b)
+  double w[NG], lam[NG];
   double phiG[NG][NG][NP];
   double phiGLL[2][NG][NG][NP];
   double ppM[NP];

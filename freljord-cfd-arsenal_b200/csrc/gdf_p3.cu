@@ -33,6 +33,7 @@
 #include "../../include/gdf_p3.h"
 #include "gdf_p3_basis.h"
 #include "gdf_charlim.cuh"
+#include "gdf_vertex.cuh"
 #include "gdf_stage.h"
 
 namespace gdf {
@@ -315,19 +316,37 @@ __global__ void __launch_bounds__(Face3<DIR>::BS, Face3<DIR>::MINB) k3_face(cons
 }
 
 // -------------------------------------------------------------- vertices ---
-__global__ void __launch_bounds__(128) k3_vertex(const __grid_constant__ K3 K, const double* __restrict__ U,
-                                                 double* __restrict__ EzV, const Scal3* __restrict__ sc) {
-  if (sc && !sc->active) return;
-  const long long v = gtid();
-  if (v >= K.vplane) return;
+// four lanes per vertex (gdf_vertex.cuh)
+template <int FLUX, class DIV>
+__device__ __forceinline__ bool vertex_lane3_as(const K3& K, const double* __restrict__ U, long long v, int q, double& Ez) {
   const int i = (int)(v % (K.nx + 1)), j = (int)(v / (K.nx + 1));
-  const long long c = i + (long long)K.nx2 * j;
-  double URU[NE], ULU[NE], URD[NE], ULD[NE];
-  trace3(K, U, c + K.nx2 + 1, K.B.phiLD, URU);   // ULD of cell (i+1, j+1)
-  trace3(K, U, c + K.nx2, K.B.phiRD, ULU);       // URD of cell (i, j+1)
-  trace3(K, U, c + 1, K.B.phiLU, URD);           // ULU of cell (i+1, j)
-  trace3(K, U, c, K.B.phiRU, ULD);               // URU of cell (i, j)
-  EzV[v] = gdf::vertex_ez(K.P, URU, ULU, URD, ULD);
+  const bool xr = !(q & 1), yu = q < 2;      // the cell is right of, above the vertex
+  double phi[NP3], u[NE];
+#pragma unroll
+  for (int d = 0; d < NP3; ++d) {   // in registers: a choice of table at each use is a branch between the loads
+    const double ru = K.B.phiRU[d], lu = K.B.phiLU[d], rd = K.B.phiRD[d], ld = K.B.phiLD[d];
+    phi[d] = xr ? (yu ? ld : lu) : (yu ? rd : ru);
+  }
+  trace3(K, U, i + xr + (long long)K.nx2 * (j + yu), phi, u);
+  return gdf::vertex_quad<FLUX, DIV>(K.P, u, Ez);
+}
+template <int FLUX>
+static __device__ __noinline__ double vertex_refused3(const K3& K, const double* __restrict__ U, long long v, int q) {
+  double Ez;
+  vertex_lane3_as<FLUX, IeeeDiv>(K, U, v, q, Ez);
+  return Ez;
+}
+template <int FLUX>
+__global__ void __launch_bounds__(128) k3_vertex(const __grid_constant__ K3 K, const double* __restrict__ U,
+                                                  double* __restrict__ EzV, const Scal3* __restrict__ sc) {
+  if (sc && !sc->active) return;
+  long long v = gtid() >> 2;
+  const int q = threadIdx.x & 3;
+  const bool live = q == 0 && v < K.vplane;
+  if (v >= K.vplane) v = K.vplane - 1;   // the whole warp takes part
+  double Ez;
+  if (!vertex_lane3_as<FLUX, SharedRcp>(K, U, v, q, Ez)) Ez = vertex_refused3<FLUX>(K, U, v, q);
+  if (live) EzV[v] = Ez;
 }
 
 // ------------------------------------------------------------------ cells --
@@ -1112,7 +1131,10 @@ int launch_lh_body(GdfP3Handle* h, int kind, const Scal3* sc) {
   const K3& K = h->K;
   int rc = run(h, [&] { k3_face<0><<<nblk(K.fxplane * NG, Face3<0>::BS), Face3<0>::BS, 0, h->st>>>(K, h->U, h->Fxh, sc); });
   if (!rc) rc = run(h, [&] { k3_face<1><<<nblk(K.fyplane, 32), Face3<1>::BS, 0, h->st>>>(K, h->U, h->Fyh, sc); });
-  if (!rc) rc = run(h, [&] { k3_vertex<<<nblk(K.vplane, 128), 128, 0, h->st>>>(K, h->U, h->EzV, sc); });
+  if (!rc) rc = run(h, [&] {
+    const auto kv = K.P.flux == 1 ? k3_vertex<1> : K.P.flux == 2 ? k3_vertex<2> : K.P.flux == 3 ? k3_vertex<3> : k3_vertex<4>;
+    kv<<<nblk(4 * K.vplane, 128), 128, 0, h->st>>>(K, h->U, h->EzV, sc);
+  });
   if (rc) return rc;
   const unsigned nc = nblk((long long)K.nx * K.ny, 64), nf = nblk(K.fxplane + K.fyplane, 128);
   h->launches++;  // the pair below is two launches

@@ -106,6 +106,19 @@ __global__ void __launch_bounds__(CELL_BS, GDF_CELL_MINB) k_cell(const __grid_co
   cell_item(K, U, U0, UI, Fxh, Fyh, duout, sc, stage, item, ms);
 }
 
+// 128 registers a thread (four blocks per SM; 150 for three were no faster at 128^2
+// and below, and 14% slower at 192^2)
+__global__ void __launch_bounds__(PAIR_BS, 4) k_cell_pair(const __grid_constant__ Consts K, const double* __restrict__ U,
+                                                  double* __restrict__ U0, double* __restrict__ UI,
+                                                  const double* __restrict__ Fxh, const double* __restrict__ Fyh,
+                                                  double* __restrict__ duout, const Scal* __restrict__ sc, int stage) {
+  __shared__ __align__(16) double ms[PAIR_SLOTS * PAIR_BS];
+  if (sc && !sc->active) return;
+  const int t = threadIdx.x;
+  const long long item = (long long)blockIdx.x * (PAIR_BS / 2) + (t >> 5) * 16 + (t & 15);
+  cell_pair(K, U, U0, UI, Fxh, Fyh, duout, sc, stage, item, (t >> 4) & 1, ms);
+}
+
 __global__ void __launch_bounds__(128) k_bface(const __grid_constant__ Consts K, const double* __restrict__ EzRL,
                                                const double* __restrict__ EzUD, const double* __restrict__ EzV,
                                                double* __restrict__ BX, double* __restrict__ BX0,
@@ -671,6 +684,20 @@ static int launch_set_bc(GdfHandle* h, double* U, int zeroB, const Scal* sc) {
   return run_kernel(h, GDF_K_SET_BC, [&] { k_set_bc<<<nblk(n, 256), 256, 0, h->st>>>(h->K, U, zeroB, sc); });
 }
 
+// Two lanes to a cell while three of k_cell_pair's blocks per SM hold the grid (12
+// warps): there one cell's chain of operations is what a launch waits for.
+// Orszag-Tang 64^2 36.5 against 43.7 us per launch, 128^2 40.7 and 45.3, 160^2 51.4
+// and 54.0; 192^2, whose blocks are four to an SM, 61.8 and 54.7; above, the
+// two are within 3% of each other either way.
+constexpr long long PAIR_CELLS = 148LL * 3 * (PAIR_BS / 2);
+static void launch_cell(const Consts& K, const double* U, double* U0, double* UI, const double* Fxh, const double* Fyh,
+                        double* duout, const Scal* sc, int stage, cudaStream_t st) {
+  if (K.plane <= PAIR_CELLS)
+    k_cell_pair<<<nblk(K.plane, PAIR_BS / 2), PAIR_BS, 0, st>>>(K, U, U0, UI, Fxh, Fyh, duout, sc, stage);
+  else
+    k_cell<<<nblk(K.plane, CELL_BS), CELL_BS, 0, st>>>(K, U, U0, UI, Fxh, Fyh, duout, sc, stage);
+}
+
 // Lh traces/Riemann (Fxhat, Fyhat, EzRL, EzUD) and LhEz vertex Ez on U
 static int launch_faces(GdfHandle* h, const double* U, const Scal* sc) {
   const Consts& K = h->K;
@@ -772,7 +799,7 @@ static int launch_stage(GdfHandle* h, int stage) {
   }
   if ((rc = launch_faces(h, h->U, h->sc))) return rc;
   rc = run_kernel(h, GDF_K_CELL, [&] {
-    k_cell<<<nblk(K.plane, CELL_BS), CELL_BS, 0, h->st>>>(K, h->U, h->U0, h->UI, h->Fxh, h->Fyh, nullptr, h->sc, stage);
+    launch_cell(K, h->U, h->U0, h->UI, h->Fxh, h->Fyh, nullptr, h->sc, stage, h->st);
   });
   if (!rc) rc = run_kernel(h, GDF_K_BFACE, [&] {
     k_bface<<<nblk(K.fxplane + K.fyplane, 128), 128, 0, h->st>>>(K, h->EzRL, h->EzUD, h->EzV, h->BX, h->BX0, h->BXI,
@@ -1215,7 +1242,7 @@ int gdf_lh_noalloc(const GdfConfig* cfg, const double* d_uh, double* d_du, void*
   CK(cudaMemsetAsync(d_du, 0, uh_bytes(*cfg), st));
   k_face<0><<<nblk(fx, 32), FACE_BS, 0, st>>>(K, d_uh, Fxh, ezx, nullptr);
   k_face<1><<<nblk(fy, 32), FACE_BS, 0, st>>>(K, d_uh, Fyh, ezy, nullptr);
-  k_cell<<<nblk(K.plane, CELL_BS), CELL_BS, 0, st>>>(K, d_uh, nullptr, nullptr, Fxh, Fyh, d_du, nullptr, 0);
+  launch_cell(K, d_uh, nullptr, nullptr, Fxh, Fyh, d_du, nullptr, 0, st);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(GDF_ERR_CUDA, std::string("gdf_lh_noalloc launch: ") + cudaGetErrorString(e));
   return GDF_OK;
@@ -1339,8 +1366,7 @@ int gdf_lh(GdfHandle* h, const double* uh, double* du) {
   CK(cudaMemsetAsync(h->UI, 0, ub, h->st));  // du (ghost and dead entries stay 0)
   if ((rc = launch_faces(h, h->UT, nullptr))) return rc;
   rc = run_kernel(h, GDF_K_CELL, [&] {
-    k_cell<<<nblk(h->K.plane, CELL_BS), CELL_BS, 0, h->st>>>(h->K, h->UT, nullptr, nullptr, h->Fxh, h->Fyh, h->UI,
-                                                             nullptr, 0);
+    launch_cell(h->K, h->UT, nullptr, nullptr, h->Fxh, h->Fyh, h->UI, nullptr, 0, h->st);
   });
   if (rc) return rc;
   CK(gdf::d2h(du, h->UI, ub, h->st));

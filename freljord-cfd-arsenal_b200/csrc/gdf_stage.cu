@@ -15,6 +15,7 @@ namespace {
 struct Ring {
   std::mutex mu;
   int holders = 0;
+  size_t asked = 0;   // bytes asked for since it was last dropped
   char* buf[STAGE_SLOTS] = {};
   cudaEvent_t ev[STAGE_SLOTS] = {};
   bool ready = false;
@@ -33,6 +34,7 @@ void drop(Ring& r) {
     r.buf[k] = nullptr;
   }
   r.ready = false;
+  r.asked = 0;
   cudaGetLastError();
 }
 
@@ -64,7 +66,10 @@ Ring* take(const void* host, size_t bytes, std::unique_lock<std::mutex>& lk) {
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEV) return nullptr;
   Ring& r = g_ring[dev];
   lk = std::unique_lock<std::mutex>(r.mu, std::try_to_lock);
-  if (!lk.owns_lock() || r.holders == 0 || !make(r)) return nullptr;
+  if (!lk.owns_lock() || r.holders == 0) return nullptr;
+  r.asked += std::min(bytes, STAGE_MAKE);
+  if (r.asked < STAGE_MAKE || !make(r)) return nullptr;
+  r.asked = STAGE_MAKE;
   return &r;
 }
 

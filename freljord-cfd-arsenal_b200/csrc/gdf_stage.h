@@ -15,7 +15,7 @@
 namespace gdf {
 
 // Keeps the current device's ring for as long as it lives: the ring (STAGE_SLOTS
-// x STAGE_CHUNK bytes, made on first use) is freed with the last of its holders.
+// x STAGE_CHUNK bytes, made after STAGE_MAKE bytes) is freed with the last of its holders.
 // Every handle holds one.
 struct StageRef {
   StageRef();
@@ -30,6 +30,10 @@ struct StageRef {
 constexpr size_t STAGE_CHUNK = (size_t)4 << 20;
 constexpr int STAGE_SLOTS = 4;
 constexpr size_t STAGE_MIN = (size_t)1 << 20;   // below: one plain copy (the ring's hand-overs cost more)
+// The ring is made once its holders have asked it for this much: making and
+// freeing it takes some 18 ms, what it saves on about this many bytes, and a
+// handle that is made, copied from once and closed would pay that each time.
+constexpr size_t STAGE_MAKE = (size_t)64 << 20;
 
 // host -> device, ordered on st; src may be reused on return
 cudaError_t h2d(void* dst, const void* src, size_t bytes, cudaStream_t st);

@@ -625,8 +625,8 @@ __global__ void __launch_bounds__(CY_CELL_BS) k_cy_cell(const __grid_constant__ 
   }
   // the stage's combination, a variable's (then the cubic slots') six values
   // at a time: their loads are all under way before the first store (192^2 x
-  // 2: 153-156 us per launch, 149-201 with each value stored before the next
-  // was loaded)
+  // 2, before the surface sums were rolled: 153-156 us per launch, 149-201 with
+  // each value stored before the next was loaded; 114-124 now)
   const double dt = sc->dt;
 #pragma unroll
   for (int n = 0; n <= NE; ++n) {

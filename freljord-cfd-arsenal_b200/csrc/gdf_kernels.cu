@@ -9,14 +9,20 @@
 //         k_face<0>, k_face<1>                Lh traces + Riemann (Fxhat,
 //                                             Fyhat) + LhEz face Ez
 //         k_vertex                            LhEz vertex Ez (2-D solvers)
-//         k_cell                              Lh volume + surface integral,
+//         k_cell or k_cell_pair               Lh volume + surface integral,
 //                                             fused with the RK combine
 //         k_bface                             LhEz dEz + face-B combine
-//         k_limit                             TVB_Limiter_P2 (+KXRCF, +pp)
-//                                             fused with div_free_Balsara
+//         k_limit                             KXRCF (or the learned gate);
+//                                             lists the gated cells
+//         k_limit_tvb                         TVB_Limiter_P2 of those
+//         k_pp                                pp_Limiter of the cells both listed
+//                                             (div_free_Balsara is fused with
+//                                             the last of the three a cell meets)
+//         k_set_bc, k_faceb_limit, k_divfree  with the face-B minmod on
 //         k_set_bc ]
-// Every kernel is one thread per item (face point, vertex, cell, face) and
-// computes that item sequentially in the reference's order, so a build with
+// Every kernel is one thread per item (face point, cell, face), four lanes per
+// vertex, two per cell of a small grid or one warp per cell of k_pp, and
+// keeps the order of the reference's operations, so a build with
 // --fmad=false reproduces the reference arithmetic value for value.
 // All device waits are stream-ordered; no kernel spins.
 
@@ -229,7 +235,7 @@ __global__ void __launch_bounds__(LIM_BS, 8) k_limit(const __grid_constant__ Con
                       nullptr, LimList<int32_t>{list, count, 0}, pp);
 }
 
-// The limiting pass, one cell per thread: the cells k_limit<LM, true> deferred
+// The limiting pass, one cell per thread: the cells k_limit<LM> listed
 // (the grid covers every interior cell; threads past the count return), or,
 // with list null (GDF_DETECT_ALL), every interior cell.
 __global__ void __launch_bounds__(LIM_BS, GDF_LIMIT_MINB) k_limit_tvb(const __grid_constant__ Consts K,

@@ -523,7 +523,7 @@ __device__ __forceinline__ void cell_item(const Consts& K, const double* __restr
 // dependent operations halve, and twice the warps run, for 15% more operations.
 // Operations and their order are those of cell_item; a sum of one lane that the
 // other one's variables do not have adds zeros.
-// A whole warp comes here together.
+// A whole warp comes here together. phix, phiy: K's tables, or the caller's copy.
 constexpr int PAIR_BS = 128, PAIR_SLOTS = 26;
 __device__ __forceinline__ double flip_if(double v, bool neg) {
   return __hiloint2double(__double2hiint(v) ^ (neg ? (int)0x80000000 : 0), __double2loint(v));
@@ -531,7 +531,8 @@ __device__ __forceinline__ double flip_if(double v, bool neg) {
 __device__ __forceinline__ void cell_pair(const Consts& K, const double* __restrict__ U, double* __restrict__ U0,
                                           double* __restrict__ UI, const double* __restrict__ Fxh,
                                           const double* __restrict__ Fyh, double* __restrict__ duout,
-                                          const Scal* __restrict__ sc, int stage, long long item, int r, double* ms) {
+                                          const Scal* __restrict__ sc, int stage, long long item, int r, double* ms,
+                                          const double (*phix)[NG][NP], const double (*phiy)[NG][NP]) {
   const int tid = threadIdx.x;
   const bool live = item < K.plane;
   if (!live) item = K.plane - 1;
@@ -611,8 +612,8 @@ __device__ __forceinline__ void cell_pair(const Consts& K, const double* __restr
         Fx[3] = r ? ez : 0.0;
         Fy[3] = r ? 0.0 : -ez;
         const double coef = 0.25 * c_basis.w[a] * c_basis.w[b];
-        const double* px = K.phix[a][b];
-        const double* py = K.phiy[a][b];
+        const double* px = phix[a][b];
+        const double* py = phiy[a][b];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           double* d = du + 6 * k;

@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(PAIR_BS, 4) k_cell_pair(const __grid_constant_
   if (sc && !sc->active) return;
   const int t = threadIdx.x;
   const long long item = (long long)blockIdx.x * (PAIR_BS / 2) + (t >> 5) * 16 + (t & 15);
-  cell_pair(K, U, U0, UI, Fxh, Fyh, duout, sc, stage, item, (t >> 4) & 1, ms);
+  cell_pair(K, U, U0, UI, Fxh, Fyh, duout, sc, stage, item, (t >> 4) & 1, ms, K.phix, K.phiy);
 }
 
 __global__ void __launch_bounds__(128) k_bface(const __grid_constant__ Consts K, const double* __restrict__ EzRL,

@@ -667,7 +667,8 @@ __device__ __forceinline__ void cell_pair(const Consts& K, const double* __restr
             add(along, l1 - l0);
             add(4, l1 + l0);
           }
-          if (k == 3) {
+          // the modes even across the face are odd along it, so zero at the middle point
+          if (k == 3 && (odd || g != 2)) {
             add(6, q1[k] * fe0 + flip_if(q0[k] * fe0, !odd));
             add(7, q1[k] * fe1 + flip_if(q0[k] * fe1, !odd));
           }

@@ -1,0 +1,55 @@
+"""Residuals of states in which some values are infinite or so large that
+fluxes overflow. The zeros of the basis decide there which entries of Lh turn
+NaN (0 x inf): every form of a residual kernel leaves out the same zeros."""
+import numpy as np
+import pytest
+
+import gdf
+
+pytestmark = pytest.mark.gpu
+
+
+def spoil(uh, live, rng, how):
+    """A smooth state of order one, then a few modes made infinite or huge."""
+    sh = uh.shape[2:]
+    for n in range(8):
+        for d in range(uh.shape[1]):
+            if live(n, d):
+                uh[n, d] = rng.normal(0, 0.05 if d else 0.3, sh)
+    uh[0, 0] += 1.2
+    uh[4, 0] += 3.0
+    uh[5, 0] += 0.5
+    for n in range(8):
+        for d in range(uh.shape[1]):
+            if live(n, d):
+                hit = rng.random(sh) < 0.003
+                if how == "inf":
+                    uh[n, d][hit] = rng.choice([np.inf, -np.inf], hit.sum())
+                else:
+                    uh[n, d][hit] *= 10.0 ** rng.uniform(150, 300, hit.sum())
+
+
+def p2_live(n, d):
+    return d < 6 or (n == 5 and d in (6, 8)) or (n == 6 and d in (7, 9))
+
+
+# up to 28416 cells, ghosts included, two lanes take a cell, above it one lane:
+# a block of a large grid and the small grid of the same cells and neighbours
+@pytest.mark.parametrize("how", ["inf", "huge"])
+@pytest.mark.parametrize("flux", [gdf.FLUX_LF, gdf.FLUX_HLL, gdf.FLUX_HLLC, gdf.FLUX_HLLD])
+def test_p2_forms_agree(flux, how):
+    def lh(uh):
+        nx, ny = uh.shape[3] - 2, uh.shape[2] - 2
+        cfg, _ = gdf.problem_config(gdf.PROB_ROTOR, nx, ny)
+        cfg.flux_type = flux
+        cfg.xa, cfg.xb, cfg.ya, cfg.yb = 0.0, nx / 128, 0.0, ny / 128   # the same cell size at any nx, ny
+        return gdf.Solver(cfg).lh(uh)
+
+    uh, _, _ = gdf._abi.new_state(200, 160)
+    spoil(uh, p2_live, np.random.default_rng(flux), how)
+    big = lh(uh)
+    assert not np.isfinite(big).all()
+    for nx, ny, i, j in ((40, 41, 0, 0), (150, 120, 31, 17), (7, 5, 190, 150)):
+        small = lh(np.ascontiguousarray(uh[:, :, j:j + ny + 2, i:i + nx + 2]))
+        inner = (slice(None), slice(None), slice(1, -1), slice(1, -1))
+        assert np.array_equal(small[inner], big[:, :, j + 1:j + ny + 1, i + 1:i + nx + 1], equal_nan=True)

@@ -449,6 +449,16 @@ __global__ void __launch_bounds__(64) k3_cell(const __grid_constant__ K3 K, doub
         }
       }
     }
+  // The products left out above are 0 x flux: NaN where the flux is not finite.
+  // Such an x (y) flux has left mode 2's (3's) sum, which has no zero, not
+  // finite either, so a cell is looked over once, not at each point.
+#pragma unroll
+  for (int n = 0; n < NE; ++n) {
+    const bool ix = n != 5 && !isfinite(du[1][n]), iy = n != 6 && !isfinite(du[2][n]);
+#pragma unroll
+    for (int d = 1; d < NQ3; ++d)
+      if ((ix && px3_zero(d)) || (iy && py3_zero(d))) du[d][n] = nan("");
+  }
   // surface integrals (main.f90:2232-2258): x faces of the cell, then y faces;
   // F1 the flux on the high face, F0 on the low one
   auto surface = [&](const double* F1, const double* F0, double cw, const double* f, bool x) {

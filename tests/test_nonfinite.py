@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 import gdf
+from oracle import OracleP3
 
 pytestmark = pytest.mark.gpu
 
@@ -53,3 +54,18 @@ def test_p2_forms_agree(flux, how):
         small = lh(np.ascontiguousarray(uh[:, :, j:j + ny + 2, i:i + nx + 2]))
         inner = (slice(None), slice(None), slice(1, -1), slice(1, -1))
         assert np.array_equal(small[inner], big[:, :, j + 1:j + ny + 1, i + 1:i + nx + 1], equal_nan=True)
+
+
+# the oracle multiplies by every zero
+@pytest.mark.parametrize("how", ["inf", "huge"])
+@pytest.mark.parametrize("flux", [gdf.FLUX_LF, gdf.FLUX_HLL, gdf.FLUX_HLLC, gdf.FLUX_HLLD])
+@pytest.mark.parametrize("nx,ny", [(7, 5), (33, 18)])
+def test_p3_equals_oracle(nx, ny, flux, how):
+    from gdf import p3
+    cfg, _ = p3.p3_problem_config(gdf.PROB_ROTOR, nx, ny)
+    cfg.flux_type = flux
+    uh, bx, by = p3.p3_new_state(nx, ny)
+    live = p3.p3_live_mask()
+    spoil(uh, lambda n, d: live[n, d], np.random.default_rng(nx + flux), how)
+    for a, b in zip(p3.P3Solver(cfg).lh(uh, bx, by), OracleP3(cfg).lh(uh, bx, by)):
+        assert np.array_equal(a, b, equal_nan=True)

@@ -163,17 +163,18 @@ __device__ __forceinline__ double fourier(const KC& K, double v, int kk, double 
   return acc;
 }
 
-// conserved (r*B1, r*B2 in slots 5, 6) -> primitives at radius rad
+// conserved (r*B1, r*B2 in slots 5, 6) -> primitives at radius rad; far: rad is
+// out of rdiv's range (0 on the axis), so rrad is not to be used
 struct PrimC {
   double rho, u, v, w, E, B1, B2, B3, rB1, rB2, rB3, S, T, K;
 };
-__device__ __forceinline__ void prim_c(const Phys& P, const double* U, double rad, const Rcp& rrad, bool dquirk,
-                                       PrimC& q) {
+__device__ __forceinline__ void prim_c(const Phys& P, const double* U, double rad, const Rcp& rrad, unsigned far,
+                                       bool dquirk, PrimC& q) {
   q.rho = U[0];
   q.E = U[4];
   q.rB1 = U[5];
   q.rB2 = U[6];
-  unsigned bad = 0;
+  unsigned bad = far;
   const Rcp rr = gdf::rcp_of(q.rho, bad);
   q.u = gdf::rdiv(U[1], rr, bad);
   q.v = gdf::rdiv(U[2], rr, bad);
@@ -345,8 +346,8 @@ __global__ void __launch_bounds__(128) k_cy_face(const __grid_constant__ KC K, c
     PrimC pa, pb;
     unsigned far = 0;
     const Rcp rre = gdf::rcp_of(re, far);
-    prim_c(K.P, UA, re, rre, false, pa);
-    prim_c(K.P, UB, re, rre, DIR == 1, pb);   // Lh.f90:284: the D side's pressure takes -w^2
+    prim_c(K.P, UA, re, rre, far, false, pa);
+    prim_c(K.P, UB, re, rre, far, DIR == 1, pb);   // Lh.f90:284: the D side's pressure takes -w^2
     double FA[NE], FB[NE];
     if (DIR == 0) { flux_r(pa, UA, FA); flux_r(pb, UB, FB); }
     else { flux_z(pa, UA, FA); flux_z(pb, UB, FB); }
@@ -516,7 +517,7 @@ __global__ void __launch_bounds__(CY_CELL_BS) k_cy_cell(const __grid_constant__ 
         Uv[n] = s;
       }
       PrimC pq;
-      prim_c(K.P, Uv, rad, rrad, false, pq);
+      prim_c(K.P, Uv, rad, rrad, far, false, pq);
       double Fx[NE], Fy[NE], Fz[NE];
       flux_r(pq, Uv, Fx);
       flux_z(pq, Uv, Fy);

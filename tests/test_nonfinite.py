@@ -5,13 +5,13 @@ import numpy as np
 import pytest
 
 import gdf
-from oracle import OracleP3
+from oracle import OracleCy, OracleP3
 
 pytestmark = pytest.mark.gpu
 
 
 def spoil(uh, live, rng, how):
-    """A smooth state of order one, then a few modes made infinite or huge."""
+    """A smooth state of order one, then (how "inf", "huge") a few modes made so."""
     sh = uh.shape[2:]
     for n in range(8):
         for d in range(uh.shape[1]):
@@ -20,6 +20,8 @@ def spoil(uh, live, rng, how):
     uh[0, 0] += 1.2
     uh[4, 0] += 3.0
     uh[5, 0] += 0.5
+    if how == "none":
+        return
     for n in range(8):
         for d in range(uh.shape[1]):
             if live(n, d):
@@ -68,4 +70,21 @@ def test_p3_equals_oracle(nx, ny, flux, how):
     live = p3.p3_live_mask()
     spoil(uh, lambda n, d: live[n, d], np.random.default_rng(nx + flux), how)
     for a, b in zip(p3.P3Solver(cfg).lh(uh, bx, by), OracleP3(cfg).lh(uh, bx, by)):
+        assert np.array_equal(a, b, equal_nan=True)
+
+
+# r B / r on the axis: a face there at an even nr
+@pytest.mark.parametrize("nr,nz,lphi", [(2, 3, 1), (16, 9, 2), (34, 20, 1)])
+@pytest.mark.parametrize("flux", [0, 1, 2], ids=["central", "lf", "hll"])
+def test_cylindrical_axis_equals_oracle(flux, nr, nz, lphi):
+    from gdf import cy
+    cfg, _ = cy.cy_problem_config(cy.CY_SMOOTH_VORTEX, nr, nz, lphi)   # r from -5 to 5
+    cfg.flux_type = flux
+    assert nr % 2 or cfg.ra + (nr // 2) * ((cfg.rb - cfg.ra) / nr) == 0.0
+    uh, br, bz = cy.cy_new_state(nr, nz, lphi)
+    live = cy.cy_live_mask()
+    spoil(uh, lambda n, d: live[n, d], np.random.default_rng(nr + flux), "none")
+    got = cy.CySolver(cfg).lh(uh, br, bz)
+    assert np.isinf(got[0]).any()
+    for a, b in zip(got, OracleCy(cfg).lh(uh.copy(), 0.0)):
         assert np.array_equal(a, b, equal_nan=True)

@@ -465,6 +465,38 @@ __device__ __forceinline__ double combine(int KIND, double u, double du, double 
 #endif
 constexpr int CY_CELL_BS = GDF_CY_STAGE ? 64 : 128;
 
+// Which fluxes of one cell plane are not finite at some Gauss point: bit n in r,
+// bit 8 + n in z. Its slots start at m, st apart. Out of line: k_cy_cell asks
+// only where a sum is not finite.
+static __device__ __noinline__ unsigned cy_flux_overflow(const KC& K, const double* m, long long st, double rc) {
+  unsigned bits = 0;
+#pragma unroll 1
+  for (int q = 0; q < NG * NG; ++q) {
+    const double* G = K.B.phiG[q / NG][q % NG];
+    const double rad = rc + K.hr1 * K.B.lam[q / NG];
+    double Uv[NE];
+#pragma unroll
+    for (int n = 0; n < NE; ++n) {
+      double s = 0.0;
+#pragma unroll
+      for (int d = 0; d < NPC; ++d) {
+        const int sl = slotc(n, d);
+        if (sl >= 0) s = s + m[sl * st] * G[d];
+      }
+      Uv[n] = s;
+    }
+    PrimC pq;
+    prim_c(K.P, Uv, rad, Rcp{rad, 0.0}, 1, false, pq);
+    double Fx[NE], Fy[NE];
+    flux_r(pq, Uv, Fx);
+    flux_z(pq, Uv, Fy);
+#pragma unroll
+    for (int n = 0; n < NE; ++n)
+      bits |= (unsigned)!isfinite(Fx[n]) << n | (unsigned)!isfinite(Fy[n]) << (8 + n);
+  }
+  return bits;
+}
+
 template <int KIND, int LP>
 __global__ void __launch_bounds__(CY_CELL_BS) k_cy_cell(const __grid_constant__ KC K, double* __restrict__ U,
                                                         double* __restrict__ X, double* __restrict__ U0,
@@ -573,6 +605,20 @@ __global__ void __launch_bounds__(CY_CELL_BS) k_cy_cell(const __grid_constant__ 
     }
   }
   if (!valid) return;
+  // The products left out above are 0 x flux: NaN where the flux is not finite.
+  // Such a flux has left mode 2's (r) or 3's (z) sum not finite either.
+  bool odd_sum = false;
+#pragma unroll
+  for (int n = 0; n < NE; ++n) odd_sum = odd_sum || !isfinite(du[n][1]) || !isfinite(du[n][2]);
+  if (odd_sum) {
+    const unsigned bits = cy_flux_overflow(K, GDF_CY_STAGE ? cms + threadIdx.x : U + cp,
+                                           GDF_CY_STAGE ? (long long)CY_CELL_BS : K.ncp, rc);
+#pragma unroll
+    for (int n = 0; n < NE; ++n) {
+      if (bits >> n & 1) du[n][2] = du[n][5] = nan("");
+      if (bits >> (8 + n) & 1) du[n][1] = du[n][3] = nan("");
+    }
+  }
   // surface terms (Lh.f90:370-407; var 8 from the edge fields, LhEz.f90:37-55),
   // x faces, then y faces, a point at a time for all variables: one copy of the
   // code per direction (unrolled over the points as well it did not fit the

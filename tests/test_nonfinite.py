@@ -88,3 +88,18 @@ def test_cylindrical_axis_equals_oracle(flux, nr, nz, lphi):
     assert np.isinf(got[0]).any()
     for a, b in zip(got, OracleCy(cfg).lh(uh.copy(), 0.0)):
         assert np.array_equal(a, b, equal_nan=True)
+
+
+# off the axis, with infinite and overflowing fluxes
+@pytest.mark.parametrize("nr,nz,lphi", [(7, 5, 2), (16, 9, 4), (33, 18, 1)])
+@pytest.mark.parametrize("how", ["inf", "huge"])
+@pytest.mark.parametrize("flux", [0, 1, 2], ids=["central", "lf", "hll"])
+def test_cylindrical_equals_oracle(flux, how, nr, nz, lphi):
+    from gdf import cy
+    cfg, _ = cy.cy_problem_config(cy.CY_SMOOTH_VORTEX, nr, nz, lphi)
+    cfg.flux_type, cfg.ra, cfg.rb = flux, 1.0, 11.0
+    uh, br, bz = cy.cy_new_state(nr, nz, lphi)
+    live = cy.cy_live_mask()
+    spoil(uh, lambda n, d: live[n, d], np.random.default_rng(nr + flux), how)
+    for a, b in zip(cy.CySolver(cfg).lh(uh, br, bz), OracleCy(cfg).lh(uh.copy(), 0.0)):
+        assert np.array_equal(a, b, equal_nan=True)

@@ -986,6 +986,8 @@ static __device__ bool kxrcf_flag(const Consts& K, const double* __restrict__ S,
   }
   const double pL = K.pow_hxhy * Lij;
   const double cd = K.ck * pL;
+  // squares are compared where theirs neither over- nor underflow
+  const bool tame = cd > 1e-100 && cd < 1e100;
 #pragma unroll 1
   for (int n = 0; n < NE; ++n) {
     const int cubic = n == 5 ? 1 : n == 6 ? 2 : 0;
@@ -1021,7 +1023,7 @@ static __device__ bool kxrcf_flag(const Consts& K, const double* __restrict__ S,
     }
     const double a = fabs(I);
     if (a > cd * (up + 1e-12) * (1.0 + 1e-9)) return true;
-    if (cd > 0.0 && (a < cd * 1e-12 * (1.0 - 1e-9) || a * a < cd * cd * ms * (1.0 - 1e-8))) continue;
+    if (tame && (a < cd * 1e-12 * (1.0 - 1e-9) || (ms < 1e200 && a * a < cd * cd * ms * (1.0 - 1e-8)))) continue;
     double uinf = 0.0;
 #pragma unroll 1
     for (int q = 0; q < NG * NG; ++q) {

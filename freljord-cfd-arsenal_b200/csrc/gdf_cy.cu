@@ -1558,7 +1558,7 @@ int upload_cells(GdfCyHandle* h, const double* uh, double* D) {
         continue;
       }
       while (e < NPC && slotc(n, e) == s + (e - d)) ++e;
-      CKC(gdf::h2d(D + pl * s, src, pl * (e - d) * sizeof(double), h->st));
+      CKC(h->stage.h2d(D + pl * s, src, pl * (e - d) * sizeof(double), h->st));
     }
   CKC(cudaStreamSynchronize(h->st));
   return GDF_OK;
@@ -1577,7 +1577,7 @@ int download_cells(GdfCyHandle* h, const double* D, double* uh) {
         continue;
       }
       while (e < NPC && slotc(n, e) == s + (e - d)) ++e;
-      CKC(gdf::d2h(dst, D + pl * s, pl * (e - d) * sizeof(double), h->st));
+      CKC(h->stage.d2h(dst, D + pl * s, pl * (e - d) * sizeof(double), h->st));
     }
   CKC(cudaStreamSynchronize(h->st));
   return GDF_OK;
@@ -1661,8 +1661,8 @@ int gdf_cy_upload(GdfCyHandle* h, const double* uh, const double* br, const doub
   if (!h || !uh || !br || !bz) return fail(GDF_ERR_ARG, "null argument");
   int rc = upload_cells(h, uh, h->U);
   if (rc) return rc;
-  CKC(gdf::h2d(h->BR, br, br_bytes(h->K), h->st));
-  CKC(gdf::h2d(h->BZ, bz, bz_bytes(h->K), h->st));
+  CKC(h->stage.h2d(h->BR, br, br_bytes(h->K), h->st));
+  CKC(h->stage.h2d(h->BZ, bz, bz_bytes(h->K), h->st));
   h->sc_host->t = 0;
   h->sc_host->dt = 0;
   h->sc_host->active = 1;
@@ -1679,8 +1679,8 @@ int gdf_cy_download(GdfCyHandle* h, double* uh, double* br, double* bz) {
   if (!h->uploaded) return fail(GDF_ERR_STATE, "no state uploaded");
   int rc = download_cells(h, h->U, uh);
   if (rc) return rc;
-  CKC(gdf::d2h(br, h->BR, br_bytes(h->K), h->st));
-  CKC(gdf::d2h(bz, h->BZ, bz_bytes(h->K), h->st));
+  CKC(h->stage.d2h(br, h->BR, br_bytes(h->K), h->st));
+  CKC(h->stage.d2h(bz, h->BZ, bz_bytes(h->K), h->st));
   CKC(cudaStreamSynchronize(h->st));
   return GDF_OK;
 }
@@ -1787,8 +1787,8 @@ int gdf_cy_lh(GdfCyHandle* h, const double* uh, const double* br, const double* 
   const KC& K = h->K;
   int rc = upload_cells(h, uh, h->U);
   if (rc) return rc;
-  CKC(gdf::h2d(h->BR, br, br_bytes(K), h->st));
-  CKC(gdf::h2d(h->BZ, bz, bz_bytes(K), h->st));
+  CKC(h->stage.h2d(h->BR, br, br_bytes(K), h->st));
+  CKC(h->stage.h2d(h->BZ, bz, bz_bytes(K), h->st));
   CKC(cudaMemsetAsync(h->T, 0, cell_plane_bytes(K) * NSC, h->st));
   if ((rc = sync_scal(h))) return rc;
   h->sc_host->trk[0] = t_rk;
@@ -1796,8 +1796,8 @@ int gdf_cy_lh(GdfCyHandle* h, const double* uh, const double* br, const double* 
   if ((rc = push_scal(h))) return rc;
   if ((rc = launch_lh(h, KIND_LH, h->sc))) return rc;
   if ((rc = download_cells(h, h->T, du))) return rc;
-  CKC(gdf::d2h(dbr, h->BRX, br_bytes(K), h->st));
-  CKC(gdf::d2h(dbz, h->BZX, bz_bytes(K), h->st));
+  CKC(h->stage.d2h(dbr, h->BRX, br_bytes(K), h->st));
+  CKC(h->stage.d2h(dbz, h->BZX, bz_bytes(K), h->st));
   CKC(cudaStreamSynchronize(h->st));
   h->uploaded = 1;
   return GDF_OK;
@@ -1808,12 +1808,12 @@ int gdf_cy_limit(GdfCyHandle* h, double* uh, double* br, double* bz) {
   const KC& K = h->K;
   int rc = upload_cells(h, uh, h->U);
   if (rc) return rc;
-  CKC(gdf::h2d(h->BR, br, br_bytes(K), h->st));
-  CKC(gdf::h2d(h->BZ, bz, bz_bytes(K), h->st));
+  CKC(h->stage.h2d(h->BR, br, br_bytes(K), h->st));
+  CKC(h->stage.h2d(h->BZ, bz, bz_bytes(K), h->st));
   if ((rc = launch_limit(h, nullptr, nullptr))) return rc;
   if ((rc = download_cells(h, h->U, uh))) return rc;
-  CKC(gdf::d2h(br, h->BR, br_bytes(K), h->st));
-  CKC(gdf::d2h(bz, h->BZ, bz_bytes(K), h->st));
+  CKC(h->stage.d2h(br, h->BR, br_bytes(K), h->st));
+  CKC(h->stage.d2h(bz, h->BZ, bz_bytes(K), h->st));
   CKC(cudaStreamSynchronize(h->st));
   h->uploaded = 1;
   return GDF_OK;
@@ -1844,7 +1844,7 @@ int gdf_cy_diagnostics(GdfCyHandle* h, double* umax, double* totaldiv, double* p
   });
   if (rc) return rc;
   std::vector<double> v((size_t)n * 3);
-  CKC(gdf::d2h(v.data(), h->diag, v.size() * sizeof(double), h->st));
+  CKC(h->stage.d2h(v.data(), h->diag, v.size() * sizeof(double), h->st));
   CKC(cudaStreamSynchronize(h->st));
   // item q = kk + nph*((i-1) + nr*(j-1)); the reference's loops: j outer, i inner
   double um = 0, td = 0, pm = 1000000;

@@ -648,7 +648,7 @@ int ens_layout(GdfEnsemble* e) {
     off[(size_t)k * (n + 1) + n] = (int)acc;
     A.total[k] = (int)acc;
   }
-  ECK(gdf::h2d(e->off, off.data(), off.size() * sizeof(int), e->st));
+  ECK(e->stage.h2d(e->off, off.data(), off.size() * sizeof(int), e->st));
   int occ = 0;
   const size_t smem = ens_smem(e->learned);
   ECK(cudaFuncSetAttribute(stage_kernel(e->learned), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -825,7 +825,7 @@ int pull_scal(GdfEnsemble* e) {
 
 int check_health(GdfEnsemble* e) {
   EnsSync s{};
-  ECK(gdf::d2h(&s, e->sync, sizeof(EnsSync), e->st));
+  ECK(e->stage.d2h(&s, e->sync, sizeof(EnsSync), e->st));
   int rc = pull_scal(e);
   if (rc) return rc;
   if (s.err) return efail(GDF_ERR_TIMEOUT, "an ensemble grid barrier timed out");
@@ -952,9 +952,9 @@ int gdf_ens_upload(GdfEnsemble* e, int32_t i, const double* uh, const double* bx
   std::string msg;
   int rc = dead_slot_error(b.cfg, uh, msg);
   if (rc) return efail(rc, msg);
-  ECK(gdf::h2d(b.d.U, uh, uh_sz(b.cfg), e->st));
-  ECK(gdf::h2d(b.d.BX, bx, bx_sz(b.cfg), e->st));
-  ECK(gdf::h2d(b.d.BY, by, by_sz(b.cfg), e->st));
+  ECK(e->stage.h2d(b.d.U, uh, uh_sz(b.cfg), e->st));
+  ECK(e->stage.h2d(b.d.BX, bx, bx_sz(b.cfg), e->st));
+  ECK(e->stage.h2d(b.d.BY, by, by_sz(b.cfg), e->st));
   ECK(cudaStreamSynchronize(e->st));
   e->uploaded = 1;
   return GDF_OK;
@@ -963,9 +963,9 @@ int gdf_ens_upload(GdfEnsemble* e, int32_t i, const double* uh, const double* bx
 int gdf_ens_download(GdfEnsemble* e, int32_t i, double* uh, double* bx, double* by) {
   if (!e || i < 0 || i >= e->n) return efail(GDF_ERR_ARG, "bad argument");
   InstBufs& b = e->in[i];
-  if (uh) ECK(gdf::d2h(uh, b.d.U, uh_sz(b.cfg), e->st));
-  if (bx) ECK(gdf::d2h(bx, b.d.BX, bx_sz(b.cfg), e->st));
-  if (by) ECK(gdf::d2h(by, b.d.BY, by_sz(b.cfg), e->st));
+  if (uh) ECK(e->stage.d2h(uh, b.d.U, uh_sz(b.cfg), e->st));
+  if (bx) ECK(e->stage.d2h(bx, b.d.BX, bx_sz(b.cfg), e->st));
+  if (by) ECK(e->stage.d2h(by, b.d.BY, by_sz(b.cfg), e->st));
   ECK(cudaStreamSynchronize(e->st));
   return GDF_OK;
 }

@@ -862,14 +862,14 @@ static int check_dead_slots(const GdfConfig& c, const double* uh) {
 
 // Copy of the 52 live slot planes of uh (the device copies' dead slots are
 // zero from allocation and no kernel writes them).
-static cudaError_t copy_live(double* dst, const double* uh, const GdfConfig& c, cudaStream_t st,
-                             cudaMemcpyKind kind) {
+static cudaError_t copy_live(GdfHandle* h, double* dst, const double* uh, cudaMemcpyKind kind) {
+  const GdfConfig& c = h->cfg;
   const size_t plane = (size_t)(c.nx + 2) * (c.ny + 2);
   auto copy = [&](int slot, int planes) {
     const size_t o = plane * slot, b = planes * plane * sizeof(double);
-    return kind == cudaMemcpyHostToDevice   ? h2d(dst + o, uh + o, b, st)
-           : kind == cudaMemcpyDeviceToHost ? d2h(dst + o, uh + o, b, st)
-                                            : cudaMemcpyAsync(dst + o, uh + o, b, kind, st);
+    return kind == cudaMemcpyHostToDevice   ? h->stage.h2d(dst + o, uh + o, b, h->st)
+           : kind == cudaMemcpyDeviceToHost ? h->stage.d2h(dst + o, uh + o, b, h->st)
+                                            : cudaMemcpyAsync(dst + o, uh + o, b, kind, h->st);
   };
   // live slots of a variable are modes 0..5 plus (Bx) 6, 8 or (By) 7, 9
   for (int n = 0; n < NE; ++n) {
@@ -1042,15 +1042,15 @@ int gdf_upload(GdfHandle* h, const double* uh, const double* bx, const double* b
   if (!h || !uh || !bx || !by) return fail(GDF_ERR_ARG, "null argument");
   // the live planes travel to a staging buffer while the host checks the
   // dead ones; the resident state changes only once the check has passed
-  CK(copy_live(h->UT, uh, h->cfg, h->st, cudaMemcpyHostToDevice));
+  CK(copy_live(h, h->UT, uh, cudaMemcpyHostToDevice));
   int rc = check_dead_slots(h->cfg, uh);
   if (rc) {
     cudaStreamSynchronize(h->st);
     return rc;
   }
-  CK(copy_live(h->U, h->UT, h->cfg, h->st, cudaMemcpyDeviceToDevice));
-  CK(gdf::h2d(h->BX, bx, bx_bytes(h->cfg), h->st));
-  CK(gdf::h2d(h->BY, by, by_bytes(h->cfg), h->st));
+  CK(copy_live(h, h->U, h->UT, cudaMemcpyDeviceToDevice));
+  CK(h->stage.h2d(h->BX, bx, bx_bytes(h->cfg), h->st));
+  CK(h->stage.h2d(h->BY, by, by_bytes(h->cfg), h->st));
   CK(cudaStreamSynchronize(h->st));
   h->uploaded = 1;
   return GDF_OK;
@@ -1059,9 +1059,9 @@ int gdf_upload(GdfHandle* h, const double* uh, const double* bx, const double* b
 int gdf_download(GdfHandle* h, double* uh, double* bx, double* by) {
   if (!h) return fail(GDF_ERR_ARG, "null handle");
   if (!h->uploaded) return fail(GDF_ERR_STATE, "no state uploaded");
-  if (uh) CK(gdf::d2h(uh, h->U, uh_bytes(h->cfg), h->st));
-  if (bx) CK(gdf::d2h(bx, h->BX, bx_bytes(h->cfg), h->st));
-  if (by) CK(gdf::d2h(by, h->BY, by_bytes(h->cfg), h->st));
+  if (uh) CK(h->stage.d2h(uh, h->U, uh_bytes(h->cfg), h->st));
+  if (bx) CK(h->stage.d2h(bx, h->BX, bx_bytes(h->cfg), h->st));
+  if (by) CK(h->stage.d2h(by, h->BY, by_bytes(h->cfg), h->st));
   CK(cudaStreamSynchronize(h->st));
   return GDF_OK;
 }
@@ -1069,9 +1069,9 @@ int gdf_download(GdfHandle* h, double* uh, double* bx, double* by) {
 int gdf_download_live(GdfHandle* h, double* uh, double* bx, double* by) {
   if (!h) return fail(GDF_ERR_ARG, "null handle");
   if (!h->uploaded) return fail(GDF_ERR_STATE, "no state uploaded");
-  if (uh) CK(copy_live(uh, h->U, h->cfg, h->st, cudaMemcpyDeviceToHost));
-  if (bx) CK(gdf::d2h(bx, h->BX, bx_bytes(h->cfg), h->st));
-  if (by) CK(gdf::d2h(by, h->BY, by_bytes(h->cfg), h->st));
+  if (uh) CK(copy_live(h, uh, h->U, cudaMemcpyDeviceToHost));
+  if (bx) CK(h->stage.d2h(bx, h->BX, bx_bytes(h->cfg), h->st));
+  if (by) CK(h->stage.d2h(by, h->BY, by_bytes(h->cfg), h->st));
   CK(cudaStreamSynchronize(h->st));
   return GDF_OK;
 }
@@ -1080,9 +1080,9 @@ int gdf_upload_state(GdfHandle* h, const double* cells, const double* bx, const 
   if (!h || !cells || !bx || !by) return fail(GDF_ERR_ARG, "null argument");
   const Consts& K = h->K;
   const long long n = 36LL * K.nx * K.ny;
-  CK(gdf::h2d(h->UT, cells, state_bytes(h->cfg), h->st));
-  CK(gdf::h2d(h->BX, bx, bx_bytes(h->cfg), h->st));
-  CK(gdf::h2d(h->BY, by, by_bytes(h->cfg), h->st));
+  CK(h->stage.h2d(h->UT, cells, state_bytes(h->cfg), h->st));
+  CK(h->stage.h2d(h->BX, bx, bx_bytes(h->cfg), h->st));
+  CK(h->stage.h2d(h->BY, by, by_bytes(h->cfg), h->st));
   int rc = run_plain(h, [&] { k_unpack_state<<<nblk(n, 256), 256, 0, h->st>>>(K, h->UT, h->U); });
   // the cell B modes from the face fields (div_free_Balsara.f90:13-79), the
   // ghosts as the end of a stage leaves them (set_bc with the ghost B
@@ -1105,10 +1105,10 @@ int gdf_download_state(GdfHandle* h, double* cells, double* bx, double* by) {
     const long long n = 36LL * h->K.nx * h->K.ny;
     int rc = run_plain(h, [&] { k_pack_state<<<nblk(n, 256), 256, 0, h->st>>>(h->K, h->U, h->UT); });
     if (rc) return rc;
-    CK(gdf::d2h(cells, h->UT, state_bytes(h->cfg), h->st));
+    CK(h->stage.d2h(cells, h->UT, state_bytes(h->cfg), h->st));
   }
-  if (bx) CK(gdf::d2h(bx, h->BX, bx_bytes(h->cfg), h->st));
-  if (by) CK(gdf::d2h(by, h->BY, by_bytes(h->cfg), h->st));
+  if (bx) CK(h->stage.d2h(bx, h->BX, bx_bytes(h->cfg), h->st));
+  if (by) CK(h->stage.d2h(by, h->BY, by_bytes(h->cfg), h->st));
   CK(cudaStreamSynchronize(h->st));
   return GDF_OK;
 }
@@ -1154,7 +1154,7 @@ int gdf_prepare(GdfHandle* h, int32_t* flags) {
   if ((rc = launch_limit(h, h->UI, h->U, 1, nullptr))) return rc;
   if ((rc = launch_set_bc(h, h->U, 1, nullptr))) return rc;
   if (flags) {
-    CK(gdf::d2h(flags, h->flags, (size_t)h->cfg.nx * h->cfg.ny * sizeof(int32_t), h->st));
+    CK(h->stage.d2h(flags, h->flags, (size_t)h->cfg.nx * h->cfg.ny * sizeof(int32_t), h->st));
   }
   rc = sync_scal(h);
   if (rc) return rc;
@@ -1169,7 +1169,7 @@ int gdf_step(GdfHandle* h, double tend, double* t, double* dt_out, int32_t* flag
   if (rc) return rc;
   if ((rc = launch_step(h))) return rc;
   if (flags) {
-    CK(gdf::d2h(flags, h->flags, (size_t)h->cfg.nx * h->cfg.ny * sizeof(int32_t), h->st));
+    CK(h->stage.d2h(flags, h->flags, (size_t)h->cfg.nx * h->cfg.ny * sizeof(int32_t), h->st));
   }
   if ((rc = sync_scal(h))) return rc;
   *t = h->sc_host->t;
@@ -1296,11 +1296,11 @@ int gdf_features(GdfHandle* h, const double* uh, float* X) {
   if (!h->QM) CK(cudaMalloc((void**)&h->QM, (size_t)QMODES * h->K.plane * sizeof(float)));
   float* dX = nullptr;
   CK(cudaMallocAsync((void**)&dX, (size_t)ncell * NFEAT * sizeof(float), h->st));
-  CK(copy_live(h->UT, uh, h->cfg, h->st, cudaMemcpyHostToDevice));
+  CK(copy_live(h, h->UT, uh, cudaMemcpyHostToDevice));
   rc = run_kernel(h, GDF_K_LIMIT, [&] { k_qmodes<<<nblk(h->K.plane, 128), 128, 0, h->st>>>(h->K, h->UT, h->QM); });
   if (!rc) rc = run_kernel(h, GDF_K_LIMIT, [&] { k_features<<<nblk(ncell, 128), 128, 0, h->st>>>(h->K, h->QM, dX); });
   if (!rc) {
-    cudaError_t e = gdf::d2h(X, dX, (size_t)ncell * NFEAT * sizeof(float), h->st);
+    cudaError_t e = h->stage.d2h(X, dX, (size_t)ncell * NFEAT * sizeof(float), h->st);
     if (e != cudaSuccess) rc = fail(GDF_ERR_CUDA, cudaGetErrorString(e));
   }
   cudaFreeAsync(dX, h->st);
@@ -1317,14 +1317,14 @@ int gdf_config_of(GdfHandle* h, GdfConfig* out) {
 // Is_Trouble_Cell (the sticky KXRCF flags), nx*ny int32 in (i-1)+nx*(j-1) order
 int gdf_get_trouble(GdfHandle* h, int32_t* trouble) {
   if (!h || !trouble) return fail(GDF_ERR_ARG, "null argument");
-  CK(gdf::d2h(trouble, h->trouble, (size_t)h->cfg.nx * h->cfg.ny * sizeof(int32_t), h->st));
+  CK(h->stage.d2h(trouble, h->trouble, (size_t)h->cfg.nx * h->cfg.ny * sizeof(int32_t), h->st));
   CK(cudaStreamSynchronize(h->st));
   return GDF_OK;
 }
 
 int gdf_set_trouble(GdfHandle* h, const int32_t* trouble) {
   if (!h || !trouble) return fail(GDF_ERR_ARG, "null argument");
-  CK(gdf::h2d(h->trouble, trouble, (size_t)h->cfg.nx * h->cfg.ny * sizeof(int32_t), h->st));
+  CK(h->stage.h2d(h->trouble, trouble, (size_t)h->cfg.nx * h->cfg.ny * sizeof(int32_t), h->st));
   CK(cudaStreamSynchronize(h->st));
   return GDF_OK;
 }
@@ -1368,14 +1368,14 @@ int gdf_lh(GdfHandle* h, const double* uh, double* du) {
   int rc = check_dead_slots(h->cfg, uh);
   if (rc) return rc;
   const size_t ub = uh_bytes(h->cfg);
-  CK(copy_live(h->UT, uh, h->cfg, h->st, cudaMemcpyHostToDevice));
+  CK(copy_live(h, h->UT, uh, cudaMemcpyHostToDevice));
   CK(cudaMemsetAsync(h->UI, 0, ub, h->st));  // du (ghost and dead entries stay 0)
   if ((rc = launch_faces(h, h->UT, nullptr))) return rc;
   rc = run_kernel(h, GDF_K_CELL, [&] {
     launch_cell(h->K, h->UT, nullptr, nullptr, h->Fxh, h->Fyh, h->UI, nullptr, 0, h->st);
   });
   if (rc) return rc;
-  CK(gdf::d2h(du, h->UI, ub, h->st));
+  CK(h->stage.d2h(du, h->UI, ub, h->st));
   CK(cudaStreamSynchronize(h->st));
   return GDF_OK;
 }
@@ -1384,7 +1384,7 @@ int gdf_lhez(GdfHandle* h, const double* uh, double* dez1, double* dez2) {
   if (!h || !uh || !dez1 || !dez2) return fail(GDF_ERR_ARG, "null argument");
   int rc = check_dead_slots(h->cfg, uh);
   if (rc) return rc;
-  CK(copy_live(h->UT, uh, h->cfg, h->st, cudaMemcpyHostToDevice));
+  CK(copy_live(h, h->UT, uh, cudaMemcpyHostToDevice));
   if ((rc = launch_faces(h, h->UT, nullptr))) return rc;
   double *d1 = h->BX0, *d2 = h->BY0;
   rc = run_kernel(h, GDF_K_BFACE, [&] {
@@ -1392,8 +1392,8 @@ int gdf_lhez(GdfHandle* h, const double* uh, double* dez1, double* dez2) {
         h->K, h->EzRL, h->EzUD, h->EzV, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, d1, d2, nullptr, 0);
   });
   if (rc) return rc;
-  CK(gdf::d2h(dez1, d1, bx_bytes(h->cfg), h->st));
-  CK(gdf::d2h(dez2, d2, by_bytes(h->cfg), h->st));
+  CK(h->stage.d2h(dez1, d1, bx_bytes(h->cfg), h->st));
+  CK(h->stage.d2h(dez2, d2, by_bytes(h->cfg), h->st));
   CK(cudaStreamSynchronize(h->st));
   return GDF_OK;
 }
@@ -1404,10 +1404,10 @@ int gdf_limit(GdfHandle* h, double* uh, double* bx, double* by, int32_t* flags) 
   if (rc) return rc;
   const size_t ub = uh_bytes(h->cfg);
   // the limiter works on the resident buffers; save and restore them
-  CK(gdf::h2d(h->UT, uh, ub, h->st));
+  CK(h->stage.h2d(h->UT, uh, ub, h->st));
   CK(cudaMemcpyAsync(h->U0, h->UT, ub, cudaMemcpyDeviceToDevice, h->st));
-  CK(gdf::h2d(h->BX0, bx, bx_bytes(h->cfg), h->st));
-  CK(gdf::h2d(h->BY0, by, by_bytes(h->cfg), h->st));
+  CK(h->stage.h2d(h->BX0, bx, bx_bytes(h->cfg), h->st));
+  CK(h->stage.h2d(h->BY0, by, by_bytes(h->cfg), h->st));
   double* sBX = h->BX;
   double* sBY = h->BY;
   h->BX = h->BX0;
@@ -1417,11 +1417,11 @@ int gdf_limit(GdfHandle* h, double* uh, double* bx, double* by, int32_t* flags) 
   h->BX = sBX;
   h->BY = sBY;
   if (rc) return rc;
-  CK(gdf::d2h(uh, h->U0, ub, h->st));
-  CK(gdf::d2h(bx, h->BX0, bx_bytes(h->cfg), h->st));
-  CK(gdf::d2h(by, h->BY0, by_bytes(h->cfg), h->st));
+  CK(h->stage.d2h(uh, h->U0, ub, h->st));
+  CK(h->stage.d2h(bx, h->BX0, bx_bytes(h->cfg), h->st));
+  CK(h->stage.d2h(by, h->BY0, by_bytes(h->cfg), h->st));
   if (flags)
-    CK(gdf::d2h(flags, h->flags, (size_t)h->cfg.nx * h->cfg.ny * sizeof(int32_t), h->st));
+    CK(h->stage.d2h(flags, h->flags, (size_t)h->cfg.nx * h->cfg.ny * sizeof(int32_t), h->st));
   CK(cudaStreamSynchronize(h->st));
   return GDF_OK;
 }
@@ -1430,7 +1430,7 @@ int gdf_dt(GdfHandle* h, const double* uh, double* dt) {
   if (!h || !uh || !dt) return fail(GDF_ERR_ARG, "null argument");
   // the cell averages only (calculate_dt reads mode 1)
   const size_t pl = (size_t)h->K.plane;
-  for (int n = 0; n < NE; ++n) CK(gdf::h2d(h->UT + 10 * n * pl, uh + 10 * n * pl, pl * sizeof(double), h->st));
+  for (int n = 0; n < NE; ++n) CK(h->stage.h2d(h->UT + 10 * n * pl, uh + 10 * n * pl, pl * sizeof(double), h->st));
   int rc = launch_dt(h, h->UT, 0);
   if (rc) return rc;
   if ((rc = sync_scal(h))) return rc;

@@ -486,7 +486,7 @@ static int mlp_ensure(GdfMlp* m, long long n, int blocks) {
 static int mlp_upload_x(GdfMlp* m, const float* X, long long n) {
   float* tmp = nullptr;
   MCK(cudaMallocAsync((void**)&tmp, (size_t)n * MLP_IN * sizeof(float), m->st));
-  MCK(gdf::h2d(tmp, X, (size_t)n * MLP_IN * sizeof(float), m->st));
+  MCK(m->stage.h2d(tmp, X, (size_t)n * MLP_IN * sizeof(float), m->st));
   const long long tot = n * MLP_INP;
   k_to_bf16<<<(unsigned)((tot + 255) / 256), 256, 0, m->st>>>(tmp, m->X, n);
   MCK(cudaGetLastError());
@@ -524,7 +524,7 @@ static int fwdbwd_launch(GdfMlp* m, const int* idx, long long nsel, float pos_w,
 // the error word of the tcgen05 tiles (read back after a synchronisation)
 static int check_err(GdfMlp* m) {
   int e = 0;
-  MCK(gdf::d2h(&e, m->err, sizeof(int), m->st));
+  MCK(m->stage.d2h(&e, m->err, sizeof(int), m->st));
   MCK(cudaStreamSynchronize(m->st));
   if (e) {
     MCK(cudaMemsetAsync(m->err, 0, sizeof(int), m->st));
@@ -594,7 +594,7 @@ int gdf_mlp_destroy(GdfMlp* m) {
 
 int gdf_mlp_set_params(GdfMlp* m, const float* params) {
   if (!m || !params) return mfail(GDF_ERR_ARG, "null argument");
-  MCK(gdf::h2d(m->P, params, MLP_NPARAM * sizeof(float), m->st));
+  MCK(m->stage.h2d(m->P, params, MLP_NPARAM * sizeof(float), m->st));
   MCK(cudaMemsetAsync(m->M, 0, MLP_NPARAM * sizeof(float), m->st));
   MCK(cudaMemsetAsync(m->V, 0, MLP_NPARAM * sizeof(float), m->st));
   m->adam_t = 0;
@@ -606,7 +606,7 @@ int gdf_mlp_set_params(GdfMlp* m, const float* params) {
 
 int gdf_mlp_get_params(GdfMlp* m, float* params) {
   if (!m || !params) return mfail(GDF_ERR_ARG, "null argument");
-  MCK(gdf::d2h(params, m->P, MLP_NPARAM * sizeof(float), m->st));
+  MCK(m->stage.d2h(params, m->P, MLP_NPARAM * sizeof(float), m->st));
   MCK(cudaStreamSynchronize(m->st));
   return GDF_OK;
 }
@@ -618,13 +618,13 @@ int gdf_mlp_grad(GdfMlp* m, const float* X, const float* y, int64_t n, float pos
   int rc = mlp_ensure(m, n, nb);
   if (rc) return rc;
   if ((rc = mlp_upload_x(m, X, n))) return rc;
-  MCK(gdf::h2d(m->y, y, (size_t)n * sizeof(float), m->st));
+  MCK(m->stage.h2d(m->y, y, (size_t)n * sizeof(float), m->st));
   std::vector<int> id((size_t)n);
   for (long long q = 0; q < n; ++q) id[q] = (int)q;
-  MCK(gdf::h2d(m->idx, id.data(), (size_t)n * sizeof(int), m->st));
+  MCK(m->stage.h2d(m->idx, id.data(), (size_t)n * sizeof(int), m->st));
   if ((rc = mlp_grad_launch(m, n, pos_weight, 1.f / (float)n))) return rc;
-  MCK(gdf::d2h(grad, m->grad, MLP_NPARAM * sizeof(float), m->st));
-  if (loss) MCK(gdf::d2h(loss, m->loss, sizeof(float), m->st));
+  MCK(m->stage.d2h(grad, m->grad, MLP_NPARAM * sizeof(float), m->st));
+  if (loss) MCK(m->stage.d2h(loss, m->loss, sizeof(float), m->st));
   MCK(cudaStreamSynchronize(m->st));
   return check_err(m);
 }
@@ -636,7 +636,7 @@ int gdf_mlp_train(GdfMlp* m, const float* X, const float* y, int64_t n, int32_t 
   int rc = mlp_ensure(m, n, nb_max);
   if (rc) return rc;
   if ((rc = mlp_upload_x(m, X, n))) return rc;
-  MCK(gdf::h2d(m->y, y, (size_t)n * sizeof(float), m->st));
+  MCK(m->stage.h2d(m->y, y, (size_t)n * sizeof(float), m->st));
   std::vector<int> id((size_t)n), next;
   for (long long q = 0; q < n; ++q) id[q] = (int)q;
   std::mt19937 rng((uint32_t)seed);
@@ -650,7 +650,7 @@ int gdf_mlp_train(GdfMlp* m, const float* X, const float* y, int64_t n, int32_t 
   std::vector<float> lossv((size_t)nbatch);
   auto epoch = [&](int ep) -> int {
     if (ep == 0) std::shuffle(id.begin(), id.end(), rng);
-    MCK(gdf::h2d(m->idx, id.data(), (size_t)n * sizeof(int), m->st));
+    MCK(m->stage.h2d(m->idx, id.data(), (size_t)n * sizeof(int), m->st));
     for (long long k = 0; k < nbatch; ++k) {
       const long long off = k * batch, nsel = std::min<long long>(batch, n - off);
       int nb = 0;
@@ -691,7 +691,7 @@ int gdf_mlp_predict(GdfMlp* m, const float* X, int64_t n, float* p) {
   MCK(cudaMallocAsync((void**)&dp, (size_t)n * sizeof(float), m->st));
   k_mlp_predict<<<(unsigned)((n + TB - 1) / TB), MLP_THREADS, 0, m->st>>>(m->D, m->X, (int)n, dp);
   MCK(cudaGetLastError());
-  MCK(gdf::d2h(p, dp, (size_t)n * sizeof(float), m->st));
+  MCK(m->stage.d2h(p, dp, (size_t)n * sizeof(float), m->st));
   MCK(cudaFreeAsync(dp, m->st));
   MCK(cudaStreamSynchronize(m->st));
   return GDF_OK;

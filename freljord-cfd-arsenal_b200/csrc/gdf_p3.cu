@@ -1281,7 +1281,7 @@ int upload_cells(GdfP3Handle* h, const double* uh, double* D) {
         continue;
       }
       while (e < NP3 && slot3(n, e) == s + (e - d)) ++e;
-      CK3(gdf::h2d(D + pl * s, src, pl * (e - d) * sizeof(double), h->st));
+      CK3(h->stage.h2d(D + pl * s, src, pl * (e - d) * sizeof(double), h->st));
     }
   CK3(cudaStreamSynchronize(h->st));
   return GDF_OK;
@@ -1300,7 +1300,7 @@ int download_cells(GdfP3Handle* h, const double* D, double* uh) {
         continue;
       }
       while (e < NP3 && slot3(n, e) == s + (e - d)) ++e;
-      CK3(gdf::d2h(dst, D + pl * s, pl * (e - d) * sizeof(double), h->st));
+      CK3(h->stage.d2h(dst, D + pl * s, pl * (e - d) * sizeof(double), h->st));
     }
   CK3(cudaStreamSynchronize(h->st));
   return GDF_OK;
@@ -1388,8 +1388,8 @@ int gdf_p3_upload(GdfP3Handle* h, const double* uh, const double* bx, const doub
   if (!h || !uh || !bx || !by) return fail(GDF_ERR_ARG, "null argument");
   int rc = upload_cells(h, uh, h->U);
   if (rc) return rc;
-  CK3(gdf::h2d(h->BX, bx, bx_bytes(h->K), h->st));
-  CK3(gdf::h2d(h->BY, by, by_bytes(h->K), h->st));
+  CK3(h->stage.h2d(h->BX, bx, bx_bytes(h->K), h->st));
+  CK3(h->stage.h2d(h->BY, by, by_bytes(h->K), h->st));
   h->sc_host->t = 0;
   h->sc_host->dt = 0;
   h->sc_host->active = 1;
@@ -1406,8 +1406,8 @@ int gdf_p3_download(GdfP3Handle* h, double* uh, double* bx, double* by) {
   if (!h->uploaded) return fail(GDF_ERR_STATE, "no state uploaded");
   int rc = download_cells(h, h->U, uh);
   if (rc) return rc;
-  CK3(gdf::d2h(bx, h->BX, bx_bytes(h->K), h->st));
-  CK3(gdf::d2h(by, h->BY, by_bytes(h->K), h->st));
+  CK3(h->stage.d2h(bx, h->BX, bx_bytes(h->K), h->st));
+  CK3(h->stage.d2h(by, h->BY, by_bytes(h->K), h->st));
   CK3(cudaStreamSynchronize(h->st));
   return GDF_OK;
 }
@@ -1573,15 +1573,15 @@ int gdf_p3_lh(GdfP3Handle* h, const double* uh, const double* bx, const double* 
   const K3& K = h->K;
   int rc = upload_cells(h, uh, h->U);
   if (rc) return rc;
-  CK3(gdf::h2d(h->BX, bx, bx_bytes(K), h->st));
-  CK3(gdf::h2d(h->BY, by, by_bytes(K), h->st));
+  CK3(h->stage.h2d(h->BX, bx, bx_bytes(K), h->st));
+  CK3(h->stage.h2d(h->BY, by, by_bytes(K), h->st));
   CK3(cudaMemsetAsync(h->T, 0, (size_t)K.plane * NS3 * sizeof(double), h->st));
   CK3(cudaMemsetAsync(h->BXT, 0, bx_bytes(K), h->st));
   CK3(cudaMemsetAsync(h->BYT, 0, by_bytes(K), h->st));
   if ((rc = launch_lh(h, KIND_LH, nullptr))) return rc;
   if ((rc = download_cells(h, h->T, du))) return rc;
-  CK3(gdf::d2h(dbx, h->BXT, bx_bytes(K), h->st));
-  CK3(gdf::d2h(dby, h->BYT, by_bytes(K), h->st));
+  CK3(h->stage.d2h(dbx, h->BXT, bx_bytes(K), h->st));
+  CK3(h->stage.d2h(dby, h->BYT, by_bytes(K), h->st));
   CK3(cudaStreamSynchronize(h->st));
   h->uploaded = 1;
   return GDF_OK;
@@ -1592,8 +1592,8 @@ int gdf_p3_limit(GdfP3Handle* h, double* uh, double* bx, double* by) {
   const K3& K = h->K;
   int rc = upload_cells(h, uh, h->T);
   if (rc) return rc;
-  CK3(gdf::h2d(h->BXT, bx, bx_bytes(K), h->st));
-  CK3(gdf::h2d(h->BYT, by, by_bytes(K), h->st));
+  CK3(h->stage.h2d(h->BXT, bx, bx_bytes(K), h->st));
+  CK3(h->stage.h2d(h->BYT, by, by_bytes(K), h->st));
   // the cells' ghosts keep the values set_bc gives them
   if ((rc = launch_set_bc(h, h->T, h->BXT, h->BYT, nullptr))) return rc;
   CK3(cudaMemcpyAsync(h->U, h->T, (size_t)K.plane * NS3 * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
@@ -1601,8 +1601,8 @@ int gdf_p3_limit(GdfP3Handle* h, double* uh, double* bx, double* by) {
   CK3(cudaMemcpyAsync(h->BY, h->BYT, by_bytes(K), cudaMemcpyDeviceToDevice, h->st));
   if ((rc = launch_limit(h, nullptr, nullptr))) return rc;
   if ((rc = download_cells(h, h->U, uh))) return rc;
-  CK3(gdf::d2h(bx, h->BX, bx_bytes(K), h->st));
-  CK3(gdf::d2h(by, h->BY, by_bytes(K), h->st));
+  CK3(h->stage.d2h(bx, h->BX, bx_bytes(K), h->st));
+  CK3(h->stage.d2h(by, h->BY, by_bytes(K), h->st));
   CK3(cudaStreamSynchronize(h->st));
   h->uploaded = 1;
   return GDF_OK;
@@ -1626,7 +1626,7 @@ int gdf_p3_diagnostics(GdfP3Handle* h, double* umax, double* totaldiv) {
   int rc = run(h, [&] { k3_diag<<<nblk(nc, 128), 128, 0, h->st>>>(K, h->U, h->diag, h->diag + nc); });
   if (rc) return rc;
   std::vector<double> v((size_t)nc * 2);
-  CK3(gdf::d2h(v.data(), h->diag, v.size() * sizeof(double), h->st));
+  CK3(h->stage.d2h(v.data(), h->diag, v.size() * sizeof(double), h->st));
   CK3(cudaStreamSynchronize(h->st));
   // the reference's loop order: i outer, j inner
   double um = 0, td = 0;

@@ -1,6 +1,7 @@
 // gdf_stage.cu -- the pinned ring behind gdf_stage.h.
 //
-// One ring per device. A copy holds the ring for its whole length; a copy that
+// One ring per device, its events made on that device (an event is recorded on
+// streams of its own device only). A copy holds the ring for its whole length; a copy that
 // finds it taken (another thread's) goes to cudaMemcpyAsync, so threads never
 // wait for each other here. A slot is reused when the event recorded behind its
 // last transfer has passed, whatever stream that was on.
@@ -38,9 +39,24 @@ void drop(Ring& r) {
   cudaGetLastError();
 }
 
-bool make(Ring& r) {
+// the device dev current in its scope
+struct OnDevice {
+  int prev = -1;
+  bool ok;
+  explicit OnDevice(int dev) {
+    ok = cudaGetDevice(&prev) == cudaSuccess;
+    if (ok && prev == dev) prev = -1;
+    else if (ok) ok = cudaSetDevice(dev) == cudaSuccess;
+  }
+  ~OnDevice() {
+    if (prev >= 0) cudaSetDevice(prev);
+  }
+};
+
+bool make(Ring& r, int dev) {
   if (r.ready) return true;
-  bool ok = true;
+  const OnDevice on(dev);
+  bool ok = on.ok;
   for (int k = 0; ok && k < STAGE_SLOTS; ++k)
     ok = cudaHostAlloc((void**)&r.buf[k], STAGE_CHUNK, cudaHostAllocPortable) == cudaSuccess &&
          cudaEventCreateWithFlags(&r.ev[k], cudaEventDisableTiming) == cudaSuccess;
@@ -52,23 +68,21 @@ bool make(Ring& r) {
   return true;
 }
 
-// the current device's ring, locked in lk, for a pageable array of this size;
-// null: copy plainly
-Ring* take(const void* host, size_t bytes, std::unique_lock<std::mutex>& lk) {
-  if (bytes < STAGE_MIN) return nullptr;
+// device dev's ring, locked in lk, for a pageable array of this size; null:
+// copy plainly
+Ring* take(int dev, const void* host, size_t bytes, std::unique_lock<std::mutex>& lk) {
+  if (dev < 0 || bytes < STAGE_MIN) return nullptr;
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
   if (a.type != cudaMemoryTypeUnregistered) return nullptr;
-  int dev = -1;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEV) return nullptr;
   Ring& r = g_ring[dev];
   lk = std::unique_lock<std::mutex>(r.mu, std::try_to_lock);
-  if (!lk.owns_lock() || r.holders == 0) return nullptr;
+  if (!lk.owns_lock()) return nullptr;
   r.asked += std::min(bytes, STAGE_MAKE);
-  if (r.asked < STAGE_MAKE || !make(r)) return nullptr;
+  if (r.asked < STAGE_MAKE || !make(r, dev)) return nullptr;
   r.asked = STAGE_MAKE;
   return &r;
 }
@@ -91,9 +105,9 @@ StageRef::~StageRef() {
   if (--g_ring[dev].holders == 0) drop(g_ring[dev]);
 }
 
-cudaError_t h2d(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+cudaError_t StageRef::h2d(void* dst, const void* src, size_t bytes, cudaStream_t st) {
   std::unique_lock<std::mutex> lk;
-  Ring* r = take(src, bytes, lk);
+  Ring* r = take(dev, src, bytes, lk);
   if (!r) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
   int k = 0;
   for (size_t o = 0; o < bytes; o += STAGE_CHUNK, k = (k + 1) % STAGE_SLOTS) {
@@ -108,9 +122,9 @@ cudaError_t h2d(void* dst, const void* src, size_t bytes, cudaStream_t st) {
   return cudaSuccess;
 }
 
-cudaError_t d2h(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+cudaError_t StageRef::d2h(void* dst, const void* src, size_t bytes, cudaStream_t st) {
   std::unique_lock<std::mutex> lk;
-  Ring* r = take(dst, bytes, lk);
+  Ring* r = take(dev, dst, bytes, lk);
   if (!r) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
   const size_t chunks = (bytes + STAGE_CHUNK - 1) / STAGE_CHUNK;
   auto issue = [&](size_t c) {

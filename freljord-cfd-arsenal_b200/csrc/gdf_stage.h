@@ -14,14 +14,23 @@
 
 namespace gdf {
 
-// Keeps the current device's ring for as long as it lives: the ring (STAGE_SLOTS
-// x STAGE_CHUNK bytes, made after STAGE_MAKE bytes) is freed with the last of its holders.
-// Every handle holds one.
+// Copies through the ring of the device that is current where it is made, and
+// keeps that ring for as long as it lives: the ring (STAGE_SLOTS x STAGE_CHUNK
+// bytes, made after STAGE_MAKE bytes) is freed with the last of its holders.
+// Every handle holds one, made with the handle's stream; the streams given to
+// h2d and d2h are that device's. Which device is current at a copy does not matter,
+// as it does not to cudaMemcpyAsync.
 struct StageRef {
   StageRef();
   ~StageRef();
   StageRef(const StageRef&) = delete;
   StageRef& operator=(const StageRef&) = delete;
+
+  // host -> device, ordered on st; src may be reused on return
+  cudaError_t h2d(void* dst, const void* src, size_t bytes, cudaStream_t st);
+  // device -> host after st's earlier work; a pageable dst of STAGE_MIN bytes or
+  // more is complete on return
+  cudaError_t d2h(void* dst, const void* src, size_t bytes, cudaStream_t st);
 
  private:
   int dev;
@@ -34,12 +43,6 @@ constexpr size_t STAGE_MIN = (size_t)1 << 20;   // below: one plain copy (the ri
 // freeing it takes some 18 ms, what it saves on about this many bytes, and a
 // handle that is made, copied from once and closed would pay that each time.
 constexpr size_t STAGE_MAKE = (size_t)64 << 20;
-
-// host -> device, ordered on st; src may be reused on return
-cudaError_t h2d(void* dst, const void* src, size_t bytes, cudaStream_t st);
-// device -> host after st's earlier work; a pageable dst of STAGE_MIN bytes or
-// more is complete on return
-cudaError_t d2h(void* dst, const void* src, size_t bytes, cudaStream_t st);
 
 // memcpy over several threads (gdf_io.cpp)
 void par_memcpy(void* dst, const void* src, size_t bytes);

@@ -87,6 +87,14 @@ Ring* take(int dev, const void* host, size_t bytes, std::unique_lock<std::mutex>
   return &r;
 }
 
+// The event behind a slot's transfer. Without one the next copy would take the
+// slot while the transfer still uses it, so a failure waits for the transfer.
+cudaError_t record(cudaEvent_t ev, cudaStream_t st) {
+  const cudaError_t e = cudaEventRecord(ev, st);
+  if (e != cudaSuccess) cudaStreamSynchronize(st);
+  return e;
+}
+
 }  // namespace
 
 StageRef::StageRef() : dev(-1) {
@@ -116,7 +124,7 @@ cudaError_t StageRef::h2d(void* dst, const void* src, size_t bytes, cudaStream_t
     if (e != cudaSuccess) return e;
     par_memcpy(r->buf[k], (const char*)src + o, n);
     e = cudaMemcpyAsync((char*)dst + o, r->buf[k], n, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaEventRecord(r->ev[k], st);
+    if (e == cudaSuccess) e = record(r->ev[k], st);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -132,7 +140,7 @@ cudaError_t StageRef::d2h(void* dst, const void* src, size_t bytes, cudaStream_t
     const size_t o = c * STAGE_CHUNK, n = std::min(STAGE_CHUNK, bytes - o);
     cudaError_t e = cudaEventSynchronize(r->ev[k]);
     if (e == cudaSuccess) e = cudaMemcpyAsync(r->buf[k], (const char*)src + o, n, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaEventRecord(r->ev[k], st);
+    if (e == cudaSuccess) e = record(r->ev[k], st);
     return e;
   };
   cudaError_t e = cudaSuccess;

@@ -22,15 +22,17 @@ namespace fake {
 struct Stream {
   int dev;
   std::deque<std::function<void()>> q;
-  void drain() {
-    while (!q.empty()) {
+  long run = 0;   // work done so far
+  void drain(long upto = -1) {
+    while (!q.empty() && (upto < 0 || run < upto)) {
       auto f = q.front();
       q.pop_front();
       f();
+      ++run;
     }
   }
 };
-struct Event { int dev; Stream* s; };
+struct Event { int dev; Stream* s; long upto; };
 inline int dev = 0, live_events = 0, record_fails = 0, pin_calls = 0;
 inline long staged = 0, plain = 0;               // copies by kind of their host memory
 inline std::map<uintptr_t, size_t> pinned;        // start -> bytes
@@ -70,7 +72,7 @@ inline cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void
   return cudaSuccess;
 }
 inline cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
-  *e = new fake::Event{fake::dev, nullptr};
+  *e = new fake::Event{fake::dev, nullptr, 0};
   ++fake::live_events;
   return cudaSuccess;
 }
@@ -83,10 +85,11 @@ inline cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
   if (e->dev != s->dev) return cudaErrorInvalidResourceHandle;
   if (fake::record_fails > 0 && --fake::record_fails == 0) return cudaErrorUnknown;
   e->s = s;
+  e->upto = s->run + (long)s->q.size();
   return cudaSuccess;
 }
 inline cudaError_t cudaEventSynchronize(cudaEvent_t e) {
-  if (e->s) e->s->drain();
+  if (e->s) e->s->drain(e->upto);
   return cudaSuccess;
 }
 inline cudaError_t cudaStreamSynchronize(cudaStream_t s) {

@@ -88,4 +88,31 @@ int check_plain() {
   REQUIRE(fake::staged == 0 && fake::plain == 2);
   return 0;
 }
+
+// an event that cannot be recorded: the error is returned and no transfer is
+// left that a later copy's slot would overtake
+int check_failed_record() {
+  fake::Stream s0{0, {}}, s1{0, {}};
+  cudaSetDevice(0);
+  StageRef a;
+  if (int r = round_trip(a, &s0, LONG, 9)) return r;
+  const size_t n = 3 * STAGE_CHUNK;
+  const Bytes x = pattern(n, 10), y = pattern(n, 11);
+  for (int fail = 1; fail <= 3; ++fail) {
+    Bytes dx(n), dy(n);
+    fake::record_fails = fail;
+    REQUIRE(a.h2d(dx.data(), x.data(), n, &s0) == cudaErrorUnknown);
+    REQUIRE(a.h2d(dy.data(), y.data(), n, &s1) == cudaSuccess);   // the same slots, on another stream
+    s1.drain();
+    s0.drain();
+    REQUIRE(dy == y);
+    REQUIRE(std::memcmp(dx.data(), x.data(), fail * STAGE_CHUNK) == 0);
+    fake::record_fails = fail;
+    REQUIRE(a.d2h(dx.data(), y.data(), n, &s0) == cudaErrorUnknown);
+    REQUIRE(a.d2h(dy.data(), x.data(), n, &s1) == cudaSuccess);
+    s0.drain();
+    REQUIRE(dy == x);
+  }
+  return 0;
+}
 }

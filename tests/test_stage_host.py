@@ -26,6 +26,6 @@ def lib():
     return C.CDLL(so)
 
 
-@pytest.mark.parametrize("check", ["other_device_current", "given_back", "plain"])
+@pytest.mark.parametrize("check", ["other_device_current", "given_back", "plain", "failed_record"])
 def test_check(lib, check):
     assert getattr(lib, "check_" + check)() == 0

@@ -1,8 +1,8 @@
 // gdf_stage.h -- copies between host arrays and the device.
 //
 // A caller's arrays are ordinary (pageable) memory as a rule. The driver copies
-// those through its own staging buffer with one host thread, 12 GB/s here (less
-// into pages not yet touched), well under the link. h2d / d2h take large
+// those through its own staging buffer with one host thread, 12 GB/s from memory, 20
+// from the host's caches, 2-3 into pages not yet touched, well under the link. h2d / d2h take large
 // pageable arrays through a ring of pinned buffers instead: several threads fill
 // (empty) one while the link moves another. Small arrays, and memory that is
 // already pinned or on a device, go to cudaMemcpyAsync as they are.
@@ -16,7 +16,7 @@ namespace gdf {
 
 // Copies through the ring of the device that is current where it is made, and
 // keeps that ring for as long as it lives: the ring (STAGE_SLOTS x STAGE_CHUNK
-// bytes, made after STAGE_MAKE bytes) is freed with the last of its holders.
+// bytes at most, made slot by slot) is freed with the last of its holders.
 // Every handle holds one, made with the handle's stream; the streams given to
 // h2d and d2h are that device's. Which device is current at a copy does not matter,
 // as it does not to cudaMemcpyAsync.
@@ -39,10 +39,17 @@ struct StageRef {
 constexpr size_t STAGE_CHUNK = (size_t)4 << 20;
 constexpr int STAGE_SLOTS = 4;
 constexpr size_t STAGE_MIN = (size_t)1 << 20;   // below: one plain copy (the ring's hand-overs cost more)
-// The ring is made once its holders have asked it for this much: making and
-// freeing it takes some 18 ms, what it saves on about this many bytes, and a
-// handle that is made, copied from once and closed would pay that each time.
-constexpr size_t STAGE_MAKE = (size_t)64 << 20;
+// When a copy makes the slots it needs (2.3 ms for all four, 0.5 ms to give them
+// back): if it is this long itself, so that it saves as much (72 MB up 5.6 ms plainly, 1.6
+// through the ring; 256 MB 23 and 5.2): the first predict of a process on 69 MB takes
+// 9.2 ms, 8.9 without the ring, the next ones 4.3 and 7 to 8 ...
+constexpr size_t STAGE_NOW = (size_t)64 << 20;
+// ... or if this much has gone past plainly while its holders lived, 27-45 ms of
+// copies: a shorter copy may then pay for the slots alone, once in that long
+// (predict on 62 MB: the tenth call 7.1 ms, 5.6 before it and 3.1 after).
+// Handles opened, loaded and closed in a loop thus stay at the plain rate until they
+// move more than they would lose.
+constexpr size_t STAGE_DUE = (size_t)512 << 20;
 
 // memcpy over several threads (gdf_io.cpp)
 void par_memcpy(void* dst, const void* src, size_t bytes);

@@ -115,4 +115,34 @@ int check_failed_record() {
   }
   return 0;
 }
+
+// one long copy makes the slots it needs; shorter ones go past plainly until
+// STAGE_DUE bytes have, and then make no more slots than they have chunks
+int check_when_made() {
+  fake::Stream s0{0, {}};
+  cudaSetDevice(0);
+  Bytes host(STAGE_NOW), devmem(STAGE_NOW);
+  auto copy = [&](StageRef& a, size_t n) { return a.h2d(devmem.data(), host.data(), n, &s0) == cudaSuccess; };
+  for (int round = 0; round < 2; ++round) {   // the count begins anew with the ring's first holder
+    StageRef a;
+    fake::staged = fake::plain = fake::pin_calls = 0;
+    const size_t n = (size_t)32 << 20;
+    for (size_t past = 0; past < STAGE_DUE; past += n) REQUIRE(copy(a, n));
+    REQUIRE(fake::staged == 0 && fake::pin_calls == 0 && fake::plain == (long)(STAGE_DUE / n));
+    REQUIRE(copy(a, STAGE_MIN));
+    REQUIRE(fake::staged == 1 && fake::pin_calls == 1);
+    REQUIRE(copy(a, 2 * STAGE_CHUNK + 1));
+    REQUIRE(fake::staged == 4 && fake::pin_calls == 3);
+    REQUIRE(copy(a, n));
+    REQUIRE(fake::pin_calls == STAGE_SLOTS);
+    s0.drain();
+  }
+  REQUIRE(fake::pinned.empty());
+  StageRef b;
+  fake::staged = fake::plain = fake::pin_calls = 0;
+  REQUIRE(copy(b, STAGE_NOW));
+  REQUIRE(fake::plain == 0 && fake::pin_calls == STAGE_SLOTS);
+  s0.drain();
+  return 0;
+}
 }

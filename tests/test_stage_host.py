@@ -26,6 +26,6 @@ def lib():
     return C.CDLL(so)
 
 
-@pytest.mark.parametrize("check", ["other_device_current", "given_back", "plain", "failed_record"])
+@pytest.mark.parametrize("check", ["other_device_current", "given_back", "plain", "failed_record", "when_made"])
 def test_check(lib, check):
     assert getattr(lib, "check_" + check)() == 0

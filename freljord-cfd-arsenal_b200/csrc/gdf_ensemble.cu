@@ -103,6 +103,8 @@ __device__ __noinline__ void call_vertex(const Consts& K, const double* U, doubl
   vertex_at(K, U, EzV, item, q);
 }
 extern __shared__ __align__(16) unsigned char ens_sm[];   // the stage kernel's dynamic shared memory
+// ens_smem sizes it for ENS_BS threads, cell_item strides it by CELL_BS
+static_assert(ENS_BS == CELL_BS, "cell_item's stride is the stage kernel's block");
 __device__ __noinline__ void call_cell(const Consts& K, const double* U, double* U0, double* UI, const double* Fxh,
                                        const double* Fyh, const Scal* sc, int stage, long long item) {
   cell_item(K, U, U0, UI, Fxh, Fyh, nullptr, sc, stage, item,
@@ -441,6 +443,9 @@ __global__ void __launch_bounds__(ENS_BS, 8) k_ep_faces(const __grid_constant__ 
 // copied to shared memory once per tile. Eight problems of 64^2-160^2 144 us per
 // launch, 206 with one lane per cell, 160 without the copy; 64 problems of 7.1 M
 // cells 70.2 ms per step against 84.5 and 72.5.
+// A tile's 2 * per lanes are whole blocks, so whole warps come to cell_pair; its
+// 4 * per vertex lanes (k_ep_faces, k_ens_stage) are whole warps of ENS_BS threads.
+static_assert(2 * ENS_BS % PAIR_BS == 0 && ENS_BS % 32 == 0, "a tile's lanes fill whole warps");
 __global__ void __launch_bounds__(PAIR_BS, 4) k_ep_cell(const __grid_constant__ EnsArgs A, int stage) {
   __shared__ __align__(16) double ms[PAIR_SLOTS * PAIR_BS];
   __shared__ double px[NG][NG][NP], py[NG][NG][NP];

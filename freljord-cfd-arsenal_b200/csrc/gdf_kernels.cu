@@ -695,10 +695,10 @@ static int launch_set_bc(GdfHandle* h, double* U, int zeroB, const Scal* sc) {
 // Orszag-Tang 64^2 36.5 against 43.7 us per launch, 128^2 40.7 and 45.3, 160^2 51.4
 // and 54.0; 192^2, whose blocks are four to an SM, 61.8 and 54.7; above, the
 // two are within 3% of each other either way.
-constexpr long long PAIR_CELLS = 148LL * 3 * (PAIR_BS / 2);
-static void launch_cell(const Consts& K, const double* U, double* U0, double* UI, const double* Fxh, const double* Fyh,
-                        double* duout, const Scal* sc, int stage, cudaStream_t st) {
-  if (K.plane <= PAIR_CELLS)
+static bool two_lanes(const GdfHandle* h) { return h->K.plane <= (long long)h->sms * 3 * (PAIR_BS / 2); }
+static void launch_cell(bool two, const Consts& K, const double* U, double* U0, double* UI, const double* Fxh,
+                        const double* Fyh, double* duout, const Scal* sc, int stage, cudaStream_t st) {
+  if (two)
     k_cell_pair<<<nblk(K.plane, PAIR_BS / 2), PAIR_BS, 0, st>>>(K, U, U0, UI, Fxh, Fyh, duout, sc, stage);
   else
     k_cell<<<nblk(K.plane, CELL_BS), CELL_BS, 0, st>>>(K, U, U0, UI, Fxh, Fyh, duout, sc, stage);
@@ -805,7 +805,7 @@ static int launch_stage(GdfHandle* h, int stage) {
   }
   if ((rc = launch_faces(h, h->U, h->sc))) return rc;
   rc = run_kernel(h, GDF_K_CELL, [&] {
-    launch_cell(K, h->U, h->U0, h->UI, h->Fxh, h->Fyh, nullptr, h->sc, stage, h->st);
+    launch_cell(two_lanes(h), K, h->U, h->U0, h->UI, h->Fxh, h->Fyh, nullptr, h->sc, stage, h->st);
   });
   if (!rc) rc = run_kernel(h, GDF_K_BFACE, [&] {
     k_bface<<<nblk(K.fxplane + K.fyplane, 128), 128, 0, h->st>>>(K, h->EzRL, h->EzUD, h->EzV, h->BX, h->BX0, h->BXI,
@@ -1248,7 +1248,8 @@ int gdf_lh_noalloc(const GdfConfig* cfg, const double* d_uh, double* d_du, void*
   CK(cudaMemsetAsync(d_du, 0, uh_bytes(*cfg), st));
   k_face<0><<<nblk(fx, 32), FACE_BS, 0, st>>>(K, d_uh, Fxh, ezx, nullptr);
   k_face<1><<<nblk(fy, 32), FACE_BS, 0, st>>>(K, d_uh, Fyh, ezy, nullptr);
-  launch_cell(K, d_uh, nullptr, nullptr, Fxh, Fyh, d_du, nullptr, 0, st);
+  // two lanes to a cell: with this scratch a grid has fewer than 23,000 cells, ghosts included
+  launch_cell(true, K, d_uh, nullptr, nullptr, Fxh, Fyh, d_du, nullptr, 0, st);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(GDF_ERR_CUDA, std::string("gdf_lh_noalloc launch: ") + cudaGetErrorString(e));
   return GDF_OK;
@@ -1372,7 +1373,7 @@ int gdf_lh(GdfHandle* h, const double* uh, double* du) {
   CK(cudaMemsetAsync(h->UI, 0, ub, h->st));  // du (ghost and dead entries stay 0)
   if ((rc = launch_faces(h, h->UT, nullptr))) return rc;
   rc = run_kernel(h, GDF_K_CELL, [&] {
-    launch_cell(h->K, h->UT, nullptr, nullptr, h->Fxh, h->Fyh, h->UI, nullptr, 0, h->st);
+    launch_cell(two_lanes(h), h->K, h->UT, nullptr, nullptr, h->Fxh, h->Fyh, h->UI, nullptr, 0, h->st);
   });
   if (rc) return rc;
   CK(h->stage.d2h(du, h->UI, ub, h->st));

@@ -10,6 +10,7 @@
 #include <sys/mman.h>
 
 #include <algorithm>
+#include <chrono>
 #include <cstdint>
 #include <mutex>
 
@@ -19,7 +20,7 @@ namespace {
 struct Ring {
   std::mutex mu;
   int holders = 0;
-  size_t past = 0;      // bytes of the copies that went plainly past it
+  int64_t past_ns = 0;  // what the copies that went plainly past it took
   int slots = 0;        // slots it has
   bool failed = false;  // a slot could not be made: no further one is tried
   char* buf[STAGE_SLOTS] = {};
@@ -56,7 +57,7 @@ void drop(Ring& r) {
     munmap(r.buf[k], STAGE_CHUNK);
   }
   r.slots = 0;
-  r.past = 0;
+  r.past_ns = 0;
   r.failed = false;
   cudaGetLastError();
 }
@@ -93,8 +94,16 @@ void make(Ring& r, int want, int dev) {
   }
 }
 
+#ifndef GDF_STAGE_CLOCK
+#define GDF_STAGE_CLOCK                                                                                \
+  std::chrono::duration_cast<std::chrono::nanoseconds>(std::chrono::steady_clock::now().time_since_epoch()) \
+      .count()
+#endif
+int64_t clock_ns() { return GDF_STAGE_CLOCK; }
+
 // device dev's ring, locked in lk, with a slot for each of the copy's chunks (as
-// many as there are at most), for a pageable array of this size; null: copy plainly
+// many as there are at most), for a pageable array of this size; null: copy
+// plainly, with lk held: add the copy's time
 Ring* take(int dev, const void* host, size_t bytes, std::unique_lock<std::mutex>& lk) {
   if (dev < 0 || bytes < STAGE_MIN) return nullptr;
   cudaPointerAttributes a;
@@ -106,12 +115,23 @@ Ring* take(int dev, const void* host, size_t bytes, std::unique_lock<std::mutex>
   Ring& r = g_ring[dev];
   lk = std::unique_lock<std::mutex>(r.mu, std::try_to_lock);
   if (!lk.owns_lock()) return nullptr;
-  if (bytes >= STAGE_NOW || r.past >= STAGE_DUE)
+  if (bytes >= STAGE_NOW || r.past_ns >= STAGE_DUE_NS)
     make(r, (int)std::min<size_t>(STAGE_SLOTS, (bytes + STAGE_CHUNK - 1) / STAGE_CHUNK), dev);
-  if (r.slots > 0) return &r;
-  r.past += std::min(bytes, STAGE_DUE);
-  r.past = std::min(r.past, STAGE_DUE);
-  return nullptr;
+  return r.slots > 0 ? &r : nullptr;
+}
+// A copy without a ring, its time counted where take left lk held. The driver is
+// done with a pageable array on return; what the stream still had to do before a
+// copy to the host is not the copy's time.
+cudaError_t plain(int dev, std::unique_lock<std::mutex>& lk, void* dst, const void* src, size_t bytes,
+                  cudaMemcpyKind kind, cudaStream_t st) {
+  if (!lk.owns_lock()) return cudaMemcpyAsync(dst, src, bytes, kind, st);
+  lk.unlock();   // other threads' copies need not wait for this one
+  if (kind == cudaMemcpyDeviceToHost) cudaStreamSynchronize(st);   // its errors are the copy's, too
+  const int64_t t0 = clock_ns();
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, kind, st);
+  const int64_t t = clock_ns() - t0;
+  if (lk.try_lock()) g_ring[dev].past_ns = std::min(g_ring[dev].past_ns + t, STAGE_DUE_NS);
+  return e;
 }
 
 // The event behind a slot's transfer. Without one the next copy would take the
@@ -143,7 +163,7 @@ StageRef::~StageRef() {
 cudaError_t StageRef::h2d(void* dst, const void* src, size_t bytes, cudaStream_t st) {
   std::unique_lock<std::mutex> lk;
   Ring* r = take(dev, src, bytes, lk);
-  if (!r) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+  if (!r) return plain(dev, lk, dst, src, bytes, cudaMemcpyHostToDevice, st);
   int k = 0;
   for (size_t o = 0; o < bytes; o += STAGE_CHUNK, k = (k + 1) % r->slots) {
     const size_t n = std::min(STAGE_CHUNK, bytes - o);
@@ -160,7 +180,7 @@ cudaError_t StageRef::h2d(void* dst, const void* src, size_t bytes, cudaStream_t
 cudaError_t StageRef::d2h(void* dst, const void* src, size_t bytes, cudaStream_t st) {
   std::unique_lock<std::mutex> lk;
   Ring* r = take(dev, dst, bytes, lk);
-  if (!r) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
+  if (!r) return plain(dev, lk, dst, src, bytes, cudaMemcpyDeviceToHost, st);
   const size_t chunks = (bytes + STAGE_CHUNK - 1) / STAGE_CHUNK, slots = r->slots;
   auto issue = [&](size_t c) {
     const int k = (int)(c % slots);

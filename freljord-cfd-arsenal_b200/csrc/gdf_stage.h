@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include <cstddef>
+#include <cstdint>
 
 namespace gdf {
 
@@ -44,12 +45,13 @@ constexpr size_t STAGE_MIN = (size_t)1 << 20;   // below: one plain copy (the ri
 // through the ring; 256 MB 23 and 5.2): the first predict of a process on 69 MB takes
 // 9.2 ms, 8.9 without the ring, the next ones 4.3 and 7 to 8 ...
 constexpr size_t STAGE_NOW = (size_t)64 << 20;
-// ... or if this much has gone past plainly while its holders lived, 27-45 ms of
-// copies: a shorter copy may then pay for the slots alone, once in that long
-// (predict on 62 MB: the tenth call 7.1 ms, 5.6 before it and 3.1 after).
-// Handles opened, loaded and closed in a loop thus stay at the plain rate until they
-// move more than they would lose.
-constexpr size_t STAGE_DUE = (size_t)512 << 20;
+// ... or if the copies of 1 MiB or more that went past plainly while its holders lived
+// took this long, ten times what the slots cost: a shorter copy may then pay for the slots
+// alone, once (predict on 62 MB: the seventh call 7.0 ms, 6.6 before it, 3.0 after), and handles opened, loaded and closed in a loop lose a tenth of their copies'
+// time at most (none where they take less than this). It is a time because the rate varies
+// by ten with where the pages are: a 512^2 state goes up in 12 ms and comes
+// down into new arrays in 40 (17 through the ring that these make).
+constexpr int64_t STAGE_DUE_NS = 28000000;
 
 // memcpy over several threads (gdf_io.cpp)
 void par_memcpy(void* dst, const void* src, size_t bytes);

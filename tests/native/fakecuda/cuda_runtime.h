@@ -35,6 +35,7 @@ struct Stream {
 struct Event { int dev; Stream* s; long upto; };
 inline int dev = 0, live_events = 0, record_fails = 0, pin_calls = 0;
 inline long staged = 0, plain = 0;               // copies by kind of their host memory
+inline int64_t now = 0;                          // ns: a byte copied plainly takes one
 inline std::map<uintptr_t, size_t> pinned;        // start -> bytes
 inline bool is_pinned(const void* p) {
   auto it = pinned.upper_bound((uintptr_t)p);
@@ -103,6 +104,7 @@ inline cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyK
     st->q.push_back([=] { std::memcpy(d, s, n); });
   } else {   // pageable: done with the host's side on return
     ++fake::plain;
+    fake::now += (int64_t)n;
     st->drain();
     std::memcpy(d, s, n);
   }

@@ -1,5 +1,7 @@
 // Host build of the pinned ring (csrc/gdf_stage.cu) on the fake runtime of
-// fakecuda/. Each check returns 0, or the line it failed at.
+// fakecuda/ and its clock. Each check returns 0, or the line it failed at.
+#include <cuda_runtime.h>
+#define GDF_STAGE_CLOCK fake::now
 #include "../../freljord-cfd-arsenal_b200/csrc/gdf_stage.cu"
 
 #include <vector>
@@ -116,8 +118,8 @@ int check_failed_record() {
   return 0;
 }
 
-// one long copy makes the slots it needs; shorter ones go past plainly until
-// STAGE_DUE bytes have, and then make no more slots than they have chunks
+// one long copy makes the slots it needs; shorter ones go past plainly until they
+// have taken STAGE_DUE_NS, and then make no more slots than they have chunks
 int check_when_made() {
   fake::Stream s0{0, {}};
   cudaSetDevice(0);
@@ -126,14 +128,15 @@ int check_when_made() {
   for (int round = 0; round < 2; ++round) {   // the count begins anew with the ring's first holder
     StageRef a;
     fake::staged = fake::plain = fake::pin_calls = 0;
-    const size_t n = (size_t)32 << 20;
-    for (size_t past = 0; past < STAGE_DUE; past += n) REQUIRE(copy(a, n));
-    REQUIRE(fake::staged == 0 && fake::pin_calls == 0 && fake::plain == (long)(STAGE_DUE / n));
+    const size_t n = (size_t)5 << 20;   // 5.2 ms each
+    int64_t past = 0;
+    for (; past < STAGE_DUE_NS; past += n) REQUIRE(copy(a, n));
+    REQUIRE(fake::staged == 0 && fake::pin_calls == 0 && fake::plain == past / (int64_t)n);
     REQUIRE(copy(a, STAGE_MIN));
     REQUIRE(fake::staged == 1 && fake::pin_calls == 1);
     REQUIRE(copy(a, 2 * STAGE_CHUNK + 1));
     REQUIRE(fake::staged == 4 && fake::pin_calls == 3);
-    REQUIRE(copy(a, n));
+    REQUIRE(copy(a, 9 * STAGE_CHUNK));
     REQUIRE(fake::pin_calls == STAGE_SLOTS);
     s0.drain();
   }

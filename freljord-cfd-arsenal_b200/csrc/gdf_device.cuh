@@ -75,12 +75,6 @@ __device__ __forceinline__ void set_bc_item(const Consts& K, double* __restrict_
   U[off + i + (long long)K.nx2 * j] = v;
 }
 
-// Products with the exact 1 and -1 entries of the basis tables written as
-// the value itself (x * 1 == x, x * -1 == -x for every double)
-#ifndef GDF_FOLD_UNIT
-#define GDF_FOLD_UNIT 1
-#endif
-
 // ---------------------------------------------------- face Riemann -------
 // Lh.f90:72-265 and LhEz.f90:6-31 for one face quadrature point.
 // DIR 0: x face (i = 0..Nx, j = 1..Ny) between cells (i,j) and (i+1,j).
@@ -107,12 +101,13 @@ __device__ __forceinline__ bool face_point(const Consts& K, ML mL, MR mR, int g,
       const double pr = DIR == 0 ? c_basis.phiGL[g][d] : c_basis.phiGD[g][d];
       // the face basis is 1 for mode 1, and for mode 2 (x faces) or 3 (y
       // faces) 1 on the low cell's face and -1 on the high cell's
-      // (get_basis.f90): those products are exact and written out
+      // (get_basis.f90): those products are exact (x * 1 == x, x * -1 == -x for
+      // every double) and written out
       const int du = DIR == 0 ? 1 : 2;
-      if (GDF_FOLD_UNIT && d == 0) {
+      if (d == 0) {
         a = a + mL(n, d);
         b = b + mR(n, d);
-      } else if (GDF_FOLD_UNIT && d == du) {
+      } else if (d == du) {
         a = a + mL(n, d);
         b = b + (-mR(n, d));
       } else {
@@ -1761,8 +1756,8 @@ __device__ __forceinline__ void limit_gate_item(const Consts& K, const double* _
   lim_flags(flags, stage, sc, item, word, mean[0], mean[4]);
 }
 
-// A cell every thread of the limiting pass limits: one limit_item<LM, true>
-// deferred, or with GDF_DETECT_ALL any. The detector bit is the one lim_gate
+// A cell of the limiting pass: one that limit_gate_item listed, or with
+// GDF_DETECT_ALL any. The detector bit is the one lim_gate
 // sets (KXRCF and the learned gate set it; GDF_DETECT_ALL does not). The modes
 // are loaded after the characteristic part, which needs few of them.
 __device__ __forceinline__ void limit_tvb_item(const Consts& K, const double* __restrict__ S, double* __restrict__ D,

@@ -34,7 +34,6 @@
 #include <cstring>
 #include <mutex>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "../../include/gdf.h"
@@ -44,20 +43,20 @@
 #ifndef GDF_EXACT
 #define GDF_EXACT 0
 #endif
-// minimum resident blocks per SM requested of the face/vertex (128-thread)
-// and residual (64-thread) kernels: the register budget per thread they
-// allow (65536 / (threads x blocks)); arithmetic is the same for any value.
-// Faces at 4 blocks (128 registers, ~300 B spilled) ran 20% faster than at
-// the unconstrained 168 registers; the residual kernel gained nothing.
+// Resident blocks per SM asked of a kernel, which bounds its registers per
+// thread (65536 / (threads x blocks)); the values are the same for any.
+// Faces, 160 threads a block: 3 blocks, 128 registers with 0.5 KB spilled: y faces of
+// the blast 2048^2 2.22 ms per launch, 2.50 with 2 blocks (spill-free).
 #ifndef GDF_FACE_MINB
 #define GDF_FACE_MINB 3
 #endif
-// vertex kernel at 3 blocks (168 registers, no spill): timed alone a
-// launch is 10% slower than at 4 blocks, but the blast 2048^2 step replayed
-// from its graph is 2% shorter (45.9 against 46.9 ms, same values)
+// Vertices, 128 threads a block: 3 blocks leave 168 registers, of which the
+// four-lane form takes 128 and spills none.
 #ifndef GDF_VERTEX_MINB
 #define GDF_VERTEX_MINB 3
 #endif
+// The residual (64 threads, 248 registers) and the limiting pass (255): one block, the
+// compiler's own choice.
 #ifndef GDF_CELL_MINB
 #define GDF_CELL_MINB 1
 #endif
@@ -158,10 +157,9 @@ __global__ void k_features(const __grid_constant__ Consts K, const float* __rest
 // resident blocks stage the BF16 weights once and walk the LIM_BS-cell
 // tiles of the grid (features gathered from QM, the two tensor-core
 // products, the sigmoid), storing each cell's probability in pnet. A tile
-// computes what the limiter block with inference computes for the same
-// cells (same features, roundings and product order per row), so the
-// stored probabilities are those of k_limit<LIM_INFER>, at the occupancy of
-// a 128-register kernel instead of the FP64 limiter's 255 registers.
+// computes what the ensemble's limiter blocks with inference (LIM_INFER) compute
+// for the same cells (same features, roundings and product order per row), so the
+// probabilities are the same.
 __global__ void __launch_bounds__(LIM_BS) k_infer(const __grid_constant__ Consts K, const MlpDev* __restrict__ net,
                                                      const float* __restrict__ QM, float* __restrict__ pnet,
                                                      const Scal* __restrict__ gate_sc) {
@@ -753,7 +751,9 @@ static int launch_limit(GdfHandle* h, const double* S, double* D, int stage, con
   }
   // two passes: the detector lists the gated cells, which the limiting pass
   // takes over full warps (a sticky KXRCF flag leaves mixed warps for most of
-  // a run)
+  // a run). With the learned gate two passes are 2% faster while few cells are gated
+  // and 2% slower once most are: the whole blast 512^2 run to step 4200 takes 3.07-3.08 ms
+  // per step, 3.05 in one pass; early steps 2.45 and 2.50, late ones 3.61 and 3.55.
   const bool all = K.detector == GDF_DETECT_ALL;   // no gate: the limiting pass over every cell
   int32_t *L = h->lim_list, *N = h->lim_count;
   const LimList<long long> pp{h->pp_list, N + 1, 0};
@@ -1040,8 +1040,9 @@ int gdf_destroy(GdfHandle* h) {
 
 int gdf_upload(GdfHandle* h, const double* uh, const double* bx, const double* by) {
   if (!h || !uh || !bx || !by) return fail(GDF_ERR_ARG, "null argument");
-  // the live planes travel to a staging buffer while the host checks the
-  // dead ones; the resident state changes only once the check has passed
+  // The live planes go to a buffer of their own (from pinned arrays while the host
+  // checks the dead ones; pageable copies are done with by then): the resident
+  // state changes only once the check has passed.
   CK(copy_live(h, h->UT, uh, cudaMemcpyHostToDevice));
   int rc = check_dead_slots(h->cfg, uh);
   if (rc) {

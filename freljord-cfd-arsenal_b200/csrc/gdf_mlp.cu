@@ -373,8 +373,9 @@ __global__ void k_mlp_reduce(const float* __restrict__ partial, int nb, float* _
 
 // One training step's end: the gradient (the block slots in block order, as
 // k_mlp_reduce), the Adam update of the FP32 parameters and their BF16 copies
-// (as k_mlp_sync), one parameter per thread; the batch's loss to *loss. Three
-// launches and a read-back of the loss before.
+// (as k_mlp_sync), one parameter per thread; the batch's loss to *loss. One
+// launch and no read-back: as three kernels and a loss copied back after each batch
+// this took some 50 us, the tile before it 18.
 __global__ void k_mlp_update(float* __restrict__ P, float* __restrict__ M, float* __restrict__ V,
                              MlpDev* __restrict__ D, const float* __restrict__ partial, int nb,
                              const float* __restrict__ loss_part, float* __restrict__ loss, float lr, float b1,

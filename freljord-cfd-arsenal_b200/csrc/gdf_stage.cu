@@ -29,9 +29,9 @@ struct Ring {
 constexpr int MAX_DEV = 64;
 Ring g_ring[MAX_DEV];
 
-// The slots are anonymous memory in huge pages, registered: 0.8 ms for one (half
-// of it the pages' zeros, by one thread), 2.3 ms for four, 0.5 ms to give four back. cudaHostAlloc took
-// 2-5 ms for one, 9-18 for four. A forked child does not get the pages, so a
+// The slots are anonymous memory in huge pages, registered: 0.8 ms for one (0.3 of
+// it the pages' zeros; in small pages 4.5 ms), 2.3 to 3 ms for four, 0.5 ms and more to give
+// four back. cudaHostAlloc took 2-5 ms for one, 9-18 for four. A forked child does not get the pages, so a
 // write of the parent's never moves them from under a transfer.
 constexpr size_t HUGE = (size_t)2 << 20;
 char* pages() {

@@ -1,10 +1,10 @@
 // gdf_stage.cu -- the pinned ring behind gdf_stage.h.
 //
 // One ring per device, its events made on that device (an event is recorded on
-// streams of its own device only). A copy holds the ring for its whole length; a copy that
-// finds it taken (another thread's) goes to cudaMemcpyAsync, so threads never
-// wait for each other here. A slot is reused when the event recorded behind its
-// last transfer has passed, whatever stream that was on.
+// streams of its own device only). A copy holds the ring for its whole length; a
+// copy that finds it taken (another thread's) goes to cudaMemcpyAsync, so threads
+// never wait for each other here. A slot is reused when the event recorded behind
+// its last transfer has passed, whatever stream that was on.
 #include "gdf_stage.h"
 
 #include <sys/mman.h>
@@ -30,9 +30,10 @@ constexpr int MAX_DEV = 64;
 Ring g_ring[MAX_DEV];
 
 // The slots are anonymous memory in huge pages, registered: 0.8 ms for one (0.3 of
-// it the pages' zeros; in small pages 4.5 ms), 2.3 to 3 ms for four, 0.5 ms and more to give
-// four back. cudaHostAlloc took 2-5 ms for one, 9-18 for four. A forked child does not get the pages, so a
-// write of the parent's never moves them from under a transfer.
+// it the pages' zeros; in small pages 4.5 ms), 2.3 to 3 ms for four, 0.5 ms and
+// more to give four back. cudaHostAlloc took 2-5 ms for one, 9-18 for four. A
+// forked child does not get the pages, so a write of the parent's never moves them
+// from under a transfer.
 constexpr size_t HUGE = (size_t)2 << 20;
 char* pages() {
   void* p = mmap(nullptr, STAGE_CHUNK + HUGE, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);

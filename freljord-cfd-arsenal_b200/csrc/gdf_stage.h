@@ -1,11 +1,11 @@
 // gdf_stage.h -- copies between host arrays and the device.
 //
 // A caller's arrays are ordinary (pageable) memory as a rule. The driver copies
-// those through its own staging buffer with one host thread, 12 GB/s from memory, 20
-// from the host's caches, 2-3 into pages not yet touched, well under the link. h2d / d2h take large
-// pageable arrays through a ring of pinned buffers instead: several threads fill
-// (empty) one while the link moves another. Small arrays, and memory that is
-// already pinned or on a device, go to cudaMemcpyAsync as they are.
+// those through its own staging buffer with one host thread, 12 GB/s from memory,
+// 20 from the host's caches, 2-3 into pages not yet touched, well under the link.
+// h2d / d2h take large pageable arrays through a ring of pinned buffers instead:
+// several threads fill (empty) one while the link moves another. Small arrays, and
+// memory that is already pinned or on a device, go to cudaMemcpyAsync as they are.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -41,16 +41,17 @@ constexpr size_t STAGE_CHUNK = (size_t)4 << 20;
 constexpr int STAGE_SLOTS = 4;
 constexpr size_t STAGE_MIN = (size_t)1 << 20;   // below: one plain copy (the ring's hand-overs cost more)
 // When a copy makes the slots it needs (2.3 ms for all four, 0.5 ms to give them
-// back): if it is this long itself, so that it saves as much (72 MB up 5.6 ms plainly, 1.6
-// through the ring; 256 MB 23 and 5.2): the first predict of a process on 69 MB takes
-// 9.2 ms, 8.9 without the ring, the next ones 4.3 and 7 to 8 ...
+// back): if it is this long itself, so that it saves as much (72 MB up 5.6 ms
+// plainly, 1.6 through the ring; 256 MB 23 and 5.2): the first predict of a process
+// on 69 MB takes 9.2 ms, 8.9 without the ring, the next ones 4.3 and 7 to 8 ...
 constexpr size_t STAGE_NOW = (size_t)64 << 20;
-// ... or if the copies of 1 MiB or more that went past plainly while its holders lived
-// took this long, ten times what the slots cost: a shorter copy may then pay for the slots
-// alone, once (predict on 62 MB: the seventh call 7.0 ms, 6.6 before it, 3.0 after), and handles opened, loaded and closed in a loop lose a tenth of their copies'
-// time at most (none where they take less than this). It is a time because the rate varies
-// by ten with where the pages are: a 512^2 state goes up in 12 ms and comes
-// down into new arrays in 40 (17 through the ring that these make).
+// ... or if the copies of 1 MiB or more that went past plainly while its holders
+// lived took this long, ten times what the slots cost. A shorter copy may then pay
+// for the slots alone, once (predict on 62 MB: the seventh call 7.0 ms, 6.6 before
+// it, 3.0 after), and handles opened, loaded and closed in a loop lose a tenth of
+// their copies' time at most (none where they take less than this). It is a time
+// because the rate varies by ten with where the pages are: a 512^2 state goes up in
+// 12 ms and comes down into new arrays in 40 (17 through the ring that these make).
 constexpr int64_t STAGE_DUE_NS = 28000000;
 
 // memcpy over several threads (gdf_io.cpp)
